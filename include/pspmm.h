@@ -62,8 +62,10 @@ typedef struct pspmm_cfg {
                                 several launches over column ranges.  0 = one launch */
     int32_t hint_CF;         /* legacy coarsening factor, validated only */
     int32_t hint_blkWarpNum; /* legacy warps per block, validated only */
-    int32_t bucketed;        /* SpMM on a split layout only: 1 = the split arrays are a length-bucketed plan (see
-                                pspmm_spmm_csr): segments in any order, flags in the two high bits of target_row */
+    int32_t bucketed;        /* SpMM only.  Split layout: 1 = the split arrays are a length-bucketed plan (see
+                                pspmm_spmm_csr): segments in any order, flags in the two high bits of target_row.
+                                Unsplit layout: 1 = the caller knows that no row is far longer than the others;
+                                with 0 the call looks for such rows and cuts them over the whole GPU */
     int32_t accumulate;      /* SpMM only: 0 = C is overwritten (every row is written, empty rows with zeros);
                                 1 = the product is added to what C holds (reduction instructions; the order in
                                 which contributions reach a row is not fixed).  Lets a caller sum products over
@@ -216,7 +218,9 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  * per lane group; combinations that are not built are rounded to the nearest built one.
  * Split layouts (rowPtr_split/target_row/n_seg as in pspmm_spmm_csr) need scratch of
  * pspmm_agnn_scratch_bytes(n_seg, dim) bytes, 16-byte aligned, for the partial results of the
- * pieces of split rows; plain CSR needs none (NULL, 0).
+ * pieces of split rows; plain CSR needs none (NULL, 0), but with pspmm_agnn_long_scratch_bytes(nnz,
+ * dim) bytes, 16-byte aligned, its long rows are cut over the whole GPU instead of being walked by one
+ * lane group each.
  *
  * pspmm_agnn_fused_apply_csr is the same pass with a separate aggregation operand:
  *     out_i = sum_j a_ij * V_j,   a_ij from A and B as above.
@@ -227,6 +231,7 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  * the alignment rules of B; this form runs with 128-bit loads and batches of 4.
  */
 PSPMM_API int pspmm_agnn_scratch_bytes(int64_t n_seg, int32_t dim, size_t *bytes);
+PSPMM_API int pspmm_agnn_long_scratch_bytes(int64_t nnz, int32_t dim, size_t *bytes);
 PSPMM_API int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *A,
                                          const float *B, const float *V, float *out, int64_t n_rows, int64_t nnz,
                                          int32_t dim, int64_t ldA, int64_t ldB, int64_t ldV, int64_t ldOut,

@@ -2,6 +2,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "pspmm_common.cuh"
 #include "vec_ops.cuh"
 
@@ -171,6 +173,7 @@ zero_shared_rows_kernel(const int32_t *__restrict__ target_row, int64_t n_seg, i
     __shared__ int q_n;
     if (threadIdx.x == 0)
         q_n = 0;
+    pdl_launch_dependents();
     __syncthreads();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -253,6 +256,7 @@ __global__ void __launch_bounds__(256)
 zero_first_pieces_kernel(const int32_t *__restrict__ target_row, int64_t n_seg, int V, float *C, int64_t ldC,
                          int dim, int vecok)
 {
+    pdl_launch_dependents();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const unsigned t = s < n_seg ? (unsigned)__ldg(target_row + s) : 0u;
@@ -307,10 +311,44 @@ static float l2_keep_fraction(double operand_bytes)
     return (float)(f < 0.02 ? 0.02 : f);
 }
 
+static int sm_count()
+{
+    static thread_local int cached_dev = -1, sms = 148;
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev != cached_dev &&
+        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) {
+        sms = v;
+        cached_dev = dev;
+    }
+    return sms;
+}
+
+// Segments one lane group owns.  Several share the pointer and entry staging, but a small matrix then
+// leaves SMs without a warp (19,717 rows at dim 16: 77 CTAs for 148 SMs) and walks its segments one
+// after the other: below half a resident wave of threads the groups take fewer segments.
+static int small_rows_per_group(int rpg, int64_t n_seg, int lpr)
+{
+    while (rpg > 1 && n_seg / rpg * lpr < (int64_t)sm_count() * 1024)
+        rpg >>= 1;
+    return rpg;
+}
+
+// Which rows of an unsplit layout are cut over the GPU: a lane group takes about a microsecond per
+// eight entries, so rows above 1/64 of an SM's share of the entries would outlast the rest; never
+// below 64 (a row's pieces must pay for their reduction) nor above 512 (half the time of the
+// smallest product that needs this many).  INT32_MAX: no row can be that long.
+int pspmm_long_row_threshold(int64_t n_entries)
+{
+    int t = 64;
+    while (t < 512 && (int64_t)t * sm_count() * 64 < n_entries)
+        t *= 2;
+    return n_entries > t ? t : INT32_MAX;
+}
+
 static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t n_seg,
                        const int32_t *colIdx, const float *val, int V, const float *B, float *C,
-                       int64_t n_out_blk_rows, int64_t n_cols, int32_t dim, int64_t ldB, int64_t ldC,
-                       const pspmm_cfg *cfg, cudaStream_t st)
+                       int64_t n_out_blk_rows, int64_t n_cols, int64_t n_entries, int32_t dim, int64_t ldB,
+                       int64_t ldC, const pspmm_cfg *cfg, cudaStream_t st)
 {
     int rc = pspmm_validate_cfg(cfg, false);
     if (rc)
@@ -334,8 +372,8 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             sub.col_tile = 0;
             if (sub.lanes_per_row * (sub.vec_width ? sub.vec_width : 4) > w)
                 sub.lanes_per_row = 0;  // let the launch pick the group width for the narrow range
-            rc = spmm_launch(segPtr, target_row, n_seg, colIdx, val, V, B + off, C + off, n_out_blk_rows, n_cols, w,
-                             ldB, ldC, &sub, st);
+            rc = spmm_launch(segPtr, target_row, n_seg, colIdx, val, V, B + off, C + off, n_out_blk_rows, n_cols,
+                             n_entries, w, ldB, ldC, &sub, st);
             if (rc)
                 return rc;
         }
@@ -355,6 +393,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             s = t;
         }
     }
+
+    if (!cfg || cfg->rows_per_group == 0)
+        s.rpg = small_rows_per_group(s.rpg, n_seg, s.lpr);
 
     const bool bucketed = target_row && cfg && cfg->bucketed;
     if (target_row && !accumulate) {
@@ -382,6 +423,12 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.rows_per_group = s.rpg;
     a.bucketed = bucketed ? 1 : 0;
     a.keep_fraction = l2_keep_fraction((double)n_cols * (double)ldB * 4.0);
+    a.n_entries = n_entries;
+    a.long_row = target_row || accumulate || (cfg && cfg->bucketed) ? INT32_MAX : pspmm_long_row_threshold(n_entries);
+    a.long_range = a.long_row < INT32_MAX ? 8 * a.long_row : 0;
+    a.sms = sm_count();
+    static std::atomic<unsigned long long> tickets{0};
+    a.long_ticket = a.long_row < INT32_MAX ? ++tickets : 0;
     const int64_t per_cta = (int64_t)(s.threads / s.lpr) * s.rpg;
     const int64_t gx = (n_seg + per_cta - 1) / per_cta;
     if (gx > INT32_MAX || s.tiles > 65535)
@@ -423,7 +470,7 @@ extern "C" int pspmm_spmm_csr(const int32_t *rowPtr, const int32_t *colIdx, cons
     if (split && n_seg >= INT32_MAX)
         return PSPMM_E_RANGE;
     return spmm_launch(split ? rowPtr_split : rowPtr, target_row, split ? n_seg : n_rows, colIdx,
-                       val, 1, B, C, n_rows, n_cols, dim, ldB, ldC, cfg, (cudaStream_t)stream);
+                       val, 1, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, (cudaStream_t)stream);
 }
 
 extern "C" int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,
@@ -447,14 +494,14 @@ extern "C" int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, c
     if (nblk > 0 && (!colIdx || !val))
         return PSPMM_E_ARG;
     return spmm_launch(split ? rowPtr_b_split : rowPtr_b, target_row, split ? n_seg : n_blk_rows,
-                       colIdx, val, V, B, C, n_blk_rows, n_cols, dim, ldB, ldC, cfg, (cudaStream_t)stream);
+                       colIdx, val, V, B, C, n_blk_rows, n_cols, nblk, dim, ldB, ldC, cfg, (cudaStream_t)stream);
 }
 
 // ----------------------------------------------------------------------------- SDDMM
 static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t n_seg,
                         const int32_t *colIdx, const float *val, int V, const float *A,
-                        const float *B, float *out, int64_t n_rows_A, int32_t dim, int64_t ldA, int64_t ldB,
-                        const pspmm_cfg *cfg, cudaStream_t st)
+                        const float *B, float *out, int64_t n_rows_A, int64_t n_entries, int32_t dim, int64_t ldA,
+                        int64_t ldB, const pspmm_cfg *cfg, cudaStream_t st)
 {
     int rc = pspmm_validate_cfg(cfg, true);
     if (rc)
@@ -465,6 +512,8 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldA, ldB, A, B), V, &s);
     if (!cfg || cfg->cta_threads == 0)
         s.threads = 128;  // measured: 128-thread CTAs are 7 % faster than 256 for this kernel
+    if (!cfg || cfg->rows_per_group == 0)
+        s.rpg = small_rows_per_group(s.rpg, n_seg, s.lpr);
     SddmmArgs a;
     a.segPtr = segPtr;
     a.target_row = target_row;
@@ -480,8 +529,16 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     a.nvec = dim / s.vw;
     a.rows_per_group = s.rpg;
     a.keep_fraction = 1.0f;  // the row count of B is not part of the call: no partial pinning
+    a.long_row = target_row ? INT32_MAX : pspmm_long_row_threshold(n_entries);
+    a.long_range = 0;
+    a.long_ctas = 0;
+    if (a.long_row < INT32_MAX) {
+        a.long_range = 8 * a.long_row;
+        const int64_t ranges = (n_entries + a.long_range - 1) / a.long_range;
+        a.long_ctas = (uint32_t)(ranges < 65536 ? ranges : 65536);
+    }
     const int64_t per_cta = (int64_t)(s.threads / s.lpr) * s.rpg;
-    const int64_t gx = (n_seg + per_cta - 1) / per_cta;
+    const int64_t gx = (n_seg + per_cta - 1) / per_cta + a.long_ctas;
     if (gx > INT32_MAX)
         return PSPMM_E_RANGE;
     dim3 grid((unsigned)gx, 1, 1);
@@ -519,7 +576,7 @@ extern "C" int pspmm_sddmm_csr(const int32_t *rowPtr, const int32_t *colIdx, con
     if (!colIdx || !out)
         return PSPMM_E_ARG;
     return sddmm_launch(split ? rowPtr_split : rowPtr, target_row, split ? n_seg : n_rows, colIdx,
-                        nullptr, 1, A, B, out, n_rows, dim, ldA, ldB, cfg, (cudaStream_t)stream);
+                        nullptr, 1, A, B, out, n_rows, nnz, dim, ldA, ldB, cfg, (cudaStream_t)stream);
 }
 
 extern "C" int pspmm_sddmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,
@@ -548,7 +605,7 @@ extern "C" int pspmm_sddmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, 
     if (!colIdx || !val || !out)
         return PSPMM_E_ARG;
     return sddmm_launch(split ? rowPtr_b_split : rowPtr_b, target_row,
-                        split ? n_seg : n_blk_rows, colIdx, val, V, A, B, out, n_rows_A, dim, ldA, ldB, cfg,
+                        split ? n_seg : n_blk_rows, colIdx, val, V, A, B, out, n_rows_A, nblk, dim, ldA, ldB, cfg,
                         (cudaStream_t)stream);
 }
 

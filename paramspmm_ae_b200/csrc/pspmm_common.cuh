@@ -9,6 +9,7 @@
 #define PSPMM_FULL_MASK 0xffffffffu
 #define PSPMM_MAX_CF 8
 #define PSPMM_RPG_MAX 16  // most consecutive segments one lane group owns
+#define PSPMM_LONG_PER_RANGE 12  // a range of 8 * long_row entries meets at most 9 rows longer than long_row
 #define PSPMM_GAP_MAX 256  // longest run of uncovered rows the SpMM kernel zeroes by itself
 
 // Records the CUDA error text for pspmm_last_cuda_error() and returns PSPMM_E_CUDA.
@@ -20,6 +21,60 @@ int pspmm_note_cuda_error(cudaError_t e);
         if (e__ != cudaSuccess)                 \
             return pspmm_note_cuda_error(e__);  \
     } while (0)
+
+// Programmatic dependent launch: a kernel launched with launch_dependent() may start while the
+// kernel before it on the stream drains; what it must not do before pdl_wait() is touch memory that
+// kernel writes.  A kernel calls pdl_launch_dependents() once its CTAs are placed.  Both are no-ops
+// outside such a pair.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename Args>
+static inline cudaError_t launch_dependent(void (*kern)(Args), dim3 grid, int threads, int smem, cudaStream_t st,
+                                           const Args &a)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+// The segment that holds entry `pos` (largest s with segPtr[s] <= pos; segPtr[0] <= pos), found by one
+// warp that probes 32 pointers per step.  The first step looks where even rows would put it, which
+// ends the search there for matrices without long rows; otherwise 3 more dependent loads for 20 K
+// segments, 4 for a million.
+__device__ __forceinline__ int find_segment(const int32_t *segPtr, int64_t n_seg, int64_t first, int64_t end, int64_t pos,
+                                            int lane)
+{
+    int64_t lo = 0, hi = n_seg;
+    if (n_seg > 32) {
+        int64_t g = (int64_t)((float)(pos - first) / (float)(end - first) * (float)n_seg) - 16;
+        g = g < 0 ? 0 : (g > n_seg - 32 ? n_seg - 32 : g);
+        const int c = __popc(__ballot_sync(PSPMM_FULL_MASK, __ldg(segPtr + g + lane) <= pos));
+        if (c == 32)
+            lo = g + 31;
+        else if (c == 0)
+            hi = g;
+        else
+            return (int)(g + c - 1);
+    }
+    while (hi - lo > 1) {
+        const int64_t step = (hi - lo + 31) / 32;
+        const int64_t p = lo + lane * step;
+        const bool ok = p < hi && __ldg(segPtr + p) <= pos;
+        const int c = __popc(__ballot_sync(PSPMM_FULL_MASK, ok));
+        lo += (int64_t)(c > 0 ? c - 1 : 0) * step;
+        hi = lo + step < hi ? lo + step : hi;
+    }
+    return (int)lo;
+}
 
 // One launch of the segment SpMM kernel.  A "segment" is a CSR row, a PCSR row piece, or
 // the block-row forms of either.
@@ -37,6 +92,11 @@ struct SpmmArgs {
     int32_t rows_per_group;
     float keep_fraction;        // share of B's lines marked evict-last in L2 (0..1]
     int32_t bucketed;           // target_row carries PSPMM_SEG_* flags, segments come in any order
+    int64_t n_entries;          // entries the caller declares
+    int32_t long_row;           // unsplit rows with more entries go to spmm_long_rows_kernel (INT32_MAX: none do)
+    int32_t long_range;         // entries one CTA of that kernel looks after at a time
+    int32_t sms;
+    unsigned long long long_ticket;  // number of this launch, for what spmm_seg_kernel tells the next one
 };
 
 // Flags in target_row of a length-bucketed plan (pspmm_cfg.bucketed): the low 30 bits are the row.
@@ -58,6 +118,9 @@ struct SddmmArgs {
     int32_t nvec;
     int32_t rows_per_group;
     float keep_fraction;
+    int32_t long_row;    // unsplit rows with more entries are dealt to the first long_ctas CTAs (INT32_MAX: none are)
+    int32_t long_range;  // entries per range of those CTAs
+    uint32_t long_ctas;
 };
 
 // Resolved launch shape.
@@ -85,6 +148,7 @@ static inline int pspmm_round_cf(int need)
     return 0;
 }
 
+int pspmm_long_row_threshold(int64_t n_entries);
 int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm);
 int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, LaunchShape *out);
 int pspmm_vw_max(int32_t dim, int64_t ld0, int64_t ld1, const void *p0, const void *p1);

@@ -36,122 +36,177 @@ __device__ __forceinline__ float transpose_reduce(float (&p)[N], int gl)
     }
 }
 
+// The entries [lb, hb) of (block-)row arow for one lane group; every lane of the warp calls this
+// together, `maxlen` is the longest of the warp's ranges and a group without work passes lb == hb.
 template <int LPR, int VW, int CF, int V>
-__global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
+__device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, int lb, int hb, int maxlen, int gl)
 {
     constexpr int ENT = (LPR >= 16) ? 1 : (16 / LPR);
     constexpr int CHUNK = LPR * ENT;
     constexpr int U0 = 8 / CF;
     constexpr int U1 = U0 < 1 ? 1 : U0;
     constexpr int U = U1 > LPR ? LPR : U1;  // entries whose gathers are batched (divides LPR)
+    const int tiles = (a.nvec + LPR * CF - 1) / (LPR * CF);
+    const int len = hb - lb;
+    const bool live = len > 0;
+    for (int off = 0; off < maxlen; off += CHUNK) {
+        int ccol[ENT];
+        float cval[ENT][V];
+        float res[ENT][V];
+#pragma unroll
+        for (int t = 0; t < ENT; ++t) {
+            const int k = lb + off + t * LPR + gl;
+            const bool ok = k < hb;
+            ccol[t] = ok ? __ldg(a.colIdx + k) : 0;
+#pragma unroll
+            for (int w = 0; w < V; ++w) {
+                cval[t][w] = (V > 1 && ok) ? __ldg(a.val + (int64_t)k * V + w) : 1.f;
+                res[t][w] = 0.f;
+            }
+        }
+        const int cnt = len - off;
+        const int wcnt = maxlen - off;
 
+        for (int tile = 0; tile < tiles; ++tile) {
+            // Slice of the A row(s) this lane is responsible for in this tile.
+            FVec<VW> av[V][CF];
+            int voff[CF];
+            bool act[CF];
+#pragma unroll
+            for (int cf = 0; cf < CF; ++cf) {
+                const int vi = (tile * CF + cf) * LPR + gl;
+                act[cf] = vi < a.nvec;
+                voff[cf] = vi * VW;
+#pragma unroll
+                for (int w = 0; w < V; ++w)
+                    // (the last block-row of an odd row count has lanes without a row of A)
+                    av[w][cf] = (live && act[cf] && arow * V + w < a.n_rows_A)
+                                    ? ldg_vec<VW>(a.A + (arow * V + w) * a.ldA + voff[cf])
+                                    : zero_vec<VW>();
+            }
+#pragma unroll
+            for (int t = 0; t < ENT; ++t) {
+                if (t * LPR >= wcnt)
+                    break;
+                float part[V][LPR];
+#pragma unroll
+                for (int j0 = 0; j0 < LPR; j0 += U) {
+                    FVec<VW> x[U][CF];
+                    const bool batch_on = (t * LPR + j0) < wcnt;  // warp-uniform
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int e = t * LPR + j0 + u;
+                        const int c = __shfl_sync(PSPMM_FULL_MASK, ccol[t], j0 + u, LPR);
+                        const float *brow = a.B + (int64_t)c * a.ldB;
+                        const bool p = batch_on && (e < cnt);
+#pragma unroll
+                        for (int cf = 0; cf < CF; ++cf)
+                            x[u][cf] = ldg_vec_if<VW>(brow + voff[cf], p && act[cf]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int w = 0; w < V; ++w) {
+                            float s = 0.f;
+#pragma unroll
+                            for (int cf = 0; cf < CF; ++cf)
+#pragma unroll
+                                for (int i = 0; i < VW; ++i)
+                                    s = fmaf(av[w][cf].v[i], x[u][cf].v[i], s);
+                            part[w][j0 + u] = s;
+                        }
+                }
+#pragma unroll
+                for (int w = 0; w < V; ++w)
+                    res[t][w] += transpose_reduce<LPR>(part[w], gl);
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < ENT; ++t) {
+            const int k = lb + off + t * LPR + gl;
+            if (k < hb) {
+#pragma unroll
+                for (int w = 0; w < V; ++w) {
+                    // Block layouts: positions whose stored value is zero are not part of
+                    // the pattern and receive zero.
+                    const float r = (V > 1 && cval[t][w] == 0.f) ? 0.f : res[t][w];
+                    __stcs(a.out + (int64_t)k * V + w, r);
+                }
+            }
+        }
+    }
+}
+
+// The first `long_ctas` CTAs look after the long rows (more than a.long_row entries), which the lane
+// groups of the others pass over: a hub row is otherwise one group's serial walk (25 K entries, dim
+// 100: 8.8 ms in a product whose other rows take 0.1 ms).  CTA c owns the entries
+// [c, c+1) * a.long_range, finds the long rows among them (find_segment, then one look at each row
+// between) and deals each one's entries to its lane groups.  Entries are independent, so nothing has
+// to be merged and one launch does both.
+template <int LPR, int VW, int CF, int V>
+__global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
+{
     const int gpc = blockDim.x / LPR;
     const int g = threadIdx.x / LPR;
     const int gl = threadIdx.x % LPR;
-    const int tiles = (a.nvec + LPR * CF - 1) / (LPR * CF);
 
-    const int64_t seg0 = (int64_t)blockIdx.x * gpc * a.rows_per_group;
+    if (blockIdx.x < a.long_ctas) {
+        __shared__ int row_list[PSPMM_LONG_PER_RANGE];
+        __shared__ int row_ends[2];
+        __shared__ int n_long;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const int64_t begin = __ldg(a.segPtr), end = __ldg(a.segPtr + a.n_seg);
+        for (int64_t s = begin + (int64_t)blockIdx.x * a.long_range; s < end; s += (int64_t)a.long_ctas * a.long_range) {
+            const int64_t e1 = s + a.long_range < end ? s + a.long_range : end;
+            if (threadIdx.x == 0)
+                n_long = 0;
+            if (warp == 0 || (warp == 1 && blockDim.x > 32)) {
+                const int r = find_segment(a.segPtr, a.n_seg, begin, end, warp == 0 ? s : e1 - 1, lane);
+                if (lane == 0)
+                    row_ends[warp] = r;
+                if (blockDim.x == 32) {
+                    const int r1 = find_segment(a.segPtr, a.n_seg, begin, end, e1 - 1, lane);
+                    if (lane == 0)
+                        row_ends[1] = r1;
+                }
+            }
+            __syncthreads();
+            for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += blockDim.x)
+                if (__ldg(a.segPtr + r + 1) - __ldg(a.segPtr + r) > a.long_row)
+                    row_list[atomicAdd(&n_long, 1)] = (int)r;
+            __syncthreads();
+            for (int i = 0; i < n_long; ++i) {
+                const int r = row_list[i];
+                const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
+                const int64_t lo = rb > s ? rb : s, hi = re < e1 ? re : e1;
+                // a share per lane group, a multiple of its width so that its stores stay coalesced
+                const int share = (int)(((hi - lo + gpc - 1) / gpc + LPR - 1) / LPR * LPR);
+                int64_t b = lo + (int64_t)g * share;
+                b = b < hi ? b : hi;
+                const int64_t e = b + share < hi ? b + share : hi;
+                sddmm_entries<LPR, VW, CF, V>(a, r, (int)b, (int)e, share, gl);
+            }
+            __syncthreads();
+        }
+        return;
+    }
+
+    const int64_t seg0 = (int64_t)(blockIdx.x - a.long_ctas) * gpc * a.rows_per_group;
     for (int it = 0; it < a.rows_per_group; ++it) {
         const int64_t seg = seg0 + (int64_t)it * gpc + g;
-        const bool live = seg < a.n_seg;
         int lb = 0, hb = 0;
         int64_t arow = 0;
-        if (live) {
+        if (seg < a.n_seg) {
             lb = __ldg(a.segPtr + seg);
             hb = __ldg(a.segPtr + seg + 1);
             arow = a.target_row ? (int64_t)__ldg(a.target_row + seg) : seg;
+            if (hb - lb > a.long_row)
+                hb = lb;
         }
-        const int len = hb - lb;
-        int maxlen = len;
+        int maxlen = hb - lb;
         if constexpr (LPR < 32)
-            maxlen = __reduce_max_sync(PSPMM_FULL_MASK, len);
-
-        for (int off = 0; off < maxlen; off += CHUNK) {
-            int ccol[ENT];
-            float cval[ENT][V];
-            float res[ENT][V];
-#pragma unroll
-            for (int t = 0; t < ENT; ++t) {
-                const int k = lb + off + t * LPR + gl;
-                const bool ok = k < hb;
-                ccol[t] = ok ? __ldg(a.colIdx + k) : 0;
-#pragma unroll
-                for (int w = 0; w < V; ++w) {
-                    cval[t][w] = (V > 1 && ok) ? __ldg(a.val + (int64_t)k * V + w) : 1.f;
-                    res[t][w] = 0.f;
-                }
-            }
-            const int cnt = len - off;
-            const int wcnt = maxlen - off;
-
-            for (int tile = 0; tile < tiles; ++tile) {
-                // Slice of the A row(s) this lane is responsible for in this tile.
-                FVec<VW> av[V][CF];
-                int voff[CF];
-                bool act[CF];
-#pragma unroll
-                for (int cf = 0; cf < CF; ++cf) {
-                    const int vi = (tile * CF + cf) * LPR + gl;
-                    act[cf] = vi < a.nvec;
-                    voff[cf] = vi * VW;
-#pragma unroll
-                    for (int w = 0; w < V; ++w)
-                        // (the last block-row of an odd row count has lanes without a row of A)
-                        av[w][cf] = (live && act[cf] && arow * V + w < a.n_rows_A)
-                                        ? ldg_vec<VW>(a.A + (arow * V + w) * a.ldA + voff[cf])
-                                        : zero_vec<VW>();
-                }
-#pragma unroll
-                for (int t = 0; t < ENT; ++t) {
-                    if (t * LPR >= wcnt)
-                        break;
-                    float part[V][LPR];
-#pragma unroll
-                    for (int j0 = 0; j0 < LPR; j0 += U) {
-                        FVec<VW> x[U][CF];
-                        const bool batch_on = (t * LPR + j0) < wcnt;  // warp-uniform
-#pragma unroll
-                        for (int u = 0; u < U; ++u) {
-                            const int e = t * LPR + j0 + u;
-                            const int c = __shfl_sync(PSPMM_FULL_MASK, ccol[t], j0 + u, LPR);
-                            const float *brow = a.B + (int64_t)c * a.ldB;
-                            const bool p = batch_on && (e < cnt);
-#pragma unroll
-                            for (int cf = 0; cf < CF; ++cf)
-                                x[u][cf] = ldg_vec_if<VW>(brow + voff[cf], p && act[cf]);
-                        }
-#pragma unroll
-                        for (int u = 0; u < U; ++u)
-#pragma unroll
-                            for (int w = 0; w < V; ++w) {
-                                float s = 0.f;
-#pragma unroll
-                                for (int cf = 0; cf < CF; ++cf)
-#pragma unroll
-                                    for (int i = 0; i < VW; ++i)
-                                        s = fmaf(av[w][cf].v[i], x[u][cf].v[i], s);
-                                part[w][j0 + u] = s;
-                            }
-                    }
-#pragma unroll
-                    for (int w = 0; w < V; ++w)
-                        res[t][w] += transpose_reduce<LPR>(part[w], gl);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < ENT; ++t) {
-                const int k = lb + off + t * LPR + gl;
-                if (k < hb) {
-#pragma unroll
-                    for (int w = 0; w < V; ++w) {
-                        // Block layouts: positions whose stored value is zero are not part of
-                        // the pattern and receive zero.
-                        const float r = (V > 1 && cval[t][w] == 0.f) ? 0.f : res[t][w];
-                        __stcs(a.out + (int64_t)k * V + w, r);
-                    }
-                }
-            }
-        }
+            maxlen = __reduce_max_sync(PSPMM_FULL_MASK, maxlen);
+        sddmm_entries<LPR, VW, CF, V>(a, arow, lb, hb, maxlen, gl);
     }
 }
 

@@ -30,6 +30,10 @@
 // segment covers lie between the target rows of consecutive segments: every group zeroes the
 // short gap that follows each of its rows (up to PSPMM_GAP_MAX rows); longer gaps are left to
 // the pre-pass.
+//
+// Long rows of an unsplit layout (more than SpmmArgs::long_row entries) are left to
+// spmm_long_rows_kernel below, which cuts them over the whole GPU; here they count as empty rows,
+// so the zeros that the second kernel adds to are stored by the same code.
 #pragma once
 
 #include "pspmm_common.cuh"
@@ -97,7 +101,14 @@ struct SpmmOcc {
 
 // ACC = true adds the product to C instead of overwriting it: every contribution is a RED, rows
 // without entries add nothing, and nothing is zeroed (no pre-pass either).
-template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false>
+// Largest ticket (SpmmArgs::long_ticket) of a launch that passed over a long row; one per device and
+// translation unit, and a launch and the one that follows it are of the same unit.
+static __device__ unsigned long long g_long_seen;
+
+// LONG = true (unsplit layouts) passes over rows of more than a.long_row entries.  Both are template
+// flags because a run-time test of either costs the 48- and 80-register shapes spills (4 - 13 % of
+// the dim sweep's products).
+template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
 __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(const SpmmArgs a)
 {
     using Tile = SpmmTile<LPR, V>;
@@ -122,6 +133,8 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
         return;  // the whole group leaves; groups only ever synchronise among themselves
     const int nrow = (a.n_seg - first < rpg) ? (int)(a.n_seg - first) : rpg;
     const bool split = a.target_row != nullptr;
+    if constexpr (LONG)
+        pdl_launch_dependents();
 
     for (int i = gl; i <= nrow; i += LPR)
         sp[i] = __ldg(a.segPtr + first + i);
@@ -159,6 +172,8 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
             for (int i = 0; i < VW; ++i)
                 acc[w][cf][i] = 0.f;
 
+    if (split)
+        pdl_wait();  // the pre-pass has zeroed the rows that are added to
     __syncwarp(gmask);
     int cur = sp[0];
     const int end = sp[nrow];
@@ -183,10 +198,12 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
         }
         __syncwarp(gmask);
         const int lim = cur + fill;
+        int resume = lim;
         while (row < nrow) {
             const int rb = sp[row], re = sp[row + 1];
+            const bool skip = LONG && re - rb > a.long_row;  // left to spmm_long_rows_kernel
             int e = (rb > cur ? rb : cur) - cur;
-            const int eh = (re < lim ? re : lim) - cur;
+            const int eh = skip ? e : (re < lim ? re : lim) - cur;
             for (; e + U <= eh; e += U)
                 spmm_batch<U, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
             if constexpr (U >= 16) {
@@ -211,7 +228,7 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                 if (e < eh)
                     spmm_batch<1, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
             }
-            if (re > lim)
+            if (re > lim && !skip)
                 break;  // the row continues in the next window
 
             // ---- the segment is complete
@@ -280,34 +297,216 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                 head_pending = false;
             }
             ++row;
+            if (skip) {  // the window restarts behind the long row
+                if (gl == 0)
+                    atomicMax(&g_long_seen, a.long_ticket);
+                resume = re;
+                break;
+            }
         }
         if (row >= nrow)
             break;
-        cur = lim;
+        cur = resume;
         __syncwarp(gmask);  // everyone is done reading the window before it is refilled
     }
 }
 
-template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false>
+// Rows of more than a.long_row entries of an unsplit (block-)CSR layout, which spmm_seg_kernel has
+// stored as zeros.  A row there is walked by one lane group, one gather batch after the other: a hub
+// row of 1,600 entries held a 197 K-entry graph at dim 16 for 310 us, 98 % of the product.  Here
+// CTA c owns the entries [c, c+1) * a.long_range whatever rows they belong to: two warps find the
+// first and last row of the range (32 pointers probed per step), all threads look for long rows
+// between them, and the eight warps share each one that is found, 32 entries per warp and step,
+// their sums meeting in shared memory and leaving as one vector RED per CTA and row.  Nothing is
+// allocated and no list is kept.  spmm_seg_kernel raises g_long_seen to this launch's ticket when it
+// passes over a row, so a matrix without long rows costs one look at that word (1.5 us behind the
+// products it was measured on; searching all ranges cost 6 us of 86).  Tickets only grow: a word that
+// a later launch has raised further makes this one search in vain, never miss a row.  Bound: gather
+// latency (8 x 16-byte loads in flight per lane, as above).
+template <int VW, int V, int LPR>
+__global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmArgs a)
+{
+    constexpr int GROUPS = 32 / LPR;
+    constexpr int U = (LPR < 8 ? LPR : 8) / (V > 1 ? 2 : 1);
+    __shared__ float sums[8][V * LPR * VW];
+    __shared__ int row_list[PSPMM_LONG_PER_RANGE];
+    __shared__ int row_ends[2];
+    __shared__ int n_long;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane / LPR, gl = lane % LPR;
+    const int v = blockIdx.y * LPR + gl;
+    const bool act = v < a.nvec;
+    const int voff = act ? v * VW : 0;
+    const char *bcol = reinterpret_cast<const char *>(a.B + voff);
+    const unsigned ldB_bytes = (unsigned)(a.ldB * 4);
+    const unsigned long long keep = l2_policy_keep(a.keep_fraction);
+    const unsigned long long stream = l2_policy_stream();
+    const int64_t begin = __ldg(a.segPtr), end = __ldg(a.segPtr + a.n_seg);
+    // (an early look lets the searches run while the kernel before this one drains)
+    bool waited = false;
+    if (*(volatile unsigned long long *)&g_long_seen < a.long_ticket) {
+        pdl_wait();
+        waited = true;
+        if (*(volatile unsigned long long *)&g_long_seen < a.long_ticket)
+            return;
+    }
+    for (int64_t s = begin + (int64_t)blockIdx.x * a.long_range; s < end; s += (int64_t)gridDim.x * a.long_range) {
+        const int64_t e1 = s + a.long_range < end ? s + a.long_range : end;
+        if (threadIdx.x == 0)
+            n_long = 0;
+        if (warp < 2) {
+            const int r = find_segment(a.segPtr, a.n_seg, begin, end, warp == 0 ? s : e1 - 1, lane);
+            if (lane == 0)
+                row_ends[warp] = r;
+        }
+        __syncthreads();
+        for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += 256)
+            if (__ldg(a.segPtr + r + 1) - __ldg(a.segPtr + r) > a.long_row)
+                row_list[atomicAdd(&n_long, 1)] = (int)r;
+        __syncthreads();
+        const int count = n_long;
+        if (count > 0 && !waited) {
+            pdl_wait();
+            waited = true;
+        }
+        for (int i = 0; i < count; ++i) {
+            const int r = row_list[i];
+            const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
+            const int64_t lo = rb > s ? rb : s, hi = re < e1 ? re : e1;
+            float acc[V][VW];
+#pragma unroll
+            for (int w = 0; w < V; ++w)
+#pragma unroll
+                for (int j = 0; j < VW; ++j)
+                    acc[w][j] = 0.f;
+            for (int64_t k0 = lo + warp * 32; k0 < hi; k0 += 256) {
+                const int64_t k = k0 + lane;
+                const bool in = k < hi;
+                const int cc = in ? ldg_stream_b32(a.colIdx + k, stream) : 0;
+                float vv[V];
+#pragma unroll
+                for (int w = 0; w < V; ++w)
+                    vv[w] = !in ? 0.f : (V == 1 && !a.val) ? 1.f : __int_as_float(ldg_stream_b32(a.val + k * V + w, stream));
+                const int left = (int)(hi - k0);
+#pragma unroll
+                for (int j0 = 0; j0 < LPR; j0 += U) {
+                    FVec<VW> x[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int c = __shfl_sync(PSPMM_FULL_MASK, cc, j0 + u, LPR);
+                        x[u] = ldg_vec_if<VW>(row_slice(bcol, c, ldB_bytes), g * LPR + j0 + u < left);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u)
+#pragma unroll
+                        for (int w = 0; w < V; ++w) {
+                            const float f = __shfl_sync(PSPMM_FULL_MASK, vv[w], j0 + u, LPR);
+                            if (V > 1 && f == 0.f)
+                                continue;  // an explicit zero of a block is no entry
+#pragma unroll
+                            for (int j = 0; j < VW; ++j)
+                                acc[w][j] = fmaf(f, x[u].v[j], acc[w][j]);
+                        }
+                }
+            }
+            // lane groups of a warp, then the warps
+#pragma unroll
+            for (int d = LPR; d < 32; d <<= 1)
+#pragma unroll
+                for (int w = 0; w < V; ++w)
+#pragma unroll
+                    for (int j = 0; j < VW; ++j)
+                        acc[w][j] += __shfl_xor_sync(PSPMM_FULL_MASK, acc[w][j], d);
+            if (g == 0) {
+#pragma unroll
+                for (int w = 0; w < V; ++w)
+#pragma unroll
+                    for (int j = 0; j < VW; ++j)
+                        sums[warp][(w * LPR + gl) * VW + j] = acc[w][j];
+            }
+            __syncthreads();
+            for (int t = threadIdx.x; t < V * LPR; t += 256) {
+                const int w = t / LPR, vi = blockIdx.y * LPR + t % LPR;
+                if (vi < a.nvec) {
+                    float tot[VW];
+#pragma unroll
+                    for (int j = 0; j < VW; ++j) {
+                        tot[j] = 0.f;
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            tot[j] += sums[q][t * VW + j];
+                    }
+                    red_add_vec<VW>(a.C + ((int64_t)r * V + w) * a.ldC + vi * VW, tot);
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+    if (!waited)
+        pdl_wait();  // this grid must not count as done before the one it follows
+}
+
+template <int VW, int V>
+static inline void spmm_launch_long_rows(const SpmmArgs &a, cudaStream_t st)
+{
+    const int lpr = a.nvec > 16 ? 32 : (a.nvec > 8 || V > 1) ? 16 : (a.nvec > 4 ? 8 : 4);
+    const int64_t ranges = (a.n_entries + a.long_range - 1) / a.long_range;
+    const unsigned tiles = (unsigned)((a.nvec + lpr - 1) / lpr);
+    const int64_t most = a.sms * 3 / tiles + 1;  // one resident wave
+    const dim3 grid((unsigned)(ranges < most ? ranges : most), tiles);
+    if (lpr == 32)
+        launch_dependent(spmm_long_rows_kernel<VW, V, 32>, grid, 256, 0, st, a);
+    else if (lpr == 16)
+        launch_dependent(spmm_long_rows_kernel<VW, V, 16>, grid, 256, 0, st, a);
+    else if constexpr (V == 1) {
+        if (lpr == 8)
+            launch_dependent(spmm_long_rows_kernel<VW, V, 8>, grid, 256, 0, st, a);
+        else
+            launch_dependent(spmm_long_rows_kernel<VW, V, 4>, grid, 256, 0, st, a);
+    }
+}
+
+// The launch that follows spmm_seg_kernel when rows may have been left to it.
+#define PSPMM_SPMM_LONG_ROWS(VW_)                                            \
+    if (a.n_entries > 0 && a.long_row < INT32_MAX) {                         \
+        if (V == 1)                                                          \
+            spmm_launch_long_rows<VW_, 1>(a, st);                            \
+        else if (V == 2)                                                     \
+            spmm_launch_long_rows<VW_, 2>(a, st);                            \
+        else                                                                 \
+            spmm_launch_long_rows<VW_, 3>(a, st);                            \
+    }
+
+template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
 static inline void spmm_launch_one(const SpmmArgs &a, dim3 grid, int threads, cudaStream_t st)
 {
     const int smem = (threads / LPR) * SpmmTile<LPR, V>::GROUP_WORDS * 4;
-    auto kern = spmm_seg_kernel<LPR, VW, CF, V, MLP, ACC>;
+    auto kern = spmm_seg_kernel<LPR, VW, CF, V, MLP, ACC, LONG>;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    kern<<<grid, threads, smem, st>>>(a);
+    if (a.target_row && !ACC)
+        launch_dependent(kern, grid, threads, smem, st, a);  // follows the zeroing pre-pass
+    else
+        kern<<<grid, threads, smem, st>>>(a);
 }
 
 // Expands to the dispatch over the instantiated (LPR, CF) pairs of one (VW, V).
-#define PSPMM_SPMM_CASE(LPR_, CF_, VW_, V_)                                  \
-    if (s.lpr == LPR_ && s.cf == CF_) {                                      \
-        spmm_launch_one<LPR_, VW_, CF_, V_, 8>(a, grid, s.threads, st);      \
-        return true;                                                         \
+// (the form that passes over long rows is built at one gather-batch depth)
+#define PSPMM_SPMM_CASE(LPR_, CF_, VW_, V_)                                               \
+    if (s.lpr == LPR_ && s.cf == CF_) {                                                   \
+        if (a.long_row < INT32_MAX)                                                       \
+            spmm_launch_one<LPR_, VW_, CF_, V_, 8, false, true>(a, grid, s.threads, st);  \
+        else                                                                              \
+            spmm_launch_one<LPR_, VW_, CF_, V_, 8>(a, grid, s.threads, st);               \
+        return true;                                                                      \
     }
 // Same, with every gather-batch depth instantiated (used for the 128-bit CSR family).
 #define PSPMM_SPMM_CASE_MLP(LPR_, CF_, VW_, V_)                              \
     if (s.lpr == LPR_ && s.cf == CF_) {                                      \
-        if (s.mlp == 2)                                                      \
+        if (a.long_row < INT32_MAX)                                          \
+            spmm_launch_one<LPR_, VW_, CF_, V_, 8, false, true>(a, grid, s.threads, st); \
+        else if (s.mlp == 2)                                                 \
             spmm_launch_one<LPR_, VW_, CF_, V_, 2>(a, grid, s.threads, st);  \
         else if (s.mlp == 4)                                                 \
             spmm_launch_one<LPR_, VW_, CF_, V_, 4>(a, grid, s.threads, st);  \

@@ -191,6 +191,8 @@ class PlannedSpMM:
     def __call__(self, out, B, accumulate=False):
         from . import _lib, ops
         kw = self.plan.kernel_cfg()
+        if self.target is None and self.plan.get("regime", "skewed").rpartition("_")[2] != "skewed":
+            kw["bucketed"] = 1  # the statistics showed no long row: nothing to look for on each call
         if accumulate:  # built for 128-bit loads at one gather-batch depth
             kw.update(vec_width=0, gather_batch=0, accumulate=1)
         dst = out

@@ -600,16 +600,18 @@ def agnn_fused(A, B, rowPtr, colIdx, beta=1.0, softmax=True, target_row=None, n_
     if out is None:
         out = torch.empty(n_out_rows, dim, dtype=torch.float32, device=A.device)
     null = ctypes.c_void_p(0)
-    scratch, sbytes = None, 0
+    scratch, need = None, ctypes.c_size_t(0)
     if split:
-        need = ctypes.c_size_t(0)
         check(lib().pspmm_agnn_scratch_bytes(n_seg, dim, ctypes.byref(need)))
-        sbytes = need.value
+    else:
+        check(lib().pspmm_agnn_long_scratch_bytes(colIdx.shape[0], dim, ctypes.byref(need)))
+    sbytes = need.value
+    if sbytes:
         scratch = torch.empty((sbytes + 15) // 16 * 4, dtype=torch.float32, device=A.device)
     seg_ptr = _ptr(rowPtr)
     tail = (float(beta), 1 if softmax else 0, int(vec_width), int(lanes_per_row), int(batch),
             seg_ptr if split else null, _ptr(target_row) if split else null, n_seg if split else 0,
-            _ptr(scratch) if split else null, sbytes, _stream())
+            _ptr(scratch), sbytes, _stream())
     if V is None:
         check(lib().pspmm_agnn_fused_csr(null if split else seg_ptr, _ptr(colIdx), _ptr(A), _ptr(B), _ptr(out),
                                          n_out_rows, colIdx.shape[0], dim, A.stride(0), B.stride(0), out.stride(0),

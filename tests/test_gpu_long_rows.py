@@ -1,0 +1,75 @@
+"""Rows of an unsplit layout that are longer than the others: the kernels cut them over the GPU from
+64 .. 512 entries on (by the matrix's size), everything else stays with one lane group."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _matrix(lengths, n_cols, seed):
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(n_cols, k, replace=False)) for k in lengths] + [[]]).astype(np.int32)
+    return rp, ci, rng.random(len(ci), dtype=np.float32)
+
+
+LAYOUTS = {
+    "around the threshold": [63, 0, 64, 65, 3, 66, 0, 0, 129, 1],
+    "long rows back to back": [600] * 9 + [0, 5] + [513] * 4,
+    "one row holds all": [0, 0, 4097, 0],
+    "first and last": [5000] + [2] * 700 + [5000],
+    "short rows between hubs": ([1, 0, 2, 900] * 40),
+}
+
+
+@pytest.mark.parametrize("dim", [1, 6, 16, 47, 64, 132])
+@pytest.mark.parametrize("name", sorted(LAYOUTS))
+def test_long_rows_match_the_oracle(oracle, name, dim):
+    from paramspmm_ae_b200 import ops
+    dev = torch.device("cuda:0")
+    n_cols = 6001
+    rp, ci, v = _matrix(LAYOUTS[name], n_cols, 3)
+    n = len(rp) - 1
+    rng = np.random.default_rng(4)
+    B = rng.uniform(-1, 1, (n_cols, dim)).astype(np.float32)
+    t = lambda x: torch.from_numpy(x).to(dev)
+    rpd, cid, vd, Bd = t(rp), t(ci), t(v), t(B)
+    out = torch.full((n, dim), float("nan"), device=dev)
+    ops.spmm_into(out, Bd, rpd, cid, vd)
+    np.testing.assert_allclose(out.cpu().numpy(), oracle.spmm_csr(rp, ci, v, B), rtol=1e-5, atol=1e-4)
+    for V in (2, 3):
+        rpb, cb, vb = ops.bcsr_from_csr(torch.from_numpy(rp), torch.from_numpy(ci), torch.from_numpy(v), n_cols, V)
+        nb = rpb.shape[0] - 1
+        out = torch.full((nb * V, dim), float("nan"), device=dev)
+        ops.spmm_into(out, Bd, rpb.to(dev), cb.to(dev), vb.to(dev), V=V)
+        np.testing.assert_allclose(out[:n].cpu().numpy(), oracle.spmm_csr(rp, ci, v, B), rtol=1e-5, atol=1e-4)
+    A = rng.uniform(-1, 1, (n, dim)).astype(np.float32)
+    got = ops.csr_sddmm(t(A), Bd, rpd, cid, vd, 1, 4)
+    np.testing.assert_allclose(got.cpu().numpy(), oracle.sddmm_csr(rp, ci, A, B), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("dim", [4, 32, 64, 132, 256])
+@pytest.mark.parametrize("softmax", [True, False])
+@pytest.mark.parametrize("name", sorted(LAYOUTS))
+def test_long_rows_of_the_fused_aggregation(oracle, name, dim, softmax):
+    from paramspmm_ae_b200 import ops
+    dev = torch.device("cuda:0")
+    n_cols = 6001
+    rp, ci, _ = _matrix(LAYOUTS[name], n_cols, 5)
+    n = len(rp) - 1
+    rng = np.random.default_rng(6)
+    A, B, V = ((rng.uniform(-1, 1, (k, dim)) / np.sqrt(dim)).astype(np.float32) for k in (n, n_cols, n_cols))
+    t = lambda x: torch.from_numpy(x).to(dev)
+    want = oracle.agnn_aggregate(rp, ci, A, B, 2.0, softmax)
+    got = ops.agnn_fused(t(A), t(B), t(rp), t(ci), 2.0, softmax)
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=1e-5, atol=1e-4)
+    rps, tr = ops.split_csr(torch.from_numpy(rp), 7)  # hundreds of pieces per row: the merge takes whole thread blocks
+    got = ops.agnn_fused(t(A), t(B), rps.to(dev), t(ci), 2.0, softmax, target_row=tr.to(dev), n_out_rows=n)
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=1e-5, atol=1e-4)
+    got = ops.agnn_fused(t(A), t(B), t(rp), t(ci), 2.0, softmax, V=t(V)).double().cpu().numpy()
+    for r in range(n):
+        c = ci[rp[r]:rp[r + 1]]
+        s = 2.0 * B[c].astype(np.float64) @ A[r].astype(np.float64)
+        w = s if not softmax else np.exp(s - s.max(initial=-np.inf)) / max(np.exp(s - s.max(initial=-np.inf)).sum(), 1e-300)
+        np.testing.assert_allclose(got[r], w @ V[c].astype(np.float64), rtol=1e-5, atol=1e-4)
