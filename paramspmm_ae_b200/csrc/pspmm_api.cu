@@ -509,7 +509,25 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     if (n_seg == 0)
         return PSPMM_OK;
     LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldA, ldB, A, B), V, &s);
+    // At most 16 lanes per row: with 32 the exchange of partial sums (31 shuffles and 62 selects per 32
+    // entries of a single row) took over, 12.6 ms against 4.1 for 115 M entries at dim 128.  Scalar and
+    // 8-byte loads fill 8 lanes up to 4 slices first (dim 17: 64 against 87 us, 4 M entries).  Rows of
+    // more than 3 slices of 16 lanes go through column tiles of 2 inside the kernel (a fourth slice
+    // leaves too few registers: dim 256 14.0 ms, two tiles of 128 9.0); scalar loads keep up to 8.
+    pspmm_cfg narrow = {};
+    if (cfg)
+        narrow = *cfg;
+    const int vw_max = pspmm_vw_max(dim, ldA, ldB, A, B);
+    const int nvec_max = dim / vw_max;
+    if (V == 1 && (narrow.lanes_per_row == 0 || narrow.lanes_per_row > 16) && nvec_max > 8)
+        narrow.lanes_per_row = vw_max < 4 && nvec_max <= 32 ? 8 : 16;
+    pspmm_resolve_shape(&narrow, dim, vw_max, V, &s);
+    if (V == 1 && s.lpr > 16) {
+        s.lpr = 16;
+        s.cf = 8;
+    }
+    if (V == 1 && s.vw == 4 && s.lpr == 16 && s.cf > 3)
+        s.cf = 2;
     if (!cfg || cfg->cta_threads == 0)
         s.threads = 128;  // measured: 128-thread CTAs are 7 % faster than 256 for this kernel
     if (!cfg || cfg->rows_per_group == 0)
@@ -529,11 +547,16 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     a.nvec = dim / s.vw;
     a.rows_per_group = s.rpg;
     a.keep_fraction = 1.0f;  // the row count of B is not part of the call: no partial pinning
-    a.long_row = target_row ? INT32_MAX : pspmm_long_row_threshold(n_entries);
+    // Unsplit rows of more than 64 entries are cut: the pieces of 32 the long-row CTAs deal out keep a
+    // warp's groups in step, which rows of very different length do not.  A range costs its CTA two
+    // searches, so it is up to 8192 entries where the matrix has enough of them to fill the chip.
+    a.long_row = target_row || n_entries <= 64 ? INT32_MAX : 64;
     a.long_range = 0;
     a.long_ctas = 0;
     if (a.long_row < INT32_MAX) {
-        a.long_range = 8 * a.long_row;
+        a.long_range = 256;
+        while (a.long_range < 8192 && n_entries / a.long_range > (int64_t)sm_count() * 24)
+            a.long_range *= 2;
         const int64_t ranges = (n_entries + a.long_range - 1) / a.long_range;
         a.long_ctas = (uint32_t)(ranges < 65536 ? ranges : 65536);
     }

@@ -10,6 +10,7 @@
 #define PSPMM_MAX_CF 8
 #define PSPMM_RPG_MAX 16  // most consecutive segments one lane group owns
 #define PSPMM_LONG_PER_RANGE 12  // a range of 8 * long_row entries meets at most 9 rows longer than long_row
+#define PSPMM_LONG_LIST 132  // rows longer than long_row that a range of 128 * long_row entries can meet, and a few
 #define PSPMM_GAP_MAX 256  // longest run of uncovered rows the SpMM kernel zeroes by itself
 
 // Records the CUDA error text for pspmm_last_cuda_error() and returns PSPMM_E_CUDA.
@@ -119,7 +120,7 @@ struct SddmmArgs {
     int32_t rows_per_group;
     float keep_fraction;
     int32_t long_row;    // unsplit rows with more entries are dealt to the first long_ctas CTAs (INT32_MAX: none are)
-    int32_t long_range;  // entries per range of those CTAs
+    int32_t long_range;  // entries per range of those CTAs, at most 128 * long_row
     uint32_t long_ctas;
 };
 

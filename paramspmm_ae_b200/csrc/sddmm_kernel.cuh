@@ -43,9 +43,10 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
 {
     constexpr int ENT = (LPR >= 16) ? 1 : (16 / LPR);
     constexpr int CHUNK = LPR * ENT;
-    constexpr int U0 = 8 / CF;
-    constexpr int U1 = U0 < 1 ? 1 : U0;
-    constexpr int U = U1 > LPR ? LPR : U1;  // entries whose gathers are batched (divides LPR)
+    // entries whose gathers are batched (divides LPR): 8 loads in flight per lane, 16 with wide rows
+    constexpr int U0 = CF >= 8 ? 2 : (CF >= 3 ? 4 : 8 / CF);
+    constexpr int U1 = V > 1 && U0 > 1 && CF > 1 ? U0 / 2 : U0;
+    constexpr int U = U1 > LPR ? LPR : U1;
     const int tiles = (a.nvec + LPR * CF - 1) / (LPR * CF);
     const int len = hb - lb;
     const bool live = len > 0;
@@ -141,8 +142,8 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
 // groups of the others pass over: a hub row is otherwise one group's serial walk (25 K entries, dim
 // 100: 8.8 ms in a product whose other rows take 0.1 ms).  CTA c owns the entries
 // [c, c+1) * a.long_range, finds the long rows among them (find_segment, then one look at each row
-// between) and deals each one's entries to its lane groups.  Entries are independent, so nothing has
-// to be merged and one launch does both.
+// between) and deals pieces of their entries to its lane groups.  Entries are independent, so nothing
+// has to be merged and one launch does both.
 template <int LPR, int VW, int CF, int V>
 __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
 {
@@ -151,7 +152,7 @@ __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
     const int gl = threadIdx.x % LPR;
 
     if (blockIdx.x < a.long_ctas) {
-        __shared__ int row_list[PSPMM_LONG_PER_RANGE];
+        __shared__ int row_list[PSPMM_LONG_LIST], row_lo[PSPMM_LONG_LIST], row_hi[PSPMM_LONG_LIST];
         __shared__ int row_ends[2];
         __shared__ int n_long;
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -160,31 +161,42 @@ __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
             const int64_t e1 = s + a.long_range < end ? s + a.long_range : end;
             if (threadIdx.x == 0)
                 n_long = 0;
-            if (warp == 0 || (warp == 1 && blockDim.x > 32)) {
-                const int r = find_segment(a.segPtr, a.n_seg, begin, end, warp == 0 ? s : e1 - 1, lane);
+            for (int q = warp; q < 2; q += blockDim.x >> 5) {
+                const int r = find_segment(a.segPtr, a.n_seg, begin, end, q == 0 ? s : e1 - 1, lane);
                 if (lane == 0)
-                    row_ends[warp] = r;
-                if (blockDim.x == 32) {
-                    const int r1 = find_segment(a.segPtr, a.n_seg, begin, end, e1 - 1, lane);
-                    if (lane == 0)
-                        row_ends[1] = r1;
+                    row_ends[q] = r;
+            }
+            __syncthreads();
+            for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += blockDim.x) {
+                const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
+                if (re - rb > a.long_row) {
+                    const int i = atomicAdd(&n_long, 1);
+                    row_list[i] = (int)r;
+                    row_lo[i] = (int)(rb > s ? rb : s);
+                    row_hi[i] = (int)(re < e1 ? re : e1);
                 }
             }
             __syncthreads();
-            for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += blockDim.x)
-                if (__ldg(a.segPtr + r + 1) - __ldg(a.segPtr + r) > a.long_row)
-                    row_list[atomicAdd(&n_long, 1)] = (int)r;
-            __syncthreads();
-            for (int i = 0; i < n_long; ++i) {
-                const int r = row_list[i];
-                const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
-                const int64_t lo = rb > s ? rb : s, hi = re < e1 ? re : e1;
-                // a share per lane group, a multiple of its width so that its stores stay coalesced
-                const int share = (int)(((hi - lo + gpc - 1) / gpc + LPR - 1) / LPR * LPR);
-                int64_t b = lo + (int64_t)g * share;
-                b = b < hi ? b : hi;
-                const int64_t e = b + share < hi ? b + share : hi;
-                sddmm_entries<LPR, VW, CF, V>(a, r, (int)b, (int)e, share, gl);
+            // Pieces of 32 entries, dealt to the lane groups in turn over all long rows of the range.
+            const int n = n_long;
+            int i = 0, piece0 = 0;  // the row the group stands in, and the number of its first piece
+            for (int p0 = 0;; p0 += gpc) {
+                const int p = p0 + g;
+                int pieces = 0;
+                while (i < n && p >= piece0 + (pieces = (row_hi[i] - row_lo[i] + 31) / 32)) {
+                    piece0 += pieces;
+                    ++i;
+                }
+                if (!__any_sync(PSPMM_FULL_MASK, i < n))
+                    break;  // (pieces are dealt in order: the warp has none left)
+                int lb = 0, hb = 0;
+                int64_t row = 0;
+                if (i < n) {
+                    row = row_list[i];
+                    lb = row_lo[i] + (p - piece0) * 32;
+                    hb = lb + 32 < row_hi[i] ? lb + 32 : row_hi[i];
+                }
+                sddmm_entries<LPR, VW, CF, V>(a, row, lb, hb, 32, gl);
             }
             __syncthreads();
         }

@@ -15,7 +15,6 @@ bool pspmm_launch_sddmm_vw2(const LaunchShape &s, int V, const SddmmArgs &a, dim
     if (V == 1) {
         CFS_ALL(8, 1)
         CFS_ALL(16, 1)
-        CFS_ALL(32, 1)
     } else if (V == 2) {
         CFS_ALL(16, 2)
         CFS_ALL(32, 2)

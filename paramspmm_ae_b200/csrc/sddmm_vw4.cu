@@ -17,7 +17,6 @@ bool pspmm_launch_sddmm_vw4(const LaunchShape &s, int V, const SddmmArgs &a, dim
         CFS_ALL(4, 1)
         CFS_ALL(8, 1)
         CFS_ALL(16, 1)
-        CFS_ALL(32, 1)
     } else if (V == 2) {
         CFS_4(4, 2)
         CFS_4(8, 2)

@@ -191,3 +191,34 @@ __device__ __forceinline__ void red_add_vec(float *p, const float *v)
         atomicAdd(p, v[0]);
     }
 }
+
+// Sum over the LPR lanes of a group of p[e], delivered to lane (gl % BS) == e.
+template <int LPR, int BS>
+__device__ __forceinline__ float group_transpose_reduce(float (&p)[BS], int gl)
+{
+    // fold the lane bits above BS first (plain butterflies on all BS values) ...
+#pragma unroll
+    for (int d = LPR / 2; d >= BS; d >>= 1)
+#pragma unroll
+        for (int e = 0; e < BS; ++e)
+            p[e] += __shfl_xor_sync(0xffffffffu, p[e], d);
+    // ... then halve the value set at every remaining step
+    float q[BS];
+#pragma unroll
+    for (int e = 0; e < BS; ++e)
+        q[e] = p[e];
+    // recursive halving, written out iteratively
+#pragma unroll
+    for (int h = BS / 2; h >= 1; h >>= 1) {
+        const bool upper = (gl & h) != 0;
+#pragma unroll
+        for (int i = 0; i < BS / 2; ++i) {
+            if (i < h) {
+                const float keep = upper ? q[i + h] : q[i];
+                const float send = upper ? q[i] : q[i + h];
+                q[i] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+            }
+        }
+    }
+    return q[0];
+}
