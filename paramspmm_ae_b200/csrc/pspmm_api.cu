@@ -333,10 +333,21 @@ static int small_rows_per_group(int rpg, int64_t n_seg, int lpr)
     return rpg;
 }
 
-// Which rows of an unsplit layout are cut over the GPU: a lane group takes about a microsecond per
-// eight entries, so rows above 1/64 of an SM's share of the entries would outlast the rest; never
-// below 64 (a row's pieces must pay for their reduction) nor above 512 (half the time of the
-// smallest product that needs this many).  INT32_MAX: no row can be that long.
+// Entries of the ranges in which a kernel deals out the long rows (PSPMM_LONG_ROW) of an unsplit
+// layout.  Finding a range's rows takes two searches, so ranges are long, up to 8192 entries, while
+// there are enough of them to fill the chip several times over.
+static int long_range(int64_t n_entries, int per_sm)
+{
+    int r = 256;
+    while (r < PSPMM_LONG_RANGE_MAX && n_entries / r > (int64_t)sm_count() * per_sm)
+        r *= 2;
+    return r;
+}
+
+// Which rows of an unsplit layout the fused aggregation cuts over the GPU: a lane group takes about a
+// microsecond per eight entries, so rows above 1/64 of an SM's share of the entries would outlast
+// the rest; never below 64 (a row's pieces must pay for their reduction) nor above 512 (half the
+// time of the smallest product that needs this many).  INT32_MAX: no row can be that long.
 int pspmm_long_row_threshold(int64_t n_entries)
 {
     int t = 64;
@@ -424,8 +435,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.bucketed = bucketed ? 1 : 0;
     a.keep_fraction = l2_keep_fraction((double)n_cols * (double)ldB * 4.0);
     a.n_entries = n_entries;
-    a.long_row = target_row || accumulate || (cfg && cfg->bucketed) ? INT32_MAX : pspmm_long_row_threshold(n_entries);
-    a.long_range = a.long_row < INT32_MAX ? 8 * a.long_row : 0;
+    a.long_row = target_row || accumulate || (cfg && cfg->bucketed) || n_entries <= PSPMM_LONG_ROW ? INT32_MAX
+                                                                                                  : PSPMM_LONG_ROW;
+    a.long_range = long_range(n_entries, 8);  // (resident CTAs take the ranges in turn)
     a.sms = sm_count();
     static std::atomic<unsigned long long> tickets{0};
     a.long_ticket = a.long_row < INT32_MAX ? ++tickets : 0;
@@ -547,16 +559,10 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     a.nvec = dim / s.vw;
     a.rows_per_group = s.rpg;
     a.keep_fraction = 1.0f;  // the row count of B is not part of the call: no partial pinning
-    // Unsplit rows of more than 64 entries are cut: the pieces of 32 the long-row CTAs deal out keep a
-    // warp's groups in step, which rows of very different length do not.  A range costs its CTA two
-    // searches, so it is up to 8192 entries where the matrix has enough of them to fill the chip.
-    a.long_row = target_row || n_entries <= 64 ? INT32_MAX : 64;
-    a.long_range = 0;
+    a.long_row = target_row || n_entries <= PSPMM_LONG_ROW ? INT32_MAX : PSPMM_LONG_ROW;
+    a.long_range = long_range(n_entries, 24);
     a.long_ctas = 0;
     if (a.long_row < INT32_MAX) {
-        a.long_range = 256;
-        while (a.long_range < 8192 && n_entries / a.long_range > (int64_t)sm_count() * 24)
-            a.long_range *= 2;
         const int64_t ranges = (n_entries + a.long_range - 1) / a.long_range;
         a.long_ctas = (uint32_t)(ranges < 65536 ? ranges : 65536);
     }

@@ -10,7 +10,11 @@
 #define PSPMM_MAX_CF 8
 #define PSPMM_RPG_MAX 16  // most consecutive segments one lane group owns
 #define PSPMM_LONG_PER_RANGE 12  // a range of 8 * long_row entries meets at most 9 rows longer than long_row
-#define PSPMM_LONG_LIST 132  // rows longer than long_row that a range of 128 * long_row entries can meet, and a few
+// Unsplit rows with more entries are not walked by one lane group: it would hold up its warp, and a
+// hub row the whole launch.  One full staging window (SpMM) or four batches of 16 (SDDMM) stay.
+#define PSPMM_LONG_ROW 64
+#define PSPMM_LONG_RANGE_MAX 8192
+#define PSPMM_LONG_LIST 132  // long rows that such a range can meet (8192 / 65 inside it and two cut), and a few
 #define PSPMM_GAP_MAX 256  // longest run of uncovered rows the SpMM kernel zeroes by itself
 
 // Records the CUDA error text for pspmm_last_cuda_error() and returns PSPMM_E_CUDA.
@@ -120,7 +124,7 @@ struct SddmmArgs {
     int32_t rows_per_group;
     float keep_fraction;
     int32_t long_row;    // unsplit rows with more entries are dealt to the first long_ctas CTAs (INT32_MAX: none are)
-    int32_t long_range;  // entries per range of those CTAs, at most 128 * long_row
+    int32_t long_range;  // entries per range of those CTAs
     uint32_t long_ctas;
 };
 

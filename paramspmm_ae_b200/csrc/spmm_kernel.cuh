@@ -91,6 +91,57 @@ __device__ __forceinline__ void spmm_batch(const int *ent, int e, const char *co
         }
 }
 
+// Entries [e, eh) of the staged window: batches of U, the tail in halves of it.
+template <int U, int LPR, int VW, int CF, int V>
+__device__ __forceinline__ void spmm_entries(const int *ent, int e, int eh, const char *const (&bcol)[CF],
+                                             unsigned ldB_bytes, unsigned long long keep, float (&acc)[V][CF][VW])
+{
+    for (; e + U <= eh; e += U)
+        spmm_batch<U, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+    if constexpr (U >= 16) {
+        if (e + 8 <= eh) {
+            spmm_batch<8, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            e += 8;
+        }
+    }
+    if constexpr (U >= 8) {
+        if (e + 4 <= eh) {
+            spmm_batch<4, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            e += 4;
+        }
+    }
+    if constexpr (U >= 4) {
+        if (e + 2 <= eh) {
+            spmm_batch<2, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            e += 2;
+        }
+    }
+    if constexpr (U >= 2) {
+        if (e < eh)
+            spmm_batch<1, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+    }
+}
+
+// Copies entries [k, k + fill) into a group's window, column and value(s) side by side.
+template <int LPR, int V>
+__device__ __forceinline__ void spmm_stage(const SpmmArgs &a, int *ent, int k0, int fill, int gl, unsigned long long stream)
+{
+    for (int i = gl; i < fill; i += LPR) {
+        const int k = k0 + i;
+        if constexpr (V == 1) {
+            // (no value array: the pattern itself, every stored entry counts as 1)
+            *reinterpret_cast<int2 *>(ent + 2 * i) =
+                make_int2(ldg_stream_b32(a.colIdx + k, stream),
+                          a.val ? ldg_stream_b32(a.val + k, stream) : __float_as_int(1.f));
+        } else {
+            ent[(1 + V) * i] = ldg_stream_b32(a.colIdx + k, stream);
+#pragma unroll
+            for (int w = 0; w < V; ++w)
+                ent[(1 + V) * i + 1 + w] = ldg_stream_b32(a.val + (int64_t)k * V + w, stream);
+        }
+    }
+}
+
 // MLP = 16-byte gathers a lane keeps in flight per batch (2, 4, 8 or 16).  It trades registers
 // (and so resident warps per SM) against memory-level parallelism inside one warp; the
 // launch bound asks for the matching number of resident 256-thread CTAs.
@@ -182,52 +233,16 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
     bool head_pending = (first == 0);  // the rows ahead of the very first segment are still to be zeroed
     while (true) {
         const int fill = (end - cur < CAP) ? (end - cur) : CAP;
-        for (int i = gl; i < fill; i += LPR) {
-            const int k = cur + i;
-            if constexpr (V == 1) {
-                // (no value array: the pattern itself, every stored entry counts as 1)
-                *reinterpret_cast<int2 *>(ent + 2 * i) =
-                    make_int2(ldg_stream_b32(a.colIdx + k, stream),
-                              a.val ? ldg_stream_b32(a.val + k, stream) : __float_as_int(1.f));
-            } else {
-                ent[(1 + V) * i] = ldg_stream_b32(a.colIdx + k, stream);
-#pragma unroll
-                for (int w = 0; w < V; ++w)
-                    ent[(1 + V) * i + 1 + w] = ldg_stream_b32(a.val + (int64_t)k * V + w, stream);
-            }
-        }
+        spmm_stage<LPR, V>(a, ent, cur, fill, gl, stream);
         __syncwarp(gmask);
         const int lim = cur + fill;
         int resume = lim;
         while (row < nrow) {
             const int rb = sp[row], re = sp[row + 1];
             const bool skip = LONG && re - rb > a.long_row;  // left to spmm_long_rows_kernel
-            int e = (rb > cur ? rb : cur) - cur;
+            const int e = (rb > cur ? rb : cur) - cur;
             const int eh = skip ? e : (re < lim ? re : lim) - cur;
-            for (; e + U <= eh; e += U)
-                spmm_batch<U, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
-            if constexpr (U >= 16) {
-                if (e + 8 <= eh) {
-                    spmm_batch<8, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
-                    e += 8;
-                }
-            }
-            if constexpr (U >= 8) {
-                if (e + 4 <= eh) {
-                    spmm_batch<4, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
-                    e += 4;
-                }
-            }
-            if constexpr (U >= 4) {
-                if (e + 2 <= eh) {
-                    spmm_batch<2, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
-                    e += 2;
-                }
-            }
-            if constexpr (U >= 2) {
-                if (e < eh)
-                    spmm_batch<1, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
-            }
+            spmm_entries<U, LPR, VW, CF, V>(ent, e, eh, bcol, ldB_bytes, keep, acc);
             if (re > lim && !skip)
                 break;  // the row continues in the next window
 
@@ -313,34 +328,44 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
 
 // Rows of more than a.long_row entries of an unsplit (block-)CSR layout, which spmm_seg_kernel has
 // stored as zeros.  A row there is walked by one lane group, one gather batch after the other: a hub
-// row of 1,600 entries held a 197 K-entry graph at dim 16 for 310 us, 98 % of the product.  Here
-// CTA c owns the entries [c, c+1) * a.long_range whatever rows they belong to: two warps find the
-// first and last row of the range (32 pointers probed per step), all threads look for long rows
-// between them, and the eight warps share each one that is found, 32 entries per warp and step,
-// their sums meeting in shared memory and leaving as one vector RED per CTA and row.  Nothing is
-// allocated and no list is kept.  spmm_seg_kernel raises g_long_seen to this launch's ticket when it
-// passes over a row, so a matrix without long rows costs one look at that word (1.5 us behind the
-// products it was measured on; searching all ranges cost 6 us of 86).  Tickets only grow: a word that
-// a later launch has raised further makes this one search in vain, never miss a row.  Bound: gather
-// latency (8 x 16-byte loads in flight per lane, as above).
+// row of 1,600 entries held a 197 K-entry graph at dim 16 for 310 us, 98 % of the product, and rows of
+// a few hundred entries still leave the groups of a warp out of step (115 M entries at dim 64, rows
+// of 490: 3.1 ms with rows up to 512 entries left there).  Here a CTA takes a range of entries,
+// whatever rows they belong to: two warps find the first and last row of the range (32 pointers
+// probed per step), all threads look for long rows between them, and the entries of those rows, end
+// to end, are dealt to the lane groups in equal spans.  A group walks its span as spmm_seg_kernel walks
+// its segments and leaves one vector RED per row it meets.  Nothing is allocated and no list
+// is kept.  spmm_seg_kernel raises g_long_seen to this launch's ticket when it passes over a row, so a
+// matrix without long rows costs one look at that word.  Tickets only grow: a word that a later launch
+// has raised further makes this one search in vain, never miss a row.  Bound: gather latency (U loads
+// of 16 bytes in flight per lane, as above).
 template <int VW, int V, int LPR>
 __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmArgs a)
 {
-    constexpr int GROUPS = 32 / LPR;
-    constexpr int U = (LPR < 8 ? LPR : 8) / (V > 1 ? 2 : 1);
-    __shared__ float sums[8][V * LPR * VW];
-    __shared__ int row_list[PSPMM_LONG_PER_RANGE];
+    constexpr int G = 256 / LPR;
+    constexpr int U = V > 1 ? 4 : 8;
+    constexpr int CAP = SpmmTile<LPR, V>::CAP;
+    __shared__ __align__(16) int windows[G * CAP * (1 + V)];
+    __shared__ int row_list[PSPMM_LONG_LIST], row_lo[PSPMM_LONG_LIST], row_off[PSPMM_LONG_LIST + 1];
     __shared__ int row_ends[2];
     __shared__ int n_long;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane / LPR, gl = lane % LPR;
+    const int g = threadIdx.x / LPR, gl = lane % LPR;
+    const unsigned gmask = (LPR == 32) ? PSPMM_FULL_MASK : (((1u << LPR) - 1u) << ((lane / LPR) * LPR));
+    int *ent = windows + g * CAP * (1 + V);
     const int v = blockIdx.y * LPR + gl;
     const bool act = v < a.nvec;
     const int voff = act ? v * VW : 0;
-    const char *bcol = reinterpret_cast<const char *>(a.B + voff);
+    const char *bcol[1] = {reinterpret_cast<const char *>(a.B + voff)};
     const unsigned ldB_bytes = (unsigned)(a.ldB * 4);
     const unsigned long long keep = l2_policy_keep(a.keep_fraction);
     const unsigned long long stream = l2_policy_stream();
+    float acc[V][1][VW];
+#pragma unroll
+    for (int w = 0; w < V; ++w)
+#pragma unroll
+        for (int j = 0; j < VW; ++j)
+            acc[w][0][j] = 0.f;
     const int64_t begin = __ldg(a.segPtr), end = __ldg(a.segPtr + a.n_seg);
     // (an early look lets the searches run while the kernel before this one drains)
     bool waited = false;
@@ -360,86 +385,65 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmArgs a
                 row_ends[warp] = r;
         }
         __syncthreads();
-        for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += 256)
-            if (__ldg(a.segPtr + r + 1) - __ldg(a.segPtr + r) > a.long_row)
-                row_list[atomicAdd(&n_long, 1)] = (int)r;
+        for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += 256) {
+            const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
+            if (re - rb > a.long_row) {
+                const int i = atomicAdd(&n_long, 1);
+                row_list[i] = (int)r;
+                row_lo[i] = (int)(rb > s ? rb : s);
+                row_off[i + 1] = (int)((re < e1 ? re : e1) - (rb > s ? rb : s));
+            }
+        }
         __syncthreads();
-        const int count = n_long;
-        if (count > 0 && !waited) {
+        const int n = n_long;
+        if (warp == 0) {  // lengths -> offsets in the concatenation
+            int base = 0;
+            for (int i0 = 0; i0 < n; i0 += 32) {
+                int x = i0 + lane < n ? row_off[i0 + lane + 1] : 0;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(PSPMM_FULL_MASK, x, d);
+                    if (lane >= d)
+                        x += o;
+                }
+                if (i0 + lane < n)
+                    row_off[i0 + lane + 1] = base + x;
+                base += __shfl_sync(PSPMM_FULL_MASK, x, 31);
+            }
+            if (lane == 0)
+                row_off[0] = 0;
+        }
+        __syncthreads();
+        if (n > 0 && !waited) {
             pdl_wait();
             waited = true;
         }
-        for (int i = 0; i < count; ++i) {
-            const int r = row_list[i];
-            const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
-            const int64_t lo = rb > s ? rb : s, hi = re < e1 ? re : e1;
-            float acc[V][VW];
+        const int total = n > 0 ? row_off[n] : 0;
+        const int span = ((total + G - 1) / G + U - 1) / U * U;
+        int p = g * span;  // position in the concatenation
+        const int stop = p + span < total ? p + span : total;
+        int i = 0;         // the row it lies in
+        while (i + 1 < n && p >= row_off[i + 1])
+            ++i;
+        while (p < stop) {
+            const int row_stop = row_off[i + 1] < stop ? row_off[i + 1] : stop;
+            while (p < row_stop) {
+                const int fill = row_stop - p < CAP ? row_stop - p : CAP;
+                spmm_stage<LPR, V>(a, ent, row_lo[i] + (p - row_off[i]), fill, gl, stream);
+                __syncwarp(gmask);
+                spmm_entries<U, LPR, VW, 1, V>(ent, 0, fill, bcol, ldB_bytes, keep, acc);
+                __syncwarp(gmask);
+                p += fill;
+            }
 #pragma unroll
-            for (int w = 0; w < V; ++w)
+            for (int w = 0; w < V; ++w) {
+                if (act)
+                    red_add_vec<VW>(a.C + ((int64_t)row_list[i] * V + w) * a.ldC + voff, acc[w][0]);
 #pragma unroll
                 for (int j = 0; j < VW; ++j)
-                    acc[w][j] = 0.f;
-            for (int64_t k0 = lo + warp * 32; k0 < hi; k0 += 256) {
-                const int64_t k = k0 + lane;
-                const bool in = k < hi;
-                const int cc = in ? ldg_stream_b32(a.colIdx + k, stream) : 0;
-                float vv[V];
-#pragma unroll
-                for (int w = 0; w < V; ++w)
-                    vv[w] = !in ? 0.f : (V == 1 && !a.val) ? 1.f : __int_as_float(ldg_stream_b32(a.val + k * V + w, stream));
-                const int left = (int)(hi - k0);
-#pragma unroll
-                for (int j0 = 0; j0 < LPR; j0 += U) {
-                    FVec<VW> x[U];
-#pragma unroll
-                    for (int u = 0; u < U; ++u) {
-                        const int c = __shfl_sync(PSPMM_FULL_MASK, cc, j0 + u, LPR);
-                        x[u] = ldg_vec_if<VW>(row_slice(bcol, c, ldB_bytes), g * LPR + j0 + u < left);
-                    }
-#pragma unroll
-                    for (int u = 0; u < U; ++u)
-#pragma unroll
-                        for (int w = 0; w < V; ++w) {
-                            const float f = __shfl_sync(PSPMM_FULL_MASK, vv[w], j0 + u, LPR);
-                            if (V > 1 && f == 0.f)
-                                continue;  // an explicit zero of a block is no entry
-#pragma unroll
-                            for (int j = 0; j < VW; ++j)
-                                acc[w][j] = fmaf(f, x[u].v[j], acc[w][j]);
-                        }
-                }
+                    acc[w][0][j] = 0.f;
             }
-            // lane groups of a warp, then the warps
-#pragma unroll
-            for (int d = LPR; d < 32; d <<= 1)
-#pragma unroll
-                for (int w = 0; w < V; ++w)
-#pragma unroll
-                    for (int j = 0; j < VW; ++j)
-                        acc[w][j] += __shfl_xor_sync(PSPMM_FULL_MASK, acc[w][j], d);
-            if (g == 0) {
-#pragma unroll
-                for (int w = 0; w < V; ++w)
-#pragma unroll
-                    for (int j = 0; j < VW; ++j)
-                        sums[warp][(w * LPR + gl) * VW + j] = acc[w][j];
-            }
-            __syncthreads();
-            for (int t = threadIdx.x; t < V * LPR; t += 256) {
-                const int w = t / LPR, vi = blockIdx.y * LPR + t % LPR;
-                if (vi < a.nvec) {
-                    float tot[VW];
-#pragma unroll
-                    for (int j = 0; j < VW; ++j) {
-                        tot[j] = 0.f;
-#pragma unroll
-                        for (int q = 0; q < 8; ++q)
-                            tot[j] += sums[q][t * VW + j];
-                    }
-                    red_add_vec<VW>(a.C + ((int64_t)r * V + w) * a.ldC + vi * VW, tot);
-                }
-            }
-            __syncthreads();
+            ++i;
         }
         __syncthreads();
     }
@@ -453,7 +457,7 @@ static inline void spmm_launch_long_rows(const SpmmArgs &a, cudaStream_t st)
     const int lpr = a.nvec > 16 ? 32 : (a.nvec > 8 || V > 1) ? 16 : (a.nvec > 4 ? 8 : 4);
     const int64_t ranges = (a.n_entries + a.long_range - 1) / a.long_range;
     const unsigned tiles = (unsigned)((a.nvec + lpr - 1) / lpr);
-    const int64_t most = a.sms * 3 / tiles + 1;  // one resident wave
+    const int64_t most = (unsigned)a.sms * 3 > tiles ? a.sms * 3 / tiles : 1;  // one resident wave, no CTA more
     const dim3 grid((unsigned)(ranges < most ? ranges : most), tiles);
     if (lpr == 32)
         launch_dependent(spmm_long_rows_kernel<VW, V, 32>, grid, 256, 0, st, a);
