@@ -283,6 +283,21 @@ PSPMM_API int pspmm_pull_rows_bulk(const pspmm_row_sources *sources, const int32
 PSPMM_API int pspmm_pull_rows_status(int32_t *status);
 
 /*
+ * C[M, N] = op(A) op(B) for the layers' dense products (what the reference leaves to cuBLAS through
+ * torch::mm, SpCONV/SpCONV.h:43-72): op(A) is M x K, op(B) is K x N, trans* != 0 means the operand is
+ * stored transposed, row-major in every case.  fp32 in and out, computed on the tensor cores from exact
+ * three-way bf16 splits with fp32 accumulation: at least as accurate as a chain of fp32 multiply-adds.
+ * Any size and alignment.  Products with few output tiles and a long K need scratch of
+ * pspmm_dense_scratch_bytes(M, N, K) bytes (0 for the others).  Every wait inside the kernel is
+ * bounded; pspmm_dense_status returns 1 once one has run out on this GPU (it synchronises).
+ */
+PSPMM_API int pspmm_dense_scratch_bytes(int64_t M, int64_t N, int64_t K, size_t *bytes);
+PSPMM_API int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A,
+                             int64_t ldA, const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch,
+                             size_t scratch_bytes, void *stream);
+PSPMM_API int pspmm_dense_status(int32_t *status);
+
+/*
  * Host-side CSR -> V x 1 block CSR, laid out exactly as scipy's tobsr((V,1)) (which the
  * reference calls at graph_input.py:245-266): blocks of a block-row appear in order of first
  * encounter while walking its V rows top to bottom.  pspmm_bcsr_count fills rowPtr_b

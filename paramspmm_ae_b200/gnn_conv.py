@@ -17,6 +17,8 @@ import math
 
 import torch
 
+from . import ops
+
 n_heads = 1
 
 
@@ -56,8 +58,8 @@ class GCNFunction(torch.autograd.Function):
             # dW = (A H)^T G with A H kept from the forward; dH = A (G W^T) (A is symmetric),
             # skipped when the layer input needs no gradient (the first layer).
             AH, weight = ctx.saved_tensors
-            d_weight = torch.mm(AH.t(), d_output)
-            d_input = _aggregate(P, torch.mm(d_output, weight.t())) if ctx.needs_input_grad[0] else None
+            d_weight = ops.dense_mm(AH, d_output, transA=True)
+            d_input = _aggregate(P, ops.dense_mm(d_output, weight, transB=True)) if ctx.needs_input_grad[0] else None
             return d_input, d_weight, None
         H, weight = ctx.saved_tensors
         if ctx.needs_input_grad[0]:
@@ -78,8 +80,8 @@ class GINFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_output):
         X_agg, weight = ctx.saved_tensors
-        d_weight = torch.mm(X_agg.t(), d_output)
-        d_input = ctx.ParamSpMM.GIN_spmm(torch.mm(d_output, weight.t()).contiguous())
+        d_weight = ops.dense_mm(X_agg, d_output, transA=True)
+        d_input = ctx.ParamSpMM.GIN_spmm(ops.dense_mm(d_output, weight, transB=True).contiguous())
         return d_input, d_weight, None
 
 
@@ -115,7 +117,7 @@ def _is_operator_colidx(P, colIdx):
 class AGNNFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, X, weights, attention_w, ParamSpMM, colIdx):
-        X_prime = torch.mm(X, weights)
+        X_prime = ops.dense_mm(X, weights)
         edge = ParamSpMM.AGNN_sddmm(X_prime)
         # [n_edges] for CSR, [n_blocks, V] for block layouts; one attention head
         edge_attentions = (edge * attention_w.reshape(())).contiguous()
@@ -130,8 +132,8 @@ class AGNNFunction(torch.autograd.Function):
         X, weights, edge_attentions = ctx.saved_tensors
         d_output = d_output.contiguous()
         d_prime = P.AGNN_spmm(edge_attentions, d_output)
-        d_input = torch.mm(d_prime, weights.t())
-        d_weights = torch.mm(X.t(), d_prime)
+        d_input = ops.dense_mm(d_prime, weights, transB=True)
+        d_weights = ops.dense_mm(X, d_prime, transA=True)
         d_att = P.AGNN_sddmm(d_output)
         if d_att.dim() != 1:
             d_att = d_att.reshape(-1)[P.mask]  # back to CSR entry order
@@ -153,8 +155,7 @@ class AGNNFusedFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, X, weights, attention_w, P, colIdx):
-        from . import ops
-        Xp = torch.mm(X, weights)
+        Xp = ops.dense_mm(X, weights)
         split = P.target_row is not None
         beta = float(attention_w.detach().reshape(()))
         out = ops.agnn_fused(Xp, Xp, P.rowPtr, P.colIdx, beta, softmax=False, target_row=P.target_row,
@@ -167,7 +168,6 @@ class AGNNFusedFunction(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, d_output):
-        from . import ops
         X, weights, Xp = ctx.saved_tensors
         P, beta = ctx.P, ctx.beta
         G = d_output.contiguous()
@@ -182,8 +182,8 @@ class AGNNFusedFunction(torch.autograd.Function):
             return o
 
         D = apply(Xp, Xp, G, beta)
-        d_input = torch.mm(D, weights.t())
-        d_weights = torch.mm(X.t(), D)
+        d_input = ops.dense_mm(D, weights, transB=True)
+        d_weights = ops.dense_mm(X, D, transA=True)
         d_att = None
         if ctx.needs_input_grad[2]:
             # The reference weights every edge's score gradient by the float value of the column-index
@@ -247,8 +247,7 @@ class AGNNConv(_Conv):
         if FUSE_AGNN_INFERENCE and not torch.is_grad_enabled() and _can_fuse(P, self.weights.size(1)):
             # No gradient will be asked for: scores, scaling and aggregation in one kernel, without
             # the per-edge array the backward would need.
-            from . import ops
-            Xp = torch.mm(X, self.weights)
+            Xp = ops.dense_mm(X, self.weights)
             split = P.target_row is not None
             return ops.agnn_fused(Xp, Xp, P.rowPtr, P.colIdx, self._beta(), softmax=False,
                                   target_row=P.target_row, n_out_rows=P.mtx_nodes if split else None)
