@@ -14,10 +14,19 @@ import os
 
 import torch
 
-from . import _lib
-from .ops import PROFILE_ITERS, PROFILE_WARMUP, _check_cuda, _gflops, _ptr, _stream
+from . import _lib, ops
+from .ops import PROFILE_ITERS, PROFILE_WARMUP, _check_cuda, _gflops
 
 _handle = None
+
+
+# (the comparator library is bound without argument types: pointers are passed as such)
+def _ptr(t):
+    return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+
+
+def _stream():
+    return ctypes.c_void_p(ops._stream())
 
 
 def _bl():

@@ -25,6 +25,10 @@ PROFILE_WARMUP = 20
 
 # ----------------------------------------------------------------------------- argument checks
 def _check_cuda(t, name, dtype=None, ndim=None):
+    # one pass over what a good operand answers; only a bad one is taken apart for its message
+    if (isinstance(t, torch.Tensor) and t.is_cuda and t.is_contiguous() and (dtype is None or t.dtype is dtype)
+            and (ndim is None or t.dim() == ndim)):
+        return
     if not isinstance(t, torch.Tensor):
         raise RuntimeError("%s must be a tensor" % name)
     if not t.is_cuda:
@@ -55,11 +59,12 @@ def _check_legacy(CF, blkWarpNum, max_cf=8):
 
 
 def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr() if t is not None else 0)
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # torch.cuda.current_stream() builds a Stream object (3 us of a 20 us call); this is the handle alone
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 # Kernel parameters chosen per call.  `tuner` (set by paramspmm_ae_b200.decider) maps
@@ -67,11 +72,33 @@ def _stream():
 tuner = None
 
 
+_legacy_cfgs = {}
+
+
 def _cfg(op, CF, W, dim, n_entries, n_seg, V, split):
-    kw = {}
-    if tuner is not None:
-        kw = tuner(op, dim, (n_entries / n_seg) if n_seg else 0.0, V, split) or {}
-    return make_cfg(CF=CF, blkWarpNum=W, **kw)
+    """Pointer to the configuration of a call through the legacy signatures."""
+    if tuner is None:
+        ref = _legacy_cfgs.get((CF, W))
+        if ref is None:
+            ref = _legacy_cfgs[(CF, W)] = ctypes.byref(make_cfg(CF=CF, blkWarpNum=W))
+        return ref
+    kw = tuner(op, dim, (n_entries / n_seg) if n_seg else 0.0, V, split) or {}
+    return ctypes.byref(make_cfg(CF=CF, blkWarpNum=W, **kw))
+
+
+_scratch_sizes = {}  # (entry point, sizes) -> bytes
+
+
+def _scratch(fn, sizes, device):
+    """(tensor, bytes) of the scratch memory an entry point asks for, (None, 0) where it needs none."""
+    need = _scratch_sizes.get((fn, sizes))
+    if need is None:
+        c = ctypes.c_size_t(0)
+        check(getattr(lib(), fn)(*sizes, ctypes.byref(c)))
+        if len(_scratch_sizes) > 4096:
+            _scratch_sizes.clear()
+        need = _scratch_sizes[(fn, sizes)] = c.value
+    return (torch.empty(need, dtype=torch.uint8, device=device), need) if need else (None, 0)
 
 
 # ----------------------------------------------------------------------------- host builders
@@ -322,23 +349,23 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
             raise RuntimeError("n_out_rows is required for split layouts")
         n_out_rows = n_seg
     _check_output(out, rowPtr, split, n_out_rows, V, dim)
-    nent = colIdx.shape[0]
-    if cfg is None:
-        cfg = _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
-    seg_ptr = _ptr(rowPtr)
-    null = ctypes.c_void_p(0)
+    ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref)
+
+
+def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref):
+    seg = rowPtr.data_ptr()
+    n, dim = X.shape
+    # row pointers of a split layout go into the split arguments
+    plain, split, target, n_seg = (seg, None, None, 0) if target_row is None else (
+        None, seg, target_row.data_ptr(), rowPtr.shape[0] - 1)
+    tail = (n_out_rows, n, colIdx.shape[0], dim, X.stride(0), out.stride(0), ref, split, target, n_seg, _stream())
     if V == 1:
-        check(lib().pspmm_spmm_csr(null if split else seg_ptr, _ptr(colIdx), _ptr(val), _ptr(X),
-                                   _ptr(out), n_out_rows, X.shape[0], nent, dim, X.stride(0),
-                                   out.stride(0), ctypes.byref(cfg), seg_ptr if split else null,
-                                   _ptr(target_row) if split else null, n_seg if split else 0,
-                                   _stream()))
+        rc = lib().pspmm_spmm_csr(plain, colIdx.data_ptr(), _ptr(val), X.data_ptr(), out.data_ptr(), *tail)
     else:
-        check(lib().pspmm_spmm_bcsr(null if split else seg_ptr, _ptr(colIdx), _ptr(val), V, _ptr(X),
-                                    _ptr(out), n_out_rows, X.shape[0], nent, dim, X.stride(0),
-                                    out.stride(0), ctypes.byref(cfg), seg_ptr if split else null,
-                                    _ptr(target_row) if split else null, n_seg if split else 0,
-                                    _stream()))
+        rc = lib().pspmm_spmm_bcsr(plain, colIdx.data_ptr(), _ptr(val), V, X.data_ptr(), out.data_ptr(), *tail)
+    if rc:
+        check(rc)
     return out
 
 
@@ -353,15 +380,16 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W):
     # features to an even row count): those extra output rows stay zero.
     padded = (n + V - 1) // V * V
     n_out = padded // V
-    out = torch.empty((padded, dim), dtype=torch.float32, device=X.device)
+    n_seg = rowPtr.shape[0] - 1
+    out = torch.empty_like(X) if padded == n else torch.empty((padded, dim), dtype=torch.float32, device=X.device)
     if target_row is None:
-        n_seg = rowPtr.shape[0] - 1
         if n_seg > n_out:
             raise RuntimeError("rowPtr describes %d (block-)rows, the input only allows %d" % (n_seg, n_out))
         if n_seg < n_out:
             out[n_seg * V:].zero_()
             n_out = n_seg
-    return spmm_into(out, X, rowPtr, colIdx, val, target_row, V, n_out, CF, W)
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out,
+                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None))
 
 
 def csr_spmm(X, rowPtr, colIdx, val, CF, blkWarpNum):
@@ -410,13 +438,12 @@ def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=No
         out = torch.empty((n_out * V, dim), dtype=torch.float32, device=X.device)
     _check_output(out, rowPtr, split, n_out, V, dim)
     nent = colIdx.shape[0]
-    if cfg is None:
-        cfg = _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
+    ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
     ms = ctypes.c_float(0.0)
-    null = ctypes.c_void_p(0)
+    null = None
     check(lib().pspmm_profile_spmm(null if split else _ptr(rowPtr), _ptr(colIdx), _ptr(val), V,
                                    _ptr(X), _ptr(out), n_out, n, nent, dim, X.stride(0),
-                                   out.stride(0), ctypes.byref(cfg),
+                                   out.stride(0), ref,
                                    _ptr(rowPtr) if split else null,
                                    _ptr(target_row) if split else null, n_seg if split else 0,
                                    warmup, iters, ctypes.byref(ms), _stream()))
@@ -480,13 +507,13 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
     nent = colIdx.shape[0]
     out = torch.empty_like(val)
     cfg = _cfg("sddmm", CF, W, dim, nent, n_seg, V, split)
-    null = ctypes.c_void_p(0)
+    null = None
     # (block-)rows of the pattern; A may stop inside the last block-row when the node count is
     # not a multiple of V, and the kernel then reads nothing past A's last row
     n_rows = n_seg if not split else (A.shape[0] + V - 1) // V
     if A.shape[0] <= (n_rows - 1) * V:
         raise RuntimeError("A has %d rows, the pattern needs more than %d" % (A.shape[0], (n_rows - 1) * V))
-    args_tail = (ctypes.byref(cfg), _ptr(rowPtr) if split else null,
+    args_tail = (cfg, _ptr(rowPtr) if split else null,
                  _ptr(target_row) if split else null, n_seg if split else 0)
     if time_only:
         ms = ctypes.c_float(0.0)
@@ -599,15 +626,11 @@ def agnn_fused(A, B, rowPtr, colIdx, beta=1.0, softmax=True, target_row=None, n_
         raise RuntimeError("A has fewer rows than the pattern")
     if out is None:
         out = torch.empty(n_out_rows, dim, dtype=torch.float32, device=A.device)
-    null = ctypes.c_void_p(0)
-    scratch, need = None, ctypes.c_size_t(0)
+    null = None
     if split:
-        check(lib().pspmm_agnn_scratch_bytes(n_seg, dim, ctypes.byref(need)))
+        scratch, sbytes = _scratch("pspmm_agnn_scratch_bytes", (n_seg, dim), A.device)
     else:
-        check(lib().pspmm_agnn_long_scratch_bytes(colIdx.shape[0], dim, ctypes.byref(need)))
-    sbytes = need.value
-    if sbytes:
-        scratch = torch.empty((sbytes + 15) // 16 * 4, dtype=torch.float32, device=A.device)
+        scratch, sbytes = _scratch("pspmm_agnn_long_scratch_bytes", (colIdx.shape[0], dim), A.device)
     seg_ptr = _ptr(rowPtr)
     tail = (float(beta), 1 if softmax else 0, int(vec_width), int(lanes_per_row), int(batch),
             seg_ptr if split else null, _ptr(target_row) if split else null, n_seg if split else 0,
@@ -703,13 +726,11 @@ def dense_mm(A, B, transA=False, transB=False, out=None):
         raise RuntimeError("mat1 and mat2 shapes cannot be multiplied (%dx%d and %dx%d)" % (M, K, Kb, N))
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=A.device)
-    handle = lib()
-    need = ctypes.c_size_t(0)
-    check(handle.pspmm_dense_scratch_bytes(M, N, K, ctypes.byref(need)))
-    scratch = torch.empty(need.value, dtype=torch.uint8, device=A.device) if need.value else None
-    check(handle.pspmm_dense_mm(1 if transA else 0, 1 if transB else 0, M, N, K, A.data_ptr(), A.stride(0), B.data_ptr(),
-                                B.stride(0), out.data_ptr(), out.stride(0), scratch.data_ptr() if need.value else None,
-                                need.value, torch.cuda.current_stream().cuda_stream))
+    scratch, need = _scratch("pspmm_dense_scratch_bytes", (M, N, K), A.device)
+    rc = lib().pspmm_dense_mm(1 if transA else 0, 1 if transB else 0, M, N, K, A.data_ptr(), A.stride(0), B.data_ptr(),
+                              B.stride(0), out.data_ptr(), out.stride(0), _ptr(scratch), need, _stream())
+    if rc:
+        check(rc)
     return out
 
 
