@@ -21,13 +21,13 @@
 // of the ring each: a group fetches the fp32 tiles of its next stage, splits them and writes A's bf16
 // parts to TMEM (a lane per row, so the MMA reads A from there) and B's to shared memory (K-major core
 // matrices without swizzle: 8 consecutive rows of 16 bytes, so the 16-byte stores of neighbouring
-// lanes never conflict).  Operands that are contiguous along M or N are read down their columns;
-// k-contiguous A passes through a raw tile in shared memory (cp.async, rows padded to 144 bytes), from
-// which each lane takes its row.  Two warps issue the MMAs; eight add finished chains out of TMEM (two
-// buffers of 128 columns) into registers and store the tile.  B of the tall products, the weights, is
-// the same for every row tile: split_weights_kernel splits it once into caller scratch, in the layout
-// of the stages, and one warp brings its tiles in with bulk copies.  Products with a long K are cut
-// into splits whose partial tiles are summed by reduce_splits_kernel.
+// lanes never conflict).  A and, where both are contiguous along M and N, B pass through raw tiles in
+// shared memory (cp.async, padded rows), from which each lane takes its row of A and its chunks of B.
+// Two warps issue the MMAs; eight add finished chains out of TMEM (two buffers of 128 columns) into
+// registers and store the tile.  B of the tall products, the weights, is the same for every row tile:
+// split_weights_kernel splits it once into caller scratch, in the layout of the stages, and one warp
+// brings its tiles in with bulk copies.  Products with a long K are cut into splits whose partial
+// tiles are summed by reduce_splits_kernel.
 //
 // What the shape rests on (2.4 M x 256 x 256; cuBLAS 5.6 ms).  All loading warps on one stage at a time
 // waited out a memory latency per stage however far ahead they loaded (a warp's scoreboard does not
@@ -50,11 +50,11 @@ constexpr int STAGES = 3, ACC_BUFS = 2;
 constexpr int PLANE = BN * BK * 2;               // one bf16 tile of B
 constexpr int STAGE_BYTES = 3 * PLANE;
 constexpr int RAW_PITCH = BK + 4;                // floats per row of a raw tile of k-contiguous A
-constexpr int RAW_PITCH_B = BN + 4;              // floats per k of a raw tile of n-contiguous B
+constexpr int RAW_PITCH_T = 128 + 4;             // floats per k of a raw tile that is contiguous along M or N
 constexpr int RAW_BYTES = BM * RAW_PITCH * 4;
+constexpr int RAW_BYTES_T = BK * RAW_PITCH_T * 4;
 constexpr int OUT_PITCH = 36;                    // floats per row of a drainer's 32 x 32 output patch
 constexpr int OUT_BYTES = 32 * OUT_PITCH * 4;
-static_assert(BK * RAW_PITCH_B * 4 <= RAW_BYTES, "either raw tile fits the slot");
 constexpr int TMEM_A = ACC_BUFS * BN;            // first column of A's parts: 16 columns per part and stage
 constexpr int TMEM_COLS = 512;
 constexpr int GROUP_WARPS = 4, LOADERS = STAGES * GROUP_WARPS, DRAINERS = 8;
@@ -62,7 +62,15 @@ constexpr int MMA_WARP = LOADERS + DRAINERS, BULK_WARP = MMA_WARP + 1;
 constexpr int THREADS = (LOADERS + DRAINERS + 4) * 32;
 // Registers per thread after the split: 768 x 80 = 61,440 at launch; 384 x 80 + 256 x 104 + 128 x 32 = 61,440.
 constexpr int DRAINER_REGS = 104, OTHER_REGS = 32;
-constexpr int SMEM_BYTES = STAGES * (STAGE_BYTES + RAW_BYTES) + DRAINERS * OUT_BYTES + 1024;
+
+// Raw tiles of one slot: k-contiguous A, or A and B that are both contiguous the other way.
+template <bool KC_A, bool KC_B, bool PRE>
+struct Raw {
+    static constexpr bool BOTH = !PRE && !KC_A && !KC_B;
+    static constexpr int BYTES = KC_A ? RAW_BYTES : (BOTH ? 2 * RAW_BYTES_T : 0);
+    static constexpr int SMEM = STAGES * (STAGE_BYTES + BYTES) + DRAINERS * OUT_BYTES + 1024;
+};
+
 
 __device__ unsigned g_dense_status;
 
@@ -77,6 +85,13 @@ struct DenseArgs {
     const unsigned char *Bs;  // B split beforehand (split_weights_kernel)
     unsigned *odd;            // with Bs: one word per block of that kernel, set when a value of B has no split
     int32_t odd_words;
+};
+
+struct ReduceArgs {
+    const float *part;
+    float *C;
+    int64_t ldC;
+    int32_t splits, M, N;
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -382,7 +397,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
         settle();
         const int row = tid;  // of the tile, as the TMEM lanes have it
         const uint32_t parts = tmem + ((uint32_t)((warp & 3) * 32) << 16) + TMEM_A + q * 48;
-        float *raw = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES + q * RAW_BYTES);
+        float *raw = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES + q * Raw<KC_A, KC_B, PRE>::BYTES);
         float x[BK];
         auto fetch_raw = [&]() {  // k-contiguous A
             const int k = k0 + j * BK, left = k1 - k;
@@ -405,27 +420,30 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
-        // B contiguous along N beside an A that needs no raw tile: [k][n]
-        constexpr bool RAW_B = !PRE && !KC_A && !KC_B;
-        auto fetch_raw_b = [&]() {
-            const int k = k0 + j * BK, n_end = n0 + a.bn < a.N ? n0 + a.bn : a.N;
-            if (a.vecB) {
+        // Tiles that are contiguous along M or N: [k][128]
+        constexpr bool BOTH = Raw<KC_A, KC_B, PRE>::BOTH;
+        float *raw_b = raw + BK * RAW_PITCH_T;
+        auto fetch_raw_t = [&](float *dst, const float *p, int64_t ld, int c0, int c_end, bool aligned, int k, int k_end) {
+            if (aligned) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int kr = (tid >> 5) + i * 4, c = (tid & 31) * 4;
-                    int n = k + kr < k1 ? n_end - (n0 + c) : 0;
+                    int n = k + kr < k_end ? c_end - (c0 + c) : 0;
                     n = n < 0 ? 0 : (n > 4 ? 4 : n);
-                    copy_async<16>(smem_addr(raw + kr * RAW_PITCH_B + c), a.B + (n ? (int64_t)(k + kr) * a.ldB + n0 + c : 0),
-                                   n * 4);
+                    copy_async<16>(smem_addr(dst + kr * RAW_PITCH_T + c), p + (n ? (int64_t)(k + kr) * ld + c0 + c : 0), n * 4);
                 }
             } else {
                 for (int kr = 0; kr < BK; ++kr) {
-                    const int n = k + kr < k1 && n0 + tid < n_end ? 1 : 0;
-                    copy_async<4>(smem_addr(raw + kr * RAW_PITCH_B + tid), a.B + (n ? (int64_t)(k + kr) * a.ldB + n0 + tid : 0),
+                    const int n = k + kr < k_end && c0 + tid < c_end ? 1 : 0;
+                    copy_async<4>(smem_addr(dst + kr * RAW_PITCH_T + tid), p + (n ? (int64_t)(k + kr) * ld + c0 + tid : 0),
                                   n * 4);
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        auto fetch_a_t = [&]() { fetch_raw_t(raw, a.A, a.ldA, m0, a.M, a.vecA, k0 + j * BK, k1); };
+        auto fetch_b_t = [&]() {
+            fetch_raw_t(raw_b, a.B, a.ldB, n0, n0 + a.bn < a.N ? n0 + a.bn : a.N, a.vecB, k0 + j * BK, k1);
         };
         auto fetch_columns = [&]() {  // A contiguous along M
             const int k = k0 + j * BK;
@@ -445,12 +463,14 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
             }
         };
         if (item < items) {
-            if constexpr (KC_A)
+            if constexpr (KC_A) {
                 fetch_raw();
-            else
+            } else if constexpr (BOTH) {
+                fetch_a_t();
+                fetch_b_t();
+            } else {
                 fetch_columns();
-            if constexpr (RAW_B)
-                fetch_raw_b();
+            }
         }
         bool ok = true;
         while (item < items) {
@@ -469,24 +489,32 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                 settle();
                 if (item < items)
                     fetch_raw();
-            } else if constexpr (RAW_B) {
+            } else if constexpr (BOTH) {
+                // Each next fetch leaves as soon as its tile has been read, so that it is in flight while
+                // this stage is split.
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
                 if (!group_all(1 + q, ok))
                     break;
+#pragma unroll
+                for (int i = 0; i < BK; ++i)
+                    x[i] = raw[i * RAW_PITCH_T + row];
+                group_all(1 + q, true);
                 settle();
+                if (item < items)
+                    fetch_a_t();
             } else {
                 settle();
             }
             ok = bar_wait(empty + 8 * q, phase ^ 1, &abort_flag);
             if (!ok) {
-                if constexpr (KC_A || RAW_B)
+                if constexpr (KC_A || BOTH)
                     continue;  // (the group leaves together)
                 else
                     break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            bool plain = split_row(x, parts);
-            if constexpr (RAW_B) {
+            bool plain = true;
+            if constexpr (BOTH) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     int r, kc;
@@ -495,11 +523,14 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                         float y[8];
 #pragma unroll
                         for (int t = 0; t < 8; ++t)
-                            y[t] = raw[(kc * 8 + t) * RAW_PITCH_B + r];
+                            y[t] = raw_b[(kc * 8 + t) * RAW_PITCH_T + r];
                         plain &= split_store(y, st + kc * (a.bn * 16) + r * 16, PLANE);
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                group_all(1 + q, true);
+                if (item < items)
+                    fetch_b_t();
             } else if constexpr (!PRE) {
                 const int n_end = n0_now + a.bn < a.N ? n0_now + a.bn : a.N;
                 const bool whole = k_now + BK <= k1_now && n0_now + BN <= n_end && (!KC_B || a.vecB);
@@ -517,6 +548,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
+            plain &= split_row(x, parts);
             if (!plain)
                 odd_flag = 1;
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -525,17 +557,12 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
             if (lane == 0)
                 bar_arrive(full + 8 * q);
             phase ^= 1;
-            if constexpr (RAW_B)
-                group_all(1 + q, true);  // the raw tile has been read
-            if constexpr (!KC_A) {
-                if (item < items) {
+            if constexpr (!KC_A && !BOTH) {
+                if (item < items)
                     fetch_columns();
-                    if constexpr (RAW_B)
-                        fetch_raw_b();
-                }
             }
         }
-        if constexpr (KC_A || RAW_B)
+        if constexpr (KC_A || BOTH)
             asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else if (warp >= MMA_WARP) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(OTHER_REGS));
@@ -629,7 +656,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
         const int quad = warp & 3, half = d >> 2;
         const int row = quad * 32 + lane;
         const int cols = a.bn / 2;  // a multiple of 8
-        float *patch = reinterpret_cast<float *>(smem + STAGES * (STAGE_BYTES + RAW_BYTES) + d * OUT_BYTES);
+        float *patch = reinterpret_cast<float *>(smem + STAGES * (STAGE_BYTES + Raw<KC_A, KC_B, PRE>::BYTES) + d * OUT_BYTES);
         int buf = 0, buf_phase = 0;
         bool ok = true;
         for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
@@ -742,22 +769,34 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-// C = sum of the partial tiles, one thread per element.
-__global__ void __launch_bounds__(256) reduce_splits_kernel(const float *part, int splits, int64_t M, int64_t N, float *C,
-                                                            int64_t ldC)
+// C = sum of the partial tiles: a block takes 32 neighbouring elements, its eight warps the splits in
+// turn (one thread per element walking 148 splits took 9 us of a 31 us product).
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const ReduceArgs a)
 {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= M * N)
-        return;
+    __shared__ float sums[8][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t total = (int64_t)a.M * a.N;
+    const int64_t i = (int64_t)blockIdx.x * 32 + lane;
+    pdl_wait();
     float s[4] = {};
-    int t = 0;
-    for (; t + 4 <= splits; t += 4)
+    if (i < total) {
+        int t = warp;
+        for (; t + 24 < a.splits; t += 32)
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            s[u] += part[(t + u) * M * N + i];
-    for (; t < splits; ++t)
-        s[0] += part[t * M * N + i];
-    C[i / N * ldC + i % N] = (s[0] + s[1]) + (s[2] + s[3]);
+            for (int u = 0; u < 4; ++u)
+                s[u] += a.part[(t + 8 * u) * total + i];
+        for (; t < a.splits; t += 8)
+            s[0] += a.part[t * total + i];
+    }
+    sums[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (warp == 0 && i < total) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+            t += sums[w][lane];
+        a.C[i / a.N * a.ldC + i % a.N] = t;
+    }
 }
 
 int device_sms()
@@ -789,8 +828,8 @@ void plan(int64_t M, int64_t N, int64_t K, DenseArgs &a)
     if (tiles >= 8 * sms)
         return;  // enough rounds
     double best = 1e30;
-    for (int64_t rounds = 1; rounds <= 8; ++rounds) {
-        int64_t splits = rounds * sms / tiles;
+    for (int64_t rounds = 0; rounds <= 8; ++rounds) {
+        int64_t splits = rounds * sms / tiles;  // (0 rounds: no split)
         splits = splits < 1 ? 1 : (splits > stages ? stages : splits);
         const int64_t len = (stages + splits - 1) / splits;
         splits = (stages + len - 1) / len;
@@ -805,8 +844,13 @@ void plan(int64_t M, int64_t N, int64_t K, DenseArgs &a)
     }
 }
 
-// The weights are worth splitting beforehand when many row tiles use them.
-bool presplit(const DenseArgs &a) { return a.m_tiles >= 16; }
+// The weights are worth splitting beforehand when many row tiles use them and a CTA goes through more
+// than a few stages (19,717 x 16 x 500: 25 us against 46; 19,717 x 16 x 3: 9.1 against 8.3).
+bool presplit(const DenseArgs &a)
+{
+    const int64_t rounds = ((int64_t)a.m_tiles * a.n_tiles * a.splits + device_sms() - 1) / device_sms();
+    return a.m_tiles >= 16 && rounds * (a.k_per_split / BK) >= 6;
+}
 
 size_t partial_bytes(const DenseArgs &a, int64_t M, int64_t N)
 {
@@ -829,19 +873,21 @@ cudaError_t launch_dense(const DenseArgs &a, unsigned grid, bool pre, cudaStream
 {
     if (!pre) {
         auto kern = dense_kernel<KC_A, KC_B, false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             Raw<KC_A, KC_B, false>::SMEM);
         if (e != cudaSuccess)
             return e;
-        kern<<<grid, THREADS, SMEM_BYTES, st>>>(a);
+        kern<<<grid, THREADS, Raw<KC_A, KC_B, false>::SMEM, st>>>(a);
         return cudaGetLastError();
     }
     auto kern = dense_kernel<KC_A, KC_B, true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         Raw<KC_A, KC_B, true>::SMEM);
     if (e != cudaSuccess)
         return e;
     split_weights_kernel<KC_B><<<(unsigned)a.odd_words, 256, 0, st>>>(a, const_cast<unsigned char *>(a.Bs));
     e = cudaGetLastError();
-    return e != cudaSuccess ? e : launch_dependent(kern, dim3(grid), THREADS, SMEM_BYTES, st, a);
+    return e != cudaSuccess ? e : launch_dependent(kern, dim3(grid), THREADS, Raw<KC_A, KC_B, true>::SMEM, st, a);
 }
 
 }  // namespace
@@ -912,8 +958,8 @@ extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t
         e = transB ? launch_dense<true, true>(a, grid, pre, st) : launch_dense<true, false>(a, grid, pre, st);
     PSPMM_CUDA_TRY(e);
     if (a.splits > 1) {
-        reduce_splits_kernel<<<(unsigned)((M * N + 255) / 256), 256, 0, st>>>(a.C, a.splits, M, N, C, ldC);
-        PSPMM_CUDA_TRY(cudaGetLastError());
+        const ReduceArgs r = {a.C, C, ldC, a.splits, a.M, a.N};
+        PSPMM_CUDA_TRY(launch_dependent(reduce_splits_kernel, dim3((unsigned)((M * N + 31) / 32)), 256, 0, st, r));
     }
     return PSPMM_OK;
 }
