@@ -121,6 +121,24 @@ PSPMM_API int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, co
                     void *stream);
 
 /*
+ * The two products with scratch memory: 16-byte aligned, pspmm_spmm_scratch_bytes(n_rows, nnz, dim, V) bytes
+ * (V = 1 for CSR; rows and entries count block-rows and blocks otherwise).  With it the rows of an
+ * unsplit layout that have more than 64 entries are cut over the whole GPU instead of being walked by
+ * one lane group each; their sums keep a fixed order.  Split layouts use no scratch.
+ */
+PSPMM_API int pspmm_spmm_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim, int32_t V, size_t *bytes);
+PSPMM_API int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
+                   const float *B, float *C, int64_t n_rows, int64_t n_cols, int64_t nnz,
+                   int32_t dim, int64_t ldB, int64_t ldC, const pspmm_cfg *cfg,
+                   const int32_t *rowPtr_split, const int32_t *target_row, int64_t n_seg,
+                   void *scratch, size_t scratch_bytes, void *stream);
+PSPMM_API int pspmm_spmm_bcsr_ws(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val, int32_t V,
+                    const float *B, float *C, int64_t n_blk_rows, int64_t n_cols, int64_t nblk,
+                    int32_t dim, int64_t ldB, int64_t ldC, const pspmm_cfg *cfg,
+                    const int32_t *rowPtr_b_split, const int32_t *target_row, int64_t n_seg,
+                    void *scratch, size_t scratch_bytes, void *stream);
+
+/*
  * out[k] = <A[row(k), :], B[colIdx[k], :]> for every stored position k of a CSR pattern.
  * Stands in for csr_sddmm / csr_split_sddmm (SDDMM/sddmm.cpp:15-117 ->
  * sddmm_kernel.cu:143-246, 917-1057).  Stored values are not read.  Any dim is accepted

@@ -2,8 +2,6 @@
 #include <stdio.h>
 #include <string.h>
 
-#include <atomic>
-
 #include "pspmm_common.cuh"
 #include "vec_ops.cuh"
 
@@ -359,7 +357,7 @@ int pspmm_long_row_threshold(int64_t n_entries)
 static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t n_seg,
                        const int32_t *colIdx, const float *val, int V, const float *B, float *C,
                        int64_t n_out_blk_rows, int64_t n_cols, int64_t n_entries, int32_t dim, int64_t ldB,
-                       int64_t ldC, const pspmm_cfg *cfg, cudaStream_t st)
+                       int64_t ldC, const pspmm_cfg *cfg, void *scratch, size_t scratch_bytes, cudaStream_t st)
 {
     int rc = pspmm_validate_cfg(cfg, false);
     if (rc)
@@ -384,7 +382,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             if (sub.lanes_per_row * (sub.vec_width ? sub.vec_width : 4) > w)
                 sub.lanes_per_row = 0;  // let the launch pick the group width for the narrow range
             rc = spmm_launch(segPtr, target_row, n_seg, colIdx, val, V, B + off, C + off, n_out_blk_rows, n_cols,
-                             n_entries, w, ldB, ldC, &sub, st);
+                             n_entries, w, ldB, ldC, &sub, scratch, scratch_bytes, st);
             if (rc)
                 return rc;
         }
@@ -419,7 +417,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
                 target_row, n_seg, n_out_blk_rows, s.rpg, V, C, ldC, dim, vecok);
     }
 
-    SpmmArgs a;
+    SpmmLongArgs a;
     a.segPtr = segPtr;
     a.target_row = target_row;
     a.colIdx = colIdx;
@@ -434,15 +432,17 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.rows_per_group = s.rpg;
     a.bucketed = bucketed ? 1 : 0;
     a.keep_fraction = l2_keep_fraction((double)n_cols * (double)ldB * 4.0);
-    a.n_entries = n_entries;
-    a.long_row = target_row || accumulate || (cfg && cfg->bucketed) || n_entries <= PSPMM_LONG_ROW ? INT32_MAX
-                                                                                                  : PSPMM_LONG_ROW;
-    a.long_range = long_range(n_entries, 8);  // (resident CTAs take the ranges in turn)
-    a.sms = sm_count();
-    static std::atomic<unsigned long long> tickets{0};
-    a.long_ticket = a.long_row < INT32_MAX ? ++tickets : 0;
+    a.lng = LongArgs{};
+    if (scratch && !target_row && !accumulate && !(cfg && cfg->bucketed) && n_entries > PSPMM_LONG_ROW) {
+        const int lanes = pspmm_long_lanes(a.nvec, V);
+        long_layout(&a.lng, n_seg, n_entries, sm_count(), 3, (a.nvec + lanes - 1) / lanes);
+        if (scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
+            long_place(&a.lng, scratch);
+        else
+            a.lng = LongArgs{};
+    }
     const int64_t per_cta = (int64_t)(s.threads / s.lpr) * s.rpg;
-    const int64_t gx = (n_seg + per_cta - 1) / per_cta;
+    const int64_t gx = (n_seg + per_cta - 1) / per_cta + a.lng.scan_ctas;
     if (gx > INT32_MAX || s.tiles > 65535)
         return PSPMM_E_RANGE;
     dim3 grid((unsigned)gx, (unsigned)s.tiles, 1);
@@ -461,11 +461,26 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     return PSPMM_OK;
 }
 
-extern "C" int pspmm_spmm_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
-                              const float *B, float *C, int64_t n_rows, int64_t n_cols,
-                              int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
-                              const pspmm_cfg *cfg, const int32_t *rowPtr_split,
-                              const int32_t *target_row, int64_t n_seg, void *stream)
+extern "C" int pspmm_spmm_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim, int32_t V, size_t *bytes)
+{
+    if (n_rows < 0 || nnz < 0 || dim <= 0 || V < 1 || V > 3 || !bytes)
+        return PSPMM_E_ARG;
+    *bytes = 0;
+    if (nnz > PSPMM_LONG_ROW && n_rows > 0) {
+        LongArgs a;
+        long_layout(&a, n_rows, nnz, sm_count(), 3, 1);
+        a.n_counters = a.shares + dim / 16 + 1;  // (shares x tiles: one wave, whatever the tiles)
+        *bytes = long_head_bytes(a) + (size_t)a.shares * 2 * V * dim * sizeof(float) + 256;
+    }
+    return PSPMM_OK;
+}
+
+extern "C" int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
+                                 const float *B, float *C, int64_t n_rows, int64_t n_cols,
+                                 int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
+                                 const pspmm_cfg *cfg, const int32_t *rowPtr_split,
+                                 const int32_t *target_row, int64_t n_seg, void *scratch,
+                                 size_t scratch_bytes, void *stream)
 {
     int rc = check_sizes(n_rows, n_cols, nnz, dim);
     if (rc)
@@ -482,14 +497,16 @@ extern "C" int pspmm_spmm_csr(const int32_t *rowPtr, const int32_t *colIdx, cons
     if (split && n_seg >= INT32_MAX)
         return PSPMM_E_RANGE;
     return spmm_launch(split ? rowPtr_split : rowPtr, target_row, split ? n_seg : n_rows, colIdx,
-                       val, 1, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, (cudaStream_t)stream);
+                       val, 1, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, scratch, scratch_bytes,
+                       (cudaStream_t)stream);
 }
 
-extern "C" int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,
-                               int32_t V, const float *B, float *C, int64_t n_blk_rows,
-                               int64_t n_cols, int64_t nblk, int32_t dim, int64_t ldB,
-                               int64_t ldC, const pspmm_cfg *cfg, const int32_t *rowPtr_b_split,
-                               const int32_t *target_row, int64_t n_seg, void *stream)
+extern "C" int pspmm_spmm_bcsr_ws(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,
+                                  int32_t V, const float *B, float *C, int64_t n_blk_rows,
+                                  int64_t n_cols, int64_t nblk, int32_t dim, int64_t ldB,
+                                  int64_t ldC, const pspmm_cfg *cfg, const int32_t *rowPtr_b_split,
+                                  const int32_t *target_row, int64_t n_seg, void *scratch,
+                                  size_t scratch_bytes, void *stream)
 {
     if (V != 2 && V != 3)
         return PSPMM_E_UNSUPPORTED;
@@ -506,7 +523,28 @@ extern "C" int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, c
     if (nblk > 0 && (!colIdx || !val))
         return PSPMM_E_ARG;
     return spmm_launch(split ? rowPtr_b_split : rowPtr_b, target_row, split ? n_seg : n_blk_rows,
-                       colIdx, val, V, B, C, n_blk_rows, n_cols, nblk, dim, ldB, ldC, cfg, (cudaStream_t)stream);
+                       colIdx, val, V, B, C, n_blk_rows, n_cols, nblk, dim, ldB, ldC, cfg, scratch, scratch_bytes,
+                       (cudaStream_t)stream);
+}
+
+extern "C" int pspmm_spmm_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
+                              const float *B, float *C, int64_t n_rows, int64_t n_cols,
+                              int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
+                              const pspmm_cfg *cfg, const int32_t *rowPtr_split,
+                              const int32_t *target_row, int64_t n_seg, void *stream)
+{
+    return pspmm_spmm_csr_ws(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, rowPtr_split,
+                             target_row, n_seg, nullptr, 0, stream);
+}
+
+extern "C" int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,
+                               int32_t V, const float *B, float *C, int64_t n_blk_rows,
+                               int64_t n_cols, int64_t nblk, int32_t dim, int64_t ldB,
+                               int64_t ldC, const pspmm_cfg *cfg, const int32_t *rowPtr_b_split,
+                               const int32_t *target_row, int64_t n_seg, void *stream)
+{
+    return pspmm_spmm_bcsr_ws(rowPtr_b, colIdx, val, V, B, C, n_blk_rows, n_cols, nblk, dim, ldB, ldC, cfg,
+                              rowPtr_b_split, target_row, n_seg, nullptr, 0, stream);
 }
 
 // ----------------------------------------------------------------------------- SDDMM
@@ -741,14 +779,22 @@ extern "C" int pspmm_profile_spmm(const int32_t *rowPtr, const int32_t *colIdx, 
                                   const int32_t *target_row, int64_t n_seg, int32_t warmup,
                                   int32_t iters, float *ms_per_iter, void *stream)
 {
+    // (the scratch that the timed entry points would be given)
+    void *scratch = nullptr;
+    size_t bytes = 0;
+    if (!target_row && pspmm_spmm_scratch_bytes(n_rows, nnz, dim, V, &bytes) == PSPMM_OK && bytes > 0)
+        PSPMM_CUDA_TRY(cudaMallocAsync(&scratch, bytes, (cudaStream_t)stream));
     auto launch = [&]() -> int {
         if (V == 1)
-            return pspmm_spmm_csr(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC,
-                                  cfg, rowPtr_split, target_row, n_seg, stream);
-        return pspmm_spmm_bcsr(rowPtr, colIdx, val, V, B, C, n_rows, n_cols, nnz, dim, ldB, ldC,
-                               cfg, rowPtr_split, target_row, n_seg, stream);
+            return pspmm_spmm_csr_ws(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC,
+                                     cfg, rowPtr_split, target_row, n_seg, scratch, bytes, stream);
+        return pspmm_spmm_bcsr_ws(rowPtr, colIdx, val, V, B, C, n_rows, n_cols, nnz, dim, ldB, ldC,
+                                  cfg, rowPtr_split, target_row, n_seg, scratch, bytes, stream);
     };
-    return time_loop(launch, warmup, iters, ms_per_iter, (cudaStream_t)stream);
+    const int rc = time_loop(launch, warmup, iters, ms_per_iter, (cudaStream_t)stream);
+    if (scratch)
+        cudaFreeAsync(scratch, (cudaStream_t)stream);
+    return rc;
 }
 
 extern "C" int pspmm_profile_sddmm(const int32_t *rowPtr, const int32_t *colIdx, const float *val,

@@ -10,9 +10,6 @@
 #define PSPMM_MAX_CF 8
 #define PSPMM_RPG_MAX 16  // most consecutive segments one lane group owns
 #define PSPMM_LONG_PER_RANGE 12  // a range of 8 * long_row entries meets at most 9 rows longer than long_row
-// Unsplit rows with more entries are not walked by one lane group: it would hold up its warp, and a
-// hub row the whole launch.  One full staging window (SpMM) or four batches of 16 (SDDMM) stay.
-#define PSPMM_LONG_ROW 64
 #define PSPMM_LONG_RANGE_MAX 8192
 #define PSPMM_LONG_LIST 132  // long rows that such a range can meet (8192 / 65 inside it and two cut), and a few
 #define PSPMM_GAP_MAX 256  // longest run of uncovered rows the SpMM kernel zeroes by itself
@@ -81,6 +78,43 @@ __device__ __forceinline__ int find_segment(const int32_t *segPtr, int64_t n_seg
     return (int)lo;
 }
 
+// Long rows of an unsplit layout, see long_rows.cuh.
+#define PSPMM_LONG_ROW 64      // longer rows are cut; one staging window, four batches of 16
+#define PSPMM_LONG_ROWS 512    // rows per total, and per look of a share
+#define PSPMM_LONG_LOOK 512    // what a look costs, in entries (3 us, at 170 - 250 entries per us and CTA)
+
+struct LongArgs {
+    int32_t *totals;    // long rows' entries per PSPMM_LONG_ROWS rows, or nullptr: rows are not cut
+    int32_t n_totals;
+    int32_t scan_ctas;  // leading CTAs of the first kernel, 8 totals each
+    int32_t *counters;  // per share and column tile: partial results that are in, of the row that starts there
+    int32_t n_counters;
+    float *partials;    // two rows per share
+    int32_t shares;     // CTAs (per column tile) of the second kernel
+};
+
+// Host side: sizes for `sms` SMs with `per_sm` resident CTAs of the second kernel: one wave of shares, more
+// when they would exceed 16 K entries (equal shares do not end together).
+static inline void long_layout(LongArgs *a, int64_t n_rows, int64_t n_entries, int sms, int per_sm, int tiles)
+{
+    a->n_totals = (int32_t)((n_rows + PSPMM_LONG_ROWS - 1) / PSPMM_LONG_ROWS);
+    a->scan_ctas = (a->n_totals + 7) / 8;
+    int waves = (int)(n_entries / 16384 / (sms * per_sm)) + 1;
+    waves = waves < 16 ? waves : 16;
+    a->shares = sms * per_sm > tiles ? sms * per_sm * waves / tiles : 1;
+    a->n_counters = a->shares * tiles;
+}
+static inline size_t long_head_bytes(const LongArgs &a)
+{
+    return (((size_t)a.n_totals + (size_t)a.n_counters) * 4 + 255) / 256 * 256;
+}
+static inline void long_place(LongArgs *a, void *scratch)
+{
+    a->totals = (int32_t *)scratch;
+    a->counters = a->totals + a->n_totals;
+    a->partials = (float *)((char *)scratch + long_head_bytes(*a));
+}
+
 // One launch of the segment SpMM kernel.  A "segment" is a CSR row, a PCSR row piece, or
 // the block-row forms of either.
 struct SpmmArgs {
@@ -97,11 +131,12 @@ struct SpmmArgs {
     int32_t rows_per_group;
     float keep_fraction;        // share of B's lines marked evict-last in L2 (0..1]
     int32_t bucketed;           // target_row carries PSPMM_SEG_* flags, segments come in any order
-    int64_t n_entries;          // entries the caller declares
-    int32_t long_row;           // unsplit rows with more entries go to spmm_long_rows_kernel (INT32_MAX: none do)
-    int32_t long_range;         // entries one CTA of that kernel looks after at a time
-    int32_t sms;
-    unsigned long long long_ticket;  // number of this launch, for what spmm_seg_kernel tells the next one
+};
+
+// The kernels that cut long rows get this one.  (Apart, because the register allocation of the others
+// changes with the size of their argument.)
+struct SpmmLongArgs : SpmmArgs {
+    LongArgs lng;  // unsplit layouts: how long rows are cut (totals == nullptr: they are not)
 };
 
 // Flags in target_row of a length-bucketed plan (pspmm_cfg.bucketed): the low 30 bits are the row.
@@ -135,10 +170,10 @@ struct LaunchShape {
 
 // Per-translation-unit dispatchers (one per vector width so the files compile in parallel).
 // Return false when (lpr, cf, V) is not instantiated for that width.
-bool pspmm_launch_spmm_vw4(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st);
-bool pspmm_launch_spmm_vw4_acc(const LaunchShape &s, const SpmmArgs &a, dim3 grid, cudaStream_t st);
-bool pspmm_launch_spmm_vw2(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st);
-bool pspmm_launch_spmm_vw1(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st);
+bool pspmm_launch_spmm_vw4(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
+bool pspmm_launch_spmm_vw4_acc(const LaunchShape &s, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
+bool pspmm_launch_spmm_vw2(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
+bool pspmm_launch_spmm_vw1(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_sddmm_vw4(const LaunchShape &s, int V, const SddmmArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_sddmm_vw2(const LaunchShape &s, int V, const SddmmArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_sddmm_vw1(const LaunchShape &s, int V, const SddmmArgs &a, dim3 grid, cudaStream_t st);
@@ -154,6 +189,8 @@ static inline int pspmm_round_cf(int need)
 }
 
 int pspmm_long_row_threshold(int64_t n_entries);
+// Lanes per row of spmm_long_rows_kernel (its column tiles are that many vectors wide).
+static inline int pspmm_long_lanes(int nvec, int V) { return nvec > 16 ? 32 : (nvec > 8 || V > 1) ? 16 : (nvec > 4 ? 8 : 4); }
 int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm);
 int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, LaunchShape *out);
 int pspmm_vw_max(int32_t dim, int64_t ld0, int64_t ld1, const void *p0, const void *p1);

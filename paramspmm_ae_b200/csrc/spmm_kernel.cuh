@@ -31,11 +31,13 @@
 // short gap that follows each of its rows (up to PSPMM_GAP_MAX rows); longer gaps are left to
 // the pre-pass.
 //
-// Long rows of an unsplit layout (more than SpmmArgs::long_row entries) are left to
-// spmm_long_rows_kernel below, which cuts them over the whole GPU; here they count as empty rows,
-// so the zeros that the second kernel adds to are stored by the same code.
+// Long rows of an unsplit layout are left to spmm_long_rows_kernel below, which cuts them over the
+// whole GPU; here they count as empty rows (their zeros are overwritten).
 #pragma once
 
+#include <type_traits>
+
+#include "long_rows.cuh"
 #include "pspmm_common.cuh"
 #include "vec_ops.cuh"
 
@@ -152,15 +154,12 @@ struct SpmmOcc {
 
 // ACC = true adds the product to C instead of overwriting it: every contribution is a RED, rows
 // without entries add nothing, and nothing is zeroed (no pre-pass either).
-// Largest ticket (SpmmArgs::long_ticket) of a launch that passed over a long row; one per device and
-// translation unit, and a launch and the one that follows it are of the same unit.
-static __device__ unsigned long long g_long_seen;
-
-// LONG = true (unsplit layouts) passes over rows of more than a.long_row entries.  Both are template
+// LONG = true (unsplit layouts) passes over rows of more than PSPMM_LONG_ROW entries
+// (long_rows.cuh); its first CTAs prepare the launch that takes them.  Both are template
 // flags because a run-time test of either costs the 48- and 80-register shapes spills (4 - 13 % of
 // the dim sweep's products).
 template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
-__global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(const SpmmArgs a)
+__global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(const std::conditional_t<LONG, SpmmLongArgs, SpmmArgs> a)
 {
     using Tile = SpmmTile<LPR, V>;
     constexpr int CAP = Tile::CAP;
@@ -179,13 +178,20 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
     int *ent = sp + Tile::HEAD_WORDS;                       // staged entries
 
     const int rpg = a.rows_per_group;
-    const int64_t first = ((int64_t)blockIdx.x * gpc + g) * rpg;
+    int64_t first = ((int64_t)blockIdx.x * gpc + g) * rpg;
+    if constexpr (LONG) {
+        pdl_launch_dependents();
+        if (blockIdx.x < (unsigned)a.lng.scan_ctas) {
+            if (blockIdx.y == 0)
+                long_scan(a.lng, a.segPtr, a.n_seg, (int)blockIdx.x);
+            return;
+        }
+        first -= (int64_t)a.lng.scan_ctas * gpc * rpg;
+    }
     if (first >= a.n_seg)
         return;  // the whole group leaves; groups only ever synchronise among themselves
     const int nrow = (a.n_seg - first < rpg) ? (int)(a.n_seg - first) : rpg;
     const bool split = a.target_row != nullptr;
-    if constexpr (LONG)
-        pdl_launch_dependents();
 
     for (int i = gl; i <= nrow; i += LPR)
         sp[i] = __ldg(a.segPtr + first + i);
@@ -239,7 +245,7 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
         int resume = lim;
         while (row < nrow) {
             const int rb = sp[row], re = sp[row + 1];
-            const bool skip = LONG && re - rb > a.long_row;  // left to spmm_long_rows_kernel
+            const bool skip = LONG && re - rb > PSPMM_LONG_ROW;  // left to spmm_long_rows_kernel
             const int e = (rb > cur ? rb : cur) - cur;
             const int eh = skip ? e : (re < lim ? re : lim) - cur;
             spmm_entries<U, LPR, VW, CF, V>(ent, e, eh, bcol, ldB_bytes, keep, acc);
@@ -313,8 +319,6 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
             }
             ++row;
             if (skip) {  // the window restarts behind the long row
-                if (gl == 0)
-                    atomicMax(&g_long_seen, a.long_ticket);
                 resume = re;
                 break;
             }
@@ -326,33 +330,26 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
     }
 }
 
-// Rows of more than a.long_row entries of an unsplit (block-)CSR layout, which spmm_seg_kernel has
-// stored as zeros.  A row there is walked by one lane group, one gather batch after the other: a hub
-// row of 1,600 entries held a 197 K-entry graph at dim 16 for 310 us, 98 % of the product, and rows of
-// a few hundred entries still leave the groups of a warp out of step (115 M entries at dim 64, rows
-// of 490: 3.1 ms with rows up to 512 entries left there).  Here a CTA takes a range of entries,
-// whatever rows they belong to: two warps find the first and last row of the range (32 pointers
-// probed per step), all threads look for long rows between them, and the entries of those rows, end
-// to end, are dealt to the lane groups in equal spans.  A group walks its span as spmm_seg_kernel walks
-// its segments and leaves one vector RED per row it meets.  Nothing is allocated and no list
-// is kept.  spmm_seg_kernel raises g_long_seen to this launch's ticket when it passes over a row, so a
-// matrix without long rows costs one look at that word.  Tickets only grow: a word that a later launch
-// has raised further makes this one search in vain, never miss a row.  Bound: gather latency (U loads
-// of 16 bytes in flight per lane, as above).
+// The long rows of an unsplit (block-)CSR layout (long_rows.cuh), which spmm_seg_kernel passes over.
+// The entries of a share are dealt to the lane groups in equal spans, which they walk as
+// spmm_seg_kernel walks its segments.  Every sum has a fixed order, as without the cut: the pieces of a
+// row inside a share meet in shared memory in the order of the entries, the shares' parts in
+// a.lng.partials.  Bound: gather latency (U loads of 16 bytes in flight per lane).
 template <int VW, int V, int LPR>
-__global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmArgs a)
+__global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongArgs a)
 {
     constexpr int G = 256 / LPR;
     constexpr int U = V > 1 ? 4 : 8;
     constexpr int CAP = SpmmTile<LPR, V>::CAP;
-    __shared__ __align__(16) int windows[G * CAP * (1 + V)];
-    __shared__ int row_list[PSPMM_LONG_LIST], row_lo[PSPMM_LONG_LIST], row_off[PSPMM_LONG_LIST + 1];
-    __shared__ int row_ends[2];
-    __shared__ int n_long;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int ROW = LPR * VW;  // columns of this CTA
+    constexpr int WINDOW_WORDS = G * CAP * (1 + V), PART_WORDS = G * 2 * V * ROW;
+    __shared__ __align__(16) int work[WINDOW_WORDS > PART_WORDS ? WINDOW_WORDS : PART_WORDS];  // windows, then parts
+    __shared__ LongShare::Shared sh;
+    float *parts = reinterpret_cast<float *>(work);
+    const int lane = threadIdx.x & 31;
     const int g = threadIdx.x / LPR, gl = lane % LPR;
     const unsigned gmask = (LPR == 32) ? PSPMM_FULL_MASK : (((1u << LPR) - 1u) << ((lane / LPR) * LPR));
-    int *ent = windows + g * CAP * (1 + V);
+    int *ent = work + g * CAP * (1 + V);
     const int v = blockIdx.y * LPR + gl;
     const bool act = v < a.nvec;
     const int voff = act ? v * VW : 0;
@@ -360,105 +357,127 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmArgs a
     const unsigned ldB_bytes = (unsigned)(a.ldB * 4);
     const unsigned long long keep = l2_policy_keep(a.keep_fraction);
     const unsigned long long stream = l2_policy_stream();
-    float acc[V][1][VW];
-#pragma unroll
-    for (int w = 0; w < V; ++w)
-#pragma unroll
-        for (int j = 0; j < VW; ++j)
-            acc[w][0][j] = 0.f;
-    const int64_t begin = __ldg(a.segPtr), end = __ldg(a.segPtr + a.n_seg);
-    // (an early look lets the searches run while the kernel before this one drains)
-    bool waited = false;
-    if (*(volatile unsigned long long *)&g_long_seen < a.long_ticket) {
-        pdl_wait();
-        waited = true;
-        if (*(volatile unsigned long long *)&g_long_seen < a.long_ticket)
-            return;
-    }
-    for (int64_t s = begin + (int64_t)blockIdx.x * a.long_range; s < end; s += (int64_t)gridDim.x * a.long_range) {
-        const int64_t e1 = s + a.long_range < end ? s + a.long_range : end;
-        if (threadIdx.x == 0)
-            n_long = 0;
-        if (warp < 2) {
-            const int r = find_segment(a.segPtr, a.n_seg, begin, end, warp == 0 ? s : e1 - 1, lane);
-            if (lane == 0)
-                row_ends[warp] = r;
-        }
-        __syncthreads();
-        for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += 256) {
-            const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
-            if (re - rb > a.long_row) {
-                const int i = atomicAdd(&n_long, 1);
-                row_list[i] = (int)r;
-                row_lo[i] = (int)(rb > s ? rb : s);
-                row_off[i + 1] = (int)((re < e1 ? re : e1) - (rb > s ? rb : s));
-            }
-        }
-        __syncthreads();
-        const int n = n_long;
-        if (warp == 0) {  // lengths -> offsets in the concatenation
-            int base = 0;
-            for (int i0 = 0; i0 < n; i0 += 32) {
-                int x = i0 + lane < n ? row_off[i0 + lane + 1] : 0;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int o = __shfl_up_sync(PSPMM_FULL_MASK, x, d);
-                    if (lane >= d)
-                        x += o;
-                }
-                if (i0 + lane < n)
-                    row_off[i0 + lane + 1] = base + x;
-                base += __shfl_sync(PSPMM_FULL_MASK, x, 31);
-            }
-            if (lane == 0)
-                row_off[0] = 0;
-        }
-        __syncthreads();
-        if (n > 0 && !waited) {
-            pdl_wait();
-            waited = true;
-        }
-        const int total = n > 0 ? row_off[n] : 0;
+    const int64_t dimv = (int64_t)a.nvec * VW;
+    const int share = blockIdx.x;
+    float acc[V][1][VW], first[V][VW];
+
+    pdl_wait();
+    LongShare job;
+    if (!job.begin(a.lng, sh, share))
+        return;
+    while (job.look(sh, a.segPtr, a.n_seg)) {
+        const int total = job.total;
+        if (total == 0)
+            continue;
+        // What a row sums up to in this share: the result, or its part of it.
+        auto emit = [&](int i, int w, int col, const float *val) {
+            int s0, s1;
+            job.shares_of(sh, i, s0, s1);
+            if (s0 == s1)
+                st_vec_hint<VW>(a.C + ((int64_t)sh.row[i] * V + w) * a.ldC + col, val, stream);
+            else
+                st_vec<VW>(a.lng.partials + (LongShare::slot(share, s0) * V + w) * dimv + col, val);
+        };
         const int span = ((total + G - 1) / G + U - 1) / U * U;
-        int p = g * span;  // position in the concatenation
-        const int stop = p + span < total ? p + span : total;
-        int i = 0;         // the row it lies in
-        while (i + 1 < n && p >= row_off[i + 1])
-            ++i;
+        const int start = g * span;
+        const int stop = start + span < total ? start + span : total;
+        int p = start;  // position in the concatenation
+        int i = p < stop ? job.row_of(sh, p) : 0;
+        bool has_first = false, has_last = false;
         while (p < stop) {
-            const int row_stop = row_off[i + 1] < stop ? row_off[i + 1] : stop;
+            const bool from_row_start = p == job.off(sh, i), from_span_start = p == start;
+            const int row_end = job.off(sh, i + 1), row_stop = row_end < stop ? row_end : stop;
+            const int from = sh.lo[i] - job.off(sh, i);
+#pragma unroll
+            for (int w = 0; w < V; ++w)
+#pragma unroll
+                for (int j = 0; j < VW; ++j)
+                    acc[w][0][j] = 0.f;
             while (p < row_stop) {
                 const int fill = row_stop - p < CAP ? row_stop - p : CAP;
-                spmm_stage<LPR, V>(a, ent, row_lo[i] + (p - row_off[i]), fill, gl, stream);
+                spmm_stage<LPR, V>(a, ent, from + p, fill, gl, stream);
                 __syncwarp(gmask);
                 spmm_entries<U, LPR, VW, 1, V>(ent, 0, fill, bcol, ldB_bytes, keep, acc);
                 __syncwarp(gmask);
                 p += fill;
             }
+            if (from_row_start && p == row_end) {  // all of the row's entries in this share
+                if (act) {
 #pragma unroll
-            for (int w = 0; w < V; ++w) {
-                if (act)
-                    red_add_vec<VW>(a.C + ((int64_t)row_list[i] * V + w) * a.ldC + voff, acc[w][0]);
+                    for (int w = 0; w < V; ++w)
+                        emit(i, w, voff, acc[w][0]);
+                }
+                has_last = false;
+            } else if (from_span_start) {
+                has_first = true;
 #pragma unroll
-                for (int j = 0; j < VW; ++j)
-                    acc[w][0][j] = 0.f;
+                for (int w = 0; w < V; ++w)
+#pragma unroll
+                    for (int j = 0; j < VW; ++j)
+                        first[w][j] = acc[w][0][j];
+            } else {
+                has_last = true;  // (only the span's last piece ends inside a row)
             }
             ++i;
         }
+        __syncthreads();  // the windows are free
+#pragma unroll
+        for (int w = 0; w < V; ++w)
+#pragma unroll
+            for (int j = 0; j < VW; ++j) {
+                if (has_first)
+                    parts[((g * 2) * V + w) * ROW + gl * VW + j] = first[w][j];
+                if (has_last)
+                    parts[((g * 2 + 1) * V + w) * ROW + gl * VW + j] = acc[w][0][j];
+            }
+        __syncthreads();
+        // Rows that several groups share, their pieces in order.
+        const int row0 = sh.edge[0], rows = sh.edge[1] - row0 + 1;
+        for (int t = threadIdx.x; t < rows * V * LPR; t += 256) {
+            const int i2 = row0 + t / (V * LPR), w = t / LPR % V, l = t % LPR;
+            const int vi = blockIdx.y * LPR + l;
+            const int off0 = job.off(sh, i2);
+            const int g0 = off0 / span, g1 = (job.off(sh, i2 + 1) - 1) / span;
+            if (g0 == g1 || vi >= a.nvec)
+                continue;  // one group had all of it
+            float sum[VW];
+#pragma unroll
+            for (int j = 0; j < VW; ++j)
+                sum[j] = 0.f;
+            for (int q = g0; q <= g1; ++q) {
+                const int slot = q > g0 || off0 == q * span ? 0 : 1;
+#pragma unroll
+                for (int j = 0; j < VW; ++j)
+                    sum[j] += parts[((q * 2 + slot) * V + w) * ROW + l * VW + j];
+            }
+            emit(i2, w, vi * VW, sum);
+        }
+        job.arrive(a.lng, sh, blockIdx.y, gridDim.y);
+        for (int q = 0; q < 2; ++q) {
+            if (!sh.last[q])
+                continue;
+            int s0, s1;
+            job.shares_of(sh, sh.edge[q], s0, s1);
+            const int64_t r = sh.row[sh.edge[q]];
+            for (int t = threadIdx.x; t < V * ROW; t += 256) {
+                const int w = t / ROW, col = blockIdx.y * ROW + t % ROW;
+                if (col >= dimv)
+                    continue;
+                float sum = 0.f;
+                for (int c = s0; c <= s1; ++c)
+                    sum += __ldcg(a.lng.partials + (LongShare::slot(c, s0) * V + w) * dimv + col);
+                a.C[(r * V + w) * a.ldC + col] = sum;
+            }
+        }
         __syncthreads();
     }
-    if (!waited)
-        pdl_wait();  // this grid must not count as done before the one it follows
 }
 
 template <int VW, int V>
-static inline void spmm_launch_long_rows(const SpmmArgs &a, cudaStream_t st)
+static inline void spmm_launch_long_rows(const SpmmLongArgs &a, cudaStream_t st)
 {
-    const int lpr = a.nvec > 16 ? 32 : (a.nvec > 8 || V > 1) ? 16 : (a.nvec > 4 ? 8 : 4);
-    const int64_t ranges = (a.n_entries + a.long_range - 1) / a.long_range;
-    const unsigned tiles = (unsigned)((a.nvec + lpr - 1) / lpr);
-    const int64_t most = (unsigned)a.sms * 3 > tiles ? a.sms * 3 / tiles : 1;  // one resident wave, no CTA more
-    const dim3 grid((unsigned)(ranges < most ? ranges : most), tiles);
+    const int lpr = pspmm_long_lanes(a.nvec, V);
+    const dim3 grid((unsigned)a.lng.shares, (unsigned)((a.nvec + lpr - 1) / lpr));
     if (lpr == 32)
         launch_dependent(spmm_long_rows_kernel<VW, V, 32>, grid, 256, 0, st, a);
     else if (lpr == 16)
@@ -473,7 +492,7 @@ static inline void spmm_launch_long_rows(const SpmmArgs &a, cudaStream_t st)
 
 // The launch that follows spmm_seg_kernel when rows may have been left to it.
 #define PSPMM_SPMM_LONG_ROWS(VW_)                                            \
-    if (a.n_entries > 0 && a.long_row < INT32_MAX) {                         \
+    if (a.lng.totals) {                                                      \
         if (V == 1)                                                          \
             spmm_launch_long_rows<VW_, 1>(a, st);                            \
         else if (V == 2)                                                     \
@@ -483,23 +502,24 @@ static inline void spmm_launch_long_rows(const SpmmArgs &a, cudaStream_t st)
     }
 
 template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
-static inline void spmm_launch_one(const SpmmArgs &a, dim3 grid, int threads, cudaStream_t st)
+static inline void spmm_launch_one(const SpmmLongArgs &a, dim3 grid, int threads, cudaStream_t st)
 {
     const int smem = (threads / LPR) * SpmmTile<LPR, V>::GROUP_WORDS * 4;
     auto kern = spmm_seg_kernel<LPR, VW, CF, V, MLP, ACC, LONG>;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const std::conditional_t<LONG, SpmmLongArgs, SpmmArgs> &args = a;
     if (a.target_row && !ACC)
-        launch_dependent(kern, grid, threads, smem, st, a);  // follows the zeroing pre-pass
+        launch_dependent(kern, grid, threads, smem, st, args);  // follows the zeroing pre-pass
     else
-        kern<<<grid, threads, smem, st>>>(a);
+        kern<<<grid, threads, smem, st>>>(args);
 }
 
 // Expands to the dispatch over the instantiated (LPR, CF) pairs of one (VW, V).
 // (the form that passes over long rows is built at one gather-batch depth)
 #define PSPMM_SPMM_CASE(LPR_, CF_, VW_, V_)                                               \
     if (s.lpr == LPR_ && s.cf == CF_) {                                                   \
-        if (a.long_row < INT32_MAX)                                                       \
+        if (a.lng.totals)                                                       \
             spmm_launch_one<LPR_, VW_, CF_, V_, 8, false, true>(a, grid, s.threads, st);  \
         else                                                                              \
             spmm_launch_one<LPR_, VW_, CF_, V_, 8>(a, grid, s.threads, st);               \
@@ -508,7 +528,7 @@ static inline void spmm_launch_one(const SpmmArgs &a, dim3 grid, int threads, cu
 // Same, with every gather-batch depth instantiated (used for the 128-bit CSR family).
 #define PSPMM_SPMM_CASE_MLP(LPR_, CF_, VW_, V_)                              \
     if (s.lpr == LPR_ && s.cf == CF_) {                                      \
-        if (a.long_row < INT32_MAX)                                          \
+        if (a.lng.totals)                                          \
             spmm_launch_one<LPR_, VW_, CF_, V_, 8, false, true>(a, grid, s.threads, st); \
         else if (s.mlp == 2)                                                 \
             spmm_launch_one<LPR_, VW_, CF_, V_, 2>(a, grid, s.threads, st);  \

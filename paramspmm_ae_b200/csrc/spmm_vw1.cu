@@ -10,7 +10,7 @@
 #define CFS_2(LPR_, V_) CASE(LPR_, 1, 1, V_) CASE(LPR_, 2, 1, V_)
 #define CASE PSPMM_SPMM_CASE
 
-static bool launch_segments(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st)
+static bool launch_segments(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st)
 {
     if (V == 1) {
         CFS_ALL(8, 1)
@@ -25,7 +25,7 @@ static bool launch_segments(const LaunchShape &s, int V, const SpmmArgs &a, dim3
     return false;
 }
 
-bool pspmm_launch_spmm_vw1(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st)
+bool pspmm_launch_spmm_vw1(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st)
 {
     if (!launch_segments(s, V, a, grid, st))
         return false;

@@ -13,7 +13,7 @@
     PSPMM_SPMM_CASE_MLP(LPR_, 1, 4, 1) PSPMM_SPMM_CASE_MLP(LPR_, 2, 4, 1) PSPMM_SPMM_CASE_MLP(LPR_, 3, 4, 1) \
     PSPMM_SPMM_CASE_MLP(LPR_, 4, 4, 1) PSPMM_SPMM_CASE_MLP(LPR_, 6, 4, 1) PSPMM_SPMM_CASE_MLP(LPR_, 8, 4, 1)
 
-static bool launch_segments(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st)
+static bool launch_segments(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st)
 {
     if (V == 1) {
         CFS_ALL(2, 1)
@@ -33,7 +33,7 @@ static bool launch_segments(const LaunchShape &s, int V, const SpmmArgs &a, dim3
     return false;
 }
 
-bool pspmm_launch_spmm_vw4(const LaunchShape &s, int V, const SpmmArgs &a, dim3 grid, cudaStream_t st)
+bool pspmm_launch_spmm_vw4(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st)
 {
     if (!launch_segments(s, V, a, grid, st))
         return false;

@@ -6,7 +6,7 @@
     PSPMM_SPMM_CASE_ACC(LPR_, 1) PSPMM_SPMM_CASE_ACC(LPR_, 2) PSPMM_SPMM_CASE_ACC(LPR_, 3) \
     PSPMM_SPMM_CASE_ACC(LPR_, 4) PSPMM_SPMM_CASE_ACC(LPR_, 6) PSPMM_SPMM_CASE_ACC(LPR_, 8)
 
-bool pspmm_launch_spmm_vw4_acc(const LaunchShape &s, const SpmmArgs &a, dim3 grid, cudaStream_t st)
+bool pspmm_launch_spmm_vw4_acc(const LaunchShape &s, const SpmmLongArgs &a, dim3 grid, cudaStream_t st)
 {
     CFS_ACC(4)
     CFS_ACC(8)

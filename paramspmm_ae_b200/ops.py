@@ -350,20 +350,23 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
         n_out_rows = n_seg
     _check_output(out, rowPtr, split, n_out_rows, V, dim)
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
-    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref)
+    long_rows = target_row is None and (cfg is None or not (cfg.bucketed or cfg.accumulate))
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows)
 
 
-def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref):
+def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows):
     seg = rowPtr.data_ptr()
     n, dim = X.shape
     # row pointers of a split layout go into the split arguments
     plain, split, target, n_seg = (seg, None, None, 0) if target_row is None else (
         None, seg, target_row.data_ptr(), rowPtr.shape[0] - 1)
-    tail = (n_out_rows, n, colIdx.shape[0], dim, X.stride(0), out.stride(0), ref, split, target, n_seg, _stream())
+    nent = colIdx.shape[0]
+    scratch, nbytes = _scratch("pspmm_spmm_scratch_bytes", (n_out_rows, nent, dim, V), X.device) if long_rows else (None, 0)
+    tail = (n_out_rows, n, nent, dim, X.stride(0), out.stride(0), ref, split, target, n_seg, _ptr(scratch), nbytes, _stream())
     if V == 1:
-        rc = lib().pspmm_spmm_csr(plain, colIdx.data_ptr(), _ptr(val), X.data_ptr(), out.data_ptr(), *tail)
+        rc = lib().pspmm_spmm_csr_ws(plain, colIdx.data_ptr(), _ptr(val), X.data_ptr(), out.data_ptr(), *tail)
     else:
-        rc = lib().pspmm_spmm_bcsr(plain, colIdx.data_ptr(), _ptr(val), V, X.data_ptr(), out.data_ptr(), *tail)
+        rc = lib().pspmm_spmm_bcsr_ws(plain, colIdx.data_ptr(), _ptr(val), V, X.data_ptr(), out.data_ptr(), *tail)
     if rc:
         check(rc)
     return out
@@ -389,7 +392,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W):
             out[n_seg * V:].zero_()
             n_out = n_seg
     return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out,
-                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None))
+                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None)
 
 
 def csr_spmm(X, rowPtr, colIdx, val, CF, blkWarpNum):

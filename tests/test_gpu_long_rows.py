@@ -73,3 +73,21 @@ def test_long_rows_of_the_fused_aggregation(oracle, name, dim, softmax):
         s = 2.0 * B[c].astype(np.float64) @ A[r].astype(np.float64)
         w = s if not softmax else np.exp(s - s.max(initial=-np.inf)) / max(np.exp(s - s.max(initial=-np.inf)).sum(), 1e-300)
         np.testing.assert_allclose(got[r], w @ V[c].astype(np.float64), rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("dim", [8, 64, 100])
+def test_sums_of_long_rows_have_a_fixed_order(dim):
+    """Equal columns stay bitwise equal and a second call gives the same bits, rows that span several
+    shares of the entries included."""
+    from paramspmm_ae_b200 import ops
+    dev = torch.device("cuda:0")
+    rp, ci, v = _matrix([30000, 3, 700, 20000] + [70] * 500 + [25000], 40001, 7)
+    t = [torch.from_numpy(x).to(dev) for x in (rp, ci, v)]
+    B = torch.rand(40001, 1, device=dev).expand(-1, dim).contiguous()
+    a = torch.empty(len(rp) - 1, dim, device=dev)
+    ops.spmm_into(a, B, *t)
+    assert bool((a == a[:, :1]).all())
+    for _ in range(5):
+        b = torch.empty_like(a)
+        ops.spmm_into(b, B, *t)
+        assert torch.equal(a, b)
