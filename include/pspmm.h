@@ -236,8 +236,8 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  * per lane group; combinations that are not built are rounded to the nearest built one.
  * Split layouts (rowPtr_split/target_row/n_seg as in pspmm_spmm_csr) need scratch of
  * pspmm_agnn_scratch_bytes(n_seg, dim) bytes, 16-byte aligned, for the partial results of the
- * pieces of split rows; plain CSR needs none (NULL, 0), but with pspmm_agnn_long_scratch_bytes(nnz,
- * dim) bytes, 16-byte aligned, its long rows are cut over the whole GPU instead of being walked by one
+ * pieces of split rows; plain CSR needs none (NULL, 0), but with pspmm_agnn_long_scratch_bytes(n_rows,
+ * nnz, dim) bytes, 16-byte aligned, its long rows are cut over the whole GPU instead of being walked by one
  * lane group each.
  *
  * pspmm_agnn_fused_apply_csr is the same pass with a separate aggregation operand:
@@ -249,7 +249,7 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  * the alignment rules of B; this form runs with 128-bit loads and batches of 4.
  */
 PSPMM_API int pspmm_agnn_scratch_bytes(int64_t n_seg, int32_t dim, size_t *bytes);
-PSPMM_API int pspmm_agnn_long_scratch_bytes(int64_t nnz, int32_t dim, size_t *bytes);
+PSPMM_API int pspmm_agnn_long_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim, size_t *bytes);
 PSPMM_API int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *A,
                                          const float *B, const float *V, float *out, int64_t n_rows, int64_t nnz,
                                          int32_t dim, int64_t ldA, int64_t ldB, int64_t ldV, int64_t ldOut,
@@ -262,6 +262,27 @@ PSPMM_API int pspmm_agnn_fused_csr(const int32_t *rowPtr, const int32_t *colIdx,
                                    int32_t vec_width, int32_t lanes_per_row, int32_t batch,
                                    const int32_t *rowPtr_split, const int32_t *target_row, int64_t n_seg,
                                    void *scratch, size_t scratch_bytes, void *stream);
+
+/*
+ * The fused aggregation as an AGNN layer trains it (gnn_conv.py:130-172 of the reference), with the
+ * attention weight read from device memory, so that no call waits for it:
+ *     forward   out_i = sum_j beta <X_i, X_j> X_j
+ *     backward  D_i = sum_j beta <X_i, X_j> G_j,  and in the same pass
+ *               *d_beta = sum over the entries (i, j) of j * <G_i, G_j>
+ * (the reference weights every score gradient by its column id).  d_beta may be NULL.  Scratch:
+ * pspmm_agnn_layer_scratch_bytes(n_rows, nnz, n_seg, dim) bytes, n_seg = 0 for unsplit layouts, 16-byte
+ * aligned; required by the backward and by split layouts.  Operands as in pspmm_agnn_fused_csr.
+ */
+PSPMM_API int pspmm_agnn_layer_scratch_bytes(int64_t n_rows, int64_t nnz, int64_t n_seg, int32_t dim, size_t *bytes);
+PSPMM_API int pspmm_agnn_layer_forward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, float *out,
+                                       int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX, int64_t ldOut,
+                                       const float *beta, const int32_t *rowPtr_split, const int32_t *target_row,
+                                       int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream);
+PSPMM_API int pspmm_agnn_layer_backward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, const float *G,
+                                        float *D, float *d_beta, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX,
+                                        int64_t ldG, int64_t ldD, const float *beta, const int32_t *rowPtr_split,
+                                        const int32_t *target_row, int64_t n_seg, void *scratch, size_t scratch_bytes,
+                                        void *stream);
 
 /*
  * Exchange step of a row-sharded SpMM across GPUs (it has no counterpart in the reference, which

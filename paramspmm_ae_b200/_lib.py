@@ -90,7 +90,12 @@ _SIGNATURES = {
     "pspmm_split_csr_device": [_vp, _i64, _i32, _vp, _vp, _i64, _vp, ctypes.c_size_t, _vp],
     "pspmm_split_csr_device_static": [_vp, _i64, _i32, _vp, _vp, _i64, _vp],
     "pspmm_agnn_scratch_bytes": [_i64, _i32, ctypes.POINTER(ctypes.c_size_t)],
-    "pspmm_agnn_long_scratch_bytes": [_i64, _i32, ctypes.POINTER(ctypes.c_size_t)],
+    "pspmm_agnn_long_scratch_bytes": [_i64, _i64, _i32, ctypes.POINTER(ctypes.c_size_t)],
+    "pspmm_agnn_layer_scratch_bytes": [_i64, _i64, _i64, _i32, ctypes.POINTER(ctypes.c_size_t)],
+    "pspmm_agnn_layer_forward": [_vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp, _vp, _vp, _i64, _vp,
+                                 ctypes.c_size_t, _vp],
+    "pspmm_agnn_layer_backward": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i64,
+                                  _vp, ctypes.c_size_t, _vp],
     "pspmm_agnn_fused_apply_csr": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, _i64,
                                    ctypes.c_float, _i32, _i32, _i32, _i32, _vp, _vp, _i64, _vp, ctypes.c_size_t, _vp],
     "pspmm_agnn_fused_csr": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, ctypes.c_float, _i32,

@@ -21,10 +21,11 @@
 // A row that is a single segment is normalised and stored directly.  Pieces of a split row leave
 // (running max, running sum, unnormalised accumulator) in caller-provided scratch and are merged
 // by agnn_combine_kernel; long rows of an unsplit layout are cut by the kernel itself when scratch is
-// given (agnn_long_rows) and merged by agnn_combine_long_kernel.  Rows that no segment covers are zeroed by a memset of the output
+// given (agnn_long_kernel).  Rows that no segment covers are zeroed by a memset of the output
 // (split layouts only; in plain CSR every row is a segment and stores its own zeros).
 #include <math_constants.h>
 
+#include "long_rows.cuh"
 #include "pspmm_common.cuh"
 #include "vec_ops.cuh"
 
@@ -43,25 +44,65 @@ struct AgnnArgs {
     int64_t ldA, ldB, ldV, ldOut;
     int32_t dim, dim_pad;
     float beta;
+    const float *beta_dev;  // where beta lies on the device, or nullptr: `beta`
     int32_t softmax;
-    int32_t long_row;    // unsplit rows with more entries are dealt to the first long_ctas CTAs (INT32_MAX: none are)
-    int32_t long_range;  // entries per range of those CTAs
-    uint32_t long_ctas;
+    double *col_sums;       // COL kernels: one partial sum per CTA
+    int32_t n_col_sums;     // CTAs of the first kernel that own segments, then the shares of long rows
+    float *col_out;
+    LongArgs lng;  // unsplit layouts: how long rows are cut (totals == nullptr: they are not)
 };
+
+// Sum over the CTA's 256 threads, stored by thread 0.
+__device__ __forceinline__ void cta_sum_to(double *dst, double x)
+{
+    __shared__ double warps[8];
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1)
+        x += __shfl_xor_sync(PSPMM_FULL_MASK, x, d);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+        warps[threadIdx.x >> 5] = x;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+            t += warps[w];
+        *dst = t;
+    }
+}
+
+// One CTA adds up the partial sums.
+__global__ void __launch_bounds__(256) agnn_col_sum_kernel(const AgnnArgs a)
+{
+    pdl_wait();
+    double x = 0.0;
+    for (int i = threadIdx.x; i < a.n_col_sums; i += 256)
+        x += __ldcg(a.col_sums + i);
+    double *sum = a.col_sums + a.n_col_sums;
+    cta_sum_to(sum, x);
+    if (threadIdx.x == 0)
+        *a.col_out = (float)*sum;
+}
 
 // Running state of one lane group: maximum and sum of the softmax (per group), the lane's slices of
 // the unnormalised accumulator.
-template <int CF, int VW>
+// With COL also the lane's part of the sum over the row's entries of column id * <V_i, V_j> (the score
+// gradient that the layer's attention weight receives), from the slices of row i in `vv`.
+template <int CF, int VW, bool COL>
 struct AgnnState {
+    float beta;
     float m, l, acc[CF][VW];
+    float t;
+    FVec<VW> vv[COL ? CF : 1];
 };
 
 // The entries [lb, hb) of one row for one lane group.  Every lane of the warp calls this together;
 // `maxlen` is the longest of the warp's ranges and a group without work passes lb == hb.
-template <int LPR, int CF, int BS, int VW, bool SEP>
+template <int LPR, int CF, int BS, int VW, bool SEP, bool COL>
 __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (&av)[CF], const bool (&act)[CF],
                                              const int (&voff)[CF], int lb, int hb, int maxlen, int gl,
-                                             AgnnState<CF, VW> &state)
+                                             AgnnState<CF, VW, COL> &state)
 {
     float m = state.m, l = state.l;
     float (&acc)[CF][VW] = state.acc;
@@ -83,7 +124,6 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
             if (off >= maxlen)
                 break;  // warp-uniform
             const bool mine = (lb + off + sub) < hb;
-            const bool full = (off + BS <= len);
             FVec<VW> x[BS][CF];
             FVec<VW> y[SEP ? BS : 1][SEP ? CF : 1];  // the rows that are aggregated, when they are not B's
             float part[BS];
@@ -91,22 +131,18 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
 #pragma unroll
             for (int e = 0; e < BS; ++e)
                 ce[e] = __shfl_sync(PSPMM_FULL_MASK, c_chunk, b * BS + e, LPR);
+            // Predicated, not branched on whether the batch is full: the groups of a warp are at different
+            // entries of their rows, and a branch issued the loads of one after those of the others
+            // (115 M entries at dim 64: 2.7 ms with the branch, 2.2 without; with two operands 5.2, 3.6).
 #pragma unroll
             for (int e = 0; e < BS; ++e) {
                 const float *brow = a.B + (int64_t)ce[e] * a.ldB;
-                if (full) {
+                const bool on = (off + e) < len;
 #pragma unroll
-                    for (int cf = 0; cf < CF; ++cf)
-                        x[e][cf] = ldg_vec<VW>(brow + voff[cf]);
-                } else {
-                    const bool on = (off + e) < len;
-#pragma unroll
-                    for (int cf = 0; cf < CF; ++cf)
-                        x[e][cf] = ldg_vec_if<VW>(brow + voff[cf], on);
-                }
+                for (int cf = 0; cf < CF; ++cf)
+                    x[e][cf] = ldg_vec_if<VW>(brow + voff[cf], on);
                 if constexpr (SEP) {
                     const float *vrow = a.Vm + (int64_t)ce[e] * a.ldV;
-                    const bool on = (off + e) < len;
 #pragma unroll
                     for (int cf = 0; cf < CF; ++cf)
                         y[e][cf] = ldg_vec_if<VW>(vrow + voff[cf], on);
@@ -124,7 +160,7 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
                     }
                 part[e] = s;
             }
-            const float score = a.beta * group_transpose_reduce<LPR, BS>(part, gl);  // entry `sub`
+            const float score = state.beta * group_transpose_reduce<LPR, BS>(part, gl);  // entry `sub`
             float p;
             if (a.softmax) {
                 float bm = mine ? score : -CUDART_INF_F;
@@ -150,6 +186,20 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
             } else {
                 p = mine ? score : 0.f;
             }
+            if constexpr (COL) {
+#pragma unroll
+                for (int e = 0; e < BS; ++e) {
+                    float d = 0.f;
+#pragma unroll
+                    for (int cf = 0; cf < CF; ++cf)
+                        if (act[cf]) {
+#pragma unroll
+                            for (int i = 0; i < VW; ++i)
+                                d = fmaf(state.vv[cf].v[i], y[e][cf].v[i], d);
+                        }
+                    state.t = fmaf((float)ce[e], d, state.t);
+                }
+            }
 #pragma unroll
             for (int e = 0; e < BS; ++e) {
                 const float pe = __shfl_sync(PSPMM_FULL_MASK, p, e, BS);
@@ -169,9 +219,9 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
     state.l = l;
 }
 
-template <int LPR, int CF, int VW>
+template <int LPR, int CF, int VW, bool COL>
 __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bool live, int gl, FVec<VW> (&av)[CF],
-                                              bool (&act)[CF], int (&voff)[CF], AgnnState<CF, VW> &state)
+                                              bool (&act)[CF], int (&voff)[CF], AgnnState<CF, VW, COL> &state)
 {
     const int nvec = a.dim / VW;
 #pragma unroll
@@ -180,6 +230,8 @@ __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bo
         act[cf] = v < nvec;
         voff[cf] = act[cf] ? v * VW : 0;
         av[cf] = (live && act[cf]) ? ldg_vec<VW>(a.A + row * a.ldA + voff[cf]) : zero_vec<VW>();
+        if constexpr (COL)
+            state.vv[cf] = (live && act[cf]) ? ldg_vec<VW>(a.Vm + row * a.ldV + voff[cf]) : zero_vec<VW>();
 #pragma unroll
         for (int i = 0; i < VW; ++i)
             state.acc[cf][i] = 0.f;
@@ -188,125 +240,26 @@ __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bo
     state.l = 0.f;
 }
 
-// Scratch slot of the piece of a long row that starts at entry p (counted from the first entry) of
-// range p / long_range: rows that start in the same stretch of long_row entries are not both long,
-// and only one row continues into a range, so (stretch, continues or starts) names a piece.
-__device__ __forceinline__ int64_t long_piece_slot(const AgnnArgs &a, int64_t p, bool starts)
-{
-    return 2 * (p / a.long_row) + (starts ? 1 : 0);
-}
+// Resident CTAs the register budget is cut for: 16 floats of a row per lane would otherwise take 142
+// registers and leave one (12 M entries at dim 128: 1,040 us instead of 570).
+template <int CF, int VW, bool SEP>
+struct AgnnOcc {
+    static constexpr int MIN_CTAS = SEP ? (CF * VW >= 16 ? 1 : 2) : (CF * VW >= 16 ? 2 : 3);
+};
 
-// The first `long_ctas` CTAs look after the long rows of an unsplit layout (more than a.long_row
-// entries), which the lane groups of the others pass over: one group walks a row's batches one after
-// the other, so a hub row of 8 K entries held a 900 K-entry graph at dim 32 for 0.8 ms of a 20 us
-// pass.  CTA c owns the entries [c, c+1) * a.long_range, finds the long rows among them, deals each
-// one's entries to its lane groups, merges their states in shared memory and leaves one partial
-// result per piece in scratch for agnn_combine_long_kernel.
-template <int LPR, int CF, int BS, int VW, bool SEP>
-__device__ __forceinline__ void agnn_long_rows(const AgnnArgs &a)
-{
-    constexpr int GROUPS = 256 / LPR;
-    extern __shared__ float part[];  // [8][dim_pad + 2]
-    const int pitch = a.dim_pad + 2;
-    __shared__ int row_list[PSPMM_LONG_PER_RANGE];
-    __shared__ int row_ends[2];
-    __shared__ int n_long;
-    const int g = threadIdx.x / LPR, gl = threadIdx.x % LPR;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t begin = __ldg(a.segPtr), end = __ldg(a.segPtr + a.n_seg);
-    for (int64_t s = begin + (int64_t)blockIdx.x * a.long_range; s < end; s += (int64_t)a.long_ctas * a.long_range) {
-        const int64_t e1 = s + a.long_range < end ? s + a.long_range : end;
-        if (threadIdx.x == 0)
-            n_long = 0;
-        if (warp < 2) {
-            const int r = find_segment(a.segPtr, a.n_seg, begin, end, warp == 0 ? s : e1 - 1, lane);
-            if (lane == 0)
-                row_ends[warp] = r;
-        }
-        __syncthreads();
-        for (int64_t r = row_ends[0] + threadIdx.x; r <= row_ends[1]; r += 256)
-            if (__ldg(a.segPtr + r + 1) - __ldg(a.segPtr + r) > a.long_row)
-                row_list[atomicAdd(&n_long, 1)] = (int)r;
-        __syncthreads();
-        for (int i = 0; i < n_long; ++i) {
-            const int r = row_list[i];
-            const int64_t rb = __ldg(a.segPtr + r), re = __ldg(a.segPtr + r + 1);
-            const int64_t lo = rb > s ? rb : s, hi = re < e1 ? re : e1;
-            const int share = (int)((hi - lo + GROUPS - 1) / GROUPS);
-            int64_t b = lo + (int64_t)g * share;
-            b = b < hi ? b : hi;
-            const int64_t e = b + share < hi ? b + share : hi;
-            FVec<VW> av[CF];
-            bool act[CF];
-            int voff[CF];
-            AgnnState<CF, VW> st;
-            agnn_load_row<LPR, CF, VW>(a, r, true, gl, av, act, voff, st);
-            agnn_entries<LPR, CF, BS, VW, SEP>(a, av, act, voff, (int)b, (int)e, share, gl, st);
-            // the lane groups of a warp merge by shuffles, the warps in shared memory
-            float M = st.m;
-#pragma unroll
-            for (int d = LPR; d < 32; d <<= 1)
-                M = fmaxf(M, __shfl_xor_sync(PSPMM_FULL_MASK, M, d));
-            const float w = !a.softmax ? 1.f : (st.m > -CUDART_INF_F ? expf(st.m - M) : 0.f);
-            float *mine = part + warp * pitch;
-            float L = st.l * w;
-#pragma unroll
-            for (int d = LPR; d < 32; d <<= 1)
-                L += __shfl_xor_sync(PSPMM_FULL_MASK, L, d);
-            if (lane == 0) {
-                mine[0] = M;
-                mine[1] = L;
-            }
-#pragma unroll
-            for (int cf = 0; cf < CF; ++cf)
-#pragma unroll
-                for (int j = 0; j < VW; ++j) {
-                    float x = st.acc[cf][j] * w;
-#pragma unroll
-                    for (int d = LPR; d < 32; d <<= 1)
-                        x += __shfl_xor_sync(PSPMM_FULL_MASK, x, d);
-                    if (lane < LPR && act[cf])
-                        mine[2 + voff[cf] + j] = x;
-                }
-            __syncthreads();
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                M = fmaxf(M, part[q * pitch]);
-            float *ps = a.scratch + long_piece_slot(a, lo - begin, rb >= s) * (int64_t)(4 + a.dim_pad);
-            for (int j = (int)threadIdx.x - 1; j < a.dim; j += 256) {  // (thread 0 starts with the sum of the weights)
-                float t = 0.f;
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const float mq = part[q * pitch];
-                    const float wq = !a.softmax ? 1.f : (mq > -CUDART_INF_F ? expf(mq - M) : 0.f);
-                    t = fmaf(wq, part[q * pitch + 2 + j], t);  // (column -1 is the warp's sum)
-                }
-                if (j < 0) {
-                    ps[0] = M;
-                    ps[1] = t;
-                } else {
-                    ps[4 + j] = t;
-                }
-            }
-            __syncthreads();
-        }
-        __syncthreads();
-    }
-}
-
-template <int LPR, int CF, int BS, int VW, bool SEP = false>
-__global__ void __launch_bounds__(256) agnn_fused_kernel(const AgnnArgs a)
+template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false>
+__global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fused_kernel(const AgnnArgs a)
 {
     static_assert(BS <= LPR, "a batch cannot be wider than the lane group");
     pdl_launch_dependents();
-    if (blockIdx.x < a.long_ctas) {
-        agnn_long_rows<LPR, CF, BS, VW, SEP>(a);
+    if (blockIdx.x < (unsigned)a.lng.scan_ctas) {
+        long_scan(a.lng, a.segPtr, a.n_seg, blockIdx.x);
         return;
     }
     const int gpc = blockDim.x / LPR;
     const int g = threadIdx.x / LPR;
     const int gl = threadIdx.x % LPR;
-    const int64_t seg = (int64_t)(blockIdx.x - a.long_ctas) * gpc + g;
+    const int64_t seg = (int64_t)(blockIdx.x - a.lng.scan_ctas) * gpc + g;
     // Lanes of dead groups run along with empty ranges: the shuffles below are full-warp.
     bool live = seg < a.n_seg;
     int lb = 0, hb = 0;
@@ -322,7 +275,7 @@ __global__ void __launch_bounds__(256) agnn_fused_kernel(const AgnnArgs a)
             const int next = seg + 1 < a.n_seg ? __ldg(a.target_row + seg + 1) : -1;
             row = me;
             single = (prev != me) && (next != me);
-        } else if (hb - lb > a.long_row) {
+        } else if (a.lng.totals && hb - lb > PSPMM_LONG_ROW) {  // agnn_long_kernel takes it
             live = false;
             hb = lb;
         }
@@ -330,12 +283,16 @@ __global__ void __launch_bounds__(256) agnn_fused_kernel(const AgnnArgs a)
     FVec<VW> av[CF];
     bool act[CF];
     int voff[CF];
-    AgnnState<CF, VW> st;
-    agnn_load_row<LPR, CF, VW>(a, row, live, gl, av, act, voff, st);
+    AgnnState<CF, VW, COL> st;
+    st.beta = a.beta_dev ? __ldg(a.beta_dev) : a.beta;
+    st.t = 0.f;
+    agnn_load_row<LPR, CF, VW, COL>(a, row, live, gl, av, act, voff, st);
     int maxlen = hb - lb;
     if constexpr (LPR < 32)
         maxlen = __reduce_max_sync(PSPMM_FULL_MASK, maxlen);
-    agnn_entries<LPR, CF, BS, VW, SEP>(a, av, act, voff, lb, hb, maxlen, gl, st);
+    agnn_entries<LPR, CF, BS, VW, SEP, COL>(a, av, act, voff, lb, hb, maxlen, gl, st);
+    if constexpr (COL)
+        cta_sum_to(a.col_sums + (blockIdx.x - a.lng.scan_ctas), (double)st.t);
     if (!live)
         return;
     if (single) {
@@ -361,6 +318,155 @@ __global__ void __launch_bounds__(256) agnn_fused_kernel(const AgnnArgs a)
             if (act[cf])
                 st_vec<VW>(ps + 4 + voff[cf], st.acc[cf]);
     }
+}
+
+// The long rows of an unsplit layout (long_rows.cuh): one lane group walks a row's batches one after the
+// other, so a hub row of 8 K entries held a 900 K-entry graph at dim 32 for 0.8 ms of a 20 us pass.
+// The entries of a share are dealt to the lane groups in equal spans; a group's states (maximum, sum,
+// accumulator) at the ends of its span and the shares' states of a row meet in shared memory and in
+// scratch as the pieces of a split row do.
+template <int LPR, int CF, int BS, int VW, bool SEP, bool COL>
+__global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long_kernel(const AgnnArgs a)
+{
+    constexpr int G = 256 / LPR;
+    constexpr int STEP = 64;  // entries per group between two looks at the row ends of a warp
+    extern __shared__ float parts[];  // [G][first or last piece][max, sum, dim_pad columns]
+    __shared__ LongShare::Shared sh;
+    const int pitch = a.dim_pad + 2;
+    const int g = threadIdx.x / LPR, gl = threadIdx.x % LPR;
+    const int share = blockIdx.x;
+    pdl_launch_dependents();
+    pdl_wait();
+    double t_sum = 0.0;
+    LongShare job;
+    const bool any = job.begin(a.lng, sh, share);
+    const int64_t stride = 4 + a.dim_pad;
+    while (any && job.look(sh, a.segPtr, a.n_seg)) {
+        const int total = job.total;
+        if (total == 0)
+            continue;
+        const int span = (total + G - 1) / G;
+        const int start = g * span;
+        const int stop = start + span < total ? start + span : total;
+        int p = start;
+        int i = p < stop ? job.row_of(sh, p) : 0;
+        FVec<VW> av[CF];
+        bool act[CF];
+        int voff[CF];
+        AgnnState<CF, VW, COL> st;
+        st.beta = a.beta_dev ? __ldg(a.beta_dev) : a.beta;
+        st.t = 0.f;
+        agnn_load_row<LPR, CF, VW, COL>(a, sh.row[i], p < stop, gl, av, act, voff, st);
+        bool from_row_start = p < stop && p == job.off(sh, i);
+        while (__any_sync(PSPMM_FULL_MASK, p < stop)) {
+            int lb = 0, count = 0, row_end = 0;
+            if (p < stop) {
+                row_end = job.off(sh, i + 1);
+                const int row_stop = row_end < stop ? row_end : stop;
+                count = row_stop - p < STEP ? row_stop - p : STEP;
+                lb = sh.lo[i] - job.off(sh, i) + p;
+            }
+            const int longest = LPR < 32 ? __reduce_max_sync(PSPMM_FULL_MASK, count) : count;
+            agnn_entries<LPR, CF, BS, VW, SEP, COL>(a, av, act, voff, lb, lb + count, longest, gl, st);
+            if (count == 0)
+                continue;
+            p += count;
+            if (p != stop && p != row_end)
+                continue;
+            if constexpr (COL) {
+                t_sum += (double)st.t;
+                st.t = 0.f;
+            }
+            // a piece is complete: all of the row in this share, or the first or last piece of the span
+            int s0, s1;
+            job.shares_of(sh, i, s0, s1);
+            if (from_row_start && p == row_end && s0 == s1) {
+                const float inv = a.softmax ? (st.l > 0.f ? 1.f / st.l : 0.f) : 1.f;
+                float *orow = a.out + (int64_t)sh.row[i] * a.ldOut;
+#pragma unroll
+                for (int cf = 0; cf < CF; ++cf)
+                    if (act[cf]) {
+                        float v[VW];
+#pragma unroll
+                        for (int j = 0; j < VW; ++j)
+                            v[j] = st.acc[cf][j] * inv;
+                        st_stream_vec<VW>(orow + voff[cf], v);
+                    }
+            } else {
+                float *mine = parts + (g * 2 + (job.off(sh, i) <= start ? 0 : 1)) * pitch;
+                if (gl == 0) {
+                    mine[0] = st.m;
+                    mine[1] = st.l;
+                }
+#pragma unroll
+                for (int cf = 0; cf < CF; ++cf)
+                    if (act[cf]) {
+#pragma unroll
+                        for (int j = 0; j < VW; ++j)
+                            mine[2 + voff[cf] + j] = st.acc[cf][j];
+                    }
+            }
+            ++i;
+            from_row_start = true;
+            agnn_load_row<LPR, CF, VW, COL>(a, p < stop ? sh.row[i] : 0, p < stop, gl, av, act, voff, st);
+        }
+        __syncthreads();
+        // Rows that several groups or shares hold: their pieces of this share, in order.
+        const int row0 = sh.edge[0], rows = sh.edge[1] - row0 + 1;
+        const int each = a.dim + 1;  // (column -1 is the sum of the weights)
+        for (int t = threadIdx.x; t < rows * each; t += 256) {
+            const int i2 = row0 + t / each, j = t % each - 1;
+            const int off0 = job.off(sh, i2);
+            const int g0 = off0 / span, g1 = (job.off(sh, i2 + 1) - 1) / span;
+            int s0, s1;
+            job.shares_of(sh, i2, s0, s1);
+            if (g0 == g1 && s0 == s1)
+                continue;
+            float M = -CUDART_INF_F, sum = 0.f, l = 0.f;
+            for (int q = g0; q <= g1; ++q)
+                M = fmaxf(M, parts[(q * 2 + (off0 <= q * span ? 0 : 1)) * pitch]);
+            for (int q = g0; q <= g1; ++q) {
+                const float *ps = parts + (q * 2 + (off0 <= q * span ? 0 : 1)) * pitch;
+                const float w = !a.softmax ? 1.f : (ps[0] > -CUDART_INF_F ? expf(ps[0] - M) : 0.f);
+                sum = fmaf(w, ps[2 + j], sum);
+                l = fmaf(w, ps[1], l);
+            }
+            if (s0 != s1) {
+                float *out = a.lng.partials + LongShare::slot(share, s0) * stride;
+                if (j < 0) {
+                    out[0] = M;
+                    out[1] = sum;
+                } else {
+                    out[4 + j] = sum;
+                }
+            } else if (j >= 0) {
+                a.out[(int64_t)sh.row[i2] * a.ldOut + j] = !a.softmax ? sum : (l > 0.f ? sum / l : 0.f);
+            }
+        }
+        job.arrive(a.lng, sh, 0, 1);
+        for (int q = 0; q < 2; ++q) {
+            if (!sh.last[q])
+                continue;
+            int s0, s1;
+            job.shares_of(sh, sh.edge[q], s0, s1);
+            for (int j = threadIdx.x; j < a.dim; j += 256) {
+                float M = -CUDART_INF_F, sum = 0.f, l = 0.f;
+                for (int c = s0; c <= s1; ++c)
+                    M = fmaxf(M, __ldcg(a.lng.partials + LongShare::slot(c, s0) * stride));
+                for (int c = s0; c <= s1; ++c) {
+                    const float *ps = a.lng.partials + LongShare::slot(c, s0) * stride;
+                    const float m = __ldcg(ps);
+                    const float w = !a.softmax ? 1.f : (m > -CUDART_INF_F ? expf(m - M) : 0.f);
+                    sum = fmaf(w, __ldcg(ps + 4 + j), sum);
+                    l = fmaf(w, __ldcg(ps + 1), l);
+                }
+                a.out[(int64_t)sh.row[sh.edge[q]] * a.ldOut + j] = !a.softmax ? sum : (l > 0.f ? sum / l : 0.f);
+            }
+        }
+        __syncthreads();
+    }
+    if constexpr (COL)
+        cta_sum_to(a.col_sums + a.n_col_sums - a.lng.shares + share, t_sum);
 }
 
 // Merges the `count` pieces of one row; slot(t) is where piece t lies.  All `warps` warps of a team
@@ -500,45 +606,15 @@ __global__ void __launch_bounds__(256) agnn_combine_kernel(const AgnnArgs a)
     }
 }
 
-__global__ void __launch_bounds__(256) agnn_combine_long_kernel(const AgnnArgs a)
-{
-    __shared__ float red[8 * 257];
-    __shared__ int list[MERGE_SPAN];
-    __shared__ int n_list;
-    if (threadIdx.x == 0)
-        n_list = 0;
-    __syncthreads();
-    const int64_t r0 = (int64_t)blockIdx.x * MERGE_SPAN + threadIdx.x;
-    if (threadIdx.x < MERGE_SPAN && r0 < a.n_seg && __ldg(a.segPtr + r0 + 1) - __ldg(a.segPtr + r0) > a.long_row)
-        list[atomicAdd(&n_list, 1)] = (int)r0;
-    __syncthreads();
-    pdl_wait();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n = n_list;
-    const int64_t begin = __ldg(a.segPtr);
-    for (int pass = 0; pass < 2; ++pass) {
-        // first the rows a warp can merge, then the long ones
-        for (int i = pass ? 0 : warp; i < n; i += pass ? 1 : 8) {
-            const int64_t row = list[i];
-            const int64_t rb = __ldg(a.segPtr + row) - begin, re = __ldg(a.segPtr + row + 1) - begin;
-            const int64_t c0 = rb / a.long_range;
-            const int64_t count = (re - 1) / a.long_range - c0 + 1;
-            if ((count > MERGE_WARP) != (pass == 1))
-                continue;
-            const auto slot = [&](int64_t t) {
-                return t == 0 ? long_piece_slot(a, rb, true) : long_piece_slot(a, (c0 + t) * a.long_range, false);
-            };
-            merge_pieces(a, row, count, slot, pass ? warp : 0, pass ? 8 : 1, lane, pass ? red : nullptr);
-        }
-    }
-}
-
-template <int LPR, int CF, int BS, int VW, bool SEP = false>
+template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false>
 void launch_fused(const AgnnArgs &a, cudaStream_t st)
 {
     const int gpc = 256 / LPR;
-    const int64_t gx = (a.n_seg + gpc - 1) / gpc + a.long_ctas;
-    agnn_fused_kernel<LPR, CF, BS, VW, SEP><<<(unsigned)gx, 256, a.long_ctas ? 8 * (a.dim_pad + 2) * 4 : 0, st>>>(a);
+    const int64_t gx = (a.n_seg + gpc - 1) / gpc + a.lng.scan_ctas;
+    agnn_fused_kernel<LPR, CF, BS, VW, SEP, COL><<<(unsigned)gx, 256, 0, st>>>(a);
+    if (a.lng.totals)
+        launch_dependent(agnn_long_kernel<LPR, CF, BS, VW, SEP, COL>, dim3((unsigned)a.lng.shares), 256,
+                         gpc * 2 * (a.dim_pad + 2) * 4, st, a);
 }
 
 }  // namespace
@@ -552,16 +628,26 @@ extern "C" int pspmm_agnn_scratch_bytes(int64_t n_seg, int32_t dim, size_t *byte
     return PSPMM_OK;
 }
 
-// Entries above which a row of an unsplit layout is cut, and the bytes its pieces may need.
-static int agnn_long_row(int64_t nnz) { return pspmm_long_row_threshold(nnz); }
-
-extern "C" int pspmm_agnn_long_scratch_bytes(int64_t nnz, int32_t dim, size_t *bytes)
+// Long rows' shares: two CTAs of agnn_long_kernel per SM.
+static void agnn_long_layout(LongArgs *a, int64_t n_rows, int64_t nnz)
 {
-    if (nnz < 0 || dim <= 0 || !bytes)
+    long_layout(a, n_rows, nnz, pspmm_sm_count(), 2, 1);
+}
+static size_t agnn_long_bytes(const LongArgs &a, int32_t dim)
+{
+    return long_head_bytes(a) + (size_t)a.shares * 2 * (4 + (dim + 3) / 4 * 4) * sizeof(float);
+}
+
+extern "C" int pspmm_agnn_long_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim, size_t *bytes)
+{
+    if (n_rows < 0 || nnz < 0 || dim <= 0 || !bytes)
         return PSPMM_E_ARG;
-    const int t = agnn_long_row(nnz);
-    const int64_t slots = t == INT32_MAX ? 0 : 2 * ((nnz + t - 1) / t);
-    *bytes = (size_t)slots * (size_t)(4 + (dim + 3) / 4 * 4) * sizeof(float);
+    *bytes = 0;
+    if (nnz > PSPMM_LONG_ROW && n_rows > 0) {
+        LongArgs a;
+        agnn_long_layout(&a, n_rows, nnz);
+        *bytes = agnn_long_bytes(a, dim);
+    }
     return PSPMM_OK;
 }
 
@@ -577,12 +663,23 @@ extern "C" int pspmm_agnn_fused_csr(const int32_t *rowPtr, const int32_t *colIdx
                                       scratch, scratch_bytes, stream);
 }
 
-extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *A,
-                                          const float *B, const float *V, float *out, int64_t n_rows, int64_t nnz,
-                                          int32_t dim, int64_t ldA, int64_t ldB, int64_t ldV, int64_t ldOut,
-                                          float beta, int32_t softmax, int32_t vec_width, int32_t lanes_per_row,
-                                          int32_t batch, const int32_t *rowPtr_split, const int32_t *target_row,
-                                          int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream)
+// Partial sums of the column-weighted scores: a CTA of 4 lanes per segment at the least, and the shares.
+static size_t agnn_sums_bytes(int64_t n_seg)
+{
+    LongArgs a;
+    long_layout(&a, n_seg, 0, pspmm_sm_count(), 2 * 16, 1);  // (at most 16 waves of shares)
+    return (size_t)((n_seg + 7) / 8 + a.shares + 2) * sizeof(double);
+}
+
+// What the entry points share.  beta_dev: beta on the device (nullptr: the value); col_out: where the sum
+// over all entries of column id * <V_i, V_j> goes (nullptr: it is not formed), with `sums` of
+// agnn_col_sums(...) + 1 doubles for it.
+static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A, const float *B, const float *V,
+                    float *out, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldA, int64_t ldB, int64_t ldV,
+                    int64_t ldOut, float beta, const float *beta_dev, int32_t softmax, int32_t vec_width,
+                    int32_t lanes_per_row, int32_t batch, const int32_t *rowPtr_split, const int32_t *target_row,
+                    int64_t n_seg, void *scratch, size_t scratch_bytes, float *col_out, double *sums, size_t sums_bytes,
+                    void *stream)
 {
     if (n_rows < 0 || nnz < 0 || dim <= 0)
         return PSPMM_E_ARG;
@@ -594,7 +691,7 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
     if (n_rows >= INT32_MAX || nnz > INT32_MAX)
         return PSPMM_E_RANGE;
     const bool split = target_row != nullptr || rowPtr_split != nullptr;
-    if (split && (!rowPtr_split || !target_row || n_seg < 0 || n_seg >= INT32_MAX))
+    if (split && (!rowPtr_split || (n_seg > 0 && !target_row) || n_seg < 0 || n_seg >= INT32_MAX))
         return PSPMM_E_ARG;
     if (!split && !rowPtr)
         return PSPMM_E_ARG;
@@ -611,6 +708,8 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
         ((uintptr_t)A) % 16 != 0 || ((uintptr_t)B) % 16 != 0 || ((uintptr_t)out) % 16 != 0)
         return PSPMM_E_UNSUPPORTED;
     cudaStream_t st = (cudaStream_t)stream;
+    if (col_out && (n_rows == 0 || (split && n_seg == 0)))
+        PSPMM_CUDA_TRY(cudaMemsetAsync(col_out, 0, sizeof(float), st));
     if (n_rows == 0)
         return PSPMM_OK;
     AgnnArgs a;
@@ -630,6 +729,10 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
     a.dim = dim;
     a.dim_pad = (dim + 3) / 4 * 4;
     a.beta = beta;
+    a.beta_dev = beta_dev;
+    a.col_sums = sums;
+    a.n_col_sums = 0;
+    a.col_out = col_out;
     a.softmax = softmax ? 1 : 0;
     if (split) {
         const size_t need = (size_t)n_seg * (size_t)(4 + a.dim_pad) * sizeof(float);
@@ -640,17 +743,13 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
         if (n_seg == 0)
             return PSPMM_OK;
     }
-    a.long_row = INT32_MAX;
-    a.long_range = 0;
-    a.long_ctas = 0;
-    if (!split && scratch && ((uintptr_t)scratch) % 16 == 0) {
-        size_t need = 0;
-        pspmm_agnn_long_scratch_bytes(nnz, dim, &need);
-        if (need > 0 && scratch_bytes >= need) {
-            a.long_row = agnn_long_row(nnz);
-            a.long_range = 8 * a.long_row;
-            a.long_ctas = (uint32_t)((nnz + a.long_range - 1) / a.long_range);
-        }
+    a.lng = LongArgs{};
+    if (!split && scratch && ((uintptr_t)scratch) % 16 == 0 && nnz > PSPMM_LONG_ROW) {
+        agnn_long_layout(&a.lng, n_rows, nnz);
+        if (scratch_bytes >= agnn_long_bytes(a.lng, dim))
+            long_place(&a.lng, scratch);
+        else
+            a.lng = LongArgs{};
     }
     // Launch shape: floats per lane per load (VW: 8 = 256-bit loads when the rows are 32-byte
     // aligned, else 4), lanes per row (LPR), slices per lane (CF = ceil(dim / VW / LPR)) and
@@ -694,6 +793,23 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
     if (cf * vw >= 8 && bs > 8)
         bs = 8;
     bool ok = false;
+    // (the column-weighted sum is built for the shapes that the rules above choose)
+    const int64_t sum_ctas = (a.n_seg + 256 / lpr - 1) / (256 / lpr);
+    if (col_out) {
+        a.n_col_sums = (int32_t)(sum_ctas + a.lng.shares);
+        if (!sums || sums_bytes < (size_t)(a.n_col_sums + 1) * sizeof(double))
+            return PSPMM_E_ARG;
+    }
+#define AGNN_CASE_COL(LPR_, CF_, VW_)                                          \
+    if (!ok && sep && col_out && vw == VW_ && lpr == LPR_ && cf == CF_) {      \
+        launch_fused<LPR_, CF_, 4, VW_, true, true>(a, st);                    \
+        ok = true;                                                             \
+    }
+    AGNN_CASE_COL(4, 1, 4) AGNN_CASE_COL(4, 2, 4) AGNN_CASE_COL(8, 2, 4) AGNN_CASE_COL(16, 2, 4) AGNN_CASE_COL(32, 2, 4)
+    AGNN_CASE_COL(4, 1, 8) AGNN_CASE_COL(8, 1, 8) AGNN_CASE_COL(16, 1, 8) AGNN_CASE_COL(32, 1, 8)
+#undef AGNN_CASE_COL
+    if (col_out && !ok)
+        return PSPMM_E_UNSUPPORTED;
 #define AGNN_CASE_SEP(LPR_, CF_, VW_)                                 \
     if (!ok && sep && vw == VW_ && lpr == LPR_ && cf == CF_ && bs == 4) { \
         launch_fused<LPR_, CF_, 4, VW_, true>(a, st);                 \
@@ -725,10 +841,65 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
     if (!ok)
         return PSPMM_E_UNSUPPORTED;
     PSPMM_CUDA_TRY(cudaGetLastError());
-    const unsigned spans = (unsigned)((a.n_seg + MERGE_SPAN - 1) / MERGE_SPAN);
     if (split)
-        PSPMM_CUDA_TRY(launch_dependent(agnn_combine_kernel, dim3(spans), 256, 0, st, a));
-    else if (a.long_ctas)
-        PSPMM_CUDA_TRY(launch_dependent(agnn_combine_long_kernel, dim3(spans), 256, 0, st, a));
+        PSPMM_CUDA_TRY(launch_dependent(agnn_combine_kernel, dim3((unsigned)((a.n_seg + MERGE_SPAN - 1) / MERGE_SPAN)),
+                                        256, 0, st, a));
+    if (col_out)
+        PSPMM_CUDA_TRY(launch_dependent(agnn_col_sum_kernel, dim3(1), 256, 0, st, a));
     return PSPMM_OK;
+}
+
+extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *A,
+                                          const float *B, const float *V, float *out, int64_t n_rows, int64_t nnz,
+                                          int32_t dim, int64_t ldA, int64_t ldB, int64_t ldV, int64_t ldOut,
+                                          float beta, int32_t softmax, int32_t vec_width, int32_t lanes_per_row,
+                                          int32_t batch, const int32_t *rowPtr_split, const int32_t *target_row,
+                                          int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream)
+{
+    return agnn_run(rowPtr, colIdx, A, B, V, out, n_rows, nnz, dim, ldA, ldB, ldV, ldOut, beta, nullptr, softmax,
+                    vec_width, lanes_per_row, batch, rowPtr_split, target_row, n_seg, scratch, scratch_bytes, nullptr,
+                    nullptr, 0, stream);
+}
+
+extern "C" int pspmm_agnn_layer_scratch_bytes(int64_t n_rows, int64_t nnz, int64_t n_seg, int32_t dim, size_t *bytes)
+{
+    if (n_rows < 0 || nnz < 0 || n_seg < 0 || dim <= 0 || !bytes)
+        return PSPMM_E_ARG;
+    size_t own = 0;
+    int rc = n_seg > 0 ? pspmm_agnn_scratch_bytes(n_seg, dim, &own) : pspmm_agnn_long_scratch_bytes(n_rows, nnz, dim, &own);
+    if (rc)
+        return rc;
+    *bytes = (own + 255) / 256 * 256 + agnn_sums_bytes(n_seg > 0 ? n_seg : n_rows);
+    return PSPMM_OK;
+}
+
+extern "C" int pspmm_agnn_layer_forward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, float *out,
+                                        int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX, int64_t ldOut,
+                                        const float *beta, const int32_t *rowPtr_split, const int32_t *target_row,
+                                        int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream)
+{
+    if (!beta)
+        return PSPMM_E_ARG;
+    return agnn_run(rowPtr, colIdx, X, X, X, out, n_rows, nnz, dim, ldX, ldX, ldX, ldOut, 0.f, beta, 0, 0, 0, 0,
+                    rowPtr_split, target_row, n_seg, scratch, scratch_bytes, nullptr, nullptr, 0, stream);
+}
+
+extern "C" int pspmm_agnn_layer_backward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, const float *G,
+                                         float *D, float *d_beta, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX,
+                                         int64_t ldG, int64_t ldD, const float *beta, const int32_t *rowPtr_split,
+                                         const int32_t *target_row, int64_t n_seg, void *scratch, size_t scratch_bytes,
+                                         void *stream)
+{
+    if (!beta || !G)
+        return PSPMM_E_ARG;
+    size_t need = 0;
+    int rc = pspmm_agnn_layer_scratch_bytes(n_rows, nnz, rowPtr_split ? n_seg : 0, dim, &need);
+    if (rc)
+        return rc;
+    if (!scratch || scratch_bytes < need || (uintptr_t)scratch % 16 != 0)
+        return PSPMM_E_ARG;
+    const size_t sums = agnn_sums_bytes(rowPtr_split ? n_seg : n_rows), own = need - sums;
+    return agnn_run(rowPtr, colIdx, X, X, G, D, n_rows, nnz, dim, ldX, ldX, ldG, ldD, 0.f, beta, 0, 0, 0, 4,
+                    rowPtr_split, target_row, n_seg, own ? scratch : nullptr, own, d_beta,
+                    (double *)((char *)scratch + own), sums, stream);
 }

@@ -799,18 +799,6 @@ __global__ void __launch_bounds__(256) reduce_splits_kernel(const ReduceArgs a)
     }
 }
 
-int device_sms()
-{
-    static thread_local int cached_dev = -1, sms = 148;
-    int dev = 0, v = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess && dev != cached_dev &&
-        cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && v > 0) {
-        sms = v;
-        cached_dev = dev;
-    }
-    return sms;
-}
-
 // Tiles and splits of a product.  The persistent CTAs take the items in turn, so a launch lasts
 // (rounds) x (stages per item + start and end of a tile, about 6 stages' time); cutting K evens out the
 // rounds and gives every SM an item, and costs the partial tiles' trip through memory (a stage lasts
@@ -821,7 +809,7 @@ void plan(int64_t M, int64_t N, int64_t K, DenseArgs &a)
     a.n_tiles = (int32_t)((N + BN - 1) / BN);
     const int64_t per = (N + a.n_tiles - 1) / a.n_tiles;
     a.bn = (int32_t)((per + 15) / 16 * 16);
-    const int64_t tiles = (int64_t)a.m_tiles * a.n_tiles, sms = device_sms();
+    const int64_t tiles = (int64_t)a.m_tiles * a.n_tiles, sms = pspmm_sm_count();
     const int64_t stages = (K + BK - 1) / BK;
     a.splits = 1;
     a.k_per_split = (int32_t)(stages * BK);
@@ -848,7 +836,7 @@ void plan(int64_t M, int64_t N, int64_t K, DenseArgs &a)
 // than a few stages (19,717 x 16 x 500: 25 us against 46; 19,717 x 16 x 3: 9.1 against 8.3).
 bool presplit(const DenseArgs &a)
 {
-    const int64_t rounds = ((int64_t)a.m_tiles * a.n_tiles * a.splits + device_sms() - 1) / device_sms();
+    const int64_t rounds = ((int64_t)a.m_tiles * a.n_tiles * a.splits + pspmm_sm_count() - 1) / pspmm_sm_count();
     return a.m_tiles >= 16 && rounds * (a.k_per_split / BK) >= 6;
 }
 
@@ -949,7 +937,7 @@ extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t
     const int64_t items = (int64_t)a.m_tiles * a.n_tiles * a.splits;
     if (items > INT32_MAX - 65536)
         return PSPMM_E_RANGE;
-    const unsigned grid = (unsigned)(items < device_sms() ? items : device_sms());
+    const unsigned grid = (unsigned)(items < pspmm_sm_count() ? items : pspmm_sm_count());
     // A is k-contiguous unless it is read transposed; B's rows are the output's columns.
     cudaError_t e;
     if (transA)

@@ -319,7 +319,7 @@ static float l2_keep_fraction(double operand_bytes)
     return (float)(f < 0.02 ? 0.02 : f);
 }
 
-static int sm_count()
+int pspmm_sm_count()
 {
     static thread_local int cached_dev = -1, sms = 148;
     int dev = 0, v = 0;
@@ -336,7 +336,7 @@ static int sm_count()
 // after the other: below half a resident wave of threads the groups take fewer segments.
 static int small_rows_per_group(int rpg, int64_t n_seg, int lpr)
 {
-    while (rpg > 1 && n_seg / rpg * lpr < (int64_t)sm_count() * 1024)
+    while (rpg > 1 && n_seg / rpg * lpr < (int64_t)pspmm_sm_count() * 1024)
         rpg >>= 1;
     return rpg;
 }
@@ -347,21 +347,9 @@ static int small_rows_per_group(int rpg, int64_t n_seg, int lpr)
 static int long_range(int64_t n_entries, int per_sm)
 {
     int r = 256;
-    while (r < PSPMM_LONG_RANGE_MAX && n_entries / r > (int64_t)sm_count() * per_sm)
+    while (r < PSPMM_LONG_RANGE_MAX && n_entries / r > (int64_t)pspmm_sm_count() * per_sm)
         r *= 2;
     return r;
-}
-
-// Which rows of an unsplit layout the fused aggregation cuts over the GPU: a lane group takes about a
-// microsecond per eight entries, so rows above 1/64 of an SM's share of the entries would outlast
-// the rest; never below 64 (a row's pieces must pay for their reduction) nor above 512 (half the
-// time of the smallest product that needs this many).  INT32_MAX: no row can be that long.
-int pspmm_long_row_threshold(int64_t n_entries)
-{
-    int t = 64;
-    while (t < 512 && (int64_t)t * sm_count() * 64 < n_entries)
-        t *= 2;
-    return n_entries > t ? t : INT32_MAX;
 }
 
 static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t n_seg,
@@ -445,7 +433,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.lng = LongArgs{};
     if (scratch && !target_row && !accumulate && !(cfg && cfg->bucketed) && n_entries > PSPMM_LONG_ROW) {
         const int lanes = pspmm_long_lanes(a.nvec, V);
-        long_layout(&a.lng, n_seg, n_entries, sm_count(), 3, (a.nvec + lanes - 1) / lanes);
+        long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
         if (scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
             long_place(&a.lng, scratch);
         else
@@ -478,7 +466,7 @@ extern "C" int pspmm_spmm_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim
     *bytes = 0;
     if (nnz > PSPMM_LONG_ROW && n_rows > 0) {
         LongArgs a;
-        long_layout(&a, n_rows, nnz, sm_count(), 3, 1);
+        long_layout(&a, n_rows, nnz, pspmm_sm_count(), 3, 1);
         a.n_counters = a.shares + dim / 16 + 1;  // (shares x tiles: one wave, whatever the tiles)
         *bytes = long_head_bytes(a) + (size_t)a.shares * 2 * V * dim * sizeof(float) + 256;
     }

@@ -9,7 +9,6 @@
 #define PSPMM_FULL_MASK 0xffffffffu
 #define PSPMM_MAX_CF 8
 #define PSPMM_RPG_MAX 16  // most consecutive segments one lane group owns
-#define PSPMM_LONG_PER_RANGE 12  // a range of 8 * long_row entries meets at most 9 rows longer than long_row
 #define PSPMM_LONG_RANGE_MAX 8192
 #define PSPMM_LONG_LIST 132  // long rows that such a range can meet (8192 / 65 inside it and two cut), and a few
 #define PSPMM_GAP_MAX 256  // longest run of uncovered rows the SpMM kernel zeroes by itself
@@ -188,7 +187,7 @@ static inline int pspmm_round_cf(int need)
     return 0;
 }
 
-int pspmm_long_row_threshold(int64_t n_entries);
+int pspmm_sm_count();  // of the current device
 // Lanes per row of spmm_long_rows_kernel (its column tiles are that many vectors wide).
 static inline int pspmm_long_lanes(int nvec, int V) { return nvec > 16 ? 32 : (nvec > 8 || V > 1) ? 16 : (nvec > 4 ? 8 : 4); }
 int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm);

@@ -96,7 +96,11 @@ FUSE_AGNN_INFERENCE = True
 # gnn_conv.py:130-180).  Outputs and gradients are the reference's up to fp32 summation order.
 # Set to False to train through the three-kernel composition (AGNNFunction).
 FUSE_AGNN_TRAINING = True
-FUSED_APPLY_VEC_WIDTH = 0  # floats per lane per load in the backward pass: 0 = the library's choice, 4 or 8
+
+
+def _beta(attention_w):
+    """The attention weight as the one float on the device that the fused passes read."""
+    return attention_w.detach().reshape(1).to(torch.float32)
 
 
 def _can_fuse(P, dim):
@@ -145,55 +149,31 @@ class AGNNFusedFunction(torch.autograd.Function):
     """AGNN layer on a CSR / split-CSR operator without edge arrays.
 
     forward   X' = X W,  out_i = sum_j beta <X'_i, X'_j> X'_j                 (one fused pass)
-    backward  D_i = sum_j beta <X'_i, X'_j> G_j   (fused pass, scores recomputed, gradient rows gathered)
+    backward  D_i = sum_j beta <X'_i, X'_j> G_j   (scores recomputed, gradient rows gathered)
               dX = D W^T,  dW = X^T D                                      (gnn_conv.py:157-160)
               d_beta = sum over edges of <G_i, G_j> * colIdx[e]              (gnn_conv.py:163-172: the
-              reference multiplies the score gradient by the column-index column it is handed); here
-              as sum_i <G_i, T_i> with T = P H, H_j = j * G_j, P the pattern with unit values: one
-              SpMM without a value array and a dot product.
+              reference multiplies the score gradient by the column-index column it is handed), summed
+              in the same pass while the gradient row is in registers.
+    The attention weight stays on the device (reading it back made every forward wait for the GPU).
     Like the reference's backward, the edge values are treated as constants with respect to X'."""
 
     @staticmethod
     def forward(ctx, X, weights, attention_w, P, colIdx):
         Xp = ops.dense_mm(X, weights)
-        split = P.target_row is not None
-        beta = float(attention_w.detach().reshape(()))
-        out = ops.agnn_fused(Xp, Xp, P.rowPtr, P.colIdx, beta, softmax=False, target_row=P.target_row,
-                             n_out_rows=Xp.shape[0] if split else None)
-        if not split and out.shape[0] != Xp.shape[0]:  # inputs padded beyond the matrix: zero rows, as the SpMM gives
-            out = torch.cat([out, out.new_zeros(Xp.shape[0] - out.shape[0], out.shape[1])])
-        ctx.save_for_backward(X, weights, Xp)
-        ctx.P, ctx.beta, ctx.colIdx = P, beta, colIdx
+        beta = _beta(attention_w).clone()  # (the backward uses the value of this forward)
+        out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, beta, P.target_row)
+        ctx.save_for_backward(X, weights, Xp, beta)
+        ctx.P = P
         return out
 
     @staticmethod
     def backward(ctx, d_output):
-        X, weights, Xp = ctx.saved_tensors
-        P, beta = ctx.P, ctx.beta
-        G = d_output.contiguous()
-        split = P.target_row is not None
-        n_out = G.shape[0] if split else None
-
-        def apply(A, B, V, b):
-            o = ops.agnn_fused(A, B, P.rowPtr, P.colIdx, b, softmax=False, target_row=P.target_row,
-                               n_out_rows=n_out, V=V, vec_width=FUSED_APPLY_VEC_WIDTH)
-            if o.shape[0] != G.shape[0]:
-                o = torch.cat([o, o.new_zeros(G.shape[0] - o.shape[0], o.shape[1])])
-            return o
-
-        D = apply(Xp, Xp, G, beta)
-        d_input = ops.dense_mm(D, weights, transB=True)
-        d_weights = ops.dense_mm(X, D, transA=True)
-        d_att = None
-        if ctx.needs_input_grad[2]:
-            # The reference weights every edge's score gradient by the float value of the column-index
-            # column it is handed, i.e. by the edge's column id j: sum_e <G_i, G_j> j = sum_i <G_i, (P H)_i>
-            # with H_j = j G_j and P the pattern with unit values.
-            H = G * torch.arange(G.shape[0], device=G.device, dtype=G.dtype)[:, None]
-            rows = G.shape[0] if split else P.rowPtr.shape[0] - 1
-            T = torch.empty(rows, G.shape[1], device=G.device, dtype=G.dtype)
-            ops.spmm_into(T, H, P.rowPtr, P.colIdx, None, target_row=P.target_row, n_out_rows=rows)
-            d_att = (G[:rows].double() * T.double()).sum().to(G.dtype).reshape(1, 1)
+        X, weights, Xp, beta = ctx.saved_tensors
+        P = ctx.P
+        D, d_att = ops.agnn_layer_backward(Xp, d_output.contiguous(), P.rowPtr, P.colIdx, beta, P.target_row,
+                                           beta_grad=ctx.needs_input_grad[2])
+        d_input = ops.dense_mm(D, weights, transB=True) if ctx.needs_input_grad[0] else None
+        d_weights = ops.dense_mm(X, D, transA=True) if ctx.needs_input_grad[1] else None
         return d_input, d_weights, d_att, None, None
 
 
@@ -231,16 +211,6 @@ class AGNNConv(_Conv):
     def __init__(self, input_dim, output_dim):
         super().__init__(input_dim, output_dim)
         self.attention_w = torch.nn.Parameter(torch.randn(1, n_heads))
-        self._beta_cache = (None, 0.0)
-
-    def _beta(self):
-        """attention_w as a host float for the fused kernel's by-value argument, read back from the
-        device only when the parameter has changed since the last call (in-place updates bump the
-        tensor's version counter)."""
-        key = (self.attention_w.data_ptr(), self.attention_w._version)
-        if self._beta_cache[0] != key:
-            self._beta_cache = (key, float(self.attention_w.detach().reshape(())))
-        return self._beta_cache[1]
 
     def forward(self, X, spmm_dict, colIdx):
         P = self._operator(spmm_dict)
@@ -248,9 +218,8 @@ class AGNNConv(_Conv):
             # No gradient will be asked for: scores, scaling and aggregation in one kernel, without
             # the per-edge array the backward would need.
             Xp = ops.dense_mm(X, self.weights)
-            split = P.target_row is not None
-            return ops.agnn_fused(Xp, Xp, P.rowPtr, P.colIdx, self._beta(), softmax=False,
-                                  target_row=P.target_row, n_out_rows=P.mtx_nodes if split else None)
+            out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, _beta(self.attention_w), P.target_row)
+            return out[: P.mtx_nodes if P.target_row is not None else P.rowPtr.shape[0] - 1]
         if (FUSE_AGNN_TRAINING and torch.is_grad_enabled() and _can_fuse(P, self.weights.size(1))
                 and _is_operator_colidx(P, colIdx)):
             return AGNNFusedFunction.apply(X, self.weights, self.attention_w, P, colIdx)

@@ -633,7 +633,7 @@ def agnn_fused(A, B, rowPtr, colIdx, beta=1.0, softmax=True, target_row=None, n_
     if split:
         scratch, sbytes = _scratch("pspmm_agnn_scratch_bytes", (n_seg, dim), A.device)
     else:
-        scratch, sbytes = _scratch("pspmm_agnn_long_scratch_bytes", (colIdx.shape[0], dim), A.device)
+        scratch, sbytes = _scratch("pspmm_agnn_long_scratch_bytes", (n_seg, colIdx.shape[0], dim), A.device)
     seg_ptr = _ptr(rowPtr)
     tail = (float(beta), 1 if softmax else 0, int(vec_width), int(lanes_per_row), int(batch),
             seg_ptr if split else null, _ptr(target_row) if split else null, n_seg if split else 0,
@@ -647,6 +647,57 @@ def agnn_fused(A, B, rowPtr, colIdx, beta=1.0, softmax=True, target_row=None, n_
                                                _ptr(out), n_out_rows, colIdx.shape[0], dim, A.stride(0), B.stride(0),
                                                ldV, out.stride(0), *tail))
     return out
+
+
+def _agnn_layer(X, rowPtr, colIdx, beta, target_row):
+    """Checks of the layer passes; (output with rows beyond the pattern zeroed, sizes and pointers)."""
+    _check_cuda(X, "X", torch.float32, 2)
+    _check_cuda(rowPtr, "rowPtr", torch.int32, 1)
+    _check_cuda(colIdx, "colIdx", torch.int32, 1)
+    _check_cuda(beta, "beta", torch.float32)
+    n, dim = X.shape
+    n_seg = rowPtr.shape[0] - 1
+    out = torch.empty_like(X)
+    if target_row is None:
+        if n < n_seg:
+            raise RuntimeError("X has fewer rows than the pattern")
+        if n > n_seg:
+            out[n_seg:].zero_()
+        sizes = (n_seg, colIdx.shape[0], 0, dim)
+        rows, plain, split, target, n_split = n_seg, rowPtr.data_ptr(), None, None, 0
+    else:
+        _check_cuda(target_row, "target_row", torch.int32, 1)
+        sizes = (n, colIdx.shape[0], n_seg, dim)
+        rows, plain, split, target, n_split = n, None, rowPtr.data_ptr(), target_row.data_ptr(), n_seg
+    scratch, nbytes = _scratch("pspmm_agnn_layer_scratch_bytes", sizes, X.device)
+    tail = (beta.data_ptr(), split, target, n_split, _ptr(scratch), nbytes, _stream())
+    return out, plain, rows, colIdx.shape[0], dim, tail, scratch
+
+
+def agnn_layer_forward(X, rowPtr, colIdx, beta, target_row=None):
+    """out_i = sum_j beta <X_i, X_j> X_j over the pattern, ``beta`` one float on the device
+    (``pspmm_agnn_layer_forward``); one output row per row of ``X``."""
+    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta, target_row)
+    rc = lib().pspmm_agnn_layer_forward(plain, colIdx.data_ptr(), X.data_ptr(), out.data_ptr(), rows, nnz, dim, X.stride(0),
+                                        out.stride(0), *tail)
+    if rc:
+        check(rc)
+    return out
+
+
+def agnn_layer_backward(X, G, rowPtr, colIdx, beta, target_row=None, beta_grad=True):
+    """D_i = sum_j beta <X_i, X_j> G_j and, in the same pass, sum over the entries of j * <G_i, G_j>
+    (the attention weight's gradient, gnn_conv.py:163-172; None without ``beta_grad``)."""
+    _check_cuda(G, "G", torch.float32, 2)
+    if G.shape != X.shape:
+        raise RuntimeError("G must have the shape of X")
+    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta, target_row)
+    d_beta = torch.empty((1, 1), dtype=torch.float32, device=X.device) if beta_grad else None
+    rc = lib().pspmm_agnn_layer_backward(plain, colIdx.data_ptr(), X.data_ptr(), G.data_ptr(), out.data_ptr(), _ptr(d_beta),
+                                         rows, nnz, dim, X.stride(0), G.stride(0), out.stride(0), *tail)
+    if rc:
+        check(rc)
+    return out, d_beta
 
 
 def pull_rows(dst, sources, first, rows, rotate=0, ctas=0, bulk=False):

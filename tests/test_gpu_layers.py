@@ -175,3 +175,34 @@ def test_agnn_layer_trains_without_edge_arrays(split):
     _close(out, out_u)
     _close(gx, gx_u)
     _close(gw, gw_u)
+
+
+@pytest.mark.parametrize("dim", [4, 20, 64, 132, 256])
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("pairs", [0, 40, 20000])
+def test_agnn_layer_passes_match_dense_algebra(dim, split, pairs):
+    """The forward and the backward pass (product and column-weighted score sum) of the layer, on empty,
+    sparse and long-row patterns, with inputs that have more rows than the pattern."""
+    from paramspmm_ae_b200 import ops, synth
+    dev = torch.device("cuda:0")
+    n = 301
+    g = synth.powerlaw_graph(n, pairs, seed=4, self_loops=pairs != 0)
+    rp, ci = g.rowPtr.to(dev), g.colIdx.to(dev)
+    rows = torch.repeat_interleave(torch.arange(n, device=dev), (rp[1:] - rp[:-1]).long())
+    mask = torch.zeros(n, n, dtype=torch.float64, device=dev)
+    mask[rows, ci.long()] = 1
+    gen = torch.Generator(device=dev).manual_seed(5)
+    X, G = (torch.randn(n + (0 if split else 2), dim, device=dev, generator=gen) / dim ** 0.5 for _ in range(2))
+    beta = torch.tensor([0.7], device=dev)
+    tr = None
+    if split:
+        rp, tr = ops.split_csr_device(rp, 9)
+    S = 0.7 * (X[:n].double() @ X[:n].double().t()) * mask
+    out = ops.agnn_layer_forward(X, rp, ci, beta, tr)
+    _close(out[:n], S @ X[:n].double())
+    D, d_beta = ops.agnn_layer_backward(X, G, rp, ci, beta, tr)
+    _close(D[:n], S @ G[:n].double())
+    terms = (G[:n].double() @ G[:n].double().t()) * mask * torch.arange(n, device=dev).double()
+    assert abs(float(d_beta) - float(terms.sum())) <= 1e-6 * float(terms.abs().sum())
+    assert float(out[n:].abs().sum()) == 0 and float(D[n:].abs().sum()) == 0
+    assert ops.agnn_layer_backward(X, G, rp, ci, beta, tr, beta_grad=False)[1] is None
