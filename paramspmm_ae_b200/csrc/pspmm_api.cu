@@ -97,7 +97,25 @@ static int cf_max_for(int vw, int V)
     return 8;
 }
 
-int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, LaunchShape *out)
+// SpMM without a plan: whether three slices on fewer lanes (2 * lanes < nvec <= 3 * lanes) beat
+// one slice per lane, which leaves up to half of the lanes idle.  On 16-byte loads they do (uniform
+// columns, 2.4 M entries, dim 80: 118 -> 82 us, dim 160: 163 -> 133), except that 9 or 10 vectors idle
+// little (4 lanes: dim 40 107 -> 121).  The segments of skewed split layouts leave the smaller groups of a warp
+// out of step: two segments per group instead of four level that (R-MAT, 6.5 entries per row, dim 72:
+// 216 us before, 241 with four, 208 with two), but not for narrower loads, which have more groups per
+// byte (R-MAT, dim 23: 133 -> 145, dim 46: 158 -> 175), nor do 33..48 vectors of 8 bytes gain.  Blocks need
+// their registers for the second row and gain only with the narrower loads.
+static bool narrow_group(int nvec, int vw, int V, bool split)
+{
+    const bool between = (nvec > 8 && nvec <= 12) || (nvec > 16 && nvec <= 24) || (nvec > 32 && nvec <= 48);
+    if (V != 1)
+        return between && V == 2 && vw < 4;
+    if (vw == 4)
+        return between && nvec > 10;
+    return between && !split && (vw == 1 ? nvec > 16 : nvec <= 24);
+}
+
+int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out)
 {
     LaunchShape s;
     s.vw = vw_max;
@@ -105,21 +123,19 @@ int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, La
         s.vw = cfg->vec_width;
     const int nvec = dim / s.vw;
     const int lmin = lpr_min_for(s.vw, V), cmax = cf_max_for(s.vw, V);
-    int lpr;
+    int lpr, rpg = 4;
     if (cfg && cfg->lanes_per_row != 0) {
         lpr = cfg->lanes_per_row;
     } else {
-        // One slice per lane, except where three slices of a quarter as many lanes leave fewer of them
-        // idle: widths of 9..12, 17..24 and 33..48 vectors (dim 80: 76 against 97 us on a power-law
-        // graph of 2.4 M entries, 174 against 203 on uniform columns; dim 160: 127 against 138).  Blocks
-        // need their registers for the second row and gain only with scalar and 8-byte loads.
         lpr = 1;
         while (lpr < nvec && lpr < 32)
             lpr <<= 1;
-        if (V == 1 || (V == 2 && s.vw < 4))
-            for (int p = 4; p <= 16; p <<= 1)
-                if (nvec > 2 * p && nvec <= 3 * p)
-                    lpr = p;
+        if (use != SHAPE_SDDMM && narrow_group(nvec, s.vw, V, use == SHAPE_SPLIT)) {
+            while (2 * lpr >= nvec)
+                lpr >>= 1;
+            if (V == 1 && (use == SHAPE_SPLIT || s.vw == 2))
+                rpg = 2;
+        }
     }
     if (lpr < lmin)
         lpr = lmin;
@@ -137,10 +153,10 @@ int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, La
         s.cf = pspmm_round_cf(need);
         s.tiles = 1;
     }
-    // (two warps' groups more or less per CTA: 128 threads are 0 - 5 % faster where nobody has measured,
-    // a plan with a shape of its own was measured with 256)
+    // (128 threads are up to 12 % faster than 256 in all SpMM shapes that the rules above choose; plans with a
+    // shape of their own were measured with 256)
     s.threads = (cfg && cfg->cta_threads) ? cfg->cta_threads : (cfg && cfg->lanes_per_row ? 256 : 128);
-    s.rpg = (cfg && cfg->rows_per_group) ? cfg->rows_per_group : 4;
+    s.rpg = (cfg && cfg->rows_per_group) ? cfg->rows_per_group : rpg;
     s.mlp = (cfg && cfg->gather_batch) ? cfg->gather_batch : 8;
     *out = s;
     return PSPMM_OK;
@@ -155,7 +171,7 @@ extern "C" int pspmm_resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64
     if (rc)
         return rc;
     LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, &s);
+    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, SHAPE_ROWS, &s);
     cfg->lanes_per_row = s.lpr;
     cfg->vec_width = s.vw;
     cfg->cta_threads = s.threads;
@@ -331,6 +347,20 @@ int pspmm_sm_count()
     return sms;
 }
 
+// Segments per lane group by what a group has to do.  A group of a half or whole warp with few entries per
+// segment waits for its pointers and columns most of the time: eight segments share them (128 columns:
+// band of 8 121 -> 105 us, power law of 8 205 -> 182, R-MAT of 6.5 216 -> 204; 64 columns, band of 8:
+// 68 -> 62).  The groups of 4 lanes are eight to a warp, and the longest holds the others up: two
+// segments each (16 columns: power law of 8 77 -> 62, R-MAT of 16 82 -> 71, band of 8 29 -> 27, but
+// band of 4 29 -> 33).
+static int rows_per_group_for(const LaunchShape &s, int dim, int64_t n_seg, int64_t n_entries)
+{
+    const bool full = 2 * s.lpr * s.cf * s.vw > dim && s.cf != 3;  // (not the three-slice groups)
+    if ((s.lpr == 32 && full && n_entries < 20 * n_seg) || (s.lpr == 16 && full && n_entries < 10 * n_seg))
+        return 8;
+    return s.lpr <= 4 && n_entries >= 6 * n_seg ? 2 : 4;
+}
+
 // Segments one lane group owns.  Several share the pointer and entry staging, but a small matrix then
 // leaves SMs without a warp (19,717 rows at dim 16: 77 CTAs for 148 SMs) and walks its segments one
 // after the other: below half a resident wave of threads the groups take fewer segments.
@@ -387,7 +417,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
         return PSPMM_OK;
     }
     LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, &s);
+    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row ? SHAPE_SPLIT : SHAPE_ROWS, &s);
     if (accumulate) {
         // built for 128-bit loads on CSR / split CSR with at least four lanes per row
         if (s.vw != 4 || V != 1)
@@ -396,13 +426,16 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             LaunchShape t = s;
             pspmm_cfg wide = *cfg;
             wide.lanes_per_row = 4;
-            pspmm_resolve_shape(&wide, dim, 4, V, &t);
+            pspmm_resolve_shape(&wide, dim, 4, V, SHAPE_ROWS, &t);
             s = t;
         }
     }
 
-    if (!cfg || cfg->rows_per_group == 0)
+    if (!cfg || cfg->rows_per_group == 0) {
+        if (V == 1 && s.rpg == 4 && (!cfg || cfg->lanes_per_row == 0))
+            s.rpg = rows_per_group_for(s, dim, n_seg, n_entries);
         s.rpg = small_rows_per_group(s.rpg, n_seg, s.lpr);
+    }
 
     const bool bucketed = target_row && cfg && cfg->bucketed;
     if (target_row && !accumulate) {
@@ -569,7 +602,7 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     const int nvec_max = dim / vw_max;
     if (V == 1 && (narrow.lanes_per_row == 0 || narrow.lanes_per_row > 16) && nvec_max > 8)
         narrow.lanes_per_row = vw_max < 4 && nvec_max <= 32 ? 8 : 16;
-    pspmm_resolve_shape(&narrow, dim, vw_max, V, &s);
+    pspmm_resolve_shape(&narrow, dim, vw_max, V, SHAPE_SDDMM, &s);
     if (V == 1 && s.lpr > 16) {
         s.lpr = 16;
         s.cf = 8;

@@ -191,5 +191,6 @@ int pspmm_sm_count();  // of the current device
 // Lanes per row of spmm_long_rows_kernel (its column tiles are that many vectors wide).
 static inline int pspmm_long_lanes(int nvec, int V) { return nvec > 16 ? 32 : (nvec > 8 || V > 1) ? 16 : (nvec > 4 ? 8 : 4); }
 int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm);
-int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, LaunchShape *out);
+enum ShapeUse { SHAPE_ROWS, SHAPE_SPLIT, SHAPE_SDDMM };
+int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out);
 int pspmm_vw_max(int32_t dim, int64_t ld0, int64_t ld1, const void *p0, const void *p1);
