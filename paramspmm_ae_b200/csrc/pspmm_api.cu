@@ -153,9 +153,10 @@ int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, Sh
         s.cf = pspmm_round_cf(need);
         s.tiles = 1;
     }
-    // (128 threads are up to 12 % faster than 256 in all SpMM shapes that the rules above choose; plans with a
-    // shape of their own were measured with 256)
-    s.threads = (cfg && cfg->cta_threads) ? cfg->cta_threads : (cfg && cfg->lanes_per_row ? 256 : 128);
+    // (128 threads are up to 12 % faster than 256 in the SpMM shapes that the rules above choose, except
+    // blocks with several slices, 3 % slower; plans with a shape of their own were measured with 256)
+    s.threads = (cfg && cfg->cta_threads) ? cfg->cta_threads
+                                          : (cfg && cfg->lanes_per_row) || (V > 1 && s.cf > 1) ? 256 : 128;
     s.rpg = (cfg && cfg->rows_per_group) ? cfg->rows_per_group : rpg;
     s.mlp = (cfg && cfg->gather_batch) ? cfg->gather_batch : 8;
     *out = s;
@@ -361,14 +362,27 @@ static int rows_per_group_for(const LaunchShape &s, int dim, int64_t n_seg, int6
     return s.lpr <= 4 && n_entries >= 6 * n_seg ? 2 : 4;
 }
 
-// Segments one lane group owns.  Several share the pointer and entry staging, but a small matrix then
-// leaves SMs without a warp (19,717 rows at dim 16: 77 CTAs for 148 SMs) and walks its segments one
-// after the other: below half a resident wave of threads the groups take fewer segments.
-static int small_rows_per_group(int rpg, int64_t n_seg, int lpr)
+// Fewer segments per lane group where that ends sooner.  A small matrix leaves SMs without a warp (19,717
+// rows at dim 16: 77 CTAs for 148 SMs), and below a few resident waves the last one counts (12,958
+// block-rows of 21 blocks on 32 lanes: 36 us with four segments in 0.7 waves, 38 with two in 1.4, 35 with
+// one in 2.7).  A wave takes as long as a group's segments and the staging they share, about five entries.
+static int small_rows_per_group(const LaunchShape &s, int V, int64_t n_seg, int64_t n_entries)
 {
-    while (rpg > 1 && n_seg / rpg * lpr < (int64_t)pspmm_sm_count() * 1024)
-        rpg >>= 1;
-    return rpg;
+    const int64_t wave = (int64_t)pspmm_sm_count() * (V == 1 || s.cf > 2 ? 768 : 1024);  // (threads, by registers)
+    const double staging = 5.0 * (double)n_seg / (double)(n_entries > 0 ? n_entries : 1);
+    auto waves = [&](int r) { return ((n_seg + r - 1) / r * s.lpr + wave - 1) / wave; };
+    int best = s.rpg;
+    if (waves(best) > 4)
+        return best;
+    double least = 0.95 * (double)waves(best) * (best + staging);
+    for (int r = best / 2; r >= 1; r /= 2) {
+        const double t = (double)waves(r) * (r + staging);
+        if (t < least) {
+            least = t;
+            best = r;
+        }
+    }
+    return best;
 }
 
 // Entries of the ranges in which a kernel deals out the long rows (PSPMM_LONG_ROW) of an unsplit
@@ -434,7 +448,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     if (!cfg || cfg->rows_per_group == 0) {
         if (V == 1 && s.rpg == 4 && (!cfg || cfg->lanes_per_row == 0))
             s.rpg = rows_per_group_for(s, dim, n_seg, n_entries);
-        s.rpg = small_rows_per_group(s.rpg, n_seg, s.lpr);
+        s.rpg = small_rows_per_group(s, V, n_seg, n_entries);
     }
 
     const bool bucketed = target_row && cfg && cfg->bucketed;
@@ -463,6 +477,10 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.rows_per_group = s.rpg;
     a.bucketed = bucketed ? 1 : 0;
     a.keep_fraction = l2_keep_fraction((double)n_cols * (double)ldB * 4.0);
+    // The product is launched behind its pre-pass as a dependent grid, which saves 2 - 5 us, except where
+    // the pieces of a bucketed plan are long: its first CTAs are the longest, and the early start packs them
+    // on the SMs that the pre-pass leaves free (32 M entries in pieces of 147: 528 us instead of 465).
+    a.dependent = target_row && !accumulate && !(bucketed && n_entries > 64 * n_seg);
     a.lng = LongArgs{};
     if (scratch && !target_row && !accumulate && !(cfg && cfg->bucketed) && n_entries > PSPMM_LONG_ROW) {
         const int lanes = pspmm_long_lanes(a.nvec, V);
@@ -612,7 +630,7 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     if (!cfg || cfg->cta_threads == 0)
         s.threads = 128;  // measured: 128-thread CTAs are 7 % faster than 256 for this kernel
     if (!cfg || cfg->rows_per_group == 0)
-        s.rpg = small_rows_per_group(s.rpg, n_seg, s.lpr);
+        s.rpg = small_rows_per_group(s, V, n_seg, n_entries);
     SddmmArgs a;
     a.segPtr = segPtr;
     a.target_row = target_row;

@@ -136,6 +136,7 @@ struct SpmmArgs {
 // changes with the size of their argument.)
 struct SpmmLongArgs : SpmmArgs {
     LongArgs lng;  // unsplit layouts: how long rows are cut (totals == nullptr: they are not)
+    bool dependent;  // (host) the launch may start while the pre-pass runs
 };
 
 // Flags in target_row of a length-bucketed plan (pspmm_cfg.bucketed): the low 30 bits are the row.

@@ -509,7 +509,7 @@ static inline void spmm_launch_one(const SpmmLongArgs &a, dim3 grid, int threads
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     const std::conditional_t<LONG, SpmmLongArgs, SpmmArgs> &args = a;
-    if (a.target_row && !ACC)
+    if (a.dependent)
         launch_dependent(kern, grid, threads, smem, st, args);  // follows the zeroing pre-pass
     else
         kern<<<grid, threads, smem, st>>>(args);
