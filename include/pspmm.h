@@ -76,10 +76,17 @@ PSPMM_API int pspmm_version(void);
 PSPMM_API const char *pspmm_strerror(int code);
 PSPMM_API const char *pspmm_last_cuda_error(void);
 
-/* Resolve a configuration exactly as the SpMM entry points would (fills the zero fields of
- * *cfg for the given dim / leading dimensions / alignment) without launching anything. */
+/* Resolve a configuration exactly as the SpMM entry points would (fills the zero fields of *cfg) without
+ * launching anything.  pspmm_resolve_spmm takes all that the choice looks at: dim, leading dimensions and
+ * alignment, whether the layout is split, its (block-)rows or pieces and its entries (blocks).  Where
+ * col_tile cuts the product it describes the launch over the first col_tile columns.  Resolving a
+ * resolved configuration changes nothing.  pspmm_resolve_cfg is the same for an unsplit layout of unknown
+ * size: lanes_per_row, vec_width and gather_batch are what a launch takes, cta_threads and
+ * rows_per_group what it starts from before it looks at the sizes. */
 PSPMM_API int pspmm_resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V,
                       const void *B, const void *C);
+PSPMM_API int pspmm_resolve_spmm(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V,
+                      const void *B, const void *C, int32_t split, int64_t n_seg, int64_t n_entries);
 
 /*
  * C[n_rows, dim] = A[n_rows, n_cols] * B[n_cols, dim], A in CSR or in PCSR (row-split CSR).

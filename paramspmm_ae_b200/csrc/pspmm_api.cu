@@ -163,24 +163,6 @@ int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, Sh
     return PSPMM_OK;
 }
 
-extern "C" int pspmm_resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V,
-                                 const void *B, const void *C)
-{
-    if (!cfg || dim <= 0 || V < 1 || V > 3)
-        return PSPMM_E_ARG;
-    int rc = pspmm_validate_cfg(cfg, false);
-    if (rc)
-        return rc;
-    LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, SHAPE_ROWS, &s);
-    cfg->lanes_per_row = s.lpr;
-    cfg->vec_width = s.vw;
-    cfg->cta_threads = s.threads;
-    cfg->rows_per_group = s.rpg;
-    cfg->gather_batch = s.mlp;
-    return PSPMM_OK;
-}
-
 // ----------------------------------------------------------------------------- zero pre-pass
 // For a split layout, before the SpMM kernel runs.  Lane groups of the SpMM kernel own `rpg`
 // consecutive segments each, so group boundaries sit at segment indices that are multiples of
@@ -385,6 +367,84 @@ static int small_rows_per_group(const LaunchShape &s, int V, int64_t n_seg, int6
     return best;
 }
 
+// Columns [off, off + w) of a product that col_tile cuts: the configuration of that launch.
+static pspmm_cfg tile_cfg(const pspmm_cfg &cfg, int32_t w)
+{
+    pspmm_cfg sub = cfg;
+    sub.col_tile = 0;
+    if (sub.lanes_per_row * (sub.vec_width ? sub.vec_width : 4) > w)
+        sub.lanes_per_row = 0;  // let the launch pick the group width for the narrow range
+    return sub;
+}
+
+// The shape of one SpMM launch.  n_seg < 0: the matrix is not known, the rules that look at its size are left out.
+static int spmm_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, bool split, int64_t n_seg, int64_t n_entries,
+                      LaunchShape *out)
+{
+    LaunchShape s;
+    pspmm_resolve_shape(cfg, dim, vw_max, V, split ? SHAPE_SPLIT : SHAPE_ROWS, &s);
+    if (cfg && cfg->accumulate) {
+        // built for 128-bit loads on CSR / split CSR with at least four lanes per row
+        if (s.vw != 4 || V != 1)
+            return PSPMM_E_UNSUPPORTED;
+        if (s.lpr < 4) {
+            pspmm_cfg wide = *cfg;
+            wide.lanes_per_row = 4;
+            pspmm_resolve_shape(&wide, dim, 4, V, SHAPE_ROWS, &s);
+        }
+    }
+    if (n_seg >= 0) {
+        // Rows of neighbouring columns share lines of L1 within a CTA: 256 threads gain 2 - 8 % on bands of 17 and
+        // more entries (28 entries, 96 columns: 86 -> 79 us) and lose up to 3 % on uniform columns.
+        if (V == 1 && s.vw == 4 && !split && n_entries >= 16 * n_seg && !(cfg && (cfg->cta_threads || cfg->lanes_per_row)))
+            s.threads = 256;
+        if (!cfg || cfg->rows_per_group == 0) {
+            if (V == 1 && s.rpg == 4 && (!cfg || cfg->lanes_per_row == 0))
+                s.rpg = rows_per_group_for(s, dim, n_seg, n_entries);
+            s.rpg = small_rows_per_group(s, V, n_seg, n_entries);
+        }
+    }
+    *out = s;
+    return PSPMM_OK;
+}
+
+static int resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V, const void *B, const void *C,
+                       bool split, int64_t n_seg, int64_t n_entries)
+{
+    if (!cfg || dim <= 0 || V < 1 || V > 3)
+        return PSPMM_E_ARG;
+    int rc = pspmm_validate_cfg(cfg, false);
+    if (rc)
+        return rc;
+    LaunchShape s;
+    const bool tiled = cfg->col_tile > 0 && cfg->col_tile < dim;
+    const pspmm_cfg sub = tiled ? tile_cfg(*cfg, cfg->col_tile) : *cfg;
+    rc = spmm_shape(&sub, tiled ? cfg->col_tile : dim, pspmm_vw_max(tiled ? cfg->col_tile : dim, ldB, ldC, B, C), V, split,
+                    n_seg, n_entries, &s);
+    if (rc)
+        return rc;
+    cfg->lanes_per_row = s.lpr;
+    cfg->vec_width = s.vw;
+    cfg->cta_threads = s.threads;
+    cfg->rows_per_group = s.rpg;
+    cfg->gather_batch = s.mlp;
+    return PSPMM_OK;
+}
+
+extern "C" int pspmm_resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V,
+                                 const void *B, const void *C)
+{
+    return resolve_cfg(cfg, dim, ldB, ldC, V, B, C, false, -1, 0);
+}
+
+extern "C" int pspmm_resolve_spmm(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V, const void *B,
+                                  const void *C, int32_t split, int64_t n_seg, int64_t n_entries)
+{
+    if (n_seg < 0 || n_entries < 0)
+        return PSPMM_E_ARG;
+    return resolve_cfg(cfg, dim, ldB, ldC, V, B, C, split != 0, n_seg, n_entries);
+}
+
 // Entries of the ranges in which a kernel deals out the long rows (PSPMM_LONG_ROW) of an unsplit
 // layout.  Finding a range's rows takes two searches, so ranges are long, up to 8192 entries, while
 // there are enough of them to fill the chip several times over.
@@ -419,10 +479,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
         // and a narrow remainder gets a narrow lane group instead of idle lanes in a wide one.
         for (int32_t off = 0; off < dim; off += cfg->col_tile) {
             const int32_t w = dim - off < cfg->col_tile ? dim - off : cfg->col_tile;
-            pspmm_cfg sub = *cfg;
-            sub.col_tile = 0;
-            if (sub.lanes_per_row * (sub.vec_width ? sub.vec_width : 4) > w)
-                sub.lanes_per_row = 0;  // let the launch pick the group width for the narrow range
+            const pspmm_cfg sub = tile_cfg(*cfg, w);
             rc = spmm_launch(segPtr, target_row, n_seg, colIdx, val, V, B + off, C + off, n_out_blk_rows, n_cols,
                              n_entries, w, ldB, ldC, &sub, scratch, scratch_bytes, st);
             if (rc)
@@ -431,30 +488,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
         return PSPMM_OK;
     }
     LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row ? SHAPE_SPLIT : SHAPE_ROWS, &s);
-    if (accumulate) {
-        // built for 128-bit loads on CSR / split CSR with at least four lanes per row
-        if (s.vw != 4 || V != 1)
-            return PSPMM_E_UNSUPPORTED;
-        if (s.lpr < 4) {
-            LaunchShape t = s;
-            pspmm_cfg wide = *cfg;
-            wide.lanes_per_row = 4;
-            pspmm_resolve_shape(&wide, dim, 4, V, SHAPE_ROWS, &t);
-            s = t;
-        }
-    }
-
-    // Rows of neighbouring columns share lines of L1 within a CTA: 256 threads gain 2 - 8 % on bands of 17 and
-    // more entries (28 entries, 96 columns: 86 -> 79 us) and lose up to 3 % on uniform columns.
-    if (V == 1 && s.vw == 4 && !target_row && n_entries >= 16 * n_seg && !(cfg && (cfg->cta_threads || cfg->lanes_per_row)))
-        s.threads = 256;
-    if (!cfg || cfg->rows_per_group == 0) {
-        if (V == 1 && s.rpg == 4 && (!cfg || cfg->lanes_per_row == 0))
-            s.rpg = rows_per_group_for(s, dim, n_seg, n_entries);
-        s.rpg = small_rows_per_group(s, V, n_seg, n_entries);
-    }
-
+    rc = spmm_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row != nullptr, n_seg, n_entries, &s);
+    if (rc)
+        return rc;
     const bool bucketed = target_row && cfg && cfg->bucketed;
     if (target_row && !accumulate) {
         const int vecok = (dim % 4 == 0 && ldC % 4 == 0 && ((uintptr_t)C) % 16 == 0) ? 1 : 0;

@@ -159,6 +159,56 @@ def test_config_resolution_covers_every_dim(pspmm_lib):
     assert cfg.vec_width == 2
 
 
+def _resolved(lib, dim, V, split, n_seg, n_entries, **kw):
+    from paramspmm_ae_b200 import _lib
+    cfg = _lib.make_cfg(**kw)
+    rc = lib.pspmm_resolve_spmm(ctypes.byref(cfg), dim, dim, dim, V, ctypes.c_void_p(256), ctypes.c_void_p(256), int(split),
+                                n_seg, n_entries)
+    return rc, tuple(getattr(cfg, f) for f, _ in cfg._fields_), cfg
+
+
+def test_resolved_shapes_see_the_layout_and_the_sizes(pspmm_lib):
+    """pspmm_resolve_spmm goes through the launch's own rules: split or not, few and many rows, short and
+    long ones.  (pspmm_resolve_cfg takes every layout for an unsplit one of unknown size.)"""
+    from paramspmm_ae_b200 import _lib
+    shape = lambda *a, **k: _resolved(pspmm_lib, *a, **k)[2]
+    assert shape(48, 1, False, 10**6, 8 * 10**6).lanes_per_row == 4
+    assert shape(46, 1, True, 10**6, 8 * 10**6).lanes_per_row == 32      # 23 vectors of 8 bytes: three slices only unsplit
+    assert shape(46, 1, False, 10**6, 8 * 10**6).lanes_per_row == 8
+    assert shape(96, 1, False, 10**6, 15 * 10**6).cta_threads == 128
+    assert shape(96, 1, False, 10**6, 16 * 10**6).cta_threads == 256     # (long rows of neighbouring columns)
+    assert shape(96, 1, True, 10**6, 16 * 10**6).cta_threads == 128
+    assert shape(128, 1, False, 10**6, 8 * 10**6).rows_per_group == 8
+    assert shape(128, 1, False, 10**6, 32 * 10**6).rows_per_group == 4
+    assert shape(128, 1, False, 1000, 8000).rows_per_group == 1          # (a small matrix fills the chip with single rows)
+    assert shape(16, 1, True, 10**6, 8 * 10**6).rows_per_group == 2
+    assert shape(8, 1, True, 10**6, 8 * 10**6, accumulate=1).lanes_per_row == 4
+    assert shape(240, 1, False, 10**6, 16 * 10**6, col_tile=64).lanes_per_row == 16
+    assert _resolved(pspmm_lib, 47, 1, False, 100, 400, accumulate=1)[0] == _lib.PSPMM_E_UNSUPPORTED
+    assert _resolved(pspmm_lib, 64, 1, False, -1, 400)[0] == _lib.PSPMM_E_ARG
+
+
+def test_a_resolved_configuration_resolves_to_itself(pspmm_lib):
+    import random
+    rng = random.Random(3)
+    for _ in range(4000):
+        V, split = rng.choice([1, 1, 1, 2, 3]), rng.random() < 0.5
+        dim, n_seg = rng.randint(1, 300), int(10 ** rng.uniform(0, 7))
+        n_entries = int(n_seg * 10 ** rng.uniform(-1, 3))
+        kw = {}
+        for field, values in (("lanes_per_row", (2, 4, 8, 16, 32)), ("vec_width", (1, 2, 4)), ("cta_threads", (64, 256)),
+                              ("rows_per_group", (1, 4, 8)), ("gather_batch", (4, 16)), ("col_tile", (32, 48, 64, 128))):
+            if rng.random() < 0.25:
+                kw[field] = rng.choice(values)
+        if V == 1 and dim % 4 == 0 and kw.get("vec_width", 4) == 4 and rng.random() < 0.2:
+            kw["accumulate"] = 1
+        rc, first, cfg = _resolved(pspmm_lib, dim, V, split, n_seg, n_entries, **kw)
+        assert rc == 0, (dim, V, split, n_seg, n_entries, kw)
+        again = {f: getattr(cfg, f) for f in ("lanes_per_row", "vec_width", "cta_threads", "rows_per_group", "gather_batch",
+                                              "col_tile", "accumulate")}
+        assert _resolved(pspmm_lib, dim, V, split, n_seg, n_entries, **again)[1] == first, (dim, V, split, n_seg, n_entries, kw)
+
+
 def test_ops_reject_cpu_tensors_and_bad_hints():
     """The torch-level operators never fall back: a CPU tensor or an invalid CF / blkWarpNum is
     an error, as in the reference (SpMM/SpMM.cpp:5-13, 110, 139)."""
