@@ -102,9 +102,9 @@ static int cf_max_for(int vw, int V)
 // columns, 2.4 M entries, dim 80: 118 -> 82 us, dim 160: 163 -> 133), except that 9 or 10 vectors idle
 // little (4 lanes: dim 40 107 -> 121).  The segments of skewed split layouts leave the smaller groups of a warp
 // out of step: two segments per group instead of four level that (R-MAT, 6.5 entries per row, dim 72:
-// 216 us before, 241 with four, 208 with two), but not for narrower loads, which have more groups per
-// byte (R-MAT, dim 23: 133 -> 145, dim 46: 158 -> 175), nor do 33..48 vectors of 8 bytes gain.  Blocks need
-// their registers for the second row and gain only with the narrower loads.
+// 216 us before, 241 with four, 208 with two; few_split_segments for small ones), but not for narrower loads,
+// which have more groups per byte (R-MAT, dim 23: 133 -> 145, dim 46: 158 -> 175), nor do 33..48 vectors of
+// 8 bytes gain.  Blocks need their registers for the second row and gain only with the narrower loads.
 static bool narrow_group(int nvec, int vw, int V, bool split)
 {
     const bool between = (nvec > 8 && nvec <= 12) || (nvec > 16 && nvec <= 24) || (nvec > 32 && nvec <= 48);
@@ -115,7 +115,19 @@ static bool narrow_group(int nvec, int vw, int V, bool split)
     return between && !split && (vw == 1 ? nvec > 16 : nvec <= 24);
 }
 
-int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out)
+// The three-slice groups of a split layout of at most this many segments end sooner with one segment each:
+// few warps hide little, so each warp waits for its longest group, and that wait grows with the segments
+// per group.  Up to about seven waves of single-segment groups one is faster or equal, beyond two are:
+//   R-MAT 1.8 M entries, 167 K segments, 48 columns: 95.3 us with two, 82.4 with one (one slice per lane: 80)
+//   R-MAT 1.2 M entries, 85 K, 76 columns: 65.3 and 57.9 (55); power law 0.2 M, 22 K, 76 columns: 21.2 and 13.8 (14.5)
+//   power law 2 M entries, 227 K, 48 columns: 49.7 with two, 54.2 with one (69); 2.5 M, 144 K, 76 columns: 75 and 82 (91)
+// The 16-lane groups are two to a warp and keep two segments (power law 0.2 M, 132 columns: 18.4 us, 19.9 with one).
+static bool few_split_segments(int64_t n_seg, int lpr)
+{
+    return n_seg >= 0 && lpr <= 8 && n_seg * lpr <= 7 * 768 * (int64_t)pspmm_sm_count();
+}
+
+int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out, int64_t n_seg)
 {
     LaunchShape s;
     s.vw = vw_max;
@@ -131,10 +143,22 @@ int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, Sh
         while (lpr < nvec && lpr < 32)
             lpr <<= 1;
         if (use != SHAPE_SDDMM && !(cfg && cfg->rows_per_group) && narrow_group(nvec, s.vw, V, use == SHAPE_SPLIT)) {
-            while (2 * lpr >= nvec)
-                lpr >>= 1;
-            if (V == 1 && (use == SHAPE_SPLIT || s.vw == 2))
-                rpg = 2;
+            int narrow = lpr;
+            while (2 * narrow >= nvec)
+                narrow >>= 1;
+            if (V == 1 && use == SHAPE_SPLIT) {
+                // (11 vectors stay on 16 lanes then: R-MAT of 167 K segments, 44 columns: 86.5 us on four lanes, 78.5;
+                // power law of 46 K: 44.4, 39.3)
+                const bool few = few_split_segments(n_seg, narrow);
+                if (!(few && nvec == 11)) {
+                    lpr = narrow;
+                    rpg = few ? 1 : 2;
+                }
+            } else {
+                lpr = narrow;
+                if (V == 1 && s.vw == 2)
+                    rpg = 2;
+            }
         }
     }
     if (lpr < lmin)
@@ -382,7 +406,7 @@ static int spmm_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, bool
                       LaunchShape *out)
 {
     LaunchShape s;
-    pspmm_resolve_shape(cfg, dim, vw_max, V, split ? SHAPE_SPLIT : SHAPE_ROWS, &s);
+    pspmm_resolve_shape(cfg, dim, vw_max, V, split ? SHAPE_SPLIT : SHAPE_ROWS, &s, n_seg);
     if (cfg && cfg->accumulate) {
         // built for 128-bit loads on CSR / split CSR with at least four lanes per row
         if (s.vw != 4 || V != 1)
@@ -390,7 +414,7 @@ static int spmm_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, bool
         if (s.lpr < 4) {
             pspmm_cfg wide = *cfg;
             wide.lanes_per_row = 4;
-            pspmm_resolve_shape(&wide, dim, 4, V, SHAPE_ROWS, &s);
+            pspmm_resolve_shape(&wide, dim, 4, V, SHAPE_ROWS, &s, n_seg);
         }
     }
     if (n_seg >= 0) {
@@ -661,7 +685,7 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     const int nvec_max = dim / vw_max;
     if (V == 1 && (narrow.lanes_per_row == 0 || narrow.lanes_per_row > 16) && nvec_max > 8)
         narrow.lanes_per_row = vw_max < 4 && nvec_max <= 32 ? 8 : 16;
-    pspmm_resolve_shape(&narrow, dim, vw_max, V, SHAPE_SDDMM, &s);
+    pspmm_resolve_shape(&narrow, dim, vw_max, V, SHAPE_SDDMM, &s, -1);
     if (V == 1 && s.lpr > 16) {
         s.lpr = 16;
         s.cf = 8;

@@ -193,5 +193,6 @@ int pspmm_sm_count();  // of the current device
 static inline int pspmm_long_lanes(int nvec, int V) { return nvec > 16 ? 32 : (nvec > 8 || V > 1) ? 16 : (nvec > 4 ? 8 : 4); }
 int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm);
 enum ShapeUse { SHAPE_ROWS, SHAPE_SPLIT, SHAPE_SDDMM };
-int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out);
+// n_seg: (block-)rows or pieces of the layout, negative when they are not known
+int pspmm_resolve_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, ShapeUse use, LaunchShape *out, int64_t n_seg);
 int pspmm_vw_max(int32_t dim, int64_t ld0, int64_t ld1, const void *p0, const void *p1);

@@ -188,6 +188,21 @@ def test_resolved_shapes_see_the_layout_and_the_sizes(pspmm_lib):
     assert _resolved(pspmm_lib, 64, 1, False, -1, 400)[0] == _lib.PSPMM_E_ARG
 
 
+def test_small_split_layouts_take_single_segments(pspmm_lib):
+    """Three slices on four or eight lanes: two segments per group, one up to about seven waves of groups
+    (the skewed layouts lost up to 20 % there), where 11 vectors keep one slice on sixteen lanes."""
+    def shape(dim, n_seg):
+        c = _resolved(pspmm_lib, dim, 1, True, n_seg, 11 * n_seg)[2]
+        return c.lanes_per_row, c.rows_per_group
+    waves7 = 7 * 768 * 148
+    assert shape(48, waves7 // 4) == (4, 1) and shape(48, waves7 // 4 + 1) == (4, 2)
+    assert shape(44, waves7 // 4)[0] == 16 and shape(44, waves7 // 4 + 1) == (4, 2)
+    for dim in (68, 76, 96):
+        assert shape(dim, waves7 // 8) == (8, 1) and shape(dim, waves7 // 8 + 1) == (8, 2)
+    assert shape(160, 40000) == (16, 2) and shape(160, 10**6) == (16, 2)  # (below that the waves decide)
+    assert shape(40, 10**5)[0] == 16
+
+
 def test_a_resolved_configuration_resolves_to_itself(pspmm_lib):
     import random
     rng = random.Random(3)
