@@ -62,14 +62,17 @@ typedef struct pspmm_cfg {
                                 several launches over column ranges.  0 = one launch */
     int32_t hint_CF;         /* legacy coarsening factor, validated only */
     int32_t hint_blkWarpNum; /* legacy warps per block, validated only */
-    int32_t bucketed;        /* SpMM only.  Split layout: 1 = the split arrays are a length-bucketed plan (see
-                                pspmm_spmm_csr): segments in any order, flags in the two high bits of target_row.
-                                Unsplit layout: 1 = the caller knows that no row is far longer than the others;
-                                with 0 the call looks for such rows and cuts them over the whole GPU */
+    int32_t bucketed;        /* SpMM only: 1 = the split arrays are a length-bucketed plan (see pspmm_spmm_csr):
+                                segments in any order, flags in the two high bits of target_row.  Unsplit layouts
+                                ignore it */
     int32_t accumulate;      /* SpMM only: 0 = C is overwritten (every row is written, empty rows with zeros);
                                 1 = the product is added to what C holds (reduction instructions; the order in
                                 which contributions reach a row is not fixed).  Lets a caller sum products over
                                 column blocks of A, e.g. as blocks of B arrive from other GPUs */
+    int32_t no_long_rows;    /* SpMM on an unsplit layout: 1 = the caller knows that no row is far longer than the
+                                others; with 0 a call that has scratch memory looks for such rows and cuts them over
+                                the whole GPU (that form of the kernel ignores gather_batch).  Split layouts
+                                ignore it */
 } pspmm_cfg;
 
 PSPMM_API int pspmm_version(void);

@@ -18,7 +18,7 @@ int pspmm_note_cuda_error(cudaError_t e)
 
 extern "C" const char *pspmm_last_cuda_error(void) { return g_cuda_err; }
 
-extern "C" int pspmm_version(void) { return 100; }
+extern "C" int pspmm_version(void) { return 101; }
 
 extern "C" const char *pspmm_strerror(int code)
 {
@@ -65,6 +65,8 @@ int pspmm_validate_cfg(const pspmm_cfg *cfg, bool sddmm)
     if (cfg->col_tile < 0 || cfg->col_tile % 4 != 0)
         return PSPMM_E_CONFIG;
     if (cfg->bucketed != 0 && (cfg->bucketed != 1 || sddmm))
+        return PSPMM_E_CONFIG;
+    if (cfg->no_long_rows != 0 && (cfg->no_long_rows != 1 || sddmm))
         return PSPMM_E_CONFIG;
     return PSPMM_OK;
 }
@@ -547,7 +549,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     // 26, 212 columns: 140 instead of 110; at most 5 us are lost elsewhere).
     a.dependent = target_row && !accumulate && !bucketed;
     a.lng = LongArgs{};
-    if (scratch && !target_row && !accumulate && !(cfg && cfg->bucketed) && n_entries > PSPMM_LONG_ROW) {
+    if (scratch && !target_row && !accumulate && !(cfg && cfg->no_long_rows) && n_entries > PSPMM_LONG_ROW) {
         const int lanes = pspmm_long_lanes(a.nvec, V);
         long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
         if (scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
@@ -896,7 +898,7 @@ extern "C" int pspmm_profile_spmm(const int32_t *rowPtr, const int32_t *colIdx, 
     // (the scratch that the timed entry points would be given)
     void *scratch = nullptr;
     size_t bytes = 0;
-    if (!target_row && pspmm_spmm_scratch_bytes(n_rows, nnz, dim, V, &bytes) == PSPMM_OK && bytes > 0)
+    if (!target_row && !(cfg && cfg->no_long_rows) && pspmm_spmm_scratch_bytes(n_rows, nnz, dim, V, &bytes) == PSPMM_OK && bytes > 0)
         PSPMM_CUDA_TRY(cudaMallocAsync(&scratch, bytes, (cudaStream_t)stream));
     auto launch = [&]() -> int {
         if (V == 1)

@@ -121,14 +121,23 @@ class Plan(dict):
     """Chosen representation and kernel parameters.
 
     Keys: if_split (0/1), vec_size (1/2), granularity (partition length or None = the
-    reference's rule), and kernel fields lanes_per_row / vec_width / cta_threads /
-    rows_per_group (0 = library default).
+    reference's rule), kernel fields lanes_per_row / vec_width / cta_threads /
+    rows_per_group (0 = library default), and no_long_rows (1: the statistics of an unsplit
+    matrix show no row far longer than the others; a plan without the key goes by its regime).
     """
 
     def kernel_cfg(self):
-        return {k: int(self.get(k, 0) or 0)
-                for k in ("lanes_per_row", "vec_width", "cta_threads", "rows_per_group", "gather_batch", "col_tile",
-                          "bucketed")}
+        """Arguments of ``_lib.make_cfg`` for the plan's launch, the same for who runs and who times it."""
+        cfg = {k: int(self.get(k, 0) or 0)
+               for k in ("lanes_per_row", "vec_width", "cta_threads", "rows_per_group", "gather_batch", "col_tile",
+                         "bucketed", "no_long_rows")}
+        if "no_long_rows" not in self:
+            cfg["no_long_rows"] = _no_long_rows(self)
+        return cfg
+
+
+def _no_long_rows(plan):
+    return int(not plan.get("if_split") and not plan.get("regime", "skewed").endswith("skewed"))
 
 
 def choose(stats, dim, op="spmm"):
@@ -159,6 +168,7 @@ def choose(stats, dim, op="spmm"):
                 rows_per_group=0, gather_batch=0, col_tile=0, bucketed=0)
     plan.update(e)
     plan["regime"] = reg
+    plan["no_long_rows"] = _no_long_rows(plan)
     if plan["if_split"] and not plan.get("granularity"):
         plan["granularity"] = auto_granularity(stats["real_avg"])
     return plan
@@ -191,8 +201,6 @@ class PlannedSpMM:
     def __call__(self, out, B, accumulate=False):
         from . import _lib, ops
         kw = self.plan.kernel_cfg()
-        if self.target is None and self.plan.get("regime", "skewed").rpartition("_")[2] != "skewed":
-            kw["bucketed"] = 1  # the statistics showed no long row: nothing to look for on each call
         if accumulate:  # built for 128-bit loads at one gather-batch depth
             kw.update(vec_width=0, gather_batch=0, accumulate=1)
         dst = out

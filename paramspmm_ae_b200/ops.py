@@ -350,7 +350,7 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
         n_out_rows = n_seg
     _check_output(out, rowPtr, split, n_out_rows, V, dim)
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
-    long_rows = target_row is None and (cfg is None or not (cfg.bucketed or cfg.accumulate))
+    long_rows = target_row is None and (cfg is None or not (cfg.no_long_rows or cfg.accumulate))
     return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows)
 
 

@@ -121,13 +121,16 @@ def candidates(dim, regime, quick=False, vecs=(1, 2), cta_threads=(64, 128, 256)
             continue  # block kernels are built with one gather depth; measured at one CTA size, untiled
         if thr == 64 and lpr == 32 and rpg == 2:
             continue
+        if skew and not gran and mlp != 8:
+            continue  # unsplit rows of any length: the kernel that leaves the long ones out has one gather depth
         if tile and (lpr * vw > tile or thr != 256 or rpg != 4):
             continue  # column ranges narrower than a lane group make no sense; tiles measured at one shape
         if tile and tile < 128 and skew:
             continue  # narrow column ranges re-read A for every range: only the even regimes try them
         base = {"vec_size": vec, "if_split": int(gran > 0), "granularity": gran or None,
                 "lanes_per_row": lpr, "vec_width": vw, "rows_per_group": rpg, "cta_threads": thr,
-                "gather_batch": mlp, "col_tile": tile, "bucketed": 0}
+                "gather_batch": mlp, "col_tile": tile, "bucketed": 0,
+                "no_long_rows": int(not gran and not skew)}  # as the plan of such a matrix
         yield base
         if skew and gran and vec == 1 and not tile:
             yield dict(base, bucketed=1)  # the same pieces ordered by length
@@ -175,11 +178,9 @@ class Timer:
         # hub rows sum thousands of terms in a different order: the floor grows with the row's length
         ln = (m.rowPtr[1:] - m.rowPtr[:-1]).double()
         self.tol = (1e-5 * self.ref.abs() + 1e-4 * torch.clamp(ln / 256.0, min=1.0)[:, None]).float()
-        self.max_row = int(ln.max())
 
     def ms(self, cand):
-        """Milliseconds per launch, or None for a candidate that is not run (hub rows without a
-        split) or that the library rejects for this width / layout."""
+        """Milliseconds per launch, or None for a candidate that the library rejects for this width / layout."""
         try:
             return self._ms(cand)
         except _lib.PspmmError as e:
@@ -189,8 +190,6 @@ class Timer:
 
     def _ms(self, cand):
         m, dim = self.m, self.dim
-        if not cand.get("if_split") and self.max_row > 4096:
-            return None  # one lane group per hub row would take milliseconds
         V = cand.get("vec_size", 1)
         rp, ci, v, tr = self.lay.get(V, cand.get("granularity") if cand.get("if_split") else None,
                                      cand.get("bucketed"))
@@ -198,7 +197,7 @@ class Timer:
         out = torch.full((nbr * V, dim), float("nan"), device=self.dev)
         cfg = _lib.make_cfg(**{k: int(cand.get(k, 0) or 0) for k in
                                ("lanes_per_row", "vec_width", "cta_threads", "rows_per_group", "gather_batch",
-                                "col_tile", "bucketed")})
+                                "col_tile", "bucketed", "no_long_rows")})
         ops.spmm_into(out, self.B, rp, ci, v, target_row=tr, V=V, n_out_rows=nbr, cfg=cfg)
         bad = int(((out[: m.n_rows] - self.ref).abs() > self.tol).sum())
         if bad or bool(torch.isnan(out[: m.n_rows]).any()):

@@ -401,3 +401,49 @@ def test_block_builder_rejects_bad_columns_and_inconsistent_counts(pspmm_lib):
     vb = np.full(12, -7.0, dtype=np.float32)
     assert pspmm_lib.pspmm_bcsr_fill(p(rp), p(ci), p(v), 3, 4, 2, p(lie), p(cb), p(vb)) == _lib.PSPMM_E_ARG
     assert (cb[2:] == -7).all() and (vb[4:] == -7).all()
+
+
+def test_timing_and_tuning_launch_what_the_operator_launches(monkeypatch):
+    """A plan becomes one configuration: the operator's product, the sweep's timer and the decider's command
+    line hand the same one to the library, and candidates of an unsplit matrix differ in what they time."""
+    from paramspmm_ae_b200 import _lib, decider, ops, sweep, synth
+    fields = lambda cfg: tuple(getattr(cfg, f) for f, _ in cfg._fields_)
+    seen = {"run": [], "time": []}
+    monkeypatch.setattr(ops, "spmm_into", lambda out, *a, cfg=None, **k: (seen["run"].append(fields(cfg)), out.zero_())[1])
+    monkeypatch.setattr(ops, "spmm_time_ms", lambda *a, cfg=None, **k: (seen["time"].append(fields(cfg)), 1.0)[1])
+    flag = [f for f, _ in _lib.PspmmCfg._fields_].index("no_long_rows")
+    for m, unsplit_flag in ((synth.uniform_rows(4000, 16, seed=1), 1), (synth.banded_rows(4000, 16, 32, seed=1), 1),
+                            (synth.powerlaw_graph(3000, 9000, seed=1), 0)):
+        stats = decider.row_stats(m.rowPtr, m.colIdx)
+        for dim in (16, 64, 128):
+            plan = decider.choose(stats, dim)
+            if plan["if_split"]:  # the layouts without a GPU: the same plan on the unsplit rows
+                plan.update(if_split=0, granularity=None, bucketed=0, no_long_rows=0)
+            X, out = torch.zeros(m.n_cols, dim), torch.zeros(m.n_rows, dim)
+            op = decider.PlannedSpMM(plan, m.rowPtr, m.colIdx, m.val, n_cols=m.n_cols)
+            seen["run"].clear()
+            op(out, X)
+            timer = sweep.Timer.__new__(sweep.Timer)
+            timer.m, timer.dim, timer.dev, timer.warmup, timer.iters = m, dim, torch.device("cpu"), 0, 1
+            timer.lay, timer.B = sweep.Layouts(m, torch.device("cpu")), X
+            timer.ref, timer.tol = torch.zeros(m.n_rows, dim), torch.ones(m.n_rows, dim)
+            seen["time"].clear()
+            timer.ms(dict(plan))
+            assert seen["time"] and seen["time"][-1] == seen["run"][0] == fields(_lib.make_cfg(**plan.kernel_cfg()))
+            assert seen["run"][0][flag] == unsplit_flag
+    old = decider.Plan({k: v for k, v in plan.items() if k != "no_long_rows"}, regime="short_even")  # (saved without the key)
+    assert old.kernel_cfg()["no_long_rows"] == 1 and decider.Plan(old, if_split=1).kernel_cfg()["no_long_rows"] == 0
+    for regime in sweep.ALL_REGIMES:
+        unsplit = [c for c in sweep.candidates(64, regime) if not c["if_split"] and c["vec_size"] == 1]
+        skewed = regime.endswith("skewed")
+        assert all(c["no_long_rows"] == int(not skewed) for c in unsplit)
+        assert {c["gather_batch"] for c in unsplit} == ({8} if skewed else {4, 8, 16})
+
+
+def test_the_long_rows_flag_is_a_flag_of_the_spmm(pspmm_lib):
+    from paramspmm_ae_b200 import _lib
+    one, null = ctypes.c_void_p(256), ctypes.c_void_p(0)
+    assert pspmm_lib.pspmm_spmm_csr(one, one, one, one, one, 4, 4, 4, 16, 16, 16,
+                                    ctypes.byref(_lib.make_cfg(no_long_rows=2)), null, null, 0, null) == _lib.PSPMM_E_CONFIG
+    assert pspmm_lib.pspmm_sddmm_csr(one, one, one, one, one, 4, 4, 16, 16, 16,
+                                     ctypes.byref(_lib.make_cfg(no_long_rows=1)), null, null, 0, null) == _lib.PSPMM_E_CONFIG
