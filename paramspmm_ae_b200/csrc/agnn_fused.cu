@@ -746,7 +746,7 @@ static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A
     a.lng = LongArgs{};
     if (!split && scratch && ((uintptr_t)scratch) % 16 == 0 && nnz > PSPMM_LONG_ROW) {
         agnn_long_layout(&a.lng, n_rows, nnz);
-        if (scratch_bytes >= agnn_long_bytes(a.lng, dim))
+        if (long_fits(a.lng, nnz) && scratch_bytes >= agnn_long_bytes(a.lng, dim))
             long_place(&a.lng, scratch);
         else
             a.lng = LongArgs{};

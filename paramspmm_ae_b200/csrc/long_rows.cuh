@@ -74,59 +74,66 @@ __device__ __forceinline__ T cta_scan(T x, T *warps, T *total)
 //
 // Positions ("units") run over the long rows' entries of the whole matrix, with PSPMM_LONG_LOOK units ahead
 // of every 512 rows for the look at them, so that a share of few long rows among many short ones is no
-// longer than the others.
+// longer than the others.  They run to the entries plus one per row, beyond 2^31 for matrices near the index
+// limit, and are 64 bits wide; what belongs to one share is not (long_fits).  Only look() knows positions: the
+// users see offsets into the share's part of the look, and the 64-bit values stay out of their registers.
 struct LongShare {
     struct Shared {
         int row[PSPMM_LONG_ROWS], lo[PSPMM_LONG_ROWS];  // the long rows of this look; their first entry in the share
-        int at[PSPMM_LONG_ROWS + 1];                    // their positions
+        int off[PSPMM_LONG_ROWS + 1];                   // where they begin among its entries of the share
         unsigned long long warps[8];
-        int found[2];
-        int edge[2];  // the rows that hold the first and the last entry of this look's part of the share
+        int64_t u0, u1, per;  // the share
+        int64_t found[2];
+        int edge[2];     // the rows that hold the first and the last entry of this look's part of the share
+        int shares[2];   // the first share of the one, the last of the other
         int last[2];
     };
-    int u0, u1, per;   // the share
-    int pos;           // position of row r
+    int64_t pos;  // position of row r
     int64_t r;
-    int n, base, total;  // long rows of this look; position and number of the entries that belong to the share
+    int share, total;  // total: entries of this look that belong to the share
 
     // False: nothing to do (no row is long, or fewer shares are needed than there are).
-    __device__ __forceinline__ bool begin(const LongArgs &a, Shared &sh, int share)
+    __device__ __forceinline__ bool begin(const LongArgs &a, Shared &sh, int share_)
     {
         const int tid = threadIdx.x;
         const int each = (a.n_totals + 255) / 256;
         unsigned long long mine = 0, all;
         bool any = false;
+        share = share_;
 #pragma unroll 8
         for (int i = 0; i < each; ++i) {
             const int t = tid * each + i;
             const int x = t < a.n_totals ? __ldcg(a.totals + t) : 0;
             any |= x > 0;
-            mine += x + (t < a.n_totals ? PSPMM_LONG_LOOK : 0);
+            mine += (unsigned long long)x + (t < a.n_totals ? PSPMM_LONG_LOOK : 0);
         }
         if (!__syncthreads_or(any))
             return false;
         const unsigned long long upto = cta_scan(mine, sh.warps, &all);
-        per = (int)((all + a.shares - 1) / a.shares + 63) / 64 * 64;
-        const unsigned long long first = (unsigned long long)share * per;
+        const unsigned long long per = long_share_size((int64_t)all, a.shares);
+        const unsigned long long first = share * per;
         if (first >= all)
             return false;
-        u0 = (int)first;
-        u1 = (int)(all - first < (unsigned)per ? all : first + per);
+        if (tid == 0) {
+            sh.u0 = (int64_t)first;
+            sh.u1 = (int64_t)(all - first < per ? all : first + per);
+            sh.per = (int64_t)per;
+        }
         if (first >= upto - mine && first < upto) {
             unsigned long long before = upto - mine;
             int t = tid * each;
             while (true) {
-                const int x = __ldcg(a.totals + t) + PSPMM_LONG_LOOK;
+                const unsigned long long x = (unsigned long long)__ldcg(a.totals + t) + PSPMM_LONG_LOOK;
                 if (before + x > first)
                     break;
                 before += x;
                 ++t;
             }
             sh.found[0] = t;
-            sh.found[1] = (int)before;
+            sh.found[1] = (int64_t)before;
         }
         __syncthreads();
-        r = (int64_t)sh.found[0] * PSPMM_LONG_ROWS;
+        r = sh.found[0] * PSPMM_LONG_ROWS;
         pos = sh.found[1];
         return true;
     }
@@ -134,6 +141,7 @@ struct LongShare {
     // Looks at the next 512 rows.  False: the share ends.  total == 0: none of its entries lie here.
     __device__ __forceinline__ bool look(Shared &sh, const int32_t *segPtr, int64_t n_seg)
     {
+        const int64_t u0 = sh.u0, u1 = sh.u1;
         if (pos >= u1)
             return false;
         int len[2], start[2];
@@ -150,59 +158,60 @@ struct LongShare {
             mine += (unsigned)len[i] + (len[i] ? 1ull << 32 : 0ull);
         }
         const unsigned long long before = cta_scan(mine, sh.warps, &all) - mine;
-        const int begin_at = pos + PSPMM_LONG_LOOK, end_at = begin_at + (int)(unsigned)all;
-        n = (int)(all >> 32);
-        base = u0 > begin_at ? u0 : begin_at;
-        total = (u1 < end_at ? u1 : end_at) - base;
-        total = total > 0 ? total : 0;
-        int idx = (int)(before >> 32), at = begin_at + (int)(unsigned)before;
+        const int64_t begin_at = pos + PSPMM_LONG_LOOK, end_at = begin_at + (unsigned)all;
+        const int64_t base = u0 > begin_at ? u0 : begin_at;
+        const int64_t part = (u1 < end_at ? u1 : end_at) - base;
+        total = part > 0 ? (int)part : 0;
+        int idx = (int)(before >> 32);
+        int64_t at = begin_at + (unsigned)before - base;  // from the share's first entry of this look
 #pragma unroll
         for (int i = 0; i < 2; ++i)
             if (len[i]) {
+                const int64_t end = at + len[i];
                 sh.row[idx] = (int)(r + 2 * threadIdx.x + i);
-                sh.lo[idx] = start[i] + (base > at ? base - at : 0);
-                sh.at[idx] = at;
+                sh.lo[idx] = start[i] + (at < 0 && end > 0 ? (int)-at : 0);
+                sh.off[idx] = at < 0 ? 0 : (at < total ? (int)at : total);
                 if (total) {
-                    if (at <= base && base < at + len[i])
+                    if (at <= 0 && end > 0) {
                         sh.edge[0] = idx;
-                    if (at < base + total && base + total <= at + len[i])
+                        sh.shares[0] = at == 0 ? share : (int)((base + at) / sh.per);
+                    }
+                    if (at < total && end >= total) {
                         sh.edge[1] = idx;
+                        sh.shares[1] = end == total ? share : (int)((base + end - 1) / sh.per);
+                    }
                 }
                 ++idx;
-                at += len[i];
+                at = end;
             }
         if (threadIdx.x == 0)
-            sh.at[n] = end_at;
+            sh.off[(int)(all >> 32)] = total;
         r += PSPMM_LONG_ROWS;
         pos = end_at;
         __syncthreads();
         return true;
     }
 
-    // Where row i begins in the concatenation of this look's entries (i == n: where they end).
-    __device__ __forceinline__ int off(const Shared &sh, int i) const
-    {
-        const int o = sh.at[i] - base;
-        return o < 0 ? 0 : (o < total ? o : total);
-    }
+    // Where row i begins in the concatenation of this look's entries (the number of rows: where they end).
+    __device__ __forceinline__ int off(const Shared &sh, int i) const { return sh.off[i]; }
     // The row that holds entry p of the concatenation.
     __device__ __forceinline__ int row_of(const Shared &sh, int p) const
     {
         int lo = sh.edge[0], hi = sh.edge[1] + 1;
         while (hi - lo > 1) {
             const int mid = (lo + hi) / 2;
-            if (sh.at[mid] - base <= p)
+            if (sh.off[mid] <= p)
                 lo = mid;
             else
                 hi = mid;
         }
         return lo;
     }
-    // First and last share that row i is part of.
+    // First and last share that row i is part of (edge[0] <= i <= edge[1]): only the outermost rows leave this one.
     __device__ __forceinline__ void shares_of(const Shared &sh, int i, int &s0, int &s1) const
     {
-        s0 = sh.at[i] / per;
-        s1 = (sh.at[i + 1] - 1) / per;
+        s0 = i == sh.edge[0] ? sh.shares[0] : share;
+        s1 = i == sh.edge[1] ? sh.shares[1] : share;
     }
     // Where a share's part of a row goes: slot 2 * share (the row began in an earlier share) or 2 * share + 1.
     __device__ __forceinline__ static int64_t slot(int share, int s0) { return 2 * (int64_t)share + (s0 == share ? 1 : 0); }

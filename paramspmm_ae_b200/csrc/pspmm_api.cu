@@ -552,7 +552,8 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     if (scratch && !target_row && !accumulate && !(cfg && cfg->no_long_rows) && n_entries > PSPMM_LONG_ROW) {
         const int lanes = pspmm_long_lanes(a.nvec, V);
         long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
-        if (scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
+        if (long_fits(a.lng, n_entries) &&
+            scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
             long_place(&a.lng, scratch);
         else
             a.lng = LongArgs{};

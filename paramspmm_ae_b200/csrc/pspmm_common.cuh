@@ -103,6 +103,17 @@ static inline void long_layout(LongArgs *a, int64_t n_rows, int64_t n_entries, i
     a->shares = sms * per_sm > tiles ? sms * per_sm * waves / tiles : 1;
     a->n_counters = a->shares * tiles;
 }
+// Positions (long_rows.cuh) per share.
+__host__ __device__ static inline int64_t long_share_size(int64_t units, int shares)
+{
+    return ((units + shares - 1) / shares + 63) / 64 * 64;
+}
+// Whether a share's entries can be counted in an int with room for the groups' spans: only a product so wide
+// that its column tiles leave one or two shares fails this.
+static inline bool long_fits(const LongArgs &a, int64_t n_entries)
+{
+    return long_share_size(n_entries + (int64_t)a.n_totals * PSPMM_LONG_LOOK, a.shares) <= 1 << 30;
+}
 static inline size_t long_head_bytes(const LongArgs &a)
 {
     return (((size_t)a.n_totals + (size_t)a.n_counters) * 4 + 255) / 256 * 256;

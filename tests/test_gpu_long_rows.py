@@ -1,5 +1,5 @@
-"""Rows of an unsplit layout that are longer than the others: the kernels cut them over the GPU from
-64 .. 512 entries on (by the matrix's size), everything else stays with one lane group."""
+"""Rows of an unsplit layout that are longer than 64 entries: the kernels cut them over the GPU; everything
+else stays with one lane group."""
 import numpy as np
 import pytest
 import torch
@@ -91,3 +91,32 @@ def test_sums_of_long_rows_have_a_fixed_order(dim):
         b = torch.empty_like(a)
         ops.spmm_into(b, B, *t)
         assert torch.equal(a, b)
+
+
+def test_positions_beyond_32_bits():
+    """Long rows of almost 2^31 entries: the positions that shares are counted in (entries plus one per row)
+    pass 2^31.  Values of 0 and 1 make every share's sum exact; a hub's fewer than 200 shares are then
+    added in fp32, 2^-24 each, 1.2e-5 in all.  A share that is lost or taken twice moves a row by 0.5 %."""
+    from paramspmm_ae_b200 import ops
+    dev = torch.device("cuda:0")
+    n, n_cols, nnz, hubs = 2_000_003, 4096, 2_147_400_000, [0, 17, 400_000, 400_001, 999_999, 2_000_002]
+    ln = (torch.arange(n) % 3 == 0).long()
+    ln[hubs] = 0
+    ln[hubs] = (nnz - int(ln.sum())) // len(hubs)
+    ln[hubs[-1]] += nnz - int(ln.sum())
+    rp = torch.cat([torch.zeros(1, dtype=torch.int64), ln.cumsum(0)])
+    assert int(rp[-1]) == nnz and int(ln[hubs].sum()) + n > 2**31
+    ci = torch.arange(nnz, dtype=torch.int32, device=dev).bitwise_and_(n_cols - 1)
+    B = torch.randint(0, 2, (n_cols, 4), generator=torch.Generator().manual_seed(2)).float()
+    B[:, 0] = 1.0
+    upto = torch.cat([torch.zeros(1, 4, dtype=torch.float64), B.double().cumsum(0)])  # sums of the first k columns
+    total = lambda e: (e // n_cols).double()[:, None] * upto[-1] + upto[e % n_cols]
+    want = (total(rp[1:]) - total(rp[:-1])).numpy()
+    rpd, Bd = rp.int().to(dev), B.to(dev)
+    out = torch.full((n, 4), float("nan"), device=dev)
+    ops.spmm_into(out, Bd, rpd, ci, None)
+    np.testing.assert_allclose(out.cpu().numpy(), want, rtol=2e-5)
+    A = torch.zeros(n, 4, device=dev)
+    A[:, 0] = 1.0  # every score is one
+    got = ops.agnn_fused(A, Bd, rpd, ci, 1.0, False)
+    np.testing.assert_allclose(got.cpu().numpy(), want, rtol=2e-5)
