@@ -338,10 +338,16 @@ PSPMM_API int pspmm_pull_rows_status(int32_t *status);
  * three-way bf16 splits with fp32 accumulation: at least as accurate as a chain of fp32 multiply-adds.
  * Any size and alignment.  Products with few output tiles and a long K need scratch of
  * pspmm_dense_scratch_bytes(M, N, K) bytes (0 for the others).  Every wait inside the kernel is
- * bounded; pspmm_dense_status returns 1 once one has run out on this GPU (it synchronises).
+ * bounded (two seconds): when one runs out, what was not computed of C becomes NaN, and
+ * pspmm_dense_status returns 1 from then on in this process (it synchronises).
+ * pspmm_dense_mm_stalled is for tests of that path: the same call with a signal withheld and waits of
+ * 20 ms, so that all of C becomes NaN.
  */
 PSPMM_API int pspmm_dense_scratch_bytes(int64_t M, int64_t N, int64_t K, size_t *bytes);
 PSPMM_API int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A,
+                             int64_t ldA, const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch,
+                             size_t scratch_bytes, void *stream);
+PSPMM_API int pspmm_dense_mm_stalled(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A,
                              int64_t ldA, const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch,
                              size_t scratch_bytes, void *stream);
 PSPMM_API int pspmm_dense_status(int32_t *status);

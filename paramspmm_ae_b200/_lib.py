@@ -107,6 +107,7 @@ _SIGNATURES = {
     "pspmm_pull_rows_status": [ctypes.POINTER(ctypes.c_int32)],
     "pspmm_dense_scratch_bytes": [_i64, _i64, _i64, ctypes.POINTER(ctypes.c_size_t)],
     "pspmm_dense_mm": [_i32, _i32, _i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, ctypes.c_size_t, _vp],
+    "pspmm_dense_mm_stalled": [_i32, _i32, _i64, _i64, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, ctypes.c_size_t, _vp],
     "pspmm_dense_status": [ctypes.POINTER(ctypes.c_int32)],
     "pspmm_bcsr_count": [_vp, _vp, _i64, _i64, _i32, _vp, ctypes.POINTER(_i64)],
     "pspmm_bcsr_fill": [_vp, _vp, _vp, _i64, _i64, _i32, _vp, _vp, _vp],

@@ -37,8 +37,8 @@
 // Infinities, NaNs and values that round to infinity in bf16 have no such split: a CTA that meets one
 // computes its tiles with fp32 FMAs from then on.
 //
-// Every wait is bounded (about two seconds); a wait that runs out raises g_dense_status, which
-// pspmm_dense_status reads, and the CTA leaves.
+// Every wait is bounded (about two seconds).  When one runs out the CTA raises g_dense_status, which
+// pspmm_dense_status reads, fills what it has not computed of C with NaN, and leaves.
 #include <type_traits>
 
 #include "pspmm_common.cuh"
@@ -85,6 +85,8 @@ struct DenseArgs {
     const unsigned char *Bs;  // B split beforehand (split_weights_kernel)
     unsigned *odd;            // with Bs: one word per block of that kernel, set when a value of B has no split
     int32_t odd_words;
+    uint32_t wait_ns;         // limit of a wait
+    int32_t withhold;         // arrivals that no one brings: 0, or 1 to make the waits for a stage run out
 };
 
 struct ReduceArgs {
@@ -113,16 +115,17 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, int parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// False when the wait ran out (or another role's did: *abort).
-__device__ __forceinline__ bool bar_wait(uint32_t bar, int parity, volatile int *abort)
+// False when the wait ran out (or another role's did: *abort).  Whole warps call it, and its lanes agree: what
+// follows are barriers and tcgen05 instructions of whole warps.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, int parity, volatile int *abort, uint32_t limit_ns)
 {
-    if (bar_try(bar, parity))
+    if (__all_sync(PSPMM_FULL_MASK, bar_try(bar, parity)))
         return true;
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    while (!bar_try(bar, parity)) {
+    while (!__all_sync(PSPMM_FULL_MASK, bar_try(bar, parity))) {
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (*abort || t - t0 > 2000000000ull) {
+        if (__any_sync(PSPMM_FULL_MASK, *abort || t - t0 > limit_ns)) {
             *abort = 1;
             atomicExch(&g_dense_status, 1u);
             return false;
@@ -343,7 +346,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                    acc_empty = acc_full + 8 * ACC_BUFS;
     if (threadIdx.x == 0) {
         for (int i = 0; i < STAGES; ++i) {
-            bar_init(full + 8 * i, GROUP_WARPS + (PRE ? 1 : 0));
+            bar_init(full + 8 * i, GROUP_WARPS + (PRE ? 1 : 0) + a.withhold);
             bar_init(empty + 8 * i, 1);
         }
         for (int i = 0; i < ACC_BUFS; ++i) {
@@ -505,8 +508,10 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
             } else {
                 settle();
             }
-            ok = bar_wait(empty + 8 * q, phase ^ 1, &abort_flag);
+            ok = bar_wait(empty + 8 * q, phase ^ 1, &abort_flag, a.wait_ns);
             if (!ok) {
+                if constexpr (BOTH)
+                    group_all(1 + q, true);  // (warps of the group that saw the stage free are at this barrier below)
                 if constexpr (KC_A || BOTH)
                     continue;  // (the group leaves together)
                 else
@@ -582,7 +587,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                 item_place(item, m0, n0, k0, k1, split);
                 const unsigned char *src = a.Bs + (int64_t)(n0 / a.bn * k_stages + k0 / BK) * (3 * plane);
                 for (int k = k0; k < k1; k += BK, src += 3 * plane) {
-                    if (!bar_wait(empty + 8 * stage, phase ^ 1, &abort_flag)) {
+                    if (!bar_wait(empty + 8 * stage, phase ^ 1, &abort_flag, a.wait_ns)) {
                         ok = false;
                         break;
                     }
@@ -620,8 +625,8 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                 item_place(item, m0, n0, k0, k1, split);
                 for (int k = k0; k < k1; k += BK, ++i) {
                     if ((i & 1) == m) {
-                        if (!bar_wait(acc_empty + 8 * m, ((i >> 1) & 1) ^ 1, &abort_flag) ||
-                            !bar_wait(full + 8 * stage, phase, &abort_flag)) {
+                        if (!bar_wait(acc_empty + 8 * m, ((i >> 1) & 1) ^ 1, &abort_flag, a.wait_ns) ||
+                            !bar_wait(full + 8 * stage, phase, &abort_flag, a.wait_ns)) {
                             ok = false;
                             break;
                         }
@@ -659,7 +664,8 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
         float *patch = reinterpret_cast<float *>(smem + STAGES * (STAGE_BYTES + Raw<KC_A, KC_B, PRE>::BYTES) + d * OUT_BYTES);
         int buf = 0, buf_phase = 0;
         bool ok = true;
-        for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+        int item = blockIdx.x;
+        for (; item < items; item += gridDim.x) {
             int m0, n0, k0, k1;
             int split;
             item_place(item, m0, n0, k0, k1, split);
@@ -668,7 +674,7 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
             for (int j = 0; j < 64; ++j)
                 acc[j] = 0.f;
             for (int k = k0; k < k1; k += BK) {
-                if (!bar_wait(acc_full + 8 * buf, buf_phase, &abort_flag)) {
+                if (!bar_wait(acc_full + 8 * buf, buf_phase, &abort_flag, a.wait_ns)) {
                     ok = false;
                     break;
                 }
@@ -757,6 +763,16 @@ __global__ void __launch_bounds__(THREADS, 1) dense_kernel(const DenseArgs a)
                             out[r * a.ldC + j0 + lane] = patch[r * OUT_PITCH + lane];
                 }
             }
+        }
+        for (; item < items; item += gridDim.x) {  // a wait ran out: no stale memory passes for a result
+            int m0, n0, k0, k1;
+            int split;
+            item_place(item, m0, n0, k0, k1, split);
+            const int c0 = n0 + half * cols;
+            const int c1 = n0 + a.bn < a.N ? n0 + a.bn : a.N;
+            if (m0 + row < a.M)
+                for (int c = c0; c < c0 + cols && c < c1; ++c)
+                    a.C[((int64_t)split * a.M + m0 + row) * a.ldC + c] = __int_as_float(0x7fffffff);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -893,9 +909,9 @@ extern "C" int pspmm_dense_scratch_bytes(int64_t M, int64_t N, int64_t K, size_t
     return PSPMM_OK;
 }
 
-extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t ldA,
-                              const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch, size_t scratch_bytes,
-                              void *stream)
+static int dense_run(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t ldA,
+                     const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch, size_t scratch_bytes,
+                     uint32_t wait_ns, int32_t withhold, void *stream)
 {
     if (M < 0 || N < 0 || K < 0 || ldC < N || ldA < (transA ? M : K) || ldB < (transB ? K : N))
         return PSPMM_E_ARG;
@@ -921,6 +937,8 @@ extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t
     a.K = (int32_t)K;
     a.C = C;
     a.ldC = ldC;
+    a.wait_ns = wait_ns;
+    a.withhold = withhold;
     const size_t need = partial_bytes(a, M, N) + split_bytes(a, K);
     if (need > 0 && (!scratch || scratch_bytes < need || (uintptr_t)scratch % 16 != 0))
         return PSPMM_E_ARG;
@@ -950,6 +968,20 @@ extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t
         PSPMM_CUDA_TRY(launch_dependent(reduce_splits_kernel, dim3((unsigned)((M * N + 31) / 32)), 256, 0, st, r));
     }
     return PSPMM_OK;
+}
+
+extern "C" int pspmm_dense_mm(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t ldA,
+                              const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch, size_t scratch_bytes,
+                              void *stream)
+{
+    return dense_run(transA, transB, M, N, K, A, ldA, B, ldB, C, ldC, scratch, scratch_bytes, 2000000000u, 0, stream);
+}
+
+extern "C" int pspmm_dense_mm_stalled(int32_t transA, int32_t transB, int64_t M, int64_t N, int64_t K, const float *A,
+                                      int64_t ldA, const float *B, int64_t ldB, float *C, int64_t ldC, void *scratch,
+                                      size_t scratch_bytes, void *stream)
+{
+    return dense_run(transA, transB, M, N, K, A, ldA, B, ldB, C, ldC, scratch, scratch_bytes, 20000000u, 1, stream);
 }
 
 extern "C" int pspmm_dense_status(int32_t *status)

@@ -796,6 +796,14 @@ def dense_mm(A, B, transA=False, transB=False, out=None):
     return out
 
 
+def dense_status():
+    """1 once a bounded wait of the dense product has run out in this process, else 0 (synchronises with the
+    device).  The rows of the result that were not computed are NaN then."""
+    v = ctypes.c_int32(0)
+    check(lib().pspmm_dense_status(ctypes.byref(v)))
+    return int(v.value)
+
+
 def _conv_forward(V, H, weight, rowPtr, colIdx, val, target_row, CF, W, product=None):
     """A @ (H @ W): dense GEMM (cuBLAS through torch.mm) then SpMM (SpCONV/SpCONV.h:43-193).
 

@@ -48,3 +48,34 @@ def test_no_wait_has_run_out():
     v = ctypes.c_int32(-1)
     _lib.check(_lib.lib().pspmm_dense_status(ctypes.byref(v)))
     assert v.value == 0
+
+
+_STALLED = """
+import ctypes, sys, torch
+sys.path.insert(0, %r)
+from paramspmm_ae_b200 import _lib, ops
+real = _lib.lib().pspmm_dense_mm
+for ta, tb, M, N, K in ((0, 0, 300, 40, 200), (0, 1, 300, 130, 64), (1, 0, 200, 50, 9000), (1, 1, 129, 17, 70),
+                        (0, 0, 40000, 256, 300), (1, 0, 40000, 47, 300)):
+    A, B = torch.randn(*((K, M) if ta else (M, K)), device="cuda"), torch.randn(*((N, K) if tb else (K, N)), device="cuda")
+    out = torch.zeros(M, N + 3, device="cuda")
+    _lib.lib().pspmm_dense_mm = _lib.lib().pspmm_dense_mm_stalled
+    ops.dense_mm(A, B, ta, tb, out=out[:, :N])
+    torch.cuda.synchronize()
+    assert ops.dense_status() == 1 and bool(out[:, :N].isnan().all()) and not bool(out[:, N:].any()), (ta, tb, M, N, K)
+    _lib.lib().pspmm_dense_mm = real  # the next product finds everything as it should be
+    want = (A.t() if ta else A).double() @ (B.t() if tb else B).double()
+    assert float((ops.dense_mm(A, B, ta, tb).double() - want).norm()) <= 1e-6 * float(want.norm()), (ta, tb, M, N, K)
+print("filled")
+"""
+
+
+def test_a_wait_that_runs_out_leaves_nan_and_the_status():
+    """One arrival per stage is withheld, so every wait gives up after 20 ms.  In a process of its own, since the
+    status stays set."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", _STALLED % root], capture_output=True, text=True, timeout=120)
+    assert p.returncode == 0 and "filled" in p.stdout, p.stdout[-500:] + p.stderr[-2000:]
