@@ -134,7 +134,8 @@ PSPMM_API int pspmm_spmm_bcsr(const int32_t *rowPtr_b, const int32_t *colIdx, co
  * The two products with scratch memory: 16-byte aligned, pspmm_spmm_scratch_bytes(n_rows, nnz, dim, V) bytes
  * (V = 1 for CSR; rows and entries count block-rows and blocks otherwise).  With it the rows of an
  * unsplit layout that have more than 64 entries are cut over the whole GPU instead of being walked by
- * one lane group each; their sums keep a fixed order.  Split layouts use no scratch.
+ * one lane group each; their sums keep a fixed order.  Split layouts use no scratch.  Scratch that is too
+ * small or not aligned is not used.
  */
 PSPMM_API int pspmm_spmm_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim, int32_t V, size_t *bytes);
 PSPMM_API int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, const float *val,

@@ -549,7 +549,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     // 26, 212 columns: 140 instead of 110; at most 5 us are lost elsewhere).
     a.dependent = target_row && !accumulate && !bucketed;
     a.lng = LongArgs{};
-    if (scratch && !target_row && !accumulate && !(cfg && cfg->no_long_rows) && n_entries > PSPMM_LONG_ROW) {
+    if (scratch && (uintptr_t)scratch % 16 == 0 && !target_row && !accumulate && !(cfg && cfg->no_long_rows) && n_entries > PSPMM_LONG_ROW) {
         const int lanes = pspmm_long_lanes(a.nvec, V);
         long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
         if (long_fits(a.lng, n_entries) &&

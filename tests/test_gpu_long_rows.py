@@ -93,6 +93,28 @@ def test_sums_of_long_rows_have_a_fixed_order(dim):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("offset, part", [(0, 1), (4, 1), (8, 1), (0, 2)])
+def test_scratch_that_cannot_be_used_is_not(oracle, offset, part):
+    """Partial sums are stored 16 bytes at a time: scratch off that boundary, or half of what is asked for,
+    leaves the plain walk, with the same product."""
+    import ctypes
+    from paramspmm_ae_b200 import _lib
+    dev, dim = torch.device("cuda:0"), 64
+    rp, ci, v = _matrix([5000, 3, 700, 2] * 3, 6001, 8)
+    n = len(rp) - 1
+    B = np.random.default_rng(9).uniform(-1, 1, (6001, dim)).astype(np.float32)
+    t = [torch.from_numpy(x).to(dev) for x in (rp, ci, v, B)]
+    need = ctypes.c_size_t(0)
+    _lib.check(_lib.lib().pspmm_spmm_scratch_bytes(n, len(ci), dim, 1, ctypes.byref(need)))
+    scratch = torch.full((need.value + 64,), 255, dtype=torch.uint8, device=dev)
+    out = torch.full((n, dim), float("nan"), device=dev)
+    _lib.check(_lib.lib().pspmm_spmm_csr_ws(*(x.data_ptr() for x in t), out.data_ptr(), n, 6001, len(ci), dim, dim, dim, None,
+                                            None, None, 0, scratch.data_ptr() + offset, need.value // part,
+                                            torch.cuda.current_stream().cuda_stream))
+    np.testing.assert_allclose(out.cpu().numpy(), oracle.spmm_csr(rp, ci, v, B), rtol=1e-5, atol=1e-4)
+    assert bool((scratch[need.value + offset:] == 255).all())
+
+
 def test_positions_beyond_32_bits():
     """Long rows of almost 2^31 entries: the positions that shares are counted in (entries plus one per row)
     pass 2^31.  Values of 0 and 1 make every share's sum exact; a hub's fewer than 200 shares are then
