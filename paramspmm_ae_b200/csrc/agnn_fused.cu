@@ -107,23 +107,24 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
     float m = state.m, l = state.l;
     float (&acc)[CF][VW] = state.acc;
     const int len = hb - lb;
+    const unsigned ub = lb, ue = hb;  // (lb and the longest range of the warp can add up to more than 2^31)
     const int sub = gl % BS;  // position inside the batch this lane answers for
 
     // Column indices are read LPR at a time (lane gl <-> entry gl of the chunk, one coalesced
     // load) and one chunk ahead, so that their latency is not part of the per-batch chain.
-    int c_next = (lb + gl < hb) ? __ldg(a.colIdx + lb + gl) : 0;
+    int c_next = (ub + gl < ue) ? __ldg(a.colIdx + (ub + gl)) : 0;
     for (int off0 = 0; off0 < maxlen; off0 += LPR) {
         const int c_chunk = c_next;
         {
-            const int kn = lb + off0 + LPR + gl;
-            c_next = (kn < hb) ? __ldg(a.colIdx + kn) : 0;
+            const unsigned kn = ub + off0 + LPR + gl;
+            c_next = (kn < ue) ? __ldg(a.colIdx + kn) : 0;
         }
 #pragma unroll
         for (int b = 0; b < LPR / BS; ++b) {
             const int off = off0 + b * BS;
             if (off >= maxlen)
                 break;  // warp-uniform
-            const bool mine = (lb + off + sub) < hb;
+            const bool mine = (ub + off + sub) < ue;
             FVec<VW> x[BS][CF];
             FVec<VW> y[SEP ? BS : 1][SEP ? CF : 1];  // the rows that are aggregated, when they are not B's
             float part[BS];

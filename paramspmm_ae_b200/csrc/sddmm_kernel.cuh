@@ -49,6 +49,7 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
     constexpr int U = U1 > LPR ? LPR : U1;
     const int tiles = (a.nvec + LPR * CF - 1) / (LPR * CF);
     const int len = hb - lb;
+    const unsigned ub = lb, ue = hb;  // (lb and maxlen can add up to more than 2^31)
     const bool live = len > 0;
     for (int off = 0; off < maxlen; off += CHUNK) {
         int ccol[ENT];
@@ -56,8 +57,8 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
         float res[ENT][V];
 #pragma unroll
         for (int t = 0; t < ENT; ++t) {
-            const int k = lb + off + t * LPR + gl;
-            const bool ok = k < hb;
+            const unsigned k = ub + off + t * LPR + gl;
+            const bool ok = k < ue;
             ccol[t] = ok ? __ldg(a.colIdx + k) : 0;
 #pragma unroll
             for (int w = 0; w < V; ++w) {
@@ -124,8 +125,8 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
         }
 #pragma unroll
         for (int t = 0; t < ENT; ++t) {
-            const int k = lb + off + t * LPR + gl;
-            if (k < hb) {
+            const unsigned k = ub + off + t * LPR + gl;
+            if (k < ue) {
 #pragma unroll
                 for (int w = 0; w < V; ++w) {
                     // Block layouts: positions whose stored value is zero are not part of
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
                 if (i < n) {
                     row = row_list[i];
                     lb = row_lo[i] + (p - piece0) * 32;
-                    hb = lb + 32 < row_hi[i] ? lb + 32 : row_hi[i];
+                    hb = row_hi[i] - lb > 32 ? lb + 32 : row_hi[i];
                 }
                 sddmm_entries<LPR, VW, CF, V>(a, row, lb, hb, 32, gl);
             }

@@ -142,3 +142,37 @@ def test_positions_beyond_32_bits():
     A[:, 0] = 1.0  # every score is one
     got = ops.agnn_fused(A, Bd, rpd, ci, 1.0, False)
     np.testing.assert_allclose(got.cpu().numpy(), want, rtol=2e-5)
+
+
+@pytest.mark.parametrize("dim", [4, 64])
+def test_ranges_that_end_near_the_index_limit(dim):
+    """A piece of 300,000 entries beside pieces of three whose entries lie 180,000 below 2^31: their groups run
+    along to the longest range of the warp, past 2^31.  (The row pointer starts high; small whole values
+    make every sum exact.)"""
+    from paramspmm_ae_b200 import ops
+    dev, n_cols, first = torch.device("cuda:0"), 4096, 2_147_000_000
+    ln = torch.tensor([300_000, 3, 3, 0, 5, 3, 1, 3, 3, 40, 3])
+    rp = first + torch.cat([torch.zeros(1, dtype=torch.int64), ln.cumsum(0)])
+    n, nnz = len(ln), int(rp[-1])
+    assert nnz < 2**31 <= nnz + 300_000
+    ci = torch.arange(nnz, dtype=torch.int32, device=dev).bitwise_and_(n_cols - 1)
+    g = torch.Generator().manual_seed(3)
+    B = torch.randint(0, 2, (n_cols, dim), generator=g).float()
+    B[:, 0] = 1.0
+    A = torch.randint(0, 4, (n, dim), generator=g).float()
+    cols, row = ci[first:].cpu().long(), torch.repeat_interleave(torch.arange(n), ln)
+    e0 = torch.zeros(n, dim)
+    e0[:, 0] = 1.0  # every score is one
+    want = torch.zeros(n, dim).index_add_(0, row, B[cols])
+    target = torch.arange(n, dtype=torch.int32, device=dev)
+    rpd, Ad, Bd = rp.int().to(dev), A.to(dev), B.to(dev)
+    got = ops.agnn_fused(e0.to(dev), Bd, rpd, ci, 1.0, False, target_row=target, n_out_rows=n)
+    assert torch.equal(got.cpu(), want)
+    got = ops.agnn_fused(e0.to(dev), Bd, rpd, ci, 1.0, False)
+    assert torch.equal(got.cpu(), want)
+    scores = (A[row] * B[cols]).sum(1)
+    val = torch.empty(nnz, device=dev)
+    got = ops.csr_split_sddmm(Ad, Bd, rpd, ci, val, target, 1, 8)[first:]
+    assert torch.equal(got.cpu(), scores)
+    got = ops.csr_sddmm(Ad, Bd, rpd, ci, val, 1, 8)[first:]
+    assert torch.equal(got.cpu(), scores)
