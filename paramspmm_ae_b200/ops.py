@@ -812,10 +812,10 @@ def _conv_forward(V, H, weight, rowPtr, colIdx, val, target_row, CF, W, product=
     SpMM runs with 128-bit accesses on 16-byte aligned rows; the extra column is dropped from the
     result.  ``product`` replaces the SpMM launch (an operator bound to a decider plan).
 
-    The projection stays an fp32 multiply-add chain in cuBLAS's order: its last bit decides which side of
-    zero some pre-activations fall on, and with a ReLU behind the layer the gradients of a 2.4 M node
-    network move by 1e-4 when it changes (``dense_mm`` is the more accurate of the two).  The backward
-    products decide nothing and run on the tensor cores."""
+    The projection is a cuBLAS fp32 product, the backward products run on the tensor cores
+    (``dense_mm``, no less accurate).  What keeps the forward there is comparability alone: its last bit
+    decides which side of zero a few pre-activations fall on, and with a ReLU behind the layer the gradients of a
+    2.4 M node network then differ in the fifth digit between builds."""
     _check_legacy(CF, W, max_cf=4)  # SpCONV/SpCONV.cpp:93-104
     fout = weight.shape[1]
     HW = torch.mm(H, _pad_cols(weight, -fout % 4))
