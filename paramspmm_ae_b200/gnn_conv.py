@@ -109,13 +109,22 @@ def _can_fuse(P, dim):
 
 def _is_operator_colidx(P, colIdx):
     """The fused backward weights edges by the operator's own column ids; callers pass them as an
-    [nnz, 1] column (GNN.py:224-225).  Checked once per (operator, tensor) pair, not per step."""
-    seen = P.__dict__.setdefault("_colidx_checked", {})
-    key = (colIdx.data_ptr(), tuple(colIdx.shape))
-    if key not in seen:
-        flat = colIdx.reshape(-1)
-        seen[key] = bool(flat.shape == P.colIdx.shape and flat.dtype == P.colIdx.dtype and torch.equal(flat, P.colIdx))
-    return seen[key]
+    [nnz, 1] column (GNN.py:224-225).  Compared once per content of a tensor, not per step: the operator holds
+    the last one it compared, so that its memory is not another tensor's meanwhile, and its version."""
+    own = P.colIdx
+    if colIdx.is_inference() or own.is_inference():  # (these keep no version)
+        return _same_entries(colIdx, own)
+    seen = P.__dict__.get("_colidx_checked")
+    if seen is None or own is not seen[1] or (colIdx._version, own._version) != seen[2] or (
+            colIdx is not seen[0] and (colIdx.data_ptr() != seen[0].data_ptr() or colIdx.shape != seen[0].shape
+                                       or colIdx.stride() != seen[0].stride() or colIdx.dtype != seen[0].dtype)):
+        seen = P._colidx_checked = (colIdx, own, (colIdx._version, own._version), _same_entries(colIdx, own))
+    return seen[3]
+
+
+def _same_entries(colIdx, own):
+    flat = colIdx.reshape(-1)
+    return bool(flat.shape == own.shape and flat.dtype == own.dtype and torch.equal(flat, own))
 
 
 class AGNNFunction(torch.autograd.Function):

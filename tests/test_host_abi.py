@@ -447,3 +447,23 @@ def test_the_long_rows_flag_is_a_flag_of_the_spmm(pspmm_lib):
                                     ctypes.byref(_lib.make_cfg(no_long_rows=2)), null, null, 0, null) == _lib.PSPMM_E_CONFIG
     assert pspmm_lib.pspmm_sddmm_csr(one, one, one, one, one, 4, 4, 16, 16, 16,
                                      ctypes.byref(_lib.make_cfg(no_long_rows=1)), null, null, 0, null) == _lib.PSPMM_E_CONFIG
+
+
+def test_edge_columns_are_compared_again_when_they_change():
+    """The fused attention layer weights edges by the operator's own columns; the tensor a caller hands in is
+    compared with them once, and again when it was written to or is another one."""
+    import types
+    from paramspmm_ae_b200 import gnn_conv
+    P = types.SimpleNamespace(colIdx=torch.arange(7, dtype=torch.int32))
+    edges = P.colIdx.clone().unsqueeze(-1)
+    assert gnn_conv._is_operator_colidx(P, edges) and gnn_conv._is_operator_colidx(P, edges)
+    held = P._colidx_checked
+    assert gnn_conv._is_operator_colidx(P, edges[:]) and P._colidx_checked is held  # (a view of the same entries)
+    edges[3] = 0
+    assert not gnn_conv._is_operator_colidx(P, edges)
+    edges[3] = 3
+    assert gnn_conv._is_operator_colidx(P, edges)
+    P.colIdx[0] = 5
+    assert not gnn_conv._is_operator_colidx(P, edges)
+    with torch.inference_mode():
+        assert gnn_conv._is_operator_colidx(P, P.colIdx.clone())
