@@ -769,22 +769,23 @@ def dense_mm(A, B, transA=False, transB=False, out=None):
     CPU tensors, column-strided views, an enabled autocast) go to ``torch.mm``, which is what the
     reference calls (SpCONV/SpCONV.h:43-72); so do operands on two devices, for its error.  Operands on
     another GPU than the current one are multiplied there."""
-    ok = True
+    gpu = A.get_device()  # (-1 on the CPU)
+    ok = A.is_cuda and B.get_device() == gpu
     for t in (A, B):
-        ok = ok and t.is_cuda and t.dtype is torch.float32 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1]
-    if not ok or A.get_device() != B.get_device() or torch.is_autocast_enabled():
+        ok = ok and t.dtype is torch.float32 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) >= t.shape[1]
+    if not ok or torch.is_autocast_enabled():
         r = torch.mm(A.t() if transA else A, B.t() if transB else B)
         return r if out is None else out.copy_(r)
     K, M = A.shape if transA else A.shape[::-1]
     N, Kb = B.shape if transB else B.shape[::-1]
     if K != Kb:
         raise RuntimeError("mat1 and mat2 shapes cannot be multiplied (%dx%d and %dx%d)" % (M, K, Kb, N))
-    if A.get_device() != torch._C._cuda_getDevice():
-        with torch.cuda.device(A.get_device()):
+    if gpu != torch._C._cuda_getDevice():
+        with torch.cuda.device(gpu):
             return dense_mm(A, B, transA, transB, out)
     if out is None:
         out = torch.empty((M, N), dtype=torch.float32, device=A.device)
-    elif (out.get_device() != A.get_device() or out.dtype is not torch.float32 or tuple(out.shape) != (M, N)
+    elif (out.get_device() != gpu or out.dtype is not torch.float32 or tuple(out.shape) != (M, N)
           or out.stride(1) != 1 or out.stride(0) < N):
         raise RuntimeError("out must be a float32 tensor of %d rows of %d columns with unit column stride on the operands' "
                            "device" % (M, N))
