@@ -110,6 +110,28 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
     const unsigned ub = lb, ue = hb;  // (lb and the longest range of the warp can add up to more than 2^31)
     const int sub = gl % BS;  // position inside the batch this lane answers for
 
+    // The rows of a batch, and those that are aggregated when they are not B's.  Beyond a row's entries the 16-byte
+    // forms with several slices per lane keep an earlier batch's and leave it out of the sums: clearing it took an
+    // instruction per float, and that, the addresses and the loads of idle lanes were a third of all
+    // (12 M entries, softmax: dim 100 584 -> 474 us, dim 148 1074 -> 867).  With one slice or 32-byte loads the
+    // zeros are free (dim 128 487, without them 489; dim 32 160 and 167, dim 16 44 and 46).
+    constexpr bool KEEP = VW == 4 && CF > 1;
+    FVec<VW> x[BS][CF];
+    FVec<VW> y[SEP ? BS : 1][SEP ? CF : 1];
+    const float *laneB = a.B + gl * VW, *laneV = a.Vm + gl * VW;
+    const unsigned ldB_lo = (unsigned)(a.ldB * 4), ldB_hi = (unsigned)((unsigned long long)(a.ldB * 4) >> 32);
+    const unsigned ldV_lo = (unsigned)(a.ldV * 4), ldV_hi = (unsigned)((unsigned long long)(a.ldV * 4) >> 32);
+    if constexpr (KEEP) {
+#pragma unroll
+        for (int e = 0; e < BS; ++e)
+#pragma unroll
+            for (int cf = 0; cf < CF; ++cf) {
+                x[e][cf] = zero_vec<VW>();
+                if constexpr (SEP)
+                    y[e][cf] = zero_vec<VW>();
+            }
+    }
+
     // Column indices are read LPR at a time (lane gl <-> entry gl of the chunk, one coalesced
     // load) and one chunk ahead, so that their latency is not part of the per-batch chain.
     int c_next = (ub + gl < ue) ? __ldg(a.colIdx + (ub + gl)) : 0;
@@ -125,8 +147,6 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
             if (off >= maxlen)
                 break;  // warp-uniform
             const bool mine = (ub + off + sub) < ue;
-            FVec<VW> x[BS][CF];
-            FVec<VW> y[SEP ? BS : 1][SEP ? CF : 1];  // the rows that are aggregated, when they are not B's
             float part[BS];
             int ce[BS];
 #pragma unroll
@@ -137,16 +157,29 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
             // (115 M entries at dim 64: 2.7 ms with the branch, 2.2 without; with two operands 5.2, 3.6).
 #pragma unroll
             for (int e = 0; e < BS; ++e) {
-                const float *brow = a.B + (int64_t)ce[e] * a.ldB;
                 const bool on = (off + e) < len;
-#pragma unroll
-                for (int cf = 0; cf < CF; ++cf)
-                    x[e][cf] = ldg_vec_if<VW>(brow + voff[cf], on);
-                if constexpr (SEP) {
-                    const float *vrow = a.Vm + (int64_t)ce[e] * a.ldV;
+                if constexpr (KEEP) {
+                    const float *brow = row_start(laneB, ce[e], ldB_lo, ldB_hi);
 #pragma unroll
                     for (int cf = 0; cf < CF; ++cf)
-                        y[e][cf] = ldg_vec_if<VW>(vrow + voff[cf], on);
+                        ldg_vec_keep<VW>(x[e][cf], brow + cf * LPR * VW, on && act[cf]);
+                    if constexpr (SEP) {
+                        const float *vrow = row_start(laneV, ce[e], ldV_lo, ldV_hi);
+#pragma unroll
+                        for (int cf = 0; cf < CF; ++cf)
+                            ldg_vec_keep<VW>(y[e][cf], vrow + cf * LPR * VW, on && act[cf]);
+                    }
+                } else {
+                    const float *brow = a.B + (int64_t)ce[e] * a.ldB;
+#pragma unroll
+                    for (int cf = 0; cf < CF; ++cf)
+                        x[e][cf] = ldg_vec_if<VW>(brow + voff[cf], on);
+                    if constexpr (SEP) {
+                        const float *vrow = a.Vm + (int64_t)ce[e] * a.ldV;
+#pragma unroll
+                        for (int cf = 0; cf < CF; ++cf)
+                            y[e][cf] = ldg_vec_if<VW>(vrow + voff[cf], on);
+                    }
                 }
             }
 #pragma unroll
@@ -198,21 +231,24 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
                             for (int i = 0; i < VW; ++i)
                                 d = fmaf(state.vv[cf].v[i], y[e][cf].v[i], d);
                         }
-                    state.t = fmaf((float)ce[e], d, state.t);
+                    if (!KEEP || (off + e) < len)
+                        state.t = fmaf((float)ce[e], d, state.t);
                 }
             }
 #pragma unroll
             for (int e = 0; e < BS; ++e) {
                 const float pe = __shfl_sync(PSPMM_FULL_MASK, p, e, BS);
 #pragma unroll
-                for (int cf = 0; cf < CF; ++cf)
+                for (int cf = 0; cf < CF; ++cf) {
+                    const FVec<VW> &r = SEP ? y[SEP ? e : 0][SEP ? cf : 0] : x[e][cf];
+                    if constexpr (KEEP) {
+                        fma_vec_if<VW>(acc[cf], pe, r.v, (off + e) < len);
+                    } else {
 #pragma unroll
-                    for (int i = 0; i < VW; ++i) {
-                        if constexpr (SEP)
-                            acc[cf][i] = fmaf(pe, y[e][cf].v[i], acc[cf][i]);
-                        else
-                            acc[cf][i] = fmaf(pe, x[e][cf].v[i], acc[cf][i]);
+                        for (int i = 0; i < VW; ++i)
+                            acc[cf][i] = fmaf(pe, r.v[i], acc[cf][i]);
                     }
+                }
             }
         }
     }

@@ -137,6 +137,38 @@ __device__ __forceinline__ FVec<VW> ldg_vec_if(const float *p, bool on)
     return r;
 }
 
+// The same load without the zeros: r keeps what it held when `on` is false.  For users that leave that out of every
+// result.
+template <int VW>
+__device__ __forceinline__ void ldg_vec_keep(FVec<VW> &r, const float *p, bool on)
+{
+    static_assert(VW == 4, "");
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3])
+        : "l"(p), "r"(on ? 1 : 0));
+}
+
+// acc[i] += s * x[i] where `on`, without a branch.
+template <int VW>
+__device__ __forceinline__ void fma_vec_if(float (&acc)[VW], float s, const float (&x)[VW], bool on)
+{
+    static_assert(VW == 4, "");
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %9, 0;\n\t@q fma.rn.f32 %0, %8, %4, %0;\n\t@q fma.rn.f32 %1, %8, %5, %1;\n\t"
+        "@q fma.rn.f32 %2, %8, %6, %2;\n\t@q fma.rn.f32 %3, %8, %7, %3;\n\t}"
+        : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+        : "f"(x[0]), "f"(x[1]), "f"(x[2]), "f"(x[3]), "f"(s), "r"(on ? 1 : 0));
+}
+
+// Address of dense row c: base + c * ld_bytes, whatever the row stride (its high word is zero below 4 GiB).
+__device__ __forceinline__ const float *row_start(const float *base, int c, unsigned ld_lo, unsigned ld_hi)
+{
+    unsigned long long r;
+    asm("{\n\t.reg .b32 l, h;\n\tmad.wide.u32 %0, %1, %2, %4;\n\tmov.b64 {l, h}, %0;\n\t"
+        "mad.lo.u32 h, %1, %3, h;\n\tmov.b64 %0, {l, h};\n\t}"
+        : "=l"(r) : "r"((unsigned)c), "r"(ld_lo), "r"(ld_hi), "l"(base));
+    return reinterpret_cast<const float *>(r);
+}
+
 template <int VW>
 __device__ __forceinline__ FVec<VW> zero_vec()
 {
