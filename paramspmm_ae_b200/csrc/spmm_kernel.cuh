@@ -50,8 +50,10 @@ struct SpmmTile {
     static constexpr int GROUP_WORDS = HEAD_WORDS + CAP * (1 + V);
 };
 
-// One batch of UU entries starting at shared-memory index e: gathers first, FMAs after.
-template <int UU, int LPR, int VW, int CF, int V>
+// One batch of UU entries starting at shared-memory index e: gathers first, FMAs after.  PACK takes two columns per
+// multiply-add: the long rows' kernel gains 3 - 7 % (R-MAT of 16 M entries unsplit, 32 columns: 478 -> 454 us; power
+// law of 2.5 M 67.6 -> 62.8), the segment kernel loses as much: its register budgets have no room for pairs.
+template <int UU, int LPR, int VW, int CF, int V, bool PACK>
 __device__ __forceinline__ void spmm_batch(const int *ent, int e, const char *const (&bcol)[CF],
                                            unsigned ldB_bytes, unsigned long long keep,
                                            float (&acc)[V][CF][VW])
@@ -86,41 +88,46 @@ __device__ __forceinline__ void spmm_batch(const int *ent, int e, const char *co
             if (V > 1 && v[u][w] == 0.f)
                 continue;
 #pragma unroll
-            for (int cf = 0; cf < CF; ++cf)
+            for (int cf = 0; cf < CF; ++cf) {
+                if constexpr (PACK) {
+                    fma_vec<VW>(acc[w][cf], v[u][w], x[u][cf].v);
+                } else {
 #pragma unroll
-                for (int i = 0; i < VW; ++i)
-                    acc[w][cf][i] = fmaf(v[u][w], x[u][cf].v[i], acc[w][cf][i]);
+                    for (int i = 0; i < VW; ++i)
+                        acc[w][cf][i] = fmaf(v[u][w], x[u][cf].v[i], acc[w][cf][i]);
+                }
+            }
         }
 }
 
 // Entries [e, eh) of the staged window: batches of U, the tail in halves of it.
-template <int U, int LPR, int VW, int CF, int V>
+template <int U, int LPR, int VW, int CF, int V, bool PACK = false>
 __device__ __forceinline__ void spmm_entries(const int *ent, int e, int eh, const char *const (&bcol)[CF],
                                              unsigned ldB_bytes, unsigned long long keep, float (&acc)[V][CF][VW])
 {
     for (; e + U <= eh; e += U)
-        spmm_batch<U, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+        spmm_batch<U, LPR, VW, CF, V, PACK>(ent, e, bcol, ldB_bytes, keep, acc);
     if constexpr (U >= 16) {
         if (e + 8 <= eh) {
-            spmm_batch<8, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            spmm_batch<8, LPR, VW, CF, V, PACK>(ent, e, bcol, ldB_bytes, keep, acc);
             e += 8;
         }
     }
     if constexpr (U >= 8) {
         if (e + 4 <= eh) {
-            spmm_batch<4, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            spmm_batch<4, LPR, VW, CF, V, PACK>(ent, e, bcol, ldB_bytes, keep, acc);
             e += 4;
         }
     }
     if constexpr (U >= 4) {
         if (e + 2 <= eh) {
-            spmm_batch<2, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            spmm_batch<2, LPR, VW, CF, V, PACK>(ent, e, bcol, ldB_bytes, keep, acc);
             e += 2;
         }
     }
     if constexpr (U >= 2) {
         if (e < eh)
-            spmm_batch<1, LPR, VW, CF, V>(ent, e, bcol, ldB_bytes, keep, acc);
+            spmm_batch<1, LPR, VW, CF, V, PACK>(ent, e, bcol, ldB_bytes, keep, acc);
     }
 }
 
@@ -397,7 +404,7 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongAr
                 const int fill = row_stop - p < CAP ? row_stop - p : CAP;
                 spmm_stage<LPR, V>(a, ent, from + p, fill, gl, stream);
                 __syncwarp(gmask);
-                spmm_entries<U, LPR, VW, 1, V>(ent, 0, fill, bcol, ldB_bytes, keep, acc);
+                spmm_entries<U, LPR, VW, 1, V, true>(ent, 0, fill, bcol, ldB_bytes, keep, acc);
                 __syncwarp(gmask);
                 p += fill;
             }

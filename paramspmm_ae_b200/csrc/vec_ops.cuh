@@ -137,6 +137,24 @@ __device__ __forceinline__ FVec<VW> ldg_vec_if(const float *p, bool on)
     return r;
 }
 
+// acc[i] = s * x[i] + acc[i] over VW floats, two of them per instruction (sm_100's packed fp32 multiply-add
+// rounds each half as fmaf does).
+template <int VW>
+__device__ __forceinline__ void fma_vec(float (&acc)[VW], float s, const float (&x)[VW])
+{
+    if constexpr (VW >= 2) {
+        unsigned long long ss;
+        asm("mov.b64 %0, {%1, %1};" : "=l"(ss) : "f"(s));
+#pragma unroll
+        for (int i = 0; i < VW; i += 2)
+            asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\t"
+                "fma.rn.f32x2 a, b, %4, a;\n\tmov.b64 {%0, %1}, a;\n\t}"
+                : "+f"(acc[i]), "+f"(acc[i + 1]) : "f"(x[i]), "f"(x[i + 1]), "l"(ss));
+    } else {
+        acc[0] = fmaf(s, x[0], acc[0]);
+    }
+}
+
 // The same load without the zeros: r keeps what it held when `on` is false.  For users that leave that out of every
 // result.
 template <int VW>
