@@ -289,6 +289,18 @@ PSPMM_API int pspmm_agnn_layer_forward(const int32_t *rowPtr, const int32_t *col
                                        int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX, int64_t ldOut,
                                        const float *beta, const int32_t *rowPtr_split, const int32_t *target_row,
                                        int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream);
+/* The same passes with the scores beta <X_i, X_j> kept between them, one float per entry: the forward writes
+ * scores[nnz] (NULL: it does not), the backward takes them instead of gathering the rows of X once more. */
+PSPMM_API int pspmm_agnn_layer_forward_scores(const int32_t *rowPtr, const int32_t *colIdx, const float *X, float *out,
+                                              float *scores, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX,
+                                              int64_t ldOut, const float *beta, const int32_t *rowPtr_split,
+                                              const int32_t *target_row, int64_t n_seg, void *scratch,
+                                              size_t scratch_bytes, void *stream);
+PSPMM_API int pspmm_agnn_layer_backward_scores(const int32_t *rowPtr, const int32_t *colIdx, const float *scores,
+                                               const float *G, float *D, float *d_beta, int64_t n_rows, int64_t nnz,
+                                               int32_t dim, int64_t ldG, int64_t ldD, const int32_t *rowPtr_split,
+                                               const int32_t *target_row, int64_t n_seg, void *scratch,
+                                               size_t scratch_bytes, void *stream);
 PSPMM_API int pspmm_agnn_layer_backward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, const float *G,
                                         float *D, float *d_beta, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX,
                                         int64_t ldG, int64_t ldD, const float *beta, const int32_t *rowPtr_split,

@@ -96,6 +96,10 @@ _SIGNATURES = {
     "pspmm_agnn_layer_scratch_bytes": [_i64, _i64, _i64, _i32, ctypes.POINTER(ctypes.c_size_t)],
     "pspmm_agnn_layer_forward": [_vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp, _vp, _vp, _i64, _vp,
                                  ctypes.c_size_t, _vp],
+    "pspmm_agnn_layer_forward_scores": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp, _vp, _vp, _i64, _vp,
+                                        ctypes.c_size_t, _vp],
+    "pspmm_agnn_layer_backward_scores": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _vp, _vp, _i64, _vp,
+                                         ctypes.c_size_t, _vp],
     "pspmm_agnn_layer_backward": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _i64,
                                   _vp, ctypes.c_size_t, _vp],
     "pspmm_agnn_fused_apply_csr": [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _i64, _i64,

@@ -46,11 +46,15 @@ struct AgnnArgs {
     float beta;
     const float *beta_dev;  // where beta lies on the device, or nullptr: `beta`
     int32_t softmax;
+    float *scores;          // scores per entry: SCORES_LEAVE kernels write them, SCORES_TAKE kernels read them
     double *col_sums;       // COL kernels: one partial sum per CTA
     int32_t n_col_sums;     // CTAs of the first kernel that own segments, then the shares of long rows
     float *col_out;
     LongArgs lng;  // unsplit layouts: how long rows are cut (totals == nullptr: they are not)
 };
+
+// What a kernel does with a.scores.
+enum { SCORES_NONE, SCORES_LEAVE, SCORES_TAKE };
 
 // Sum over the CTA's 256 threads, stored by thread 0.
 __device__ __forceinline__ void cta_sum_to(double *dst, double x)
@@ -99,7 +103,7 @@ struct AgnnState {
 
 // The entries [lb, hb) of one row for one lane group.  Every lane of the warp calls this together;
 // `maxlen` is the longest of the warp's ranges and a group without work passes lb == hb.
-template <int LPR, int CF, int BS, int VW, bool SEP, bool COL>
+template <int LPR, int CF, int BS, int VW, bool SEP, bool COL, int SCORES>
 __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (&av)[CF], const bool (&act)[CF],
                                              const int (&voff)[CF], int lb, int hb, int maxlen, int gl,
                                              AgnnState<CF, VW, COL> &state)
@@ -220,6 +224,10 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
             } else {
                 p = mine ? score : 0.f;
             }
+            if constexpr (SCORES == SCORES_LEAVE) {
+                if (mine && gl < BS)
+                    __stcs(a.scores + (ub + off + sub), score);
+            }
             if constexpr (COL) {
 #pragma unroll
                 for (int e = 0; e < BS; ++e) {
@@ -256,7 +264,71 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
     state.l = l;
 }
 
-template <int LPR, int CF, int VW, bool COL>
+// The same for scores that lie in a.scores: one gather per entry (the rows of a.Vm) and no exchange.  A training
+// step's backward pass takes the forward's: 115 M entries, dim 64: 3.64 ms with the scores recomputed from a
+// second gather, 1.77 (16.5 TB/s of gathered rows; the bare gather takes 1.4); the forward writes them in 0.09 ms of 1.89.
+// Bound: the latency of eight 32-byte loads in flight per lane at two resident CTAs.
+template <int LPR, int CF, int BS, int VW, bool COL>
+__device__ __forceinline__ void agnn_scored_entries(const AgnnArgs &a, const bool (&act)[CF], const int (&voff)[CF], int lb,
+                                                    int hb, int maxlen, int gl, AgnnState<CF, VW, COL> &state)
+{
+    const int len = hb - lb;
+    const unsigned ub = lb, ue = hb;
+    int c_next = 0;
+    float p_next = 0.f;
+    auto fetch = [&](unsigned k) {  // lane gl <-> entry gl of a chunk, one chunk ahead
+        c_next = k < ue ? __ldg(a.colIdx + k) : 0;
+        p_next = k < ue ? __ldcs(a.scores + k) : 0.f;
+    };
+    fetch(ub + gl);
+    for (int off0 = 0; off0 < maxlen; off0 += LPR) {
+        const int c_chunk = c_next;
+        const float p_chunk = p_next;
+        fetch(ub + off0 + LPR + gl);
+#pragma unroll
+        for (int b = 0; b < LPR / BS; ++b) {
+            const int off = off0 + b * BS;
+            if (off >= maxlen)
+                break;  // warp-uniform
+            FVec<VW> y[BS][CF];
+            float pe[BS];
+            int ce[BS];
+#pragma unroll
+            for (int e = 0; e < BS; ++e) {
+                ce[e] = __shfl_sync(PSPMM_FULL_MASK, c_chunk, b * BS + e, LPR);
+                pe[e] = __shfl_sync(PSPMM_FULL_MASK, p_chunk, b * BS + e, LPR);
+            }
+#pragma unroll
+            for (int e = 0; e < BS; ++e) {
+                const float *vrow = a.Vm + (int64_t)ce[e] * a.ldV;
+#pragma unroll
+                for (int cf = 0; cf < CF; ++cf)
+                    y[e][cf] = ldg_vec_if<VW>(vrow + voff[cf], (off + e) < len);
+            }
+#pragma unroll
+            for (int e = 0; e < BS; ++e) {
+                if constexpr (COL) {
+                    float d = 0.f;
+#pragma unroll
+                    for (int cf = 0; cf < CF; ++cf)
+                        if (act[cf]) {
+#pragma unroll
+                            for (int i = 0; i < VW; ++i)
+                                d = fmaf(state.vv[cf].v[i], y[e][cf].v[i], d);
+                        }
+                    state.t = fmaf((float)ce[e], d, state.t);
+                }
+#pragma unroll
+                for (int cf = 0; cf < CF; ++cf)
+#pragma unroll
+                    for (int i = 0; i < VW; ++i)
+                        state.acc[cf][i] = fmaf(pe[e], y[e][cf].v[i], state.acc[cf][i]);
+            }
+        }
+    }
+}
+
+template <int LPR, int CF, int VW, bool COL, int SCORES>
 __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bool live, int gl, FVec<VW> (&av)[CF],
                                               bool (&act)[CF], int (&voff)[CF], AgnnState<CF, VW, COL> &state)
 {
@@ -266,7 +338,8 @@ __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bo
         const int v = cf * LPR + gl;
         act[cf] = v < nvec;
         voff[cf] = act[cf] ? v * VW : 0;
-        av[cf] = (live && act[cf]) ? ldg_vec<VW>(a.A + row * a.ldA + voff[cf]) : zero_vec<VW>();
+        if constexpr (SCORES != SCORES_TAKE)
+            av[cf] = (live && act[cf]) ? ldg_vec<VW>(a.A + row * a.ldA + voff[cf]) : zero_vec<VW>();
         if constexpr (COL)
             state.vv[cf] = (live && act[cf]) ? ldg_vec<VW>(a.Vm + row * a.ldV + voff[cf]) : zero_vec<VW>();
 #pragma unroll
@@ -284,7 +357,7 @@ struct AgnnOcc {
     static constexpr int MIN_CTAS = SEP ? (CF * VW >= 16 ? 1 : 2) : (CF * VW >= 16 ? 2 : 3);
 };
 
-template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false>
+template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false, int SCORES = SCORES_NONE>
 __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fused_kernel(const AgnnArgs a)
 {
     static_assert(BS <= LPR, "a batch cannot be wider than the lane group");
@@ -323,11 +396,14 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fuse
     AgnnState<CF, VW, COL> st;
     st.beta = a.beta_dev ? __ldg(a.beta_dev) : a.beta;
     st.t = 0.f;
-    agnn_load_row<LPR, CF, VW, COL>(a, row, live, gl, av, act, voff, st);
+    agnn_load_row<LPR, CF, VW, COL, SCORES>(a, row, live, gl, av, act, voff, st);
     int maxlen = hb - lb;
     if constexpr (LPR < 32)
         maxlen = __reduce_max_sync(PSPMM_FULL_MASK, maxlen);
-    agnn_entries<LPR, CF, BS, VW, SEP, COL>(a, av, act, voff, lb, hb, maxlen, gl, st);
+    if constexpr (SCORES == SCORES_TAKE)
+        agnn_scored_entries<LPR, CF, BS, VW, COL>(a, act, voff, lb, hb, maxlen, gl, st);
+    else
+        agnn_entries<LPR, CF, BS, VW, SEP, COL, SCORES>(a, av, act, voff, lb, hb, maxlen, gl, st);
     if constexpr (COL)
         cta_sum_to(a.col_sums + (blockIdx.x - a.lng.scan_ctas), (double)st.t);
     if (!live)
@@ -362,7 +438,7 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fuse
 // The entries of a share are dealt to the lane groups in equal spans; a group's states (maximum, sum,
 // accumulator) at the ends of its span and the shares' states of a row meet in shared memory and in
 // scratch as the pieces of a split row do.
-template <int LPR, int CF, int BS, int VW, bool SEP, bool COL>
+template <int LPR, int CF, int BS, int VW, bool SEP, bool COL, int SCORES>
 __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long_kernel(const AgnnArgs a)
 {
     constexpr int G = 256 / LPR;
@@ -393,7 +469,7 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long
         AgnnState<CF, VW, COL> st;
         st.beta = a.beta_dev ? __ldg(a.beta_dev) : a.beta;
         st.t = 0.f;
-        agnn_load_row<LPR, CF, VW, COL>(a, sh.row[i], p < stop, gl, av, act, voff, st);
+        agnn_load_row<LPR, CF, VW, COL, SCORES>(a, sh.row[i], p < stop, gl, av, act, voff, st);
         bool from_row_start = p < stop && p == job.off(sh, i);
         while (__any_sync(PSPMM_FULL_MASK, p < stop)) {
             int lb = 0, count = 0, row_end = 0;
@@ -404,7 +480,10 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long
                 lb = sh.lo[i] - job.off(sh, i) + p;
             }
             const int longest = LPR < 32 ? __reduce_max_sync(PSPMM_FULL_MASK, count) : count;
-            agnn_entries<LPR, CF, BS, VW, SEP, COL>(a, av, act, voff, lb, lb + count, longest, gl, st);
+            if constexpr (SCORES == SCORES_TAKE)
+                agnn_scored_entries<LPR, CF, BS, VW, COL>(a, act, voff, lb, lb + count, longest, gl, st);
+            else
+                agnn_entries<LPR, CF, BS, VW, SEP, COL, SCORES>(a, av, act, voff, lb, lb + count, longest, gl, st);
             if (count == 0)
                 continue;
             p += count;
@@ -445,7 +524,7 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long
             }
             ++i;
             from_row_start = true;
-            agnn_load_row<LPR, CF, VW, COL>(a, p < stop ? sh.row[i] : 0, p < stop, gl, av, act, voff, st);
+            agnn_load_row<LPR, CF, VW, COL, SCORES>(a, p < stop ? sh.row[i] : 0, p < stop, gl, av, act, voff, st);
         }
         __syncthreads();
         // Rows that several groups or shares hold: their pieces of this share, in order.
@@ -643,14 +722,14 @@ __global__ void __launch_bounds__(256) agnn_combine_kernel(const AgnnArgs a)
     }
 }
 
-template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false>
+template <int LPR, int CF, int BS, int VW, bool SEP = false, bool COL = false, int SCORES = SCORES_NONE>
 void launch_fused(const AgnnArgs &a, cudaStream_t st)
 {
     const int gpc = 256 / LPR;
     const int64_t gx = (a.n_seg + gpc - 1) / gpc + a.lng.scan_ctas;
-    agnn_fused_kernel<LPR, CF, BS, VW, SEP, COL><<<(unsigned)gx, 256, 0, st>>>(a);
+    agnn_fused_kernel<LPR, CF, BS, VW, SEP, COL, SCORES><<<(unsigned)gx, 256, 0, st>>>(a);
     if (a.lng.totals)
-        launch_dependent(agnn_long_kernel<LPR, CF, BS, VW, SEP, COL>, dim3((unsigned)a.lng.shares), 256,
+        launch_dependent(agnn_long_kernel<LPR, CF, BS, VW, SEP, COL, SCORES>, dim3((unsigned)a.lng.shares), 256,
                          gpc * 2 * (a.dim_pad + 2) * 4, st, a);
 }
 
@@ -716,7 +795,7 @@ static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A
                     int64_t ldOut, float beta, const float *beta_dev, int32_t softmax, int32_t vec_width,
                     int32_t lanes_per_row, int32_t batch, const int32_t *rowPtr_split, const int32_t *target_row,
                     int64_t n_seg, void *scratch, size_t scratch_bytes, float *col_out, double *sums, size_t sums_bytes,
-                    void *stream)
+                    float *scores, bool take_scores, void *stream)
 {
     if (n_rows < 0 || nnz < 0 || dim <= 0)
         return PSPMM_E_ARG;
@@ -767,6 +846,7 @@ static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A
     a.dim_pad = (dim + 3) / 4 * 4;
     a.beta = beta;
     a.beta_dev = beta_dev;
+    a.scores = scores;
     a.col_sums = sums;
     a.n_col_sums = 0;
     a.col_out = col_out;
@@ -812,7 +892,7 @@ static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A
         lpr *= 2;
         cf = (nvec + lpr - 1) / lpr;
     }
-    if (sep && lanes_per_row == 0) {  // two gathered rows per entry: at most two slices per lane (one of 32 bytes) keeps them in registers
+    if ((sep || take_scores) && lanes_per_row == 0) {  // two gathered rows per entry: at most two slices per lane (one of 32 bytes) keeps them in registers
         while (cf > (vw == 8 ? 1 : 2) && lpr < 32) {
             lpr *= 2;
             cf = (nvec + lpr - 1) / lpr;
@@ -837,6 +917,27 @@ static int agnn_run(const int32_t *rowPtr, const int32_t *colIdx, const float *A
         if (!sums || sums_bytes < (size_t)(a.n_col_sums + 1) * sizeof(double))
             return PSPMM_E_ARG;
     }
+#define AGNN_CASE_TAKE(LPR_, CF_, VW_)                                                   \
+    if (!ok && take_scores && vw == VW_ && lpr == LPR_ && cf == CF_) {                   \
+        if (col_out)                                                                     \
+            launch_fused<LPR_, CF_, LPR_ < 8 ? 4 : 8, VW_, true, true, SCORES_TAKE>(a, st);  \
+        else                                                                             \
+            launch_fused<LPR_, CF_, LPR_ < 8 ? 4 : 8, VW_, true, false, SCORES_TAKE>(a, st); \
+        ok = true;                                                                       \
+    }
+    AGNN_CASE_TAKE(4, 1, 4) AGNN_CASE_TAKE(4, 2, 4) AGNN_CASE_TAKE(8, 2, 4) AGNN_CASE_TAKE(16, 2, 4) AGNN_CASE_TAKE(32, 2, 4)
+    AGNN_CASE_TAKE(4, 1, 8) AGNN_CASE_TAKE(8, 1, 8) AGNN_CASE_TAKE(16, 1, 8) AGNN_CASE_TAKE(32, 1, 8)
+#undef AGNN_CASE_TAKE
+#define AGNN_CASE_LEAVE(LPR_, CF_, VW_)                                          \
+    if (!ok && scores && vw == VW_ && lpr == LPR_ && cf == CF_) {                \
+        launch_fused<LPR_, CF_, 4, VW_, false, false, SCORES_LEAVE>(a, st);      \
+        ok = true;                                                               \
+    }
+    AGNN_CASE_LEAVE(4, 1, 4) AGNN_CASE_LEAVE(4, 2, 4) AGNN_CASE_LEAVE(4, 4, 4) AGNN_CASE_LEAVE(8, 4, 4) AGNN_CASE_LEAVE(16, 4, 4)
+    AGNN_CASE_LEAVE(4, 1, 8) AGNN_CASE_LEAVE(4, 2, 8) AGNN_CASE_LEAVE(8, 2, 8) AGNN_CASE_LEAVE(16, 2, 8)
+#undef AGNN_CASE_LEAVE
+    if (scores && !ok)
+        return PSPMM_E_UNSUPPORTED;
 #define AGNN_CASE_COL(LPR_, CF_, VW_)                                          \
     if (!ok && sep && col_out && vw == VW_ && lpr == LPR_ && cf == CF_) {      \
         launch_fused<LPR_, CF_, 4, VW_, true, true>(a, st);                    \
@@ -895,7 +996,7 @@ extern "C" int pspmm_agnn_fused_apply_csr(const int32_t *rowPtr, const int32_t *
 {
     return agnn_run(rowPtr, colIdx, A, B, V, out, n_rows, nnz, dim, ldA, ldB, ldV, ldOut, beta, nullptr, softmax,
                     vec_width, lanes_per_row, batch, rowPtr_split, target_row, n_seg, scratch, scratch_bytes, nullptr,
-                    nullptr, 0, stream);
+                    nullptr, 0, nullptr, false, stream);
 }
 
 extern "C" int pspmm_agnn_layer_scratch_bytes(int64_t n_rows, int64_t nnz, int64_t n_seg, int32_t dim, size_t *bytes)
@@ -915,10 +1016,38 @@ extern "C" int pspmm_agnn_layer_forward(const int32_t *rowPtr, const int32_t *co
                                         const float *beta, const int32_t *rowPtr_split, const int32_t *target_row,
                                         int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream)
 {
+    return pspmm_agnn_layer_forward_scores(rowPtr, colIdx, X, out, nullptr, n_rows, nnz, dim, ldX, ldOut, beta, rowPtr_split,
+                                           target_row, n_seg, scratch, scratch_bytes, stream);
+}
+
+extern "C" int pspmm_agnn_layer_forward_scores(const int32_t *rowPtr, const int32_t *colIdx, const float *X, float *out,
+                                               float *scores, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX,
+                                               int64_t ldOut, const float *beta, const int32_t *rowPtr_split,
+                                               const int32_t *target_row, int64_t n_seg, void *scratch,
+                                               size_t scratch_bytes, void *stream)
+{
     if (!beta)
         return PSPMM_E_ARG;
     return agnn_run(rowPtr, colIdx, X, X, X, out, n_rows, nnz, dim, ldX, ldX, ldX, ldOut, 0.f, beta, 0, 0, 0, 0,
-                    rowPtr_split, target_row, n_seg, scratch, scratch_bytes, nullptr, nullptr, 0, stream);
+                    rowPtr_split, target_row, n_seg, scratch, scratch_bytes, nullptr, nullptr, 0, scores, false, stream);
+}
+
+// What the two backward passes share: the scores are recomputed from X, or taken.
+static int agnn_backward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, const float *scores, const float *G,
+                         float *D, float *d_beta, int64_t n_rows, int64_t nnz, int32_t dim, int64_t ldX, int64_t ldG,
+                         int64_t ldD, const float *beta, const int32_t *rowPtr_split, const int32_t *target_row,
+                         int64_t n_seg, void *scratch, size_t scratch_bytes, void *stream)
+{
+    size_t need = 0;
+    int rc = pspmm_agnn_layer_scratch_bytes(n_rows, nnz, rowPtr_split ? n_seg : 0, dim, &need);
+    if (rc)
+        return rc;
+    if (!scratch || scratch_bytes < need || (uintptr_t)scratch % 16 != 0)
+        return PSPMM_E_ARG;
+    const size_t sums = agnn_sums_bytes(rowPtr_split ? n_seg : n_rows), own = need - sums;
+    return agnn_run(rowPtr, colIdx, X, X, G, D, n_rows, nnz, dim, ldX, ldX, ldG, ldD, 0.f, beta, 0, 0, 0, 4,
+                    rowPtr_split, target_row, n_seg, own ? scratch : nullptr, own, d_beta,
+                    (double *)((char *)scratch + own), sums, const_cast<float *>(scores), scores != nullptr, stream);
 }
 
 extern "C" int pspmm_agnn_layer_backward(const int32_t *rowPtr, const int32_t *colIdx, const float *X, const float *G,
@@ -929,14 +1058,20 @@ extern "C" int pspmm_agnn_layer_backward(const int32_t *rowPtr, const int32_t *c
 {
     if (!beta || !G)
         return PSPMM_E_ARG;
-    size_t need = 0;
-    int rc = pspmm_agnn_layer_scratch_bytes(n_rows, nnz, rowPtr_split ? n_seg : 0, dim, &need);
-    if (rc)
-        return rc;
-    if (!scratch || scratch_bytes < need || (uintptr_t)scratch % 16 != 0)
+    return agnn_backward(rowPtr, colIdx, X, nullptr, G, D, d_beta, n_rows, nnz, dim, ldX, ldG, ldD, beta, rowPtr_split,
+                         target_row, n_seg, scratch, scratch_bytes, stream);
+}
+
+extern "C" int pspmm_agnn_layer_backward_scores(const int32_t *rowPtr, const int32_t *colIdx, const float *scores,
+                                                const float *G, float *D, float *d_beta, int64_t n_rows, int64_t nnz,
+                                                int32_t dim, int64_t ldG, int64_t ldD, const int32_t *rowPtr_split,
+                                                const int32_t *target_row, int64_t n_seg, void *scratch,
+                                                size_t scratch_bytes, void *stream)
+{
+    if (!G || (nnz > 0 && !scores))
         return PSPMM_E_ARG;
-    const size_t sums = agnn_sums_bytes(rowPtr_split ? n_seg : n_rows), own = need - sums;
-    return agnn_run(rowPtr, colIdx, X, X, G, D, n_rows, nnz, dim, ldX, ldX, ldG, ldD, 0.f, beta, 0, 0, 0, 4,
-                    rowPtr_split, target_row, n_seg, own ? scratch : nullptr, own, d_beta,
-                    (double *)((char *)scratch + own), sums, stream);
+    // (the operands of the scores are not read: G stands in for them in what the passes check)
+    static const float none = 0.f;
+    return agnn_backward(rowPtr, colIdx, G, scores ? scores : &none, G, D, d_beta, n_rows, nnz, dim, ldG, ldG, ldD, nullptr,
+                         rowPtr_split, target_row, n_seg, scratch, scratch_bytes, stream);
 }

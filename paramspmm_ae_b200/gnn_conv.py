@@ -89,11 +89,10 @@ class GINFunction(torch.autograd.Function):
 # (SDDMM -> scale -> SpMM in one pass).  Set to False to always use the three-kernel composition.
 FUSE_AGNN_INFERENCE = True
 
-# With gradients enabled the same layers run AGNNFusedFunction: the forward is the fused kernel, and
-# the backward recomputes the edge scores inside the kernel instead of reading a saved edge array,
-# so a training step writes no per-edge array at all (the reference's composition writes the
-# attention values in the forward and the score gradient in the backward, 4 bytes per edge each,
-# gnn_conv.py:130-180).  Outputs and gradients are the reference's up to fp32 summation order.
+# With gradients enabled the same layers run AGNNFusedFunction: the forward is the fused kernel, which leaves
+# the edge scores for the backward (4 bytes per edge; the reference's composition writes the attention values in
+# the forward and the score gradient in the backward, gnn_conv.py:130-180).  Outputs and gradients are the
+# reference's up to fp32 summation order.
 # Set to False to train through the three-kernel composition (AGNNFunction).
 FUSE_AGNN_TRAINING = True
 
@@ -155,10 +154,11 @@ class AGNNFunction(torch.autograd.Function):
 
 
 class AGNNFusedFunction(torch.autograd.Function):
-    """AGNN layer on a CSR / split-CSR operator without edge arrays.
+    """AGNN layer on a CSR / split-CSR operator in one pass over the pattern per direction.
 
-    forward   X' = X W,  out_i = sum_j beta <X'_i, X'_j> X'_j                 (one fused pass)
-    backward  D_i = sum_j beta <X'_i, X'_j> G_j   (scores recomputed, gradient rows gathered)
+    forward   X' = X W,  out_i = sum_j beta <X'_i, X'_j> X'_j     (one fused pass, which leaves the scores)
+    backward  D_i = sum_j beta <X'_i, X'_j> G_j           (gradient rows gathered, scores read; where there
+              is no room for them the rows of X' are gathered again and the scores recomputed)
               dX = D W^T,  dW = X^T D                                      (gnn_conv.py:157-160)
               d_beta = sum over edges of <G_i, G_j> * colIdx[e]              (gnn_conv.py:163-172: the
               reference multiplies the score gradient by the column-index column it is handed), summed
@@ -170,17 +170,22 @@ class AGNNFusedFunction(torch.autograd.Function):
     def forward(ctx, X, weights, attention_w, P, colIdx):
         Xp = ops.dense_mm(X, weights)
         beta = _beta(attention_w).clone()  # (the backward uses the value of this forward)
-        out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, beta, P.target_row)
-        ctx.save_for_backward(X, weights, Xp, beta)
+        try:
+            scores = torch.empty(P.colIdx.shape[0], dtype=torch.float32, device=Xp.device)
+        except torch.cuda.OutOfMemoryError:
+            scores = None
+        out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, beta, P.target_row, scores)
+        ctx.save_for_backward(X, weights, *((Xp, beta) if scores is None else (scores,)))
         ctx.P = P
         return out
 
     @staticmethod
     def backward(ctx, d_output):
-        X, weights, Xp, beta = ctx.saved_tensors
+        X, weights, *rest = ctx.saved_tensors
+        Xp, beta, scores = (*rest, None) if len(rest) == 2 else (None, None, *rest)
         P = ctx.P
         D, d_att = ops.agnn_layer_backward(Xp, d_output.contiguous(), P.rowPtr, P.colIdx, beta, P.target_row,
-                                           beta_grad=ctx.needs_input_grad[2])
+                                           beta_grad=ctx.needs_input_grad[2], scores=scores)
         d_input = ops.dense_mm(D, weights, transB=True) if ctx.needs_input_grad[0] else None
         d_weights = ops.dense_mm(X, D, transA=True) if ctx.needs_input_grad[1] else None
         return d_input, d_weights, d_att, None, None

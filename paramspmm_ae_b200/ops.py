@@ -649,12 +649,17 @@ def agnn_fused(A, B, rowPtr, colIdx, beta=1.0, softmax=True, target_row=None, n_
     return out
 
 
-def _agnn_layer(X, rowPtr, colIdx, beta, target_row):
+def _agnn_layer(X, rowPtr, colIdx, beta, target_row, scores=None):
     """Checks of the layer passes; (output with rows beyond the pattern zeroed, sizes and pointers)."""
     _check_cuda(X, "X", torch.float32, 2)
     _check_cuda(rowPtr, "rowPtr", torch.int32, 1)
     _check_cuda(colIdx, "colIdx", torch.int32, 1)
-    _check_cuda(beta, "beta", torch.float32)
+    if beta is not None:
+        _check_cuda(beta, "beta", torch.float32)
+    if scores is not None:
+        _check_cuda(scores, "scores", torch.float32, 1)
+        if scores.shape[0] != colIdx.shape[0]:
+            raise RuntimeError("scores must have one entry per column index")
     n, dim = X.shape
     n_seg = rowPtr.shape[0] - 1
     out = torch.empty_like(X)
@@ -670,29 +675,38 @@ def _agnn_layer(X, rowPtr, colIdx, beta, target_row):
         sizes = (n, colIdx.shape[0], n_seg, dim)
         rows, plain, split, target, n_split = n, None, rowPtr.data_ptr(), target_row.data_ptr(), n_seg
     scratch, nbytes = _scratch("pspmm_agnn_layer_scratch_bytes", sizes, X.device)
-    tail = (beta.data_ptr(), split, target, n_split, _ptr(scratch), nbytes, _stream())
+    tail = (_ptr(beta), split, target, n_split, _ptr(scratch), nbytes, _stream())
     return out, plain, rows, colIdx.shape[0], dim, tail, scratch
 
 
-def agnn_layer_forward(X, rowPtr, colIdx, beta, target_row=None):
+def agnn_layer_forward(X, rowPtr, colIdx, beta, target_row=None, scores=None):
     """out_i = sum_j beta <X_i, X_j> X_j over the pattern, ``beta`` one float on the device
-    (``pspmm_agnn_layer_forward``); one output row per row of ``X``."""
-    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta, target_row)
-    rc = lib().pspmm_agnn_layer_forward(plain, colIdx.data_ptr(), X.data_ptr(), out.data_ptr(), rows, nnz, dim, X.stride(0),
-                                        out.stride(0), *tail)
+    (``pspmm_agnn_layer_forward``); one output row per row of ``X``.  ``scores`` (one float per entry) receives
+    beta <X_i, X_j> for :func:`agnn_layer_backward`."""
+    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta, target_row, scores)
+    rc = lib().pspmm_agnn_layer_forward_scores(plain, colIdx.data_ptr(), X.data_ptr(), out.data_ptr(), _ptr(scores), rows,
+                                               nnz, dim, X.stride(0), out.stride(0), *tail)
     if rc:
         check(rc)
     return out
 
 
-def agnn_layer_backward(X, G, rowPtr, colIdx, beta, target_row=None, beta_grad=True):
+def agnn_layer_backward(X, G, rowPtr, colIdx, beta, target_row=None, beta_grad=True, scores=None):
     """D_i = sum_j beta <X_i, X_j> G_j and, in the same pass, sum over the entries of j * <G_i, G_j>
-    (the attention weight's gradient, gnn_conv.py:163-172; None without ``beta_grad``)."""
+    (the attention weight's gradient, gnn_conv.py:163-172; None without ``beta_grad``).  With the ``scores`` that
+    :func:`agnn_layer_forward` left, ``X`` and ``beta`` are not used."""
     _check_cuda(G, "G", torch.float32, 2)
-    if G.shape != X.shape:
+    if scores is None and G.shape != X.shape:
         raise RuntimeError("G must have the shape of X")
-    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta, target_row)
+    X = G if scores is not None else X
+    out, plain, rows, nnz, dim, tail, _keep = _agnn_layer(X, rowPtr, colIdx, beta if scores is None else None, target_row, scores)
     d_beta = torch.empty((1, 1), dtype=torch.float32, device=X.device) if beta_grad else None
+    if scores is not None:
+        rc = lib().pspmm_agnn_layer_backward_scores(plain, colIdx.data_ptr(), scores.data_ptr(), G.data_ptr(), out.data_ptr(),
+                                                    _ptr(d_beta), rows, nnz, dim, G.stride(0), out.stride(0), *tail[1:])
+        if rc:
+            check(rc)
+        return out, d_beta
     rc = lib().pspmm_agnn_layer_backward(plain, colIdx.data_ptr(), X.data_ptr(), G.data_ptr(), out.data_ptr(), _ptr(d_beta),
                                          rows, nnz, dim, X.stride(0), G.stride(0), out.stride(0), *tail)
     if rc:

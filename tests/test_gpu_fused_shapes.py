@@ -61,3 +61,70 @@ def test_infinite_rows_reach_only_the_rows_that_hold_them(dim, softmax, sep):
             if not extra:  # (pieces of a cut row meet with weights of their own: 0 * inf there is not the plain row's)
                 np.testing.assert_array_equal(np.isfinite(got), np.isfinite(want))
         target[inf_col] = keep
+
+
+@pytest.mark.parametrize("dim", [4, 16, 24, 32, 40, 64, 68, 128, 132, 256])
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("pairs", [0, 40, 20000])
+def test_scores_kept_between_the_layer_passes(dim, split, pairs):
+    """The scores that the forward leaves and the backward that takes them, against dense fp64 algebra: empty,
+    sparse and long-row patterns, every default shape of the two kernels."""
+    from paramspmm_ae_b200 import ops, synth
+    dev = torch.device("cuda:0")
+    n = 301
+    g = synth.powerlaw_graph(n, pairs, seed=4, self_loops=pairs != 0)
+    rp, ci = g.rowPtr.to(dev), g.colIdx.to(dev)
+    rows = torch.repeat_interleave(torch.arange(n, device=dev), (rp[1:] - rp[:-1]).long())
+    cols = ci.long()
+    gen = torch.Generator(device=dev).manual_seed(5)
+    X, G = (torch.randn(n + (0 if split else 2), dim, device=dev, generator=gen) / dim ** 0.5 for _ in range(2))
+    beta = torch.tensor([0.7], device=dev)
+    tr = None
+    if split:
+        rp, tr = ops.split_csr_device(rp, 9)
+    scores = torch.full((ci.shape[0],), float("nan"), device=dev)
+    out = ops.agnn_layer_forward(X, rp, ci, beta, tr, scores)
+    assert torch.equal(out, ops.agnn_layer_forward(X, rp, ci, beta, tr))
+    X64, G64 = X.double(), G.double()
+    # dot products of dim terms below 1: a few roundings of their absolute sum
+    want = 0.7 * (X64[rows] * X64[cols]).sum(1)
+    bound = 1e-6 * (X64[rows] * X64[cols]).abs().sum(1)
+    assert bool(((scores.double() - want).abs() <= bound).all())
+    D, d_beta = ops.agnn_layer_backward(None, G, rp, ci, None, tr, scores=scores)
+    terms = scores.double()[:, None] * G64[cols]
+    want = torch.zeros(n, dim, dtype=torch.float64, device=dev).index_add_(0, rows, terms)
+    scale = torch.zeros(n, dim, dtype=torch.float64, device=dev).index_add_(0, rows, terms.abs())
+    assert bool(((D[:n].double() - want).abs() <= 2e-6 * scale + 1e-30).all())
+    assert float(D[n:].abs().sum()) == 0
+    terms = (G64[rows] * G64[cols]).sum(1) * cols.double()
+    assert abs(float(d_beta) - float(terms.sum())) <= 1e-6 * float(terms.abs().sum())
+    assert ops.agnn_layer_backward(None, G, rp, ci, None, tr, beta_grad=False, scores=scores)[1] is None
+
+
+def test_agnn_layer_trains_without_room_for_the_scores(monkeypatch):
+    """Where the score array cannot be allocated the backward recomputes the scores."""
+    from paramspmm_ae_b200 import gnn_conv, pcsr, synth
+    dev = torch.device("cuda:0")
+    g = synth.powerlaw_graph(301, 3000, seed=4)
+    P = pcsr.pcsr_sddmm(None, 1, False, 301, g.nnz, g.rowPtr, g.colIdx, g.val, None, CF=1, blkWarpNum=8)
+    layer = gnn_conv.AGNNConv(16, 32).to(dev)
+    X, G = torch.randn(301, 16, device=dev), torch.randn(301, 32, device=dev)
+
+    def step():
+        x = X.clone().requires_grad_(True)
+        layer.zero_grad()
+        out = layer(x, {32: P}, P.colIdx.unsqueeze(-1))
+        out.backward(G)
+        return out.detach(), x.grad, layer.weights.grad.clone(), layer.attention_w.grad.clone()
+
+    kept = step()
+    empty = torch.empty
+
+    def refuse(*size, **kw):
+        if size == (g.nnz,):
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(gnn_conv.torch, "empty", refuse)
+    for a, b in zip(kept, step()):
+        assert float((a - b).norm()) <= 1e-5 * float(b.norm())
