@@ -78,6 +78,9 @@ _SIGNATURES = {
     "pspmm_spmm_scratch_bytes": [_i64, _i64, _i32, _i32, ctypes.POINTER(ctypes.c_size_t)],
     "pspmm_spmm_csr_ws": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _i64, _i64, _cfgp, _vp, _vp,
                           _i64, _vp, ctypes.c_size_t, _vp],
+    "pspmm_spmm_csr_padded": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _i64, _i64, _cfgp, _vp, _vp,
+                          _i64, _vp, ctypes.c_size_t, _vp],
+    "pspmm_pad_rows": [_vp, _vp, _i64, _i32, _i64, _i64, _vp],
     "pspmm_spmm_bcsr_ws": [_vp, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i32, _i64, _i64, _cfgp,
                            _vp, _vp, _i64, _vp, ctypes.c_size_t, _vp],
     "pspmm_sddmm_csr": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i32, _i64, _i64, _cfgp, _vp, _vp, _i64,

@@ -485,7 +485,8 @@ static int long_range(int64_t n_entries, int per_sm)
 static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t n_seg,
                        const int32_t *colIdx, const float *val, int V, const float *B, float *C,
                        int64_t n_out_blk_rows, int64_t n_cols, int64_t n_entries, int32_t dim, int64_t ldB,
-                       int64_t ldC, const pspmm_cfg *cfg, void *scratch, size_t scratch_bytes, cudaStream_t st)
+                       int64_t ldC, const pspmm_cfg *cfg, void *scratch, size_t scratch_bytes, cudaStream_t st,
+                       bool ragged = false)
 {
     int rc = pspmm_validate_cfg(cfg, false);
     if (rc)
@@ -507,16 +508,26 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             const int32_t w = dim - off < cfg->col_tile ? dim - off : cfg->col_tile;
             const pspmm_cfg sub = tile_cfg(*cfg, w);
             rc = spmm_launch(segPtr, target_row, n_seg, colIdx, val, V, B + off, C + off, n_out_blk_rows, n_cols,
-                             n_entries, w, ldB, ldC, &sub, scratch, scratch_bytes, st);
+                             n_entries, w, ldB, ldC, &sub, scratch, scratch_bytes, st, ragged);
             if (rc)
                 return rc;
         }
         return PSPMM_OK;
     }
     LaunchShape s;
-    rc = spmm_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row != nullptr, n_seg, n_entries, &s);
+    const int32_t wide = ragged ? (dim + 3) / 4 * 4 : dim;  // columns that are gathered
+    rc = spmm_shape(cfg, wide, ragged ? 4 : pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row != nullptr, n_seg, n_entries, &s);
     if (rc)
         return rc;
+    if (ragged && s.lpr < 4) {  // (built for at least four lanes and up to four slices)
+        s.lpr = 4;
+        s.cf = pspmm_round_cf((wide / 4 + 3) / 4);
+    }
+    if (ragged && (s.cf > 4 || s.tiles > 1)) {
+        s.lpr = 32;
+        s.cf = 4;
+        s.tiles = (wide / 4 + 127) / 128;
+    }
     const bool bucketed = target_row && cfg && cfg->bucketed;
     if (target_row && !accumulate) {
         const int vecok = (dim % 4 == 0 && ldC % 4 == 0 && ((uintptr_t)C) % 16 == 0) ? 1 : 0;
@@ -528,7 +539,8 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
                 target_row, n_seg, n_out_blk_rows, s.rpg, V, C, ldC, dim, vecok);
     }
 
-    SpmmLongArgs a;
+    SpmmRaggedArgs a;
+    a.dim = dim;
     a.segPtr = segPtr;
     a.target_row = target_row;
     a.colIdx = colIdx;
@@ -539,7 +551,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.n_out = n_out_blk_rows;
     a.ldB = ldB;
     a.ldC = ldC;
-    a.nvec = dim / s.vw;
+    a.nvec = wide / s.vw;
     a.rows_per_group = s.rpg;
     a.bucketed = bucketed ? 1 : 0;
     a.keep_fraction = l2_keep_fraction((double)n_cols * (double)ldB * 4.0);
@@ -553,7 +565,7 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
         const int lanes = pspmm_long_lanes(a.nvec, V);
         long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
         if (long_fits(a.lng, n_entries) &&
-            scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * dim * sizeof(float))
+            scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * wide * sizeof(float))
             long_place(&a.lng, scratch);
         else
             a.lng = LongArgs{};
@@ -564,7 +576,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
         return PSPMM_E_RANGE;
     dim3 grid((unsigned)gx, (unsigned)s.tiles, 1);
     bool ok = false;
-    if (accumulate)
+    if (ragged)
+        ok = pspmm_launch_spmm_ragged(s, a, grid, st);
+    else if (accumulate)
         ok = pspmm_launch_spmm_vw4_acc(s, a, grid, st);
     else if (s.vw == 4)
         ok = pspmm_launch_spmm_vw4(s, V, a, grid, st);
@@ -592,12 +606,10 @@ extern "C" int pspmm_spmm_scratch_bytes(int64_t n_rows, int64_t nnz, int32_t dim
     return PSPMM_OK;
 }
 
-extern "C" int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
-                                 const float *B, float *C, int64_t n_rows, int64_t n_cols,
-                                 int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
-                                 const pspmm_cfg *cfg, const int32_t *rowPtr_split,
-                                 const int32_t *target_row, int64_t n_seg, void *scratch,
-                                 size_t scratch_bytes, void *stream)
+static int spmm_csr(const int32_t *rowPtr, const int32_t *colIdx, const float *val, const float *B, float *C,
+                    int64_t n_rows, int64_t n_cols, int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
+                    const pspmm_cfg *cfg, const int32_t *rowPtr_split, const int32_t *target_row, int64_t n_seg,
+                    void *scratch, size_t scratch_bytes, void *stream, bool ragged)
 {
     int rc = check_sizes(n_rows, n_cols, nnz, dim);
     if (rc)
@@ -615,7 +627,33 @@ extern "C" int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, c
         return PSPMM_E_RANGE;
     return spmm_launch(split ? rowPtr_split : rowPtr, target_row, split ? n_seg : n_rows, colIdx,
                        val, 1, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, scratch, scratch_bytes,
-                       (cudaStream_t)stream);
+                       (cudaStream_t)stream, ragged);
+}
+
+extern "C" int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
+                                 const float *B, float *C, int64_t n_rows, int64_t n_cols,
+                                 int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
+                                 const pspmm_cfg *cfg, const int32_t *rowPtr_split,
+                                 const int32_t *target_row, int64_t n_seg, void *scratch,
+                                 size_t scratch_bytes, void *stream)
+{
+    return spmm_csr(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, rowPtr_split, target_row, n_seg,
+                    scratch, scratch_bytes, stream, false);
+}
+
+extern "C" int pspmm_spmm_csr_padded(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
+                                     const float *B, float *C, int64_t n_rows, int64_t n_cols,
+                                     int64_t nnz, int32_t dim, int64_t ldB, int64_t ldC,
+                                     const pspmm_cfg *cfg, const int32_t *rowPtr_split,
+                                     const int32_t *target_row, int64_t n_seg, void *scratch,
+                                     size_t scratch_bytes, void *stream)
+{
+    if (ldB % 4 != 0 || (uintptr_t)B % 16 != 0 || ldB < (dim + 3) / 4 * 4)
+        return PSPMM_E_ARG;
+    if (cfg && (cfg->accumulate || (cfg->vec_width != 0 && cfg->vec_width != 4)))
+        return PSPMM_E_UNSUPPORTED;
+    return spmm_csr(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, rowPtr_split, target_row, n_seg,
+                    scratch, scratch_bytes, stream, true);
 }
 
 extern "C" int pspmm_spmm_bcsr_ws(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val,

@@ -150,6 +150,11 @@ struct SpmmLongArgs : SpmmArgs {
     bool dependent;  // (host) the launch may start while the pre-pass runs
 };
 
+// Operands whose width is no multiple of 4: B's rows are padded to 16 bytes, C's are not (spmm_ragged.cu).
+struct SpmmRaggedArgs : SpmmLongArgs {
+    int32_t dim;  // columns of C; nvec counts the padded ones
+};
+
 // Flags in target_row of a length-bucketed plan (pspmm_cfg.bucketed): the low 30 bits are the row.
 #define PSPMM_SEG_MULTI 0x80000000u  // the row is cut into several segments: every one of them adds with REDs
 #define PSPMM_SEG_FIRST 0x40000000u  // the first of them: the pre-pass zeroes the row when it meets this one
@@ -183,6 +188,7 @@ struct LaunchShape {
 // Return false when (lpr, cf, V) is not instantiated for that width.
 bool pspmm_launch_spmm_vw4(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_spmm_vw4_acc(const LaunchShape &s, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
+bool pspmm_launch_spmm_ragged(const LaunchShape &s, const SpmmRaggedArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_spmm_vw2(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_spmm_vw1(const LaunchShape &s, int V, const SpmmLongArgs &a, dim3 grid, cudaStream_t st);
 bool pspmm_launch_sddmm_vw4(const LaunchShape &s, int V, const SddmmArgs &a, dim3 grid, cudaStream_t st);

@@ -151,6 +151,16 @@ __device__ __forceinline__ void spmm_stage(const SpmmArgs &a, int *ent, int k0, 
     }
 }
 
+// What a launch hands its kernel: no more than the kernel reads (SpmmLongArgs).
+template <bool LONG, bool RAGGED>
+using SpmmKernelArgs = std::conditional_t<RAGGED, SpmmRaggedArgs, std::conditional_t<LONG, SpmmLongArgs, SpmmArgs>>;
+
+// Words of shared memory per lane group.  A RAGGED row passes through a row of them on its way out, so that the lanes store
+// neighbouring floats: the four of a lane one by one are four times the sectors (3.2 M entries at 47 columns, split: 96 us,
+// this way 85; shifted to whole 16-byte vectors with single floats at the ends 92: bank conflicts and divergence).
+template <int LPR, int VW, int CF, int V, bool RAGGED>
+constexpr int spmm_group_words = SpmmTile<LPR, V>::GROUP_WORDS + (RAGGED ? LPR * CF * VW : 0);
+
 // MLP = 16-byte gathers a lane keeps in flight per batch (2, 4, 8 or 16).  It trades registers
 // (and so resident warps per SM) against memory-level parallelism inside one warp; the
 // launch bound asks for the matching number of resident 256-thread CTAs.
@@ -165,8 +175,9 @@ struct SpmmOcc {
 // (long_rows.cuh); its first CTAs prepare the launch that takes them.  Both are template
 // flags because a run-time test of either costs the 48- and 80-register shapes spills (4 - 13 % of
 // the dim sweep's products).
-template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
-__global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(const std::conditional_t<LONG, SpmmLongArgs, SpmmArgs> a)
+// RAGGED = true: see SpmmRaggedArgs.  Only what is stored differs.
+template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false, bool RAGGED = false>
+__global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(const SpmmKernelArgs<LONG, RAGGED> a)
 {
     using Tile = SpmmTile<LPR, V>;
     constexpr int CAP = Tile::CAP;
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
     const int gl = threadIdx.x % LPR;
     const unsigned gmask =
         (LPR == 32) ? PSPMM_FULL_MASK : (((1u << LPR) - 1u) << (((threadIdx.x & 31) / LPR) * LPR));
-    int *sp = smem_words + g * Tile::GROUP_WORDS;            // segment pointers
+    int *sp = smem_words + g * spmm_group_words<LPR, VW, CF, V, RAGGED>;  // segment pointers
     int *st = sp + (PSPMM_RPG_MAX + 1);                     // target rows: [0] previous, [1..] own, then next
     int *ent = sp + Tile::HEAD_WORDS;                       // staged entries
 
@@ -292,7 +303,9 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                 float *crow = a.C + (orow * V + w) * a.ldC;
 #pragma unroll
                 for (int cf = 0; cf < CF; ++cf) {
-                    if (act[cf] && emit) {
+                    if constexpr (RAGGED) {
+                        st_vec<VW>(reinterpret_cast<float *>(ent + CAP * (1 + V)) + (cf * LPR + gl) * VW, acc[w][cf]);
+                    } else if (act[cf] && emit) {
                         if (ACC || shared)
                             red_add_vec<VW>(crow + voff[cf], acc[w][cf]);
                         else
@@ -301,6 +314,19 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
 #pragma unroll
                     for (int i = 0; i < VW; ++i)
                         acc[w][cf][i] = 0.f;
+                }
+                if constexpr (RAGGED) {
+                    const float *out = reinterpret_cast<float *>(ent + CAP * (1 + V));
+                    const int left = a.dim - vec0 * VW, cols = left < LPR * CF * VW ? left : LPR * CF * VW;
+                    float *to = crow + vec0 * VW;
+                    __syncwarp(gmask);
+                    for (int j = gl; j < cols; j += LPR) {
+                        if (shared)
+                            red_add_vec<1>(to + j, out + j);
+                        else
+                            st_vec_hint<1>(to + j, out + j, stream);
+                    }
+                    __syncwarp(gmask);
                 }
             }
             if (!ACC && split && !a.bucketed) {
@@ -313,8 +339,13 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                         float *crow = a.C + r * a.ldC;
 #pragma unroll
                         for (int cf = 0; cf < CF; ++cf)
-                            if (act[cf])
-                                st_vec_hint<VW>(crow + voff[cf], zero, stream);
+                            if (act[cf]) {
+                                if constexpr (RAGGED)
+                                    for (int i = 0; i < VW && voff[cf] + i < a.dim; ++i)
+                                        st_vec_hint<1>(crow + voff[cf] + i, zero, stream);
+                                else
+                                    st_vec_hint<VW>(crow + voff[cf], zero, stream);
+                            }
                     }
                 };
                 const int64_t after = (int64_t)next - orow - 1;
@@ -342,8 +373,8 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
 // spmm_seg_kernel walks its segments.  Every sum has a fixed order, as without the cut: the pieces of a
 // row inside a share meet in shared memory in the order of the entries, the shares' parts in
 // a.lng.partials.  Bound: gather latency (U loads of 16 bytes in flight per lane).
-template <int VW, int V, int LPR>
-__global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongArgs a)
+template <int VW, int V, int LPR, bool RAGGED = false>
+__global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmKernelArgs<true, RAGGED> a)
 {
     constexpr int G = 256 / LPR;
     constexpr int U = V > 1 ? 4 : 8;
@@ -364,7 +395,10 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongAr
     const unsigned ldB_bytes = (unsigned)(a.ldB * 4);
     const unsigned long long keep = l2_policy_keep(a.keep_fraction);
     const unsigned long long stream = l2_policy_stream();
-    const int64_t dimv = (int64_t)a.nvec * VW;
+    const int64_t dimv = (int64_t)a.nvec * VW;  // columns of a partial result
+    int64_t dim = dimv;
+    if constexpr (RAGGED)
+        dim = a.dim;
     const int share = blockIdx.x;
     float acc[V][1][VW], first[V][VW];
 
@@ -380,8 +414,18 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongAr
         auto emit = [&](int i, int w, int col, const float *val) {
             int s0, s1;
             job.shares_of(sh, i, s0, s1);
+            float *to = a.C + ((int64_t)sh.row[i] * V + w) * a.ldC + col;
+            if constexpr (RAGGED) {
+                if (s0 == s1) {
+#pragma unroll
+                    for (int j = 0; j < VW; ++j)
+                        if (col + j < dim)
+                            st_vec_hint<1>(to + j, val + j, stream);
+                    return;
+                }
+            }
             if (s0 == s1)
-                st_vec_hint<VW>(a.C + ((int64_t)sh.row[i] * V + w) * a.ldC + col, val, stream);
+                st_vec_hint<VW>(to, val, stream);
             else
                 st_vec<VW>(a.lng.partials + (LongShare::slot(share, s0) * V + w) * dimv + col, val);
         };
@@ -468,7 +512,7 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongAr
             const int64_t r = sh.row[sh.edge[q]];
             for (int t = threadIdx.x; t < V * ROW; t += 256) {
                 const int w = t / ROW, col = blockIdx.y * ROW + t % ROW;
-                if (col >= dimv)
+                if (col >= dim)
                     continue;
                 float sum = 0.f;
                 for (int c = s0; c <= s1; ++c)
@@ -480,20 +524,20 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmLongAr
     }
 }
 
-template <int VW, int V>
-static inline void spmm_launch_long_rows(const SpmmLongArgs &a, cudaStream_t st)
+template <int VW, int V, bool RAGGED = false>
+static inline void spmm_launch_long_rows(const SpmmKernelArgs<true, RAGGED> &a, cudaStream_t st)
 {
     const int lpr = pspmm_long_lanes(a.nvec, V);
     const dim3 grid((unsigned)a.lng.shares, (unsigned)((a.nvec + lpr - 1) / lpr));
     if (lpr == 32)
-        launch_dependent(spmm_long_rows_kernel<VW, V, 32>, grid, 256, 0, st, a);
+        launch_dependent(spmm_long_rows_kernel<VW, V, 32, RAGGED>, grid, 256, 0, st, a);
     else if (lpr == 16)
-        launch_dependent(spmm_long_rows_kernel<VW, V, 16>, grid, 256, 0, st, a);
+        launch_dependent(spmm_long_rows_kernel<VW, V, 16, RAGGED>, grid, 256, 0, st, a);
     else if constexpr (V == 1) {
         if (lpr == 8)
-            launch_dependent(spmm_long_rows_kernel<VW, V, 8>, grid, 256, 0, st, a);
+            launch_dependent(spmm_long_rows_kernel<VW, V, 8, RAGGED>, grid, 256, 0, st, a);
         else
-            launch_dependent(spmm_long_rows_kernel<VW, V, 4>, grid, 256, 0, st, a);
+            launch_dependent(spmm_long_rows_kernel<VW, V, 4, RAGGED>, grid, 256, 0, st, a);
     }
 }
 
@@ -508,14 +552,14 @@ static inline void spmm_launch_long_rows(const SpmmLongArgs &a, cudaStream_t st)
             spmm_launch_long_rows<VW_, 3>(a, st);                            \
     }
 
-template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false>
-static inline void spmm_launch_one(const SpmmLongArgs &a, dim3 grid, int threads, cudaStream_t st)
+template <int LPR, int VW, int CF, int V, int MLP, bool ACC = false, bool LONG = false, bool RAGGED = false>
+static inline void spmm_launch_one(const SpmmKernelArgs<true, RAGGED> &a, dim3 grid, int threads, cudaStream_t st)
 {
-    const int smem = (threads / LPR) * SpmmTile<LPR, V>::GROUP_WORDS * 4;
-    auto kern = spmm_seg_kernel<LPR, VW, CF, V, MLP, ACC, LONG>;
+    const int smem = (threads / LPR) * spmm_group_words<LPR, VW, CF, V, RAGGED> * 4;
+    auto kern = spmm_seg_kernel<LPR, VW, CF, V, MLP, ACC, LONG, RAGGED>;
     if (smem > 48 * 1024)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    const std::conditional_t<LONG, SpmmLongArgs, SpmmArgs> &args = a;
+    const SpmmKernelArgs<LONG, RAGGED> &args = a;
     if (a.dependent)
         launch_dependent(kern, grid, threads, smem, st, args);  // follows the zeroing pre-pass
     else
@@ -546,6 +590,18 @@ static inline void spmm_launch_one(const SpmmLongArgs &a, dim3 grid, int threads
         else                                                                 \
             spmm_launch_one<LPR_, VW_, CF_, V_, 8>(a, grid, s.threads, st);  \
         return true;                                                         \
+    }
+#define PSPMM_SPMM_CASE_RAGGED(LPR_, CF_)                                                        \
+    if (s.lpr == LPR_ && s.cf == CF_) {                                                          \
+        if (a.lng.totals)                                                                        \
+            spmm_launch_one<LPR_, 4, CF_, 1, 8, false, true, true>(a, grid, s.threads, st);      \
+        else if (s.mlp <= 4)                                                                     \
+            spmm_launch_one<LPR_, 4, CF_, 1, 4, false, false, true>(a, grid, s.threads, st);     \
+        else if (s.mlp == 16)                                                                    \
+            spmm_launch_one<LPR_, 4, CF_, 1, 16, false, false, true>(a, grid, s.threads, st);    \
+        else                                                                                     \
+            spmm_launch_one<LPR_, 4, CF_, 1, 8, false, false, true>(a, grid, s.threads, st);     \
+        return true;                                                                             \
     }
 // The accumulating form is built for the 128-bit CSR family at one gather-batch depth.
 #define PSPMM_SPMM_CASE_ACC(LPR_, CF_)                                       \

@@ -198,7 +198,8 @@ class PlannedSpMM:
             self.segPtr, self.target = ops.split_csr_device(rowPtr, int(plan["granularity"]))
         self.n_seg = self.segPtr.shape[0] - 1
 
-    def __call__(self, out, B, accumulate=False):
+    def __call__(self, out, B, accumulate=False, dim=None):
+        """out = A B (or += with ``accumulate``); ``dim``: columns of the product where ``B`` is padded (``ops.spmm_into``)."""
         from . import _lib, ops
         kw = self.plan.kernel_cfg()
         if accumulate:  # built for 128-bit loads at one gather-batch depth
@@ -207,7 +208,8 @@ class PlannedSpMM:
         if out.shape[0] < self.n_seg_rows * self.V:  # block layouts write whole blocks: an odd row count needs a pad row
             dst = torch.empty(self.n_seg_rows * self.V, out.shape[1], dtype=out.dtype, device=out.device)
         ops.spmm_into(dst, B, self.segPtr, self.colIdx, self.val, target_row=self.target, V=self.V,
-                      n_out_rows=self.n_seg_rows, cfg=_lib.make_cfg(**kw))
+                      n_out_rows=self.n_seg_rows, cfg=_lib.make_cfg(**kw),
+                      dim=dim)
         if dst is not out:
             out.copy_(dst[: out.shape[0]])
         return out

@@ -333,15 +333,51 @@ def _check_output(out, rowPtr, split, n_out_rows, V, dim):
         raise RuntimeError("rowPtr must have one entry per output row plus one")
 
 
+def _pad_rows(X):
+    """[n, dim] -> [n, dim rounded up to 4] with zeros in the new columns (one pass, ``pspmm_pad_rows``)."""
+    n, dim = X.shape
+    out = torch.empty((n, dim + -dim % 4), dtype=torch.float32, device=X.device)
+    rc = lib().pspmm_pad_rows(X.data_ptr(), out.data_ptr(), n, dim, X.stride(0), out.stride(0), _stream())
+    if rc:
+        check(rc)
+    return out
+
+
+def _padding_pays(n, n_entries, dim, split):
+    """Whether an (odd) width is gathered from a copy padded to 16-byte rows: one pass over the operand (9 us of
+    launch and 5 TB/s) against gathers of 4 bytes per lane.  us without / with the copy:
+    unsplit: 100 K rows of 16, 101 columns 89 / 81, power law 130 / 100; 32, 255 columns 347 / 278 and 504 / 271; 64, 23
+    columns 96 / 75; but 16, 47 columns 41 / 44 and 500 K rows of 32, 47 columns 385 / 408: three slices of 16 lanes
+    leave few lanes idle there (power law 703 / 470, but the layout does not say so).
+    split: power law of 100 K rows of 32, 101 columns 142 / 132, 255 305 / 241; 64, 47 columns 139 / 130; but 16, 101
+    columns 87 / 95.  Widths of 2 modulo 4 gather 8 bytes per lane and gain nothing (split, 32, 70 columns 98 / 109)."""
+    work = dim * n_entries
+    if work < 6e7:
+        return False
+    if split:
+        return work >= 2400 * n
+    return work >= 1000 * n and (dim > 48 or n_entries >= 48 * n)
+
+
+def _sddmm_padding_pays(n, n_entries, dim):
+    """The same for edge scores (100 K rows of 32: 31 columns 64 / 46 us, 47 73 / 67, 23 52 / 45; 64: 31 columns 125 / 78; but
+    of 16 at 47 columns 42 / 44, of 32 at 101 columns 133 / 126 and with 500 K rows 1077 / 1187)."""
+    return dim <= 64 and n_entries >= 24 * n and dim * n_entries >= 6e7
+
+
 def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None, CF=0, W=0,
-              cfg=None):
+              cfg=None, dim=None):
     """Launch the SpMM into a caller-provided output (also used by the multi-GPU row shards).
 
     ``n_out_rows`` counts (block-)rows of the output; it defaults to the number of segments
     when there is no split and must be given for split layouts.  ``val=None`` (CSR layouts)
-    multiplies by the pattern itself: every stored entry counts as 1.
+    multiplies by the pattern itself: every stored entry counts as 1.  ``dim``: columns of the product where ``X``
+    carries more, up to the next multiple of 4 (CSR layouts).
     """
-    dim = X.shape[1]
+    if dim is None:
+        dim = X.shape[1]
+    elif V != 1 or X.shape[1] != dim + -dim % 4:
+        raise RuntimeError("input must have the columns of the product, padded to a multiple of 4")
     n_seg = rowPtr.shape[0] - 1
     split = target_row is not None
     if n_out_rows is None:
@@ -351,20 +387,24 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
     _check_output(out, rowPtr, split, n_out_rows, V, dim)
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
     long_rows = target_row is None and (cfg is None or not (cfg.no_long_rows or cfg.accumulate))
-    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows)
+    pad = cfg is None or (not cfg.accumulate and cfg.vec_width in (0, 4))
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, pad)
 
 
-def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows):
+def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, pad=True):
     seg = rowPtr.data_ptr()
-    n, dim = X.shape
+    n, dim = X.shape[0], out.shape[1]
+    if dim & 1 and V == 1 and pad and X.shape[1] == dim and _padding_pays(n, colIdx.shape[0], dim, target_row is not None):
+        X = _pad_rows(X)
+    cols = X.shape[1]
     # row pointers of a split layout go into the split arguments
     plain, split, target, n_seg = (seg, None, None, 0) if target_row is None else (
         None, seg, target_row.data_ptr(), rowPtr.shape[0] - 1)
     nent = colIdx.shape[0]
-    scratch, nbytes = _scratch("pspmm_spmm_scratch_bytes", (n_out_rows, nent, dim, V), X.device) if long_rows else (None, 0)
+    scratch, nbytes = _scratch("pspmm_spmm_scratch_bytes", (n_out_rows, nent, cols, V), X.device) if long_rows else (None, 0)
     tail = (n_out_rows, n, nent, dim, X.stride(0), out.stride(0), ref, split, target, n_seg, _ptr(scratch), nbytes, _stream())
     if V == 1:
-        rc = lib().pspmm_spmm_csr_ws(plain, colIdx.data_ptr(), _ptr(val), X.data_ptr(), out.data_ptr(), *tail)
+        rc = (lib().pspmm_spmm_csr_ws if cols == dim else lib().pspmm_spmm_csr_padded)(plain, colIdx.data_ptr(), _ptr(val), X.data_ptr(), out.data_ptr(), *tail)
     else:
         rc = lib().pspmm_spmm_bcsr_ws(plain, colIdx.data_ptr(), _ptr(val), V, X.data_ptr(), out.data_ptr(), *tail)
     if rc:
@@ -372,10 +412,11 @@ def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, lo
     return out
 
 
-def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W):
+def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
     _check_legacy(CF, W)
     _spmm_inputs(X, rowPtr, colIdx, val, target_row, V)
-    n, dim = X.shape
+    n = X.shape[0]
+    dim = X.shape[1] if dim is None else dim  # (fewer: X is padded, see spmm_into)
     # The reference sizes the output from the dense input, zeros_like(input) for CSR
     # (SpMM/SpMM_kernel.cu:136) and the input's row count rounded up to a multiple of V for the
     # block layouts (:281-282, 427-428), and walks as many (block-)rows as the row pointer has.
@@ -384,7 +425,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W):
     padded = (n + V - 1) // V * V
     n_out = padded // V
     n_seg = rowPtr.shape[0] - 1
-    out = torch.empty_like(X) if padded == n else torch.empty((padded, dim), dtype=torch.float32, device=X.device)
+    out = torch.empty_like(X) if padded == n and dim == X.shape[1] else torch.empty((padded, dim), dtype=torch.float32, device=X.device)
     if target_row is None:
         if n_seg > n_out:
             raise RuntimeError("rowPtr describes %d (block-)rows, the input only allows %d" % (n_seg, n_out))
@@ -442,6 +483,8 @@ def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=No
     _check_output(out, rowPtr, split, n_out, V, dim)
     nent = colIdx.shape[0]
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
+    if dim & 1 and V == 1 and _padding_pays(n, nent, dim, split):  # (the copy is part of the call)
+        return _loop_ms(lambda: spmm_into(out, X, rowPtr, colIdx, val, target_row, V, n_out, CF, W, cfg), warmup, iters)
     ms = ctypes.c_float(0.0)
     null = None
     check(lib().pspmm_profile_spmm(null if split else _ptr(rowPtr), _ptr(colIdx), _ptr(val), V,
@@ -451,6 +494,18 @@ def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=No
                                    _ptr(target_row) if split else null, n_seg if split else 0,
                                    warmup, iters, ctypes.byref(ms), _stream()))
     return ms.value
+
+
+def _loop_ms(call, warmup, iters):
+    for _ in range(warmup):
+        call()
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    begin.record()
+    for _ in range(iters):
+        call()
+    end.record()
+    end.synchronize()
+    return begin.elapsed_time(end) / iters
 
 
 def _gflops(nnz, dim, ms):
@@ -509,6 +564,11 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
     n_seg = rowPtr.shape[0] - 1
     nent = colIdx.shape[0]
     out = torch.empty_like(val)
+    if dim & 1 and V == 1 and not time_only and _sddmm_padding_pays(B.shape[0], nent, dim):
+        same = A.data_ptr() == B.data_ptr() and A.shape == B.shape
+        A = _pad_rows(A)
+        B = A if same else _pad_rows(B)
+        dim = A.shape[1]
     cfg = _cfg("sddmm", CF, W, dim, nent, n_seg, V, split)
     null = None
     # (block-)rows of the pattern; A may stop inside the last block-row when the node count is
@@ -518,6 +578,8 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
         raise RuntimeError("A has %d rows, the pattern needs more than %d" % (A.shape[0], (n_rows - 1) * V))
     args_tail = (cfg, _ptr(rowPtr) if split else null,
                  _ptr(target_row) if split else null, n_seg if split else 0)
+    if time_only and dim & 1 and V == 1 and _sddmm_padding_pays(B.shape[0], nent, dim):
+        return _loop_ms(lambda: _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W), PROFILE_WARMUP, PROFILE_ITERS)
     if time_only:
         ms = ctypes.c_float(0.0)
         check(lib().pspmm_profile_sddmm(null if split else _ptr(rowPtr), _ptr(colIdx), _ptr(val), V,
@@ -823,19 +885,20 @@ def _conv_forward(V, H, weight, rowPtr, colIdx, val, target_row, CF, W, product=
     """A @ (H @ W): dense GEMM (cuBLAS through torch.mm) then SpMM (SpCONV/SpCONV.h:43-193).
 
     An output width that is not a multiple of 4 (class counts: 47, 41, ...) is carried as the next
-    multiple of 4 through both products, by a zero column appended to the weights, so that the
-    SpMM runs with 128-bit accesses on 16-byte aligned rows; the extra column is dropped from the
-    result.  ``product`` replaces the SpMM launch (an operator bound to a decider plan).
+    multiple of 4 between the products, so that the SpMM gathers 16-byte aligned rows; it stores the columns that
+    exist.  (Block layouts store the padded width, which is cut back.)  ``product`` replaces the SpMM launch (an operator
+    bound to a decider plan).
 
     The projection is a cuBLAS fp32 product, the backward products run on the tensor cores
     (``dense_mm``, no less accurate).  What keeps the forward there is comparability alone: its last bit
     decides which side of zero a few pre-activations fall on, and with a ReLU behind the layer the gradients of a
-    2.4 M node network then differ in the fifth digit between builds."""
+    2.4 M node network then differ by 1e-4 between builds (a step with it there: 82.9 -> 76.5 ms)."""
     _check_legacy(CF, W, max_cf=4)  # SpCONV/SpCONV.cpp:93-104
     fout = weight.shape[1]
     HW = torch.mm(H, _pad_cols(weight, -fout % 4))
     n = HW.shape[0]
-    out = product(HW) if product else _spmm(HW, rowPtr, colIdx, val, target_row, V, CF, W)
+    dim = fout if V == 1 and HW.shape[1] != fout else None
+    out = product(HW, dim) if product else _spmm(HW, rowPtr, colIdx, val, target_row, V, CF, W, dim)
     if out.shape[0] != n:
         out = out[:n]  # block variants slice back (SpCONV.h:115-118)
     return out[:, :fout].contiguous() if out.shape[1] != fout else out
@@ -847,7 +910,10 @@ def _conv_backward(V, g_out, H, weight, rowPtr, colIdx, val, target_row, CF, W, 
     ``input_grad=False`` leaves dH out (None): the first layer of a network has no use for it."""
     _check_legacy(CF, W, max_cf=4)
     n, fout = g_out.shape
-    g_out = _pad_cols(g_out, -fout % 4).contiguous()
+    if fout % 4 and g_out.is_cuda and g_out.dtype is torch.float32 and g_out.stride(1) == 1 and g_out.stride(0) >= fout:
+        g_out = _pad_rows(g_out)
+    else:
+        g_out = _pad_cols(g_out, -fout % 4).contiguous()
     AG = product(g_out) if product else _spmm(g_out, rowPtr, colIdx, val, target_row, V, CF, W)
     AG = AG[:n, :fout]
     d_weight = dense_mm(H, AG, transA=True)

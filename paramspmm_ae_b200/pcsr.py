@@ -141,19 +141,23 @@ class pcsr_spmm(object):
         self._planned = decider.PlannedSpMM(plan, self.rowPtr, self.colIdx, self.val, n_cols=n)
         return self
 
-    def _planned_product(self, X):
+    def _planned_product(self, X, dim=None):
         """One output row per input row, as the legacy operators give (rows beyond the matrix zero);
-        a width that is not a multiple of 4 is padded for the launch and cut back."""
-        n, dim = X.shape
-        Xp = ops._pad_cols(X, -dim % 4).contiguous()
+        a width that is not a multiple of 4 is padded for the launch (``dim``: it is already, from ``dim`` columns)."""
+        n, dim = X.shape[0], X.shape[1] if dim is None else dim
+        if X.shape[1] == dim and dim % 4 and X.is_cuda and X.dtype is torch.float32 and X.is_contiguous():
+            Xp = ops._pad_rows(X)
+        else:
+            Xp = ops._pad_cols(X, -X.shape[1] % 4).contiguous()
         rows = self._planned.n_rows
         if n < rows:
             raise RuntimeError("the matrix has %d rows, the input only %d" % (rows, n))
-        out = torch.empty((n, Xp.shape[1]), dtype=torch.float32, device=X.device)
+        cut = Xp.shape[1] != dim and self._planned.V != 1  # (block layouts store what they gather)
+        out = torch.empty((n, Xp.shape[1] if cut else dim), dtype=torch.float32, device=X.device)
         if n > rows:
             out[rows:].zero_()
-        self._planned(out[:rows], Xp)
-        return out[:, :dim].contiguous() if Xp.shape[1] != dim else out
+        self._planned(out[:rows], Xp, dim=None if out.shape[1] == Xp.shape[1] else dim)
+        return out[:, :dim].contiguous() if cut else out
 
     # -- helpers ------------------------------------------------------------------------
     def _key(self):
