@@ -51,6 +51,20 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
     const int len = hb - lb;
     const unsigned ub = lb, ue = hb;  // (lb and maxlen can add up to more than 2^31)
     const bool live = len > 0;
+    const unsigned ldB_lo = (unsigned)(a.ldB * 4), ldB_hi = (unsigned)((unsigned long long)(a.ldB * 4) >> 32);
+    // With several slices per lane a row that is not loaded keeps what was there, and what comes of it is not stored
+    // (the scores of entries beyond the segment) or left out (slices beyond the last column).  Clearing it took an
+    // instruction per float: 4 M entries, dim 100 170 -> 158 us, 256 378 -> 317; 0.9 M unsplit, dim 256 158 -> 109.  With one
+    // slice the compiler overlaps batches if it may clear (band of 24 at dim 16: 60 us, without 75).
+    constexpr bool KEEP = V == 1 && CF > 1 && (CF <= 4 || VW < 4);
+    FVec<VW> kept[KEEP ? U : 1][KEEP ? CF : 1];
+    if constexpr (KEEP) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int cf = 0; cf < CF; ++cf)
+                kept[u][cf] = zero_vec<VW>();
+    }
     for (int off = 0; off < maxlen; off += CHUNK) {
         int ccol[ENT];
         float cval[ENT][V];
@@ -93,17 +107,30 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
                 float part[V][LPR];
 #pragma unroll
                 for (int j0 = 0; j0 < LPR; j0 += U) {
-                    FVec<VW> x[U][CF];
+                    FVec<VW> cleared[KEEP ? 1 : U][KEEP ? 1 : CF];
+                    auto x = [&](int u, int cf) -> FVec<VW> & {
+                        if constexpr (KEEP)
+                            return kept[u][cf];
+                        else
+                            return cleared[u][cf];
+                    };
                     const bool batch_on = (t * LPR + j0) < wcnt;  // warp-uniform
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         const int e = t * LPR + j0 + u;
                         const int c = __shfl_sync(PSPMM_FULL_MASK, ccol[t], j0 + u, LPR);
-                        const float *brow = a.B + (int64_t)c * a.ldB;
                         const bool p = batch_on && (e < cnt);
+                        if constexpr (KEEP) {
+                            const float *brow = row_start(a.B + voff[0], c, ldB_lo, ldB_hi);
 #pragma unroll
-                        for (int cf = 0; cf < CF; ++cf)
-                            x[u][cf] = ldg_vec_if<VW>(brow + voff[cf], p && act[cf]);
+                            for (int cf = 0; cf < CF; ++cf)
+                                ldg_vec_keep<VW>(x(u, cf), brow + cf * LPR * VW, p && act[cf]);
+                        } else {
+                            const float *brow = a.B + (int64_t)c * a.ldB;
+#pragma unroll
+                            for (int cf = 0; cf < CF; ++cf)
+                                x(u, cf) = ldg_vec_if<VW>(brow + voff[cf], p && act[cf]);
+                        }
                     }
 #pragma unroll
                     for (int u = 0; u < U; ++u)
@@ -112,9 +139,11 @@ __device__ __forceinline__ void sddmm_entries(const SddmmArgs &a, int64_t arow, 
                             float s = 0.f;
 #pragma unroll
                             for (int cf = 0; cf < CF; ++cf)
+                                if (!KEEP || act[cf]) {
 #pragma unroll
-                                for (int i = 0; i < VW; ++i)
-                                    s = fmaf(av[w][cf].v[i], x[u][cf].v[i], s);
+                                    for (int i = 0; i < VW; ++i)
+                                        s = fmaf(av[w][cf].v[i], x(u, cf).v[i], s);
+                                }
                             part[w][j0 + u] = s;
                         }
                 }

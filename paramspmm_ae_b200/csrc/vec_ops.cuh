@@ -160,10 +160,16 @@ __device__ __forceinline__ void fma_vec(float (&acc)[VW], float s, const float (
 template <int VW>
 __device__ __forceinline__ void ldg_vec_keep(FVec<VW> &r, const float *p, bool on)
 {
-    static_assert(VW == 4, "");
-    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
-        : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3])
-        : "l"(p), "r"(on ? 1 : 0));
+    const int flag = on ? 1 : 0;
+    if constexpr (VW == 4)
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+            : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]) : "l"(p), "r"(flag));
+    else if constexpr (VW == 2)
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q ld.global.nc.v2.f32 {%0, %1}, [%2];\n\t}"
+            : "+f"(r.v[0]), "+f"(r.v[1]) : "l"(p), "r"(flag));
+    else
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+            : "+f"(r.v[0]) : "l"(p), "r"(flag));
 }
 
 // acc[i] += s * x[i] where `on`, without a branch.

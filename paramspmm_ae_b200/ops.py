@@ -360,9 +360,9 @@ def _padding_pays(n, n_entries, dim, split):
 
 
 def _sddmm_padding_pays(n, n_entries, dim):
-    """The same for edge scores (100 K rows of 32: 31 columns 64 / 46 us, 47 73 / 67, 23 52 / 45; 64: 31 columns 125 / 78; but
-    of 16 at 47 columns 42 / 44, of 32 at 101 columns 133 / 126 and with 500 K rows 1077 / 1187)."""
-    return dim <= 64 and n_entries >= 24 * n and dim * n_entries >= 6e7
+    """The same for edge scores (100 K rows of 32: 23 columns 52 / 46 us, 31 62 / 45, 63 77 / 69, 101 131 / 114; 500 K of 16: 31
+    columns 132 / 112; but 47 columns 62 / 65, and of 16 101 columns 70 / 73)."""
+    return dim * n_entries >= 6e7 and (n_entries >= 16 * n if dim <= 32 else dim > 48 and n_entries >= 32 * n)
 
 
 def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None, CF=0, W=0,

@@ -128,3 +128,27 @@ def test_agnn_layer_trains_without_room_for_the_scores(monkeypatch):
     monkeypatch.setattr(gnn_conv.torch, "empty", refuse)
     for a, b in zip(kept, step()):
         assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+
+
+@pytest.mark.parametrize("dim", [5, 20, 47, 68, 70, 100, 132, 200, 256, 260])
+@pytest.mark.parametrize("split", [False, True])
+def test_scores_of_finite_rows_stay_finite_beside_infinite_ones(dim, split):
+    """Edge scores of rows that end inside a batch of gathers, and of widths that leave lanes without a column."""
+    from paramspmm_ae_b200 import ops
+    n, inf_col = 301, 5
+    g = torch.Generator().manual_seed(dim)
+    A, B = (torch.rand(n, dim, generator=g) - 0.3 for _ in range(2))
+    rp, ci, cols = _rows_of_one_to_nine(n, inf_col, dim)
+    B[inf_col, :: 2] = float("inf")
+    rows = torch.repeat_interleave(torch.arange(n), (rp[1:] - rp[:-1]).long())
+    want = (A.double()[rows] * B.double()[ci.long()]).sum(1)
+    bound = 1e-6 * (A.double()[rows] * B.double()[ci.long()]).abs().sum(1)
+    val = torch.ones(ci.shape[0])
+    args = [t.cuda() for t in (A, B)]
+    if split:
+        rps, tr = ops.split_csr(rp, 4)
+        got = ops.csr_split_sddmm(*args, rps.cuda(), ci.cuda(), val.cuda(), tr.cuda(), 1, 8).cpu().double()
+    else:
+        got = ops.csr_sddmm(*args, rp.cuda(), ci.cuda(), val.cuda(), 1, 8).cpu().double()
+    clean = ci != inf_col
+    assert bool(((got - want).abs() <= bound)[clean].all()) and not bool(torch.isfinite(got[~clean]).any())
