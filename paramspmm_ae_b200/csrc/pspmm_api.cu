@@ -715,8 +715,12 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
         return PSPMM_OK;
     LaunchShape s;
     // At most 16 lanes per row: with 32 the exchange of partial sums (31 shuffles and 62 selects per 32
-    // entries of a single row) took over, 12.6 ms against 4.1 for 115 M entries at dim 128.  Scalar and
-    // 8-byte loads fill 8 lanes up to 4 slices first (dim 17: 64 against 87 us, 4 M entries).  Rows of
+    // entries of a single row) took over, 12.6 ms against 4.1 for 115 M entries at dim 128.  Fewer lanes
+    // with up to 4 slices each take fewer steps of it: scalar and 8-byte loads fill 8 lanes first (dim 17: 64 against 87 us,
+    // 4 M entries), 9 to 12 vectors of 16 bytes go on 4 lanes and up to 32 on 8 (4 M entries, 48 columns: 93 us on 16
+    // lanes, 75; 64 93 and 84; 100 160 and 147; band of 24 at 80 columns 293 and 194; 64 threads per CTA gain another 4 % on
+    // scattered columns and lose 10 % on bands).  Few entries unsplit are left on 16 up to 64 columns: their long rows
+    // end last, and a narrow group walks its piece longer (power law of 0.9 M, 48 columns: 41 us, on 4 lanes 45).  Rows of
     // more than 3 slices of 16 lanes go through column tiles of 2 inside the kernel (a fourth slice
     // leaves too few registers: dim 256 14.0 ms, two tiles of 128 9.0); scalar loads keep up to 8.
     pspmm_cfg narrow = {};
@@ -724,8 +728,11 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
         narrow = *cfg;
     const int vw_max = pspmm_vw_max(dim, ldA, ldB, A, B);
     const int nvec_max = dim / vw_max;
-    if (V == 1 && (narrow.lanes_per_row == 0 || narrow.lanes_per_row > 16) && nvec_max > 8)
-        narrow.lanes_per_row = vw_max < 4 && nvec_max <= 32 ? 8 : 16;
+    if (V == 1 && (narrow.lanes_per_row == 0 || narrow.lanes_per_row > 16) && nvec_max > 8) {
+        const bool chosen = narrow.lanes_per_row > 16;  // by the caller, for more lanes than there are
+        const bool few = !target_row && nvec_max <= 16 && n_entries < 2000000;
+        narrow.lanes_per_row = nvec_max > 32 || (vw_max == 4 && (chosen || few)) ? 16 : (vw_max == 4 && nvec_max <= 12 ? 4 : 8);
+    }
     pspmm_resolve_shape(&narrow, dim, vw_max, V, SHAPE_SDDMM, &s, -1);
     if (V == 1 && s.lpr > 16) {
         s.lpr = 16;

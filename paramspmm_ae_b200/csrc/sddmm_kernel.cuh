@@ -207,13 +207,15 @@ __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
                 }
             }
             __syncthreads();
-            // Pieces of 32 entries, dealt to the lane groups in turn over all long rows of the range.
+            // Pieces of 32 entries, dealt to the lane groups in turn over all long rows of the range.  (16 for narrow groups of
+            // several slices: they are more to a CTA, and each takes longer.)
+            constexpr int PIECE = LPR <= 8 && CF > 1 && V == 1 ? 16 : 32;
             const int n = n_long;
             int i = 0, piece0 = 0;  // the row the group stands in, and the number of its first piece
             for (int p0 = 0;; p0 += gpc) {
                 const int p = p0 + g;
                 int pieces = 0;
-                while (i < n && p >= piece0 + (pieces = (row_hi[i] - row_lo[i] + 31) / 32)) {
+                while (i < n && p >= piece0 + (pieces = (row_hi[i] - row_lo[i] + PIECE - 1) / PIECE)) {
                     piece0 += pieces;
                     ++i;
                 }
@@ -223,10 +225,10 @@ __global__ void __launch_bounds__(512) sddmm_seg_kernel(const SddmmArgs a)
                 int64_t row = 0;
                 if (i < n) {
                     row = row_list[i];
-                    lb = row_lo[i] + (p - piece0) * 32;
-                    hb = row_hi[i] - lb > 32 ? lb + 32 : row_hi[i];
+                    lb = row_lo[i] + (p - piece0) * PIECE;
+                    hb = row_hi[i] - lb > PIECE ? lb + PIECE : row_hi[i];
                 }
-                sddmm_entries<LPR, VW, CF, V>(a, row, lb, hb, 32, gl);
+                sddmm_entries<LPR, VW, CF, V>(a, row, lb, hb, PIECE, gl);
             }
             __syncthreads();
         }
