@@ -140,8 +140,44 @@ def _no_long_rows(plan):
     return int(not plan.get("if_split") and not plan.get("regime", "skewed").endswith("skewed"))
 
 
-def choose(stats, dim, op="spmm"):
-    """Table lookup (regime x dim); falls back to a rule when the table has no entry."""
+_NO_SHAPE = dict(lanes_per_row=0, vec_width=0, cta_threads=0, rows_per_group=0, gather_batch=0, col_tile=0, bucketed=0,
+                 vec_size=1)  # the launch's own rules
+
+
+def _fit_to_size(plan, stats, dim, n_cols):
+    """The table is fitted on matrices of about a million rows; smaller ones do not fill the GPU with its plans.
+
+    Skewed: a lane group walks its `granularity x rows_per_group` entries one gather batch after the other, which takes 0.16 us
+    per entry in batches of one, 0.12 of two, 0.08 of four and 0.06 of eight.  Where that is longer than 0.42 of what all
+    gathers take at 12 TB/s, the group gets pieces of 32 and fewer of
+    them; below 8 us of gathers the plain split is as good.  us with the table's plan / so: power law of 100 K rows of 25, 256
+    columns 298 / 154, 128 127 / 90, 16 58 / 31; R-MAT of 300 K rows of 8, 128 columns 153 / 117, 16 55 / 37; power law of 30 K rows of
+    25, 256 columns 146 / 51; of 8 K rows of 8, 32 columns 47 / 8.4.  (100 K rows of 100, 64 columns, ratio 0.29: 152 / 166 if it did.)
+    Even and local: column tiles pay while the dense operand exceeds the L2 (uniform 300 K rows of 16, 128 columns 211 us, untiled
+    242), not below (100 K, 192 columns 111 and 90; 8 K, 256 columns 41 and 14); up to 1.7 M output values the launch's own
+    rules, which see the size, are up to twice as fast (8 K rows of 16 at 32 columns 12.4 and 6.0; 30 K of 8 in a band at 16 8.3 and 6.2;
+    but 30 K rows of 24 in a band at 64 14.4 and 18.5)."""
+    n, gathers = stats["n_rows"], stats["nnz"] * dim * 4 / 12e6
+    if not plan["regime"].endswith("skewed"):
+        if n * dim <= 1.7e6 or (plan["col_tile"] and n_cols * dim * 4 <= 110e6):
+            plan.update(_NO_SHAPE, if_split=0, granularity=None, no_long_rows=1)
+        return
+    if not plan["if_split"] or not plan["rows_per_group"]:
+        return
+    slices = -(-dim // (4 * (plan["lanes_per_row"] or 32)))
+    batch = max(1, (plan["gather_batch"] or 8) // slices)
+    per_entry = 0.16 if batch == 1 else (0.12 if batch < 4 else (0.08 if batch < 8 else 0.06))
+    if plan["granularity"] * plan["rows_per_group"] * per_entry <= 0.42 * gathers:
+        return
+    if gathers < 8:
+        plan.update(_NO_SHAPE, granularity=32)
+    elif plan["granularity"] * plan["rows_per_group"] > (128 if gathers >= 20 else 64):
+        plan.update(granularity=32, rows_per_group=4 if gathers >= 20 else 2, col_tile=0)
+
+
+def choose(stats, dim, op="spmm", n_cols=None):
+    """Table lookup (regime x dim), fitted to the matrix's size; falls back to a rule when the table has no entry.
+    ``n_cols``: rows of the dense operand where they are not those of the matrix (a shard)."""
     reg = regime(stats)
     per_regime = table().get("entries", {}).get(op, {})
     ent = per_regime.get(reg, {})
@@ -171,6 +207,8 @@ def choose(stats, dim, op="spmm"):
     plan["no_long_rows"] = _no_long_rows(plan)
     if plan["if_split"] and not plan.get("granularity"):
         plan["granularity"] = auto_granularity(stats["real_avg"])
+    if op == "spmm":
+        _fit_to_size(plan, stats, dim, stats["n_rows"] if n_cols is None else n_cols)
     return plan
 
 

@@ -666,7 +666,7 @@ class ShardedSpMM:
         bound = {}
 
         def local_spmm(out, B, rowPtr, colIdx, val, accumulate=False):
-            p = decider.choose(stats, B.shape[1])
+            p = decider.choose(stats, B.shape[1], n_cols=B.shape[0])
             # (a bucketed plan permutes the entries, so it belongs to one column / value array pair)
             key = (int(p["if_split"]), p.get("granularity"), int(p.get("bucketed", 0)), colIdx.data_ptr(), val.data_ptr())
             if key not in bound:  # layout arrays of this plan, built once on the device and kept

@@ -315,6 +315,30 @@ def test_table_measures_every_regime_and_the_decider_reaches_them():
     assert decider.regime(st) == "long_local" and decider.choose(st, 64)["regime"] == "long_local"
 
 
+def test_plans_fit_the_size_of_the_matrix():
+    """Plans of the table stand for matrices that fill the GPU; smaller ones get shorter groups, or the launch's own rules."""
+    from paramspmm_ae_b200 import decider
+
+    def plan(n, k, dim, cov=2.0, n_cols=None):
+        stats = {"n_rows": n, "nnz": n * k, "avg": float(k), "cov": cov, "max": k * (300 if cov else 1), "real_avg": float(k), "near_diag": 0.0}
+        p = decider.choose(stats, dim, n_cols=n_cols)
+        assert (p["granularity"] is not None) == bool(p["if_split"]) and p["no_long_rows"] == int(not cov)
+        return p
+
+    table = decider.table()["entries"]["spmm"]
+    for dim in (16, 64, 128, 256):
+        full = table["medium_skewed"][str(dim)]
+        assert all(plan(4_000_000, 25, dim)[k] == full[k] for k in ("granularity", "rows_per_group", "bucketed", "lanes_per_row"))
+        p = plan(100_000, 25, dim)
+        assert p["bucketed"] and p["granularity"] * p["rows_per_group"] <= 128 and p["lanes_per_row"] == full["lanes_per_row"]
+        p = plan(5_000, 8, dim)
+        assert p["if_split"] and not p["bucketed"] and not p["lanes_per_row"] and p["granularity"] == 32
+        p = plan(8_000, 16, dim, cov=0.0)
+        assert not p["if_split"] and not p["col_tile"] and (dim > 212 or not p["lanes_per_row"])
+    assert plan(1_000_000, 16, 256, cov=0.0)["col_tile"] and not plan(100_000, 16, 256, cov=0.0)["col_tile"]
+    assert plan(100_000, 16, 256, cov=0.0, n_cols=1_000_000)["col_tile"]      # (a shard: the dense operand is the whole one)
+
+
 def test_header_is_plain_c_and_declares_what_the_python_shim_binds(tmp_path):
     """include/pspmm.h must compile as C99 and as C++ on its own (it is what a foreign-language
     binding includes), and every function the ctypes shim binds must be declared in it."""
