@@ -45,6 +45,24 @@ __device__ __forceinline__ void long_scan(const LongArgs &a, const int32_t *segP
     }
 }
 
+// The same totals, all of them, by one CTA for itself.  One barrier is needed before they are read.
+__device__ __forceinline__ void long_own_totals(int *totals, const LongArgs &a, const int32_t *segPtr, int64_t n_seg)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int t = warp; t < a.n_totals; t += blockDim.x >> 5) {
+        int sum = 0;
+#pragma unroll 8
+        for (int i = 0; i < PSPMM_LONG_ROWS / 32; ++i) {
+            const int64_t r = (int64_t)t * PSPMM_LONG_ROWS + i * 32 + lane;
+            const int len = r < n_seg ? __ldg(segPtr + r + 1) - __ldg(segPtr + r) : 0;
+            sum += len > PSPMM_LONG_ROW ? len : 0;
+        }
+        sum = __reduce_add_sync(PSPMM_FULL_MASK, sum);
+        if (lane == 0)
+            totals[t] = sum;
+    }
+}
+
 // Inclusive sum over the 256 threads of a CTA; `warps` is scratch for 8 words.  One barrier before the
 // result, and one is needed before the next use of `warps`.
 template <typename T>
@@ -92,8 +110,9 @@ struct LongShare {
     int64_t r;
     int share, total;  // total: entries of this look that belong to the share
 
-    // False: nothing to do (no row is long, or fewer shares are needed than there are).
-    __device__ __forceinline__ bool begin(const LongArgs &a, Shared &sh, int share_)
+    // False: nothing to do (no row is long, or fewer shares are needed than there are).  `own`: totals of
+    // long_own_totals in shared memory, or nullptr.
+    __device__ __forceinline__ bool begin(const LongArgs &a, Shared &sh, int share_, const int *own = nullptr)
     {
         const int tid = threadIdx.x;
         const int each = (a.n_totals + 255) / 256;
@@ -103,7 +122,7 @@ struct LongShare {
 #pragma unroll 8
         for (int i = 0; i < each; ++i) {
             const int t = tid * each + i;
-            const int x = t < a.n_totals ? __ldcg(a.totals + t) : 0;
+            const int x = t >= a.n_totals ? 0 : (own ? own[t] : __ldcg(a.totals + t));
             any |= x > 0;
             mine += (unsigned long long)x + (t < a.n_totals ? PSPMM_LONG_LOOK : 0);
         }
@@ -123,7 +142,7 @@ struct LongShare {
             unsigned long long before = upto - mine;
             int t = tid * each;
             while (true) {
-                const unsigned long long x = (unsigned long long)__ldcg(a.totals + t) + PSPMM_LONG_LOOK;
+                const unsigned long long x = (unsigned long long)(own ? own[t] : __ldcg(a.totals + t)) + PSPMM_LONG_LOOK;
                 if (before + x > first)
                     break;
                 before += x;

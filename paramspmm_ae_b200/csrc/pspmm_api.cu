@@ -569,6 +569,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
             long_place(&a.lng, scratch);
         else
             a.lng = LongArgs{};
+        // (the look at all rows by every share pays while the segments are short of it: 19.7 K rows with hubs, dim 16 22.5 -> 20.4
+        // us, 32 24.9 -> 20.8, 8 K rows at 64 24.1 -> 18.8; but at 128 24.9 -> 26.7, and 20 K rows without any 16.0 -> 18.7)
+        a.lng.own_totals = a.lng.n_totals <= PSPMM_OWN_TOTALS && dim <= 64;
     }
     const int64_t per_cta = (int64_t)(s.threads / s.lpr) * s.rpg;
     const int64_t gx = (n_seg + per_cta - 1) / per_cta + a.lng.scan_ctas;

@@ -90,7 +90,9 @@ struct LongArgs {
     int32_t n_counters;
     float *partials;    // two rows per share
     int32_t shares;     // CTAs (per column tile) of the second kernel
+    int32_t own_totals; // 1: these add up the totals themselves (n_totals <= PSPMM_OWN_TOTALS) and need not wait for the first
 };
+#define PSPMM_OWN_TOTALS 64
 
 // Host side: sizes for `sms` SMs with `per_sm` resident CTAs of the second kernel: one wave of shares, more
 // when they would exceed 16 K entries (equal shares do not end together).
@@ -102,6 +104,7 @@ static inline void long_layout(LongArgs *a, int64_t n_rows, int64_t n_entries, i
     waves = waves < 16 ? waves : 16;
     a->shares = sms * per_sm > tiles ? sms * per_sm * waves / tiles : 1;
     a->n_counters = a->shares * tiles;
+    a->own_totals = 0;
 }
 // Positions (long_rows.cuh) per share.
 __host__ __device__ static inline int64_t long_share_size(int64_t units, int shares)

@@ -32,7 +32,7 @@
 // the pre-pass.
 //
 // Long rows of an unsplit layout are left to spmm_long_rows_kernel below, which cuts them over the
-// whole GPU; here they count as empty rows (their zeros are overwritten).
+// whole GPU; here they are passed over.
 #pragma once
 
 #include <type_traits>
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                 run_start = row + 1;
             }
             // (pieces of a split layout are never empty)
-            const bool emit = !ACC || split || re > rb;
+            const bool emit = (!ACC || split || re > rb) && !skip;
 #pragma unroll
             for (int w = 0; w < V; ++w) {
                 float *crow = a.C + (orow * V + w) * a.ldC;
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256, SpmmOcc<MLP>::MIN_CTAS) spmm_seg_kernel(c
                     const int left = a.dim - vec0 * VW, cols = left < LPR * CF * VW ? left : LPR * CF * VW;
                     float *to = crow + vec0 * VW;
                     __syncwarp(gmask);
-                    for (int j = gl; j < cols; j += LPR) {
+                    for (int j = emit ? gl : cols; j < cols; j += LPR) {
                         if (shared)
                             red_add_vec<1>(to + j, out + j);
                         else
@@ -402,10 +402,21 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmKernel
     const int share = blockIdx.x;
     float acc[V][1][VW], first[V][VW];
 
-    pdl_wait();
+    // Few rows: the CTAs find their shares without the segment kernel and gather beside it; only the counters, which it
+    // clears, are waited for.  (It writes none of these rows.  19.7 K rows, 197 K entries, dim 16: the two took 9.5 and 8 us
+    // one behind the other.)  Every CTA waits for it once, so that this launch does not end before it.
+    __shared__ int own[PSPMM_OWN_TOTALS];
+    if (a.lng.own_totals) {
+        long_own_totals(own, a.lng, a.segPtr, a.n_seg);
+        __syncthreads();
+    } else {
+        pdl_wait();
+    }
     LongShare job;
-    if (!job.begin(a.lng, sh, share))
+    if (!job.begin(a.lng, sh, share, a.lng.own_totals ? own : nullptr)) {
+        pdl_wait();
         return;
+    }
     while (job.look(sh, a.segPtr, a.n_seg)) {
         const int total = job.total;
         if (total == 0)
@@ -503,6 +514,7 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmKernel
             }
             emit(i2, w, vi * VW, sum);
         }
+        pdl_wait();  // (the counters; no wait but the first)
         job.arrive(a.lng, sh, blockIdx.y, gridDim.y);
         for (int q = 0; q < 2; ++q) {
             if (!sh.last[q])
@@ -522,6 +534,7 @@ __global__ void __launch_bounds__(256, 3) spmm_long_rows_kernel(const SpmmKernel
         }
         __syncthreads();
     }
+    pdl_wait();
 }
 
 template <int VW, int V, bool RAGGED = false>

@@ -169,11 +169,11 @@ class AGNNFusedFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, X, weights, attention_w, P, colIdx):
         Xp = ops.dense_mm(X, weights)
-        beta = _beta(attention_w).clone()  # (the backward uses the value of this forward)
+        beta = _beta(attention_w)
         try:
             scores = torch.empty(P.colIdx.shape[0], dtype=torch.float32, device=Xp.device)
         except torch.cuda.OutOfMemoryError:
-            scores = None
+            scores, beta = None, beta.clone()  # (the backward uses the value of this forward)
         out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, beta, P.target_row, scores)
         ctx.save_for_backward(X, weights, *((Xp, beta) if scores is None else (scores,)))
         ctx.P = P

@@ -388,15 +388,15 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
     long_rows = target_row is None and (cfg is None or not (cfg.no_long_rows or cfg.accumulate))
     pad = cfg is None or (not cfg.accumulate and cfg.vec_width in (0, 4))
-    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, pad)
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, dim, pad)
 
 
-def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, pad=True):
+def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, dim, pad=True):
     seg = rowPtr.data_ptr()
-    n, dim = X.shape[0], out.shape[1]
-    if dim & 1 and V == 1 and pad and X.shape[1] == dim and _padding_pays(n, colIdx.shape[0], dim, target_row is not None):
+    n, cols = X.shape
+    if dim & 1 and V == 1 and pad and cols == dim and _padding_pays(n, colIdx.shape[0], dim, target_row is not None):
         X = _pad_rows(X)
-    cols = X.shape[1]
+        cols = X.shape[1]
     # row pointers of a split layout go into the split arguments
     plain, split, target, n_seg = (seg, None, None, 0) if target_row is None else (
         None, seg, target_row.data_ptr(), rowPtr.shape[0] - 1)
@@ -415,8 +415,8 @@ def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, lo
 def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
     _check_legacy(CF, W)
     _spmm_inputs(X, rowPtr, colIdx, val, target_row, V)
-    n = X.shape[0]
-    dim = X.shape[1] if dim is None else dim  # (fewer: X is padded, see spmm_into)
+    n, cols = X.shape
+    dim = cols if dim is None else dim  # (fewer: X is padded, see spmm_into)
     # The reference sizes the output from the dense input, zeros_like(input) for CSR
     # (SpMM/SpMM_kernel.cu:136) and the input's row count rounded up to a multiple of V for the
     # block layouts (:281-282, 427-428), and walks as many (block-)rows as the row pointer has.
@@ -425,7 +425,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
     padded = (n + V - 1) // V * V
     n_out = padded // V
     n_seg = rowPtr.shape[0] - 1
-    out = torch.empty_like(X) if padded == n and dim == X.shape[1] else torch.empty((padded, dim), dtype=torch.float32, device=X.device)
+    out = torch.empty_like(X) if padded == n and dim == cols else torch.empty((padded, dim), dtype=torch.float32, device=X.device)
     if target_row is None:
         if n_seg > n_out:
             raise RuntimeError("rowPtr describes %d (block-)rows, the input only allows %d" % (n_seg, n_out))
@@ -433,7 +433,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
             out[n_seg * V:].zero_()
             n_out = n_seg
     return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out,
-                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None)
+                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None, dim)
 
 
 def csr_spmm(X, rowPtr, colIdx, val, CF, blkWarpNum):

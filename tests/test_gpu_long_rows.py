@@ -176,3 +176,32 @@ def test_ranges_that_end_near_the_index_limit(dim):
     assert torch.equal(got.cpu(), scores)
     got = ops.csr_sddmm(Ad, Bd, rpd, ci, val, 1, 8)[first:]
     assert torch.equal(got.cpu(), scores)
+
+
+@pytest.mark.parametrize("rows", [1, 511, 512, 513, 32768, 32769])
+@pytest.mark.parametrize("dim", [16, 47, 64, 68])
+def test_long_rows_beside_the_segments(rows, dim):
+    """Row counts on both sides of what a share looks at by itself (64 x 512 rows): first, last and neighbouring rows long,
+    repeated calls on one scratch-sized allocation, rows of the threshold's length."""
+    from paramspmm_ae_b200 import ops
+    dev = torch.device("cuda")
+    n_cols = max(rows, 700)
+    ln = torch.zeros(rows, dtype=torch.int64)
+    ln[::7] = 3
+    ln[rows // 2:rows // 2 + 3] = torch.tensor([64, 65, 600])[: min(3, rows - rows // 2)]
+    ln[0], ln[-1] = 300, 700
+    rp = torch.cat([torch.zeros(1, dtype=torch.int64), ln.cumsum(0)]).to(torch.int32).to(dev)
+    gen = torch.Generator().manual_seed(rows + dim)
+    ci = torch.cat([torch.randperm(n_cols, generator=gen)[:k].sort().values for k in ln.tolist() if k]).to(torch.int32).to(dev)
+    val = torch.rand(ci.shape[0], generator=gen).to(dev)
+    X = torch.randn(n_cols, dim, generator=gen).to(dev)
+    r = torch.repeat_interleave(torch.arange(rows, device=dev), ln.to(dev))
+    terms = val.double()[:, None] * X.double()[ci.long()]
+    want = torch.zeros(rows, dim, dtype=torch.float64, device=dev).index_add_(0, r, terms)
+    scale = torch.zeros(rows, dim, dtype=torch.float64, device=dev).index_add_(0, r, terms.abs())
+    first = None
+    for _ in range(5):
+        got = ops.csr_spmm(X, rp, ci, val, 1, 8)[:rows]
+        assert bool(((got.double() - want).abs() <= 1e-5 * scale + 1e-12).all())
+        first = got if first is None else first
+        assert torch.equal(got, first)
