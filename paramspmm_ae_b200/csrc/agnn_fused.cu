@@ -279,7 +279,7 @@ __device__ __forceinline__ float agnn_weight_sum(float l, unsigned lanes)
 
 // The same for scores that lie in a.scores: one gather per entry (the rows of a.Vm) and no exchange.  A training
 // step's backward pass takes the forward's: 115 M entries, dim 64: 3.64 ms with the scores recomputed from a
-// second gather, 1.77 (16.5 TB/s of gathered rows; the bare gather takes 1.4); the forward writes them in 0.09 ms of 1.89.
+// second gather, 1.72 (17 TB/s of gathered rows; the bare gather takes 1.4); the forward writes them in 0.09 ms of 1.89.
 // Bound: the latency of eight 32-byte loads in flight per lane at two resident CTAs.
 template <int LPR, int CF, int BS, int VW, bool COL>
 __device__ __forceinline__ void agnn_scored_entries(const AgnnArgs &a, const bool (&act)[CF], const int (&voff)[CF], int lb,
@@ -364,14 +364,16 @@ __device__ __forceinline__ void agnn_load_row(const AgnnArgs &a, int64_t row, bo
 }
 
 // Resident CTAs the register budget is cut for: 16 floats of a row per lane would otherwise take 142
-// registers and leave one (12 M entries at dim 128: 1,040 us instead of 570).
+// registers and leave one (12 M entries at dim 128: 1,040 us instead of 570).  Taking scores, three CTAs of 80 registers
+// and eight rows in flight beat two of 128 up to 16 lanes (steps of 4 M entries, dim 128 677 -> 640 us, 12 M 1011 -> 970; 115 M,
+// dim 64: the kernel 1.77 -> 1.72 ms); on 32 lanes they spill, and the long rows' kernel, with more state, loses 3 %.
 template <int CF, int VW, bool SEP>
 struct AgnnOcc {
     static constexpr int MIN_CTAS = SEP ? (CF * VW >= 16 ? 1 : 2) : (CF * VW >= 16 ? 2 : 3);
 };
 
 template <int LPR, int CF, int BS, int VW, bool SEP, bool COL, int SCORES, bool SOFTMAX>
-__global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fused_kernel(const AgnnArgs a)
+__global__ void __launch_bounds__(256, SCORES == SCORES_TAKE && LPR <= 16 ? 3 : AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_fused_kernel(const AgnnArgs a)
 {
     static_assert(BS <= LPR, "a batch cannot be wider than the lane group");
     pdl_launch_dependents();
