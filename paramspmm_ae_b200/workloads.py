@@ -168,7 +168,7 @@ def agnn_layer(n=232_965, pairs=57_180_000, dim=64, seed=41, iters=10, grans=(0,
     out["fused_softmax_best_ms"] = min(f["fused_softmax_ms"] for f in fused)
     # One training step of the layer (projection, propagation, backward to the input, the weights and
     # the attention weight): the reference's three-kernel composition, which writes the attention
-    # values and the score gradient per edge, against the fused function, which writes neither.
+    # values and the score gradient per edge, against the fused function, which writes the scores once.
     from . import gnn_conv, pcsr
     gfast = min((f for f in fused if (f["vec_width"], f["lanes_per_row"], f["batch"]) == (0, 0, 0)),
                 key=lambda f: f["fused_ms"])["granularity"]
