@@ -157,7 +157,10 @@ def _fit_to_size(plan, stats, dim, n_cols):
     242), not below (100 K, 192 columns 111 and 90; 8 K, 256 columns 41 and 14); up to 1.7 M output values the launch's own
     rules, which see the size, are up to twice as fast (8 K rows of 16 at 32 columns 12.4 and 6.0; 30 K of 8 in a band at 16 8.3 and 6.2;
     but 30 K rows of 24 in a band at 64 14.4 and 18.5)."""
+    if "n_rows" not in stats or "nnz" not in stats:
+        return
     n, gathers = stats["n_rows"], stats["nnz"] * dim * 4 / 12e6
+    n_cols = n if n_cols is None else n_cols
     if not plan["regime"].endswith("skewed"):
         if n * dim <= 1.7e6 or (plan["col_tile"] and n_cols * dim * 4 <= 110e6):
             plan.update(_NO_SHAPE, if_split=0, granularity=None, no_long_rows=1)
@@ -208,7 +211,7 @@ def choose(stats, dim, op="spmm", n_cols=None):
     if plan["if_split"] and not plan.get("granularity"):
         plan["granularity"] = auto_granularity(stats["real_avg"])
     if op == "spmm":
-        _fit_to_size(plan, stats, dim, stats["n_rows"] if n_cols is None else n_cols)
+        _fit_to_size(plan, stats, dim, n_cols)
     return plan
 
 

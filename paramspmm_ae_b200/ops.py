@@ -413,6 +413,8 @@ def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, lo
 
 
 def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
+    if dim is not None and tuner is not None:  # (its configurations may ask for narrower loads)
+        return _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W)[:, :dim].contiguous()
     _check_legacy(CF, W)
     _spmm_inputs(X, rowPtr, colIdx, val, target_row, V)
     n, cols = X.shape
@@ -433,7 +435,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
             out[n_seg * V:].zero_()
             n_out = n_seg
     return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out,
-                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None, dim)
+                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None, dim, tuner is None)
 
 
 def csr_spmm(X, rowPtr, colIdx, val, CF, blkWarpNum):
@@ -483,7 +485,8 @@ def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=No
     _check_output(out, rowPtr, split, n_out, V, dim)
     nent = colIdx.shape[0]
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
-    if dim & 1 and V == 1 and _padding_pays(n, nent, dim, split):  # (the copy is part of the call)
+    if (dim & 1 and V == 1 and _padding_pays(n, nent, dim, split)  # (the copy is part of the call)
+            and (tuner is None if cfg is None else not cfg.accumulate and cfg.vec_width in (0, 4))):
         return _loop_ms(lambda: spmm_into(out, X, rowPtr, colIdx, val, target_row, V, n_out, CF, W, cfg), warmup, iters)
     ms = ctypes.c_float(0.0)
     null = None

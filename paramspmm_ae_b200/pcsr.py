@@ -152,7 +152,8 @@ class pcsr_spmm(object):
         rows = self._planned.n_rows
         if n < rows:
             raise RuntimeError("the matrix has %d rows, the input only %d" % (rows, n))
-        cut = Xp.shape[1] != dim and self._planned.V != 1  # (block layouts store what they gather)
+        # (block layouts, and plans with narrower loads, store what they gather)
+        cut = Xp.shape[1] != dim and (self._planned.V != 1 or self._planned.plan.get("vec_width") in (1, 2))
         out = torch.empty((n, Xp.shape[1] if cut else dim), dtype=torch.float32, device=X.device)
         if n > rows:
             out[rows:].zero_()

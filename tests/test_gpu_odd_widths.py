@@ -91,3 +91,21 @@ def test_legacy_calls_on_both_sides_of_the_rule(dim, split, monkeypatch):
         results.append(run())
     for a, b in zip(*results):
         assert a.shape == b.shape and float((a - b).norm()) <= 1e-6 * float(a.norm())
+
+
+@pytest.mark.parametrize("vec_width", [0, 1, 2, 4])
+def test_plans_and_tuners_with_narrower_loads_take_odd_widths(vec_width, monkeypatch):
+    """Configurations of the caller that ask for narrower loads go the way they went, without the padded product."""
+    from paramspmm_ae_b200 import decider, ops, pcsr, synth
+    m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
+    X = torch.randn(3000, 255, device="cuda")
+    want = ops.csr_spmm(X, m.rowPtr, m.colIdx, m.val, 1, 8)
+    plan = decider.Plan(vec_size=1, lanes_per_row=0, vec_width=vec_width, cta_threads=0, rows_per_group=0, gather_batch=0, col_tile=0,
+                        if_split=1, granularity=32, bucketed=0)
+    P = pcsr.pcsr_spmm.from_plan(plan, m.rowPtr, m.colIdx, m.val)
+    H, W = torch.randn(3000, 16, device="cuda"), torch.randn(16, 47, device="cuda")
+    conv = ops.csr_spmm_forward(H, W, m.rowPtr, m.colIdx, m.val, 1, 8)
+    monkeypatch.setattr(ops, "tuner", lambda *a: dict(vec_width=vec_width))
+    for got, ref in ((P.GIN_spmm(X), want), (ops.csr_spmm(X, m.rowPtr, m.colIdx, m.val, 1, 8), want),
+                     (ops.csr_spmm_forward(H, W, m.rowPtr, m.colIdx, m.val, 1, 8), conv), (P.forward(H, W), conv)):
+        assert got.shape == ref.shape and got.is_contiguous() and float((got - ref).norm()) <= 1e-5 * float(ref.norm())
