@@ -395,7 +395,10 @@ def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, lo
     seg = rowPtr.data_ptr()
     n, cols = X.shape
     if dim & 1 and V == 1 and pad and cols == dim and _padding_pays(n, colIdx.shape[0], dim, target_row is not None):
-        X = _pad_rows(X)
+        try:
+            X = _pad_rows(X)
+        except torch.cuda.OutOfMemoryError:
+            pass  # no room for the copy: the width's own loads
         cols = X.shape[1]
     # row pointers of a split layout go into the split arguments
     plain, split, target, n_seg = (seg, None, None, 0) if target_row is None else (
@@ -569,9 +572,12 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
     out = torch.empty_like(val)
     if dim & 1 and V == 1 and not time_only and _sddmm_padding_pays(B.shape[0], nent, dim):
         same = A.data_ptr() == B.data_ptr() and A.shape == B.shape
-        A = _pad_rows(A)
-        B = A if same else _pad_rows(B)
-        dim = A.shape[1]
+        try:
+            Ap = _pad_rows(A)
+            A, B = Ap, Ap if same else _pad_rows(B)
+            dim = A.shape[1]
+        except torch.cuda.OutOfMemoryError:
+            pass
     cfg = _cfg("sddmm", CF, W, dim, nent, n_seg, V, split)
     null = None
     # (block-)rows of the pattern; A may stop inside the last block-row when the node count is

@@ -109,3 +109,24 @@ def test_plans_and_tuners_with_narrower_loads_take_odd_widths(vec_width, monkeyp
     for got, ref in ((P.GIN_spmm(X), want), (ops.csr_spmm(X, m.rowPtr, m.colIdx, m.val, 1, 8), want),
                      (ops.csr_spmm_forward(H, W, m.rowPtr, m.colIdx, m.val, 1, 8), conv), (P.forward(H, W), conv)):
         assert got.shape == ref.shape and got.is_contiguous() and float((got - ref).norm()) <= 1e-5 * float(ref.norm())
+
+
+def test_products_run_without_room_for_the_copy(monkeypatch):
+    from paramspmm_ae_b200 import ops, synth
+    m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
+    X, Y = (torch.randn(3000, 31, device="cuda") for _ in range(2))
+    monkeypatch.setattr(ops, "_padding_pays", lambda *a: True)
+    monkeypatch.setattr(ops, "_sddmm_padding_pays", lambda *a: True)
+    call = lambda: (ops.csr_spmm(X, m.rowPtr, m.colIdx, m.val, 1, 8), ops.csr_sddmm(X, Y, m.rowPtr, m.colIdx, m.val, 1, 8))
+    padded, pad, seen = call(), ops._pad_rows, []
+
+    def refuse(t):
+        seen.append(t)
+        if len(seen) == 2:  # (the first operand of the scores fits, the second does not)
+            return pad(t)
+        raise torch.cuda.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(ops, "_pad_rows", refuse)
+    for a, b in zip(padded, call()):
+        assert float((a - b).norm()) <= 1e-6 * float(b.norm())
+    assert len(seen) == 3
