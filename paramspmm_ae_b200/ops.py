@@ -359,6 +359,12 @@ def _padding_pays(n, n_entries, dim, split):
     return work >= 1000 * n and (dim > 48 or n_entries >= 48 * n)
 
 
+def _takes_padding(cfg):
+    """Whether a call's configuration (None: the tuner's, if there is one) leaves the padded product open: it has 16-byte
+    loads only and does not accumulate."""
+    return tuner is None if cfg is None else not cfg.accumulate and cfg.vec_width in (0, 4)
+
+
 def _sddmm_padding_pays(n, n_entries, dim):
     """The same for edge scores (100 K rows of 32: 23 columns 52 / 46 us, 31 62 / 45, 63 77 / 69, 101 131 / 114; 500 K of 16: 31
     columns 132 / 112; but 47 columns 62 / 65, and of 16 101 columns 70 / 73)."""
@@ -387,8 +393,7 @@ def spmm_into(out, X, rowPtr, colIdx, val, target_row=None, V=1, n_out_rows=None
     _check_output(out, rowPtr, split, n_out_rows, V, dim)
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, split)
     long_rows = target_row is None and (cfg is None or not (cfg.no_long_rows or cfg.accumulate))
-    pad = cfg is None or (not cfg.accumulate and cfg.vec_width in (0, 4))
-    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, dim, pad)
+    return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, dim, _takes_padding(cfg))
 
 
 def _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out_rows, ref, long_rows, dim, pad=True):
@@ -438,7 +443,7 @@ def _spmm(X, rowPtr, colIdx, val, target_row, V, CF, W, dim=None):
             out[n_seg * V:].zero_()
             n_out = n_seg
     return _spmm_launch(out, X, rowPtr, colIdx, val, target_row, V, n_out,
-                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None, dim, tuner is None)
+                        _cfg("spmm", CF, W, dim, colIdx.shape[0], n_seg, V, target_row is not None), target_row is None, dim, _takes_padding(None))
 
 
 def csr_spmm(X, rowPtr, colIdx, val, CF, blkWarpNum):
@@ -488,8 +493,7 @@ def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=No
     _check_output(out, rowPtr, split, n_out, V, dim)
     nent = colIdx.shape[0]
     ref = ctypes.byref(cfg) if cfg is not None else _cfg("spmm", CF, W, dim, nent, n_seg, V, split)
-    if (dim & 1 and V == 1 and _padding_pays(n, nent, dim, split)  # (the copy is part of the call)
-            and (tuner is None if cfg is None else not cfg.accumulate and cfg.vec_width in (0, 4))):
+    if dim & 1 and V == 1 and _padding_pays(n, nent, dim, split) and _takes_padding(cfg):  # (the copy is part of the call)
         return _loop_ms(lambda: spmm_into(out, X, rowPtr, colIdx, val, target_row, V, n_out, CF, W, cfg), warmup, iters)
     ms = ctypes.c_float(0.0)
     null = None

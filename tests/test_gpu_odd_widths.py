@@ -111,6 +111,21 @@ def test_plans_and_tuners_with_narrower_loads_take_odd_widths(vec_width, monkeyp
         assert got.shape == ref.shape and got.is_contiguous() and float((got - ref).norm()) <= 1e-5 * float(ref.norm())
 
 
+@pytest.mark.parametrize("vec_width", [0, 1, 2, 4])
+@pytest.mark.parametrize("split", [False, True])
+def test_tuners_with_narrower_loads_take_odd_widths_into_an_output(vec_width, split, monkeypatch):
+    from paramspmm_ae_b200 import ops, synth
+    m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
+    rp, tr = ops.split_csr_device(m.rowPtr, 32) if split else (m.rowPtr, None)
+    X = torch.randn(3000, 255, device="cuda")
+    want = ops.csr_spmm(X, m.rowPtr, m.colIdx, m.val, 1, 8)
+    monkeypatch.setattr(ops, "_padding_pays", lambda *a: True)
+    monkeypatch.setattr(ops, "tuner", lambda *a: dict(vec_width=vec_width))
+    got = ops.spmm_into(torch.full_like(X, float("nan")), X, rp, m.colIdx, m.val, tr, n_out_rows=3000)
+    assert float((got - want).norm()) <= 1e-5 * float(want.norm())
+    assert ops.spmm_time_ms(X, rp, m.colIdx, m.val, tr, iters=2, n_out_rows=3000) > 0
+
+
 def test_products_run_without_room_for_the_copy(monkeypatch):
     from paramspmm_ae_b200 import ops, synth
     m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
