@@ -123,7 +123,8 @@ class Plan(dict):
     Keys: if_split (0/1), vec_size (1/2), granularity (partition length or None = the
     reference's rule), kernel fields lanes_per_row / vec_width / cta_threads /
     rows_per_group (0 = library default), and no_long_rows (1: the statistics of an unsplit
-    matrix show no row far longer than the others; a plan without the key goes by its regime).
+    matrix show no row that its lane group would walk for long after the others; a plan without the key goes by
+    its regime).
     """
 
     def kernel_cfg(self):
@@ -138,6 +139,22 @@ class Plan(dict):
 
 def _no_long_rows(plan):
     return int(not plan.get("if_split") and not plan.get("regime", "skewed").endswith("skewed"))
+
+
+def _walk_ends_late(stats, dim):
+    """Whether the longest row, walked by one lane group (0.05 - 0.08 us per entry), ends well after the rest of an unsplit
+    product.  The form of the kernel that cuts such rows costs 3 - 12 us where it has little to cut.
+    us walked / cut, 8 long rows among the mean: 5 K rows of 400, 16 columns, longest 600 67 / 36, 128 columns, 5,000 247 / 64;
+    20 K of 50, 64 columns, 800 48 / 36, 256 98 / 70; but 200 25 / 37 and 60 / 70; 6 K of 100, 128 columns, 400 31 / 33, 1,600
+    76 / 33; 50 K of 400, 16 columns, 600 178 / 231, 6,000 565 / 229."""
+    if "n_rows" not in stats or "nnz" not in stats:
+        return False
+    return 0.06 * stats["max"] > 20 + 0.2 * _gather_us(stats, dim)
+
+
+def _gather_us(stats, dim):
+    """What all gathers of a product take at 12 TB/s."""
+    return stats["nnz"] * dim * 4 / 12e6
 
 
 _NO_SHAPE = dict(lanes_per_row=0, vec_width=0, cta_threads=0, rows_per_group=0, gather_batch=0, col_tile=0, bucketed=0,
@@ -156,14 +173,18 @@ def _fit_to_size(plan, stats, dim, n_cols):
     Even and local: column tiles pay while the dense operand exceeds the L2 (uniform 300 K rows of 16, 128 columns 211 us, untiled
     242), not below (100 K, 192 columns 111 and 90; 8 K, 256 columns 41 and 14); up to 1.7 M output values the launch's own
     rules, which see the size, are up to twice as fast (8 K rows of 16 at 32 columns 12.4 and 6.0; 30 K of 8 in a band at 16 8.3 and 6.2;
-    but 30 K rows of 24 in a band at 64 14.4 and 18.5)."""
+    but 30 K rows of 24 in a band at 64 14.4 and 18.5).  A split without column tiles stays where a row ends late (30 K rows of
+    60, longest 900, 16 columns 39, walked 90, cut 51)."""
     if "n_rows" not in stats or "nnz" not in stats:
         return
-    n, gathers = stats["n_rows"], stats["nnz"] * dim * 4 / 12e6
+    n, gathers = stats["n_rows"], _gather_us(stats, dim)
     n_cols = n if n_cols is None else n_cols
     if not plan["regime"].endswith("skewed"):
+        late = _walk_ends_late(stats, dim)
+        if plan["if_split"] and not plan["col_tile"] and late:
+            return
         if n * dim <= 1.7e6 or (plan["col_tile"] and n_cols * dim * 4 <= 110e6):
-            plan.update(_NO_SHAPE, if_split=0, granularity=None, no_long_rows=1)
+            plan.update(_NO_SHAPE, if_split=0, granularity=None, no_long_rows=int(not late))
         return
     if not plan["if_split"] or not plan["rows_per_group"]:
         return
@@ -207,7 +228,7 @@ def choose(stats, dim, op="spmm", n_cols=None):
                 rows_per_group=0, gather_batch=0, col_tile=0, bucketed=0)
     plan.update(e)
     plan["regime"] = reg
-    plan["no_long_rows"] = _no_long_rows(plan)
+    plan["no_long_rows"] = int(_no_long_rows(plan) and not _walk_ends_late(stats, dim))
     if plan["if_split"] and not plan.get("granularity"):
         plan["granularity"] = auto_granularity(stats["real_avg"])
     if op == "spmm":

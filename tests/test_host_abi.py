@@ -339,6 +339,27 @@ def test_plans_fit_the_size_of_the_matrix():
     assert plan(100_000, 16, 256, cov=0.0, n_cols=1_000_000)["col_tile"]      # (a shard: the dense operand is the whole one)
 
 
+def test_plans_of_even_matrices_cut_rows_that_end_late():
+    """A matrix counts as even up to rows of 16 times the mean.  Where one lane group would walk such a row long after the product's
+    other rows, the plan keeps its split or lets the launch cut the row, in small matrices and in large ones."""
+    from paramspmm_ae_b200 import decider
+
+    def plan(n, k, longest, dim, drop=()):
+        stats = {"n_rows": n, "nnz": n * k, "avg": float(k), "cov": 0.2, "max": longest, "real_avg": float(k), "near_diag": 0.0}
+        p = decider.choose({f: v for f, v in stats.items() if f not in drop}, dim)
+        assert p["regime"].endswith("_even")
+        assert p.kernel_cfg()["no_long_rows"] == p["no_long_rows"]
+        return p
+
+    cut = lambda p: bool(p["if_split"]) or not p["no_long_rows"]
+    for n, k, longest in ((5000, 400, 5000), (20000, 50, 800), (6000, 100, 1600), (30000, 60, 900), (50000, 400, 6000)):
+        assert all(cut(plan(n, k, longest, dim)) for dim in (16, 64, 128, 256) if n * dim <= 4e6)
+    for n, k in ((5000, 16), (20000, 50), (100000, 16), (1000000, 16)):
+        assert all(plan(n, k, 16 * k if k == 16 else 2 * k, dim)["no_long_rows"] for dim in (64, 128))
+    assert cut(plan(100000, 100, 1600, 64)) and not cut(plan(100000, 100, 300, 64))
+    assert plan(20000, 50, 800, 64, drop=("nnz",))["no_long_rows"]  # (statistics without sizes go by the regime)
+
+
 def test_header_is_plain_c_and_declares_what_the_python_shim_binds(tmp_path):
     """include/pspmm.h must compile as C99 and as C++ on its own (it is what a foreign-language
     binding includes), and every function the ctypes shim binds must be declared in it."""
