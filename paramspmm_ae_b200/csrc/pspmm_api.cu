@@ -563,16 +563,26 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     a.dependent = target_row && !accumulate && !bucketed;
     a.lng = LongArgs{};
     if (scratch && (uintptr_t)scratch % 16 == 0 && !target_row && !accumulate && !(cfg && cfg->no_long_rows) && n_entries > PSPMM_LONG_ROW) {
-        const int lanes = pspmm_long_lanes(a.nvec, V);
-        long_layout(&a.lng, n_seg, n_entries, pspmm_sm_count(), 3, (a.nvec + lanes - 1) / lanes);
+        const int lanes = pspmm_long_lanes(a.nvec, V), tiles = (a.nvec + lanes - 1) / lanes, sms = pspmm_sm_count();
+        long_layout(&a.lng, n_seg, n_entries, sms, 3, tiles);
+        // Few rows: every share looks at all of them itself, beside the segments.  One share per SM up to 2048 entries per
+        // SM, two up to twice that where rows of 16 entries and more hide the look; for more work too few shares, and three per SM cost
+        // 16 - 27 % where no row is long.  us without this look / so: power law of 197 K entries, 16 columns 22.4 / 16.4, 64 30.7 / 22.6;
+        // 12 K rows, 312 K 22.7 / 16.4, 24.6 / 22.3; 20 K rows, 520 K 26.0 / 22.1, 27.5 / 29.4; 128 columns 24.9 / 26.7.  No long rows: 20 K of 10
+        // 7.2 / 9.4, 10.3 / 12.3; 20 K of 30 12.3 / 12.3, 16.6 / 18.4; 32 K of 18 12.1 / 14.4, 20.5 / 22.6; 32 K of 10 would be 8.3 / 12.3.
+        const int64_t one = (int64_t)PSPMM_OWN_ENTRIES * sms;
+        const int per_sm = n_entries <= one ? 1 : (n_entries <= 2 * one && n_entries >= 16 * n_seg ? 2 : 0);
+        if (per_sm && a.lng.n_totals <= PSPMM_OWN_TOTALS && dim <= 64 && (uintptr_t)segPtr % 16 == 0) {
+            a.lng.own_totals = 1;
+            if (a.lng.shares > per_sm * sms)
+                a.lng.shares = per_sm * sms;
+            a.lng.n_counters = a.lng.shares * tiles;
+        }
         if (long_fits(a.lng, n_entries) &&
             scratch_bytes >= long_head_bytes(a.lng) + (size_t)a.lng.shares * 2 * V * wide * sizeof(float))
             long_place(&a.lng, scratch);
         else
             a.lng = LongArgs{};
-        // (the look at all rows by every share pays while the segments are short of it: 19.7 K rows with hubs, dim 16 22.5 -> 20.4
-        // us, 32 24.9 -> 20.8, 8 K rows at 64 24.1 -> 18.8; but at 128 24.9 -> 26.7, and 20 K rows without any 16.0 -> 18.7)
-        a.lng.own_totals = a.lng.n_totals <= PSPMM_OWN_TOTALS && dim <= 64;
     }
     const int64_t per_cta = (int64_t)(s.threads / s.lpr) * s.rpg;
     const int64_t gx = (n_seg + per_cta - 1) / per_cta + a.lng.scan_ctas;

@@ -93,6 +93,7 @@ struct LongArgs {
     int32_t own_totals; // 1: these add up the totals themselves (n_totals <= PSPMM_OWN_TOTALS) and need not wait for the first
 };
 #define PSPMM_OWN_TOTALS 64
+#define PSPMM_OWN_ENTRIES 2048  // per SM and share of it, up to which they do
 
 // Host side: sizes for `sms` SMs with `per_sm` resident CTAs of the second kernel: one wave of shares, more
 // when they would exceed 16 K entries (equal shares do not end together).

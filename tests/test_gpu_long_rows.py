@@ -205,3 +205,33 @@ def test_long_rows_beside_the_segments(rows, dim):
         assert bool(((got.double() - want).abs() <= 1e-5 * scale + 1e-12).all())
         first = got if first is None else first
         assert torch.equal(got, first)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+@pytest.mark.parametrize("rows, mean", [(1536, 3), (4099, 9), (8193, 40), (8193, 80)])
+def test_own_look_and_its_limits(rows, mean, offset):
+    """Shares that look for long rows themselves, four row pointers at a time: row pointers off that boundary and more entries
+    than that is done for; long rows at the edges of a look's 512, of its quarters and of the matrix."""
+    from paramspmm_ae_b200 import ops
+    dev, dim, n_cols = torch.device("cuda:0"), 32, 4000
+    ln = torch.full((rows,), mean)
+    for r in (0, 1, 3, 4, 127, 128, 511, 512, 1023, rows - 2, rows - 1):
+        ln[r] = 65 + r % 300
+    rp = torch.zeros(rows + 1, dtype=torch.int64)
+    rp[1:] = ln.cumsum(0)
+    buf = torch.zeros(rows + 4, dtype=torch.int32, device=dev)
+    ptr = buf[offset:offset + rows + 1]
+    ptr.copy_(rp)
+    assert ptr.data_ptr() % 16 == 4 * offset
+    gen = torch.Generator().manual_seed(rows)
+    ci = torch.randint(0, n_cols, (int(rp[-1]),), generator=gen).int().to(dev)
+    val, X = torch.rand(ci.shape[0], generator=gen).to(dev), torch.randn(n_cols, dim, generator=gen).to(dev)
+    r = torch.repeat_interleave(torch.arange(rows, device=dev), ln.to(dev))
+    terms = val.double()[:, None] * X.double()[ci.long()]
+    want = torch.zeros(rows, dim, dtype=torch.float64, device=dev).index_add_(0, r, terms)
+    scale = torch.zeros(rows, dim, dtype=torch.float64, device=dev).index_add_(0, r, terms.abs())
+    out = torch.full((rows, dim), float("nan"), device=dev)
+    for _ in range(3):
+        ops.spmm_into(out, X, ptr, ci, val)
+        # (sums of up to 364 terms in another order: 1e-5 of the terms' absolute sum)
+        assert bool(((out.double() - want).abs() <= 1e-5 * scale + 1e-12).all())
