@@ -251,7 +251,8 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  * ParamSDDMM, a multiplication by the attention weight and ParamSpMM (gnn_conv.py:130-151:
  * AGNN_sddmm, `* attention_w`, AGNN_spmm), computed in one pass without the per-edge array; with
  * softmax != 0 the per-row edge softmax sits between the two.  Stored values are ignored (the
- * pattern is a mask, as in pspmm_sddmm_csr).  Rows without entries give zero rows.
+ * pattern is a mask, as in pspmm_sddmm_csr).  Rows without entries give zero rows.  The softmax's weighted sums
+ * stay below the row's entries times its largest |B_j| (or |V_j|); terms below 5e-35 in magnitude lose digits.
  * dim must be a multiple of 4 and at most 256, A, B and out 16-byte aligned with leading
  * dimensions that are multiples of 4 (PSPMM_E_UNSUPPORTED otherwise).  `vec_width` = floats per lane
  * per load: 0 (library's choice), 4, or 8 (256-bit loads; needs dim a multiple of 8 and 32-byte

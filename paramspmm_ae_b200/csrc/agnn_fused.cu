@@ -204,7 +204,8 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
                 // m: what the exponentials are taken against, at most 8 below the largest score so far.  It moves when a
                 // score exceeds it by more (a vote of the warp, mostly no), and l stays with the lanes until the end: two
                 // exchanges, an exponential and the accumulator's scaling leave the chain of every batch (12 M entries, split: dim 128
-                // 487 -> 468 us, 64 264 -> 250, 32 160 -> 148).  e^8 costs no accuracy: all terms of a row carry the same factor.
+                // 487 -> 468 us, 64 264 -> 250, 32 160 -> 148; moved by every larger score, 480, 256 and 153).  The weights, up to e^8, are
+                // scaled by 2^-12, exactly, so that the sums have the range that weights up to 1 leave them (no time).
                 const float over = score - m;
                 if (__any_sync(PSPMM_FULL_MASK, mine && over > 8.f)) {
                     float bm = mine ? score : -CUDART_INF_F;
@@ -222,7 +223,7 @@ __device__ __forceinline__ void agnn_entries(const AgnnArgs &a, const FVec<VW> (
                             acc[cf][i] *= sc;
                 }
                 // (a group whose scores so far are all -inf keeps an empty state)
-                p = mine && m > -CUDART_INF_F ? expf(score - m) : 0.f;
+                p = mine && m > -CUDART_INF_F ? expf(score - m) * 0x1p-12f : 0.f;
                 l += p;
             } else {
                 p = mine ? score : 0.f;

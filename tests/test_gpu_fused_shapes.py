@@ -152,3 +152,51 @@ def test_scores_of_finite_rows_stay_finite_beside_infinite_ones(dim, split):
         got = ops.csr_sddmm(*args, rp.cuda(), ci.cuda(), val.cuda(), 1, 8).cpu().double()
     clean = ci != inf_col
     assert bool(((got - want).abs() <= bound)[clean].all()) and not bool(torch.isfinite(got[~clean]).any())
+
+
+def _moving_scores(n):
+    """Scores of one row that rise and fall by more and by less than what moves the reference of the exponentials."""
+    t = np.linspace(-20.0, 20.0, n) if n > 1 else np.array([3.0])
+    spike, steps = np.zeros(n), np.full(n, 7.9)
+    spike[-1] = 30.0
+    steps[: min(4, n)] = 0.0  # (all weights of the later batches are e^7.9 of the first reference)
+    return [t, t[::-1], 20.0 * (-1.0) ** np.arange(n), spike, spike[::-1], steps, np.repeat(np.arange(-(n // 8) - 1.0, 0.0), 8)[:n] * 8.1]
+
+
+def _moving_case(dim, lengths, seed):
+    """Every row has columns of its own; column 0 of B is the score, A takes it alone, so scores are exact."""
+    rows = [s for k in lengths for s in _moving_scores(k)]
+    rp = np.concatenate([[0], np.cumsum([len(s) for s in rows])]).astype(np.int32)
+    g = torch.Generator().manual_seed(seed)
+    A, B = torch.zeros(len(rows), dim), torch.rand(int(rp[-1]), dim, generator=g) - 0.3
+    A[:, 0] = 1.0
+    B[:, 0] = torch.from_numpy(np.concatenate(rows)).float()
+    return rp, torch.arange(int(rp[-1]), dtype=torch.int32), A, B
+
+
+def _softmax_rows(rp, scores, V):
+    """Results in fp64, and their terms' absolute sums."""
+    out, scale = np.zeros((len(rp) - 1, V.shape[1])), np.zeros((len(rp) - 1, V.shape[1]))
+    for i in range(len(rp) - 1):
+        s = scores[rp[i]:rp[i + 1]]
+        w = np.exp(s - s.max())
+        w /= w.sum()
+        out[i], scale[i] = w @ V[rp[i]:rp[i + 1]], w @ np.abs(V[rp[i]:rp[i + 1]])
+    return out, scale
+
+
+@pytest.mark.parametrize("dim", [16, 100, 128, 256])
+@pytest.mark.parametrize("granularity", [None, 32])
+def test_softmax_of_values_near_the_largest(dim, granularity):
+    """Weighted averages of values of 4e33: weights above one would leave sums of 64 terms no room."""
+    from paramspmm_ae_b200 import ops
+    rp, ci, A, B = _moving_case(dim, (64, 300), dim)
+    n = len(rp) - 1
+    V = 4e33 * (torch.rand(B.shape, generator=torch.Generator().manual_seed(1)) + 0.5)
+    want, scale = _softmax_rows(rp, B[:, 0].double().numpy(), V.double().numpy())
+    ptr, extra = torch.from_numpy(rp), {}
+    if granularity:
+        ptr, tr = ops.split_csr(ptr, granularity)
+        extra = dict(target_row=tr.cuda(), n_out_rows=n)
+    got = ops.agnn_fused(A.cuda(), B.cuda(), ptr.cuda(), ci.cuda(), 1.0, True, V=V.cuda(), **extra).cpu().double().numpy()
+    assert (np.abs(got - want) <= (1e-5 + 600 * 2.0 ** -24) * scale).all()
