@@ -185,6 +185,33 @@ def _softmax_rows(rp, scores, V):
     return out, scale
 
 
+@pytest.mark.parametrize("dim", [4, 16, 20, 64, 100, 128, 132, 256])
+@pytest.mark.parametrize("sep", [False, True])
+@pytest.mark.parametrize("lengths", [(1, 2, 4, 5, 9, 33, 64), (65, 300, 1500)], ids=["short", "long"])
+def test_softmax_whose_scores_move_within_a_row(dim, sep, lengths):
+    """Rows of several batches, long rows cut over shares, split rows whose pieces' references lie far apart."""
+    from paramspmm_ae_b200 import ops
+    rp, ci, A, B = _moving_case(dim, lengths, dim)
+    n = len(rp) - 1
+    V = torch.rand(B.shape, generator=torch.Generator().manual_seed(1)) + 0.5 if sep else B
+    want, scale = _softmax_rows(rp, B[:, 0].double().numpy(), V.double().numpy())
+    # an exponent of up to 50 is off by half of its last bit, 2e-6, once for the entry and once for each move of the reference that
+    # still counts; then one rounding per term of two sums
+    bound = (1e-5 + 2 * max(lengths) * 2.0 ** -24) * scale
+    kw = dict(V=V.cuda()) if sep else {}
+    rpt = torch.from_numpy(rp)
+    for granularity in (None, 4, 32):
+        ptr, extra = rpt, {}
+        if granularity:
+            ptr, tr = ops.split_csr(rpt, granularity)
+            extra = dict(target_row=tr.cuda(), n_out_rows=n)
+        got = ops.agnn_fused(A.cuda(), B.cuda(), ptr.cuda(), ci.cuda(), 1.0, True, **kw, **extra).cpu().double().numpy()
+        assert (np.abs(got - want) <= bound).all(), (granularity, np.abs(got - want).max())
+        if granularity is None and lengths[0] == 1:  # (the weight of an only entry is one)
+            one = np.flatnonzero(np.diff(rp) == 1)
+            np.testing.assert_array_equal(got[one], V.double().numpy()[rp[one]])
+
+
 @pytest.mark.parametrize("dim", [16, 100, 128, 256])
 @pytest.mark.parametrize("granularity", [None, 32])
 def test_softmax_of_values_near_the_largest(dim, granularity):
