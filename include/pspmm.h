@@ -147,6 +147,7 @@ PSPMM_API int pspmm_spmm_csr_ws(const int32_t *rowPtr, const int32_t *colIdx, co
  * The CSR product for a dim that is no multiple of 4: every row of B holds the next multiple of 4 columns (their
  * content does not matter), B is 16-byte aligned and ldB a multiple of 4; C is as narrow as dim and need not
  * be aligned.  Scratch is sized for the padded dim.  PSPMM_E_UNSUPPORTED with cfg->accumulate or a vec_width below 4.
+ * pspmm_resolve_spmm_padded is pspmm_resolve_spmm for it.
  * pspmm_pad_rows makes such a B: dst[n, dim rounded up to 4] from src[n, dim], zeros in the new columns.
  */
 PSPMM_API int pspmm_spmm_csr_padded(const int32_t *rowPtr, const int32_t *colIdx, const float *val,
@@ -156,6 +157,8 @@ PSPMM_API int pspmm_spmm_csr_padded(const int32_t *rowPtr, const int32_t *colIdx
                    void *scratch, size_t scratch_bytes, void *stream);
 PSPMM_API int pspmm_pad_rows(const float *src, float *dst, int64_t n, int32_t dim, int64_t ld_src, int64_t ld_dst,
                              void *stream);
+PSPMM_API int pspmm_resolve_spmm_padded(pspmm_cfg *cfg, int32_t dim, int64_t ldB, const void *B, int32_t split, int64_t n_seg,
+                                        int64_t n_entries);
 PSPMM_API int pspmm_spmm_bcsr_ws(const int32_t *rowPtr_b, const int32_t *colIdx, const float *val, int32_t V,
                     const float *B, float *C, int64_t n_blk_rows, int64_t n_cols, int64_t nblk,
                     int32_t dim, int64_t ldB, int64_t ldC, const pspmm_cfg *cfg,

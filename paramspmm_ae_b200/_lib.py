@@ -71,6 +71,7 @@ _cfgp = ctypes.POINTER(PspmmCfg)
 _SIGNATURES = {
     "pspmm_resolve_cfg": [_cfgp, _i32, _i64, _i64, _i32, _vp, _vp],
     "pspmm_resolve_spmm": [_cfgp, _i32, _i64, _i64, _i32, _vp, _vp, _i32, _i64, _i64],
+    "pspmm_resolve_spmm_padded": [_cfgp, _i32, _i64, _vp, _i32, _i64, _i64],
     "pspmm_spmm_csr": [_vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i32, _i64, _i64, _cfgp, _vp, _vp,
                        _i64, _vp],
     "pspmm_spmm_bcsr": [_vp, _vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _i32, _i64, _i64, _cfgp,

@@ -404,10 +404,15 @@ static pspmm_cfg tile_cfg(const pspmm_cfg &cfg, int32_t w)
 }
 
 // The shape of one SpMM launch.  n_seg < 0: the matrix is not known, the rules that look at its size are left out.
+// `ragged`: the product of spmm_ragged.cu, whose dim is rounded up.
 static int spmm_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, bool split, int64_t n_seg, int64_t n_entries,
-                      LaunchShape *out)
+                      LaunchShape *out, bool ragged = false)
 {
     LaunchShape s;
+    if (ragged) {
+        dim = (dim + 3) / 4 * 4;
+        vw_max = 4;
+    }
     pspmm_resolve_shape(cfg, dim, vw_max, V, split ? SHAPE_SPLIT : SHAPE_ROWS, &s, n_seg);
     if (cfg && cfg->accumulate) {
         // built for 128-bit loads on CSR / split CSR with at least four lanes per row
@@ -430,12 +435,34 @@ static int spmm_shape(const pspmm_cfg *cfg, int32_t dim, int vw_max, int V, bool
             s.rpg = small_rows_per_group(s, V, n_seg, n_entries);
         }
     }
+    if (ragged && (s.lpr < 4 || s.cf > 4)) {
+        // Built for at least four lanes and up to four slices: as many lanes as that takes.  (A plan of 8 lanes and five slices
+        // at 142 columns, uniform 300 K rows of 12: 537 us on 32 lanes and four slices, 363 on 16 and three.)
+        const int nvec = dim / 4;
+        while (s.lpr < 4 || (s.lpr < 32 && (nvec + s.lpr - 1) / s.lpr > 4))
+            s.lpr *= 2;
+        const int need = (nvec + s.lpr - 1) / s.lpr;
+        s.cf = need < 4 ? need : 4;
+        s.tiles = (need + 3) / 4;
+    }
+    if (ragged && s.mlp == 2)
+        s.mlp = 4;  // (the least it is built for)
     *out = s;
     return PSPMM_OK;
 }
 
+// What the product on padded rows asks of its operand and its configuration.
+static int check_padded(const pspmm_cfg *cfg, int32_t dim, int64_t ldB, const void *B)
+{
+    if (ldB % 4 != 0 || (uintptr_t)B % 16 != 0 || ldB < (dim + 3) / 4 * 4)
+        return PSPMM_E_ARG;
+    if (cfg && (cfg->accumulate || (cfg->vec_width != 0 && cfg->vec_width != 4)))
+        return PSPMM_E_UNSUPPORTED;
+    return PSPMM_OK;
+}
+
 static int resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, int32_t V, const void *B, const void *C,
-                       bool split, int64_t n_seg, int64_t n_entries)
+                       bool split, int64_t n_seg, int64_t n_entries, bool ragged = false)
 {
     if (!cfg || dim <= 0 || V < 1 || V > 3)
         return PSPMM_E_ARG;
@@ -446,7 +473,7 @@ static int resolve_cfg(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int64_t ldC, in
     const bool tiled = cfg->col_tile > 0 && cfg->col_tile < dim;
     const pspmm_cfg sub = tiled ? tile_cfg(*cfg, cfg->col_tile) : *cfg;
     rc = spmm_shape(&sub, tiled ? cfg->col_tile : dim, pspmm_vw_max(tiled ? cfg->col_tile : dim, ldB, ldC, B, C), V, split,
-                    n_seg, n_entries, &s);
+                    n_seg, n_entries, &s, ragged);
     if (rc)
         return rc;
     cfg->lanes_per_row = s.lpr;
@@ -469,6 +496,15 @@ extern "C" int pspmm_resolve_spmm(pspmm_cfg *cfg, int32_t dim, int64_t ldB, int6
     if (n_seg < 0 || n_entries < 0)
         return PSPMM_E_ARG;
     return resolve_cfg(cfg, dim, ldB, ldC, V, B, C, split != 0, n_seg, n_entries);
+}
+
+extern "C" int pspmm_resolve_spmm_padded(pspmm_cfg *cfg, int32_t dim, int64_t ldB, const void *B, int32_t split, int64_t n_seg,
+                                         int64_t n_entries)
+{
+    if (n_seg < 0 || n_entries < 0 || !cfg || dim <= 0)
+        return PSPMM_E_ARG;
+    const int rc = check_padded(cfg, dim, ldB, B);
+    return rc ? rc : resolve_cfg(cfg, dim, ldB, dim, 1, B, B, split != 0, n_seg, n_entries, true);
 }
 
 // Entries of the ranges in which a kernel deals out the long rows (PSPMM_LONG_ROW) of an unsplit
@@ -516,19 +552,9 @@ static int spmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_t
     }
     LaunchShape s;
     const int32_t wide = ragged ? (dim + 3) / 4 * 4 : dim;  // columns that are gathered
-    rc = spmm_shape(cfg, wide, ragged ? 4 : pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row != nullptr, n_seg, n_entries, &s);
+    rc = spmm_shape(cfg, dim, pspmm_vw_max(dim, ldB, ldC, B, C), V, target_row != nullptr, n_seg, n_entries, &s, ragged);
     if (rc)
         return rc;
-    if (ragged && (s.lpr < 4 || s.cf > 4)) {
-        // Built for at least four lanes and up to four slices: as many lanes as that takes.  (A plan of 8 lanes and five slices
-        // at 142 columns, uniform 300 K rows of 12: 537 us on 32 lanes and four slices, 363 on 16 and three.)
-        const int nvec = wide / 4;
-        while (s.lpr < 4 || (s.lpr < 32 && (nvec + s.lpr - 1) / s.lpr > 4))
-            s.lpr *= 2;
-        const int need = (nvec + s.lpr - 1) / s.lpr;
-        s.cf = need < 4 ? need : 4;
-        s.tiles = (need + 3) / 4;
-    }
     const bool bucketed = target_row && cfg && cfg->bucketed;
     if (target_row && !accumulate) {
         const int vecok = (dim % 4 == 0 && ldC % 4 == 0 && ((uintptr_t)C) % 16 == 0) ? 1 : 0;
@@ -662,10 +688,9 @@ extern "C" int pspmm_spmm_csr_padded(const int32_t *rowPtr, const int32_t *colId
                                      const int32_t *target_row, int64_t n_seg, void *scratch,
                                      size_t scratch_bytes, void *stream)
 {
-    if (ldB % 4 != 0 || (uintptr_t)B % 16 != 0 || ldB < (dim + 3) / 4 * 4)
-        return PSPMM_E_ARG;
-    if (cfg && (cfg->accumulate || (cfg->vec_width != 0 && cfg->vec_width != 4)))
-        return PSPMM_E_UNSUPPORTED;
+    const int rc = check_padded(cfg, dim, ldB, B);
+    if (rc)
+        return rc;
     return spmm_csr(rowPtr, colIdx, val, B, C, n_rows, n_cols, nnz, dim, ldB, ldC, cfg, rowPtr_split, target_row, n_seg,
                     scratch, scratch_bytes, stream, true);
 }

@@ -224,6 +224,37 @@ def test_a_resolved_configuration_resolves_to_itself(pspmm_lib):
         assert _resolved(pspmm_lib, dim, V, split, n_seg, n_entries, **again)[1] == first, (dim, V, split, n_seg, n_entries, kw)
 
 
+def test_odd_widths_resolve_to_the_padded_product(pspmm_lib):
+    """The product on padded rows has a resolution of its own: 16-byte loads, at least four lanes, at most four slices on them
+    below a whole warp, and a resolved configuration resolves to itself."""
+    import random
+    from paramspmm_ae_b200 import _lib
+    B = ctypes.c_void_p(256)
+
+    def shape(dim, split, n_seg, n_entries, **kw):
+        cfg = _lib.make_cfg(**kw)
+        rc = pspmm_lib.pspmm_resolve_spmm_padded(ctypes.byref(cfg), dim, dim + -dim % 4, B, int(split), n_seg, n_entries)
+        return rc, cfg, tuple(getattr(cfg, f) for f, _ in cfg._fields_)
+
+    rng = random.Random(4)
+    for _ in range(3000):
+        dim, n_seg = rng.randint(1, 1100), int(10 ** rng.uniform(0, 7))
+        kw = {f: rng.choice(v) for f, v in (("lanes_per_row", (2, 4, 8, 16, 32)), ("vec_width", (0, 4)), ("gather_batch", (2, 4, 16)),
+                                            ("rows_per_group", (1, 8)), ("col_tile", (32, 64))) if rng.random() < 0.3}
+        sizes = rng.random() < 0.5, n_seg, int(n_seg * 10 ** rng.uniform(-1, 3))
+        rc, cfg, first = shape(dim, *sizes, **kw)
+        wide = min(dim + 3, kw.get("col_tile", dim + 3)) // 4
+        assert rc == 0 and cfg.vec_width == 4 and cfg.lanes_per_row >= 4 and cfg.gather_batch in (4, 8, 16)
+        assert cfg.lanes_per_row == 32 or wide <= 4 * cfg.lanes_per_row, (dim, kw)
+        again = {f: getattr(cfg, f) for f in ("lanes_per_row", "vec_width", "cta_threads", "rows_per_group", "gather_batch", "col_tile")}
+        assert shape(dim, *sizes, **again)[2] == first, (dim, kw)
+    assert shape(142, False, 300000, 3600000, lanes_per_row=8)[1].lanes_per_row == 16  # (five slices of 8 lanes)
+    assert shape(47, False, 100, 400, accumulate=1)[0] == shape(47, False, 100, 400, vec_width=2)[0] == _lib.PSPMM_E_UNSUPPORTED
+    cfg = _lib.make_cfg()
+    for ld, ptr in ((47, 256), (44, 256), (48, 260)):
+        assert pspmm_lib.pspmm_resolve_spmm_padded(ctypes.byref(cfg), 47, ld, ctypes.c_void_p(ptr), 0, 10, 10) == _lib.PSPMM_E_ARG
+
+
 def test_ops_reject_cpu_tensors_and_bad_hints():
     """The torch-level operators never fall back: a CPU tensor or an invalid CF / blkWarpNum is
     an error, as in the reference (SpMM/SpMM.cpp:5-13, 110, 139)."""
