@@ -93,8 +93,25 @@ FUSE_AGNN_INFERENCE = True
 # the edge scores for the backward (4 bytes per edge; the reference's composition writes the attention values in
 # the forward and the score gradient in the backward, gnn_conv.py:130-180).  Outputs and gradients are the
 # reference's up to fp32 summation order.
-# Set to False to train through the three-kernel composition (AGNNFunction).
+# Set to False to train through the three-kernel composition (AGNNFunction).  ``AGNNConv.keep_scores`` chooses per layer
+# whether the scores are kept.
 FUSE_AGNN_TRAINING = True
+_SCORES_UNASKED = 16 << 20  # bytes up to which scores are kept without a look at the free memory (12 us of host time)
+
+
+def _room(device):
+    """Bytes of a device that torch has not handed out, within the limit of the process.  (The driver's own figure for free memory
+    takes 0.2 ms, at times several.)"""
+    limit = torch.cuda.get_per_process_memory_fraction(device) * torch.cuda.get_device_properties(device).total_memory
+    return limit - torch.cuda.memory_stats_as_nested_dict(device)["allocated_bytes"]["all"]["current"]
+
+
+def _keeps_scores(nnz, Xp):
+    """Whether the scores of ``nnz`` edges may take memory until the backward.  They stand in for the projected features, up to
+    whose size a step takes no more than without; beyond it up to a 32nd of what is free, so that the layers behind this one find
+    the room they found without (a second gather per edge instead: 115 M edges, 64 columns, a step of 4.1 ms becomes 6.1)."""
+    nbytes = 4 * nnz
+    return nbytes <= max(Xp.numel() * Xp.element_size(), _SCORES_UNASKED) or 32 * nbytes <= _room(Xp.device)
 
 
 def _beta(attention_w):
@@ -157,8 +174,8 @@ class AGNNFusedFunction(torch.autograd.Function):
     """AGNN layer on a CSR / split-CSR operator in one pass over the pattern per direction.
 
     forward   X' = X W,  out_i = sum_j beta <X'_i, X'_j> X'_j     (one fused pass, which leaves the scores)
-    backward  D_i = sum_j beta <X'_i, X'_j> G_j           (gradient rows gathered, scores read; where there
-              is no room for them the rows of X' are gathered again and the scores recomputed)
+    backward  D_i = sum_j beta <X'_i, X'_j> G_j           (gradient rows gathered, scores read; with ``keep_scores=False``, or
+              little room for them, the rows of X' are kept and gathered again and the scores recomputed)
               dX = D W^T,  dW = X^T D                                      (gnn_conv.py:157-160)
               d_beta = sum over edges of <G_i, G_j> * colIdx[e]              (gnn_conv.py:163-172: the
               reference multiplies the score gradient by the column-index column it is handed), summed
@@ -167,13 +184,16 @@ class AGNNFusedFunction(torch.autograd.Function):
     Like the reference's backward, the edge values are treated as constants with respect to X'."""
 
     @staticmethod
-    def forward(ctx, X, weights, attention_w, P, colIdx):
+    def forward(ctx, X, weights, attention_w, P, colIdx, keep_scores=True):
         Xp = ops.dense_mm(X, weights)
-        beta = _beta(attention_w)
-        try:
-            scores = torch.empty(P.colIdx.shape[0], dtype=torch.float32, device=Xp.device)
-        except torch.cuda.OutOfMemoryError:
-            scores, beta = None, beta.clone()  # (the backward uses the value of this forward)
+        beta, scores = _beta(attention_w), None
+        if keep_scores and _keeps_scores(P.colIdx.shape[0], Xp):
+            try:
+                scores = torch.empty(P.colIdx.shape[0], dtype=torch.float32, device=Xp.device)
+            except torch.cuda.OutOfMemoryError:
+                pass
+        if scores is None:
+            beta = beta.clone()  # (the backward uses the value of this forward)
         out = ops.agnn_layer_forward(Xp, P.rowPtr, P.colIdx, beta, P.target_row, scores)
         ctx.save_for_backward(X, weights, *((Xp, beta) if scores is None else (scores,)))
         ctx.P = P
@@ -188,7 +208,7 @@ class AGNNFusedFunction(torch.autograd.Function):
                                            beta_grad=ctx.needs_input_grad[2], scores=scores)
         d_input = ops.dense_mm(D, weights, transB=True) if ctx.needs_input_grad[0] else None
         d_weights = ops.dense_mm(X, D, transA=True) if ctx.needs_input_grad[1] else None
-        return d_input, d_weights, d_att, None, None
+        return d_input, d_weights, d_att, None, None, None
 
 
 class _Conv(torch.nn.Module):
@@ -222,6 +242,10 @@ class GINConv(_Conv):
 
 
 class AGNNConv(_Conv):
+    # False: a fused training step keeps the projected features and recomputes the edge scores in the backward, for a
+    # network that has no room for 4 bytes per edge and layer
+    keep_scores = True
+
     def __init__(self, input_dim, output_dim):
         super().__init__(input_dim, output_dim)
         self.attention_w = torch.nn.Parameter(torch.randn(1, n_heads))
@@ -236,5 +260,5 @@ class AGNNConv(_Conv):
             return out[: P.mtx_nodes if P.target_row is not None else P.rowPtr.shape[0] - 1]
         if (FUSE_AGNN_TRAINING and torch.is_grad_enabled() and _can_fuse(P, self.weights.size(1))
                 and _is_operator_colidx(P, colIdx)):
-            return AGNNFusedFunction.apply(X, self.weights, self.attention_w, P, colIdx)
+            return AGNNFusedFunction.apply(X, self.weights, self.attention_w, P, colIdx, self.keep_scores)
         return AGNNFunction.apply(X, self.weights, self.attention_w, P, colIdx)

@@ -130,6 +130,81 @@ def test_agnn_layer_trains_without_room_for_the_scores(monkeypatch):
         assert float((a - b).norm()) <= 1e-5 * float(b.norm())
 
 
+def _agnn_network(n, pairs, dim, layers, classes):
+    from paramspmm_ae_b200 import gnn_conv, pcsr, synth
+    dev = torch.device("cuda:0")
+    g = synth.powerlaw_graph(n, pairs, seed=4, device=dev)
+    P = pcsr.pcsr_sddmm(None, 1, False, n, g.nnz, g.rowPtr, g.colIdx, g.val, None, CF=1, blkWarpNum=8)
+    torch.manual_seed(5)
+    net = torch.nn.ModuleList([gnn_conv.AGNNConv(dim, dim) for _ in range(layers)]).to(dev)
+    last = torch.nn.Linear(dim, classes, bias=False).to(dev)
+    X = torch.nn.functional.normalize(torch.randn(n, dim, device=dev))
+
+    def step():
+        net.zero_grad(set_to_none=True)
+        h = X
+        for layer in net:
+            h = torch.nn.functional.normalize(torch.relu(layer(h, {dim: P}, P.colIdx.unsqueeze(-1))))
+        torch.relu(last(h)).sum().backward()
+        return [p.grad.clone() for p in net.parameters()]
+
+    return net, P, step
+
+
+def _close(got, want):
+    # (scores kept and recomputed are sums of the same products in another order)
+    return all(0 < float(b.norm()) < float("inf") and float((a - b).norm()) <= 1e-4 * float(b.norm()) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("pairs, dim", [(3000, 16), (40000, 16), (3000, 256)])
+def test_agnn_layers_keep_no_scores_when_told(pairs, dim):
+    net, P, step = _agnn_network(301, pairs, dim, 2, 8)
+    saved = []
+
+    def pack(t):
+        saved.append(tuple(t.shape))
+        return t
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        kept = step()
+        assert saved.count((P.colIdx.shape[0],)) == 2
+        saved.clear()
+        for layer in net:
+            layer.keep_scores = False
+        assert _close(step(), kept) and saved.count((P.colIdx.shape[0],)) == 0
+
+
+def test_agnn_network_trains_in_the_memory_it_took_without_scores(monkeypatch):
+    """Scores of 40 MB per layer in a network whose last layer needs a few hundred: a limit that it keeps to with recomputed scores
+    is kept to by default."""
+    from paramspmm_ae_b200 import gnn_conv
+    net, P, step = _agnn_network(20000, 5000000, 16, 2, 4096)
+    dev = torch.device("cuda:0")
+    total = torch.cuda.get_device_properties(dev).total_memory
+    empty, nnz = torch.empty, P.colIdx.shape[0]
+
+    def refuse(*size, **kw):
+        if size == (nnz,):
+            raise torch.cuda.OutOfMemoryError("no room")
+        return empty(*size, **kw)
+
+    try:
+        with monkeypatch.context() as m:
+            m.setattr(gnn_conv.torch, "empty", refuse)
+            step()
+            torch.cuda.reset_peak_memory_stats(dev)
+            step()
+            limit = torch.cuda.max_memory_allocated(dev) + (40 << 20)  # (the allocator takes memory in pieces of 20 MB)
+            torch.cuda.empty_cache()
+            torch.cuda.set_per_process_memory_fraction(limit / total, dev)
+            want = step()
+        torch.cuda.empty_cache()
+        assert _close(step(), want)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, dev)
+        torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("dim", [5, 20, 47, 68, 70, 100, 132, 200, 256, 260])
 @pytest.mark.parametrize("split", [False, True])
 def test_scores_of_finite_rows_stay_finite_beside_infinite_ones(dim, split):
