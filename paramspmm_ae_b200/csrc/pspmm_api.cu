@@ -758,7 +758,10 @@ static int sddmm_launch(const int32_t *segPtr, const int32_t *target_row, int64_
     // with up to 4 slices each take fewer steps of it: scalar and 8-byte loads fill 8 lanes first (dim 17: 64 against 87 us,
     // 4 M entries), 9 to 12 vectors of 16 bytes go on 4 lanes and up to 32 on 8 (4 M entries, 48 columns: 93 us on 16
     // lanes, 75; 64 93 and 84; 100 160 and 147; band of 24 at 80 columns 293 and 194; 64 threads per CTA gain another 4 % on
-    // scattered columns and lose 10 % on bands).  Few entries unsplit are left on 16 up to 64 columns: their long rows
+    // scattered columns and lose 10 % on bands).  13 to 16 vectors lose by it on scattered columns in even rows of 12 to 16 or 32, one or two
+    // batches of 16 lanes (300 K rows of 16, 52 columns 96 -> 100 us, 64 104 -> 108; of 12 94 -> 98; of 32 188 -> 193), and gain otherwise: rows of
+    // 20 154 -> 132 and 159 -> 139, band of 16 89 -> 84, power law of 12 120 -> 104, of 16 134 -> 120.  The mean length, all that a call
+    // knows of its rows, does not tell them apart, so there is no bound by it.  Few entries unsplit are left on 16 up to 64 columns: their long rows
     // end last, and a narrow group walks its piece longer (power law of 0.9 M, 48 columns: 41 us, on 4 lanes 45).  Rows of
     // more than 3 slices of 16 lanes go through column tiles of 2 inside the kernel (a fourth slice
     // leaves too few registers: dim 256 14.0 ms, two tiles of 128 9.0); scalar loads keep up to 8.
