@@ -102,8 +102,11 @@ _SCORES_UNASKED = 16 << 20  # bytes up to which scores are kept without a look a
 def _room(device):
     """Bytes of a device that torch has not handed out, within the limit of the process.  (The driver's own figure for free memory
     takes 0.2 ms, at times several.)"""
-    limit = torch.cuda.get_per_process_memory_fraction(device) * torch.cuda.get_device_properties(device).total_memory
-    return limit - torch.cuda.memory_stats_as_nested_dict(device)["allocated_bytes"]["all"]["current"]
+    try:
+        limit = torch.cuda.get_per_process_memory_fraction(device) * torch.cuda.get_device_properties(device).total_memory
+        return limit - torch.cuda.memory_stats_as_nested_dict(device)["allocated_bytes"]["all"]["current"]
+    except (RuntimeError, KeyError):  # an allocator of the host's, which keeps no figures: its allocation tells
+        return float("inf")
 
 
 def _keeps_scores(nnz, Xp):

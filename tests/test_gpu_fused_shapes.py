@@ -130,11 +130,12 @@ def test_agnn_layer_trains_without_room_for_the_scores(monkeypatch):
         assert float((a - b).norm()) <= 1e-5 * float(b.norm())
 
 
-def _agnn_network(n, pairs, dim, layers, classes):
-    from paramspmm_ae_b200 import gnn_conv, pcsr, synth
+def _agnn_network(n, mean, dim, layers, classes):
+    from paramspmm_ae_b200 import gnn_conv, pcsr
     dev = torch.device("cuda:0")
-    g = synth.powerlaw_graph(n, pairs, seed=4, device=dev)
-    P = pcsr.pcsr_sddmm(None, 1, False, n, g.nnz, g.rowPtr, g.colIdx, g.val, None, CF=1, blkWarpNum=8)
+    ci = torch.randint(0, n, (n * mean,), generator=torch.Generator().manual_seed(4), dtype=torch.int32)
+    P = pcsr.pcsr_sddmm(None, 1, False, n, n * mean, torch.arange(n + 1, dtype=torch.int32) * mean, ci, torch.ones(n * mean), None, CF=1,
+                        blkWarpNum=8)
     torch.manual_seed(5)
     net = torch.nn.ModuleList([gnn_conv.AGNNConv(dim, dim) for _ in range(layers)]).to(dev)
     last = torch.nn.Linear(dim, classes, bias=False).to(dev)
@@ -156,9 +157,9 @@ def _close(got, want):
     return all(0 < float(b.norm()) < float("inf") and float((a - b).norm()) <= 1e-4 * float(b.norm()) for a, b in zip(got, want))
 
 
-@pytest.mark.parametrize("pairs, dim", [(3000, 16), (40000, 16), (3000, 256)])
-def test_agnn_layers_keep_no_scores_when_told(pairs, dim):
-    net, P, step = _agnn_network(301, pairs, dim, 2, 8)
+@pytest.mark.parametrize("mean, dim", [(20, 16), (200, 16), (20, 256)])
+def test_agnn_layers_keep_no_scores_when_told(mean, dim):
+    net, P, step = _agnn_network(301, mean, dim, 2, 8)
     saved = []
 
     def pack(t):
@@ -175,10 +176,11 @@ def test_agnn_layers_keep_no_scores_when_told(pairs, dim):
 
 
 def test_agnn_network_trains_in_the_memory_it_took_without_scores(monkeypatch):
-    """Scores of 40 MB per layer in a network whose last layer needs a few hundred: a limit that it keeps to with recomputed scores
+    """Scores of 80 MB per layer in a network whose last layer needs several hundred: a limit that it keeps to with recomputed scores
     is kept to by default."""
     from paramspmm_ae_b200 import gnn_conv
-    net, P, step = _agnn_network(20000, 5000000, 16, 2, 4096)
+    torch.cuda.empty_cache()
+    net, P, step = _agnn_network(20000, 1000, 8, 2, 4096)
     dev = torch.device("cuda:0")
     total = torch.cuda.get_device_properties(dev).total_memory
     empty, nnz = torch.empty, P.colIdx.shape[0]
@@ -194,7 +196,7 @@ def test_agnn_network_trains_in_the_memory_it_took_without_scores(monkeypatch):
             step()
             torch.cuda.reset_peak_memory_stats(dev)
             step()
-            limit = torch.cuda.max_memory_allocated(dev) + (40 << 20)  # (the allocator takes memory in pieces of 20 MB)
+            limit = torch.cuda.max_memory_allocated(dev) + (90 << 20)  # (what the allocator may hold in parts; rows of 8 stay out of its large blocks)
             torch.cuda.empty_cache()
             torch.cuda.set_per_process_memory_fraction(limit / total, dev)
             want = step()

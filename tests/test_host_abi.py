@@ -543,3 +543,24 @@ def test_edge_columns_are_compared_again_when_they_change():
     assert not gnn_conv._is_operator_colidx(P, edges)
     with torch.inference_mode():
         assert gnn_conv._is_operator_colidx(P, P.colIdx.clone())
+
+
+def test_scores_are_kept_by_what_memory_they_take(monkeypatch):
+    """Up to what they replace, up to a fixed size, up to a 32nd of the room; an allocator without figures is not asked."""
+    from paramspmm_ae_b200 import gnn_conv
+    asked = []
+    monkeypatch.setattr(gnn_conv, "_room", lambda device: asked.append(device) or 32 * 4 * 5_000_000)
+    few, many = torch.zeros(10, 4), torch.zeros(1).expand(1_500_000, 4)
+    assert gnn_conv._keeps_scores(4_000_000, few) and gnn_conv._keeps_scores(6_000_000, many) and not asked
+    assert gnn_conv._keeps_scores(5_000_000, few) and not gnn_conv._keeps_scores(5_000_001, few) and len(asked) == 2
+    monkeypatch.undo()
+
+    def no_figures(*a):
+        raise RuntimeError("not supported")
+
+    monkeypatch.setattr(torch.cuda, "get_per_process_memory_fraction", lambda d: 0.5)
+    monkeypatch.setattr(torch.cuda, "get_device_properties", lambda d: type("P", (), {"total_memory": 1000}))
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", lambda d: {"allocated_bytes": {"all": {"current": 400}}})
+    assert gnn_conv._room(None) == 100
+    monkeypatch.setattr(torch.cuda, "memory_stats_as_nested_dict", no_figures)
+    assert gnn_conv._room(None) == float("inf") and gnn_conv._keeps_scores(2**30, few)
