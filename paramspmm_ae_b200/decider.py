@@ -278,8 +278,9 @@ class PlannedSpMM:
 
     @property
     def launches(self):
-        """Kernels per product: the SpMM, plus the zeroing pre-pass of a split layout."""
-        return 2 if self.target is not None else 1
+        """Kernels per product: the SpMM, plus the zeroing pre-pass of a split layout or the launch that takes the long rows of
+        an unsplit one."""
+        return 2 if self.target is not None or not self.plan.kernel_cfg()["no_long_rows"] else 1
 
 
 def legacy_tuple(plan, dim):
