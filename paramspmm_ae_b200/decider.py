@@ -171,7 +171,9 @@ def _fit_to_size(plan, stats, dim, n_cols):
     columns 298 / 154, 128 127 / 90, 16 58 / 31; R-MAT of 300 K rows of 8, 128 columns 153 / 117, 16 55 / 37; power law of 30 K rows of
     25, 256 columns 146 / 51; of 8 K rows of 8, 32 columns 47 / 8.4.  (100 K rows of 100, 64 columns, ratio 0.29: 152 / 166 if it did.)
     Even and local: column tiles pay while the dense operand exceeds the L2 (uniform 300 K rows of 16, 128 columns 211 us, untiled
-    242), not below (100 K, 192 columns 111 and 90; 8 K, 256 columns 41 and 14); up to 1.7 M output values the launch's own
+    242), not below (100 K, 192 columns 111 and 90; 8 K, 256 columns 41 and 14); local ones, whose
+    gathers the L1 answers, gain by them from half of that on (band of 30, 160 columns: 20 K rows 35 and 27, 60 K 74 and 74, 120 K 148
+    and 157; of 77, 120 K, 144 columns 292 and 341); up to 1.7 M output values the launch's own
     rules, which see the size, are up to twice as fast (8 K rows of 16 at 32 columns 12.4 and 6.0; 30 K of 8 in a band at 16 8.3 and 6.2;
     but 30 K rows of 24 in a band at 64 14.4 and 18.5).  A split without column tiles stays where a row ends late (30 K rows of
     60, longest 900, 16 columns 39, walked 90, cut 51)."""
@@ -183,7 +185,8 @@ def _fit_to_size(plan, stats, dim, n_cols):
         late = _walk_ends_late(stats, dim)
         if plan["if_split"] and not plan["col_tile"] and late:
             return
-        if n * dim <= 1.7e6 or (plan["col_tile"] and n_cols * dim * 4 <= 110e6):
+        fits = 36e6 if plan["regime"].endswith("local") else 110e6
+        if n * dim <= 1.7e6 or (plan["col_tile"] and n_cols * dim * 4 <= fits):
             plan.update(_NO_SHAPE, if_split=0, granularity=None, no_long_rows=int(not late))
         return
     if not plan["if_split"] or not plan["rows_per_group"]:

@@ -114,7 +114,7 @@ def _keeps_scores(nnz, Xp):
     whose size a step takes no more than without; beyond it up to a 32nd of what is free, so that the layers behind this one find
     the room they found without (a second gather per edge instead: 115 M edges, 64 columns, a step of 4.1 ms becomes 6.1)."""
     nbytes = 4 * nnz
-    return nbytes <= max(Xp.numel() * Xp.element_size(), _SCORES_UNASKED) or 32 * nbytes <= _room(Xp.device)
+    return nbytes <= _SCORES_UNASKED or nbytes <= Xp.numel() * Xp.element_size() or 32 * nbytes <= _room(Xp.device)
 
 
 def _beta(attention_w):

@@ -370,6 +370,14 @@ def test_plans_fit_the_size_of_the_matrix():
     assert plan(100_000, 16, 256, cov=0.0, n_cols=1_000_000)["col_tile"]      # (a shard: the dense operand is the whole one)
 
 
+def test_column_tiles_of_local_matrices_stay_from_a_third_of_the_l2_on():
+    from paramspmm_ae_b200 import decider
+    for n, tiled in ((20_000, False), (50_000, False), (60_000, True), (120_000, True), (1_000_000, True)):
+        for k in (30, 77):
+            stats = {"n_rows": n, "nnz": n * k, "avg": float(k), "cov": 0.0, "max": k, "real_avg": float(k), "near_diag": 1.0}
+            assert bool(decider.choose(stats, 160)["col_tile"]) == tiled, (n, k)
+
+
 def test_plans_of_even_matrices_cut_rows_that_end_late():
     """A matrix counts as even up to rows of 16 times the mean.  Where one lane group would walk such a row long after the product's
     other rows, the plan keeps its split or lets the launch cut the row, in small matrices and in large ones."""
