@@ -2,7 +2,8 @@
 // single floats.  (A row of 47 floats admits no wider load than 4 bytes, and the L1 takes a request per row and
 // slice: power law of 3.2 M entries, unsplit, 101 columns 210 us, with the copy 144; 255 columns 504 and 271.)
 // pad_rows_kernel makes the padded copy; the layers' projections come padded.  Against products of the next multiple of 4 it
-// costs 10 - 25 % (stores of single floats, two barriers per row), and saves them the pass that cuts the result back.
+// costs up to 9 % on even rows and 3 - 20 % on a power law (stores of single floats, two barriers per row: 100 K rows of 32, 101 columns 103 and
+// 98 us, split power law of it, 47 columns 79 and 66), and saves them the pass that cuts the result back.
 #include "spmm_kernel.cuh"
 
 #define CFS(LPR_) \
