@@ -117,17 +117,26 @@ def test_agnn_layer_trains_without_room_for_the_scores(monkeypatch):
         out.backward(G)
         return out.detach(), x.grad, layer.weights.grad.clone(), layer.attention_w.grad.clone()
 
+    taken, backward = [], gnn_conv.ops.agnn_layer_backward
+
+    def watched(*args, scores=None, **kw):
+        taken.append(scores is not None)
+        return backward(*args, scores=scores, **kw)
+
+    monkeypatch.setattr(gnn_conv.ops, "agnn_layer_backward", watched)
     kept = step()
-    empty = torch.empty
+    empty, refused = torch.empty, []
 
     def refuse(*size, **kw):
         if size == (g.nnz,):
+            refused.append(size)
             raise torch.cuda.OutOfMemoryError("no room")
         return empty(*size, **kw)
 
     monkeypatch.setattr(gnn_conv.torch, "empty", refuse)
     for a, b in zip(kept, step()):
         assert float((a - b).norm()) <= 1e-5 * float(b.norm())
+    assert len(refused) == 1 and taken == [True, False]
 
 
 def _agnn_network(n, mean, dim, layers, classes):
