@@ -478,7 +478,8 @@ def vec_split_spmm(X, rowPtr_bcsr_split, colIdx, val, target_row, CF, blkWarpNum
 
 def spmm_time_ms(X, rowPtr, colIdx, val, target_row=None, V=1, CF=0, W=0, cfg=None,
                  warmup=PROFILE_WARMUP, iters=PROFILE_ITERS, out=None, n_out_rows=None):
-    """Mean milliseconds per launch over `iters` back-to-back launches (CUDA events).
+    """Mean milliseconds per launch over `iters` back-to-back launches (CUDA events).  Odd widths that run on a padded
+    copy (``_padding_pays``) are timed as whole calls of :func:`spmm_into`, the copy and its allocation among them.
 
     ``n_out_rows`` counts (block-)rows of the output; it defaults to the square case
     ceil(input rows / V) that the reference's profile functions assume.
@@ -573,8 +574,11 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
     dim = A.shape[1]
     n_seg = rowPtr.shape[0] - 1
     nent = colIdx.shape[0]
+    pad = dim & 1 and V == 1 and _sddmm_padding_pays(B.shape[0], nent, dim)
+    if pad and time_only:  # (as whole calls: the copies are part of them)
+        return _loop_ms(lambda: _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W), PROFILE_WARMUP, PROFILE_ITERS)
     out = torch.empty_like(val)
-    if dim & 1 and V == 1 and not time_only and _sddmm_padding_pays(B.shape[0], nent, dim):
+    if pad:
         same = A.data_ptr() == B.data_ptr() and A.shape == B.shape
         try:
             Ap = _pad_rows(A)
@@ -591,8 +595,6 @@ def _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W, time_only=False):
         raise RuntimeError("A has %d rows, the pattern needs more than %d" % (A.shape[0], (n_rows - 1) * V))
     args_tail = (cfg, _ptr(rowPtr) if split else null,
                  _ptr(target_row) if split else null, n_seg if split else 0)
-    if time_only and dim & 1 and V == 1 and _sddmm_padding_pays(B.shape[0], nent, dim):
-        return _loop_ms(lambda: _sddmm(A, B, rowPtr, colIdx, val, target_row, V, CF, W), PROFILE_WARMUP, PROFILE_ITERS)
     if time_only:
         ms = ctypes.c_float(0.0)
         check(lib().pspmm_profile_sddmm(null if split else _ptr(rowPtr), _ptr(colIdx), _ptr(val), V,

@@ -126,6 +126,18 @@ def test_tuners_with_narrower_loads_take_odd_widths_into_an_output(vec_width, sp
     assert ops.spmm_time_ms(X, rp, m.colIdx, m.val, tr, iters=2, n_out_rows=3000) > 0
 
 
+def test_timing_of_scores_at_odd_widths_holds_nothing_beside_its_calls(monkeypatch):
+    from paramspmm_ae_b200 import ops, synth
+    m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
+    X = torch.randn(3000, 63, device="cuda")
+    monkeypatch.setattr(ops, "_sddmm_padding_pays", lambda *a: True)
+    assert ops.csr_sddmm_profile(X, X, m.rowPtr, m.colIdx, m.val, 1, 8) > 0
+    held, before = [], torch.cuda.memory_allocated()
+    monkeypatch.setattr(ops, "_loop_ms", lambda *a: held.append(torch.cuda.memory_allocated()) or 1.0)
+    ops.csr_sddmm_profile(X, X, m.rowPtr, m.colIdx, m.val, 1, 8)
+    assert held == [before]
+
+
 def test_products_run_without_room_for_the_copy(monkeypatch):
     from paramspmm_ae_b200 import ops, synth
     m = synth.powerlaw_graph(3000, 120000, seed=3).to("cuda")
