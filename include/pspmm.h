@@ -272,7 +272,7 @@ PSPMM_API int pspmm_split_csr_device_static(const int32_t *rowPtr, int64_t n_row
  *     out_i = sum_j a_ij * V_j,   a_ij from A and B as above.
  * With A = B = the projected features and V = the upstream gradient G it yields the layer's backward
  * product sum_j a_ij G_j (what gnn_conv.py:157 computes from the saved edge array, AGNN_spmm) from
- * recomputed scores, so training keeps no per-edge array either.  ldV = 0 makes every column use the
+ * recomputed scores, so training need not keep a per-edge array either.  ldV = 0 makes every column use the
  * one row V[0, :] (a row of ones turns the pass into per-row sums of the scores).  V and ldV follow
  * the alignment rules of B; this form runs with 128-bit loads and batches of 4.
  */

@@ -5,21 +5,23 @@
 //     out_i = sum_j a_ij * V_j        (V = B in the forward pass)                 (the SpMM)
 //
 // in ONE pass over the pattern: every gathered row B_j is used for its score and for the
-// aggregation while it sits in registers, the per-edge values never reach memory, and the
-// softmax is the running-maximum ("online") form, so a row needs no second sweep.  This is the
+// aggregation while it sits in registers, the per-edge values reach memory only where a training forward
+// leaves its scores, and the softmax's weights are taken against a reference that follows the largest score so far
+// ("online" form), so a row needs no second sweep.  This is the
 // AGNN propagation (A = B = the projected node features) without the two edge-array round trips
 // and with half the gathers of SDDMM followed by SpMM.  With a separate aggregation operand V
 // (template flag SEP: a second gather per entry) the same pass gives the layer's backward products
-// from recomputed scores: sum_j a_ij G_j for an upstream gradient G, again without an edge array.
+// from recomputed scores: sum_j a_ij G_j for an upstream gradient G, again without an edge array.  Where the
+// forward left its scores (SCORES_LEAVE), the backward takes them and gathers G alone (SCORES_TAKE).
 //
 // Work unit = segment (CSR row or PCSR row piece); a group of LPR lanes owns one segment, lane gl
 // holds the slice [(cf*LPR + gl)*4, +4) of A_i and of the accumulator.  Entries are taken BS at a
 // time: BS gathers (128-bit loads), BS lane-partial dot products, a recursive-halving exchange
 // after which lane e holds the complete score of entry e (about one shuffle per entry), one
-// max / exp / sum step for the batch, then BS broadcasts of the weights and the FMAs.
+// exp per lane (and a vote on whether the reference moves) for the batch, then BS broadcasts of the weights and the FMAs.
 //
 // A row that is a single segment is normalised and stored directly.  Pieces of a split row leave
-// (running max, running sum, unnormalised accumulator) in caller-provided scratch and are merged
+// (reference, sum of weights, unnormalised accumulator) in caller-provided scratch and are merged
 // by agnn_combine_kernel; long rows of an unsplit layout are cut by the kernel itself when scratch is
 // given (agnn_long_kernel).  Rows that no segment covers are zeroed by a memset of the output
 // (split layouts only; in plain CSR every row is a segment and stores its own zeros).
@@ -39,7 +41,7 @@ struct AgnnArgs {
     const float *B;
     const float *Vm;  // aggregated rows (SEP kernels); row stride ldV, 0 = one row shared by all columns
     float *out;
-    float *scratch;  // [n_seg][4 + dim_pad] partials of split rows: max, sum, 2 unused, accumulator
+    float *scratch;  // [n_seg][4 + dim_pad] partials of split rows: reference, sum, 2 unused, accumulator
     int64_t n_seg;
     int64_t ldA, ldB, ldV, ldOut;
     int32_t dim, dim_pad;
@@ -461,7 +463,7 @@ __global__ void __launch_bounds__(256, AgnnOcc<CF, VW, SEP>::MIN_CTAS) agnn_long
 {
     constexpr int G = 256 / LPR;
     constexpr int STEP = 64;  // entries per group between two looks at the row ends of a warp
-    extern __shared__ float parts[];  // [G][first or last piece][max, sum, dim_pad columns]
+    extern __shared__ float parts[];  // [G][first or last piece][reference, sum, dim_pad columns]
     __shared__ LongShare::Shared sh;
     const int pitch = a.dim_pad + 2;
     const int g = threadIdx.x / LPR, gl = threadIdx.x % LPR;
